@@ -12,10 +12,10 @@
 //                   sum_rest Wmax * prod Gmax skips jobs whose every contribution would
 //                   fail the threshold (the role of upper_bound_thread, :897-1023; skipping
 //                   changes no result), the survivors are compacted;
-//   expand_jobs_kernel  persistent CTAs take the surviving (ket, term) jobs from a counter,
-//                   stage the job's W block and TDM columns in shared memory, contract
-//                   W with the first TDM once per job and evaluate every bra tuple from
-//                   there (threshold per contribution, as the reference), then insert into
+//   expand_jobs_kernel  persistent warps take the surviving (ket, term) jobs from a counter,
+//                   stage the job's W block and TDM columns in shared memory, screen every
+//                   bra tuple in float with a rigorous margin, evaluate the few that can pass
+//                   exactly (threshold per contribution, as the reference), and insert into
 //                   an open-addressed table keyed by (bra sector, mixed-radix local-state
 //                   index) with atomic accumulation of the R values;
 //   compact_kernel  occupied slots -> (key, values).
@@ -37,7 +37,7 @@ constexpr int kMaxProbe = 1 << 16;
 constexpr int kKeyIdxBits = 40;
 
 // counters: [0] kept jobs, [1] elements of kept jobs, [2] table overflow, [3] output rows,
-// [4] next job of the expand CTAs
+// [4] next job of the expand warps
 struct OpenParams {
   const OpenTerm* ot;
   const OpenItem* items;
@@ -127,7 +127,7 @@ __global__ void screen_kernel(OpenParams p, const double* __restrict__ wmax, con
 }
 
 __device__ __forceinline__ void table_add(unsigned long long* keys, double* vals, unsigned long long cap_mask,
-                                          unsigned long long key, const double* add, int R,
+                                          unsigned long long key, double x, const double* crow, int R,
                                           unsigned long long* overflow) {
   unsigned long long h = key * 0x9E3779B97F4A7C15ull;
   h ^= h >> 29;
@@ -140,7 +140,7 @@ __device__ __forceinline__ void table_add(unsigned long long* keys, double* vals
       else cur = prev;
     }
     if (cur == key) {
-      for (int r = 0; r < R; ++r) atomicAdd(vals + slot * R + r, add[r]);
+      for (int r = 0; r < R; ++r) atomicAdd(vals + slot * R + r, x * crow[r]);
       return;
     }
     slot = (slot + 1) & cap_mask;
@@ -148,50 +148,53 @@ __device__ __forceinline__ void table_add(unsigned long long* keys, double* vals
   atomicExch(overflow, 1ull);
 }
 
-constexpr int kExpThreads = 256;
-constexpr int kOpenMaxR = 16;  // roots of one open sigma at most (checked on the host)
-constexpr int kExpSmemBytes = 96 * 1024;  // shared-memory budget of one expand CTA
+constexpr int kExpWarps = 8;      // warps of an expand CTA at most
+constexpr int kOpenMaxR = 16;     // roots of one open sigma at most (checked on the host)
+constexpr int kExpSlice = 36 * 1024;      // largest float tiles of one job a warp keeps in shared memory
+constexpr int kExpCtaBytes = 104 * 1024;  // shared-memory budget of one expand CTA (two per SM)
+constexpr int kQueue = 64;        // candidates a warp holds: flushed 32 at a time, so 31 + 32 always fit
 // The float pre-filter keeps a contribution for the exact double evaluation unless
 // |x32| + kFilterMargin * s32 <= thresh / max|c|, where s32 = sum of |products| of the same
 // sum.  The float evaluation differs from the exact value by at most about
 // (number of factors + summed terms) * 2^-24 * s (below 1e-5 s for every shape here), so
 // the margin of 1e-4 s never drops a contribution the double evaluation would keep.
 constexpr float kFilterMargin = 1e-4f;
+// Whole tiles and units are skipped on an upper bound of s32 (the column maxima in place of the
+// columns not looked at yet); this factor covers the bound's own float rounding and the margin.
+constexpr float kBoundSlack = 1.002f;
 
-// Shared-memory tiles of one job.  Doubles: the W block of the ket's dressed-cluster state
-// for every bra state of that cluster [rest][mb0] and the TDM columns of the remaining
-// clusters [d_r][mb_{r+1}] (for the exact evaluations).  Floats: the same tiles, and
-// T1[pair + P*jl] = sum_i W[i + d0*jl, b0] G0[i, b1] with its absolute-value twin T1a
-// (pair = b0 + mb0*b1, P = mb0*mb1, jl < rest/d0).
+// Shared memory of one warp, in floats: the W block of the ket's dressed-cluster state
+// [rest][mb0 | 1] (bra states fastest, so that a warp's lanes read consecutive words; an odd
+// stride, so that it is written without bank conflicts too), the TDM
+// columns of the remaining clusters [mb_{r+1}][d_r], and for clusters of more than
+// kExpMaxD orbital indices (D = 0) the per-lane sums T1, T1a [JL][32] and u, ua [d2][32].
 struct ExpandTiles {
-  int w64, g64[3];           // offsets in doubles
-  int w32, g32[3], t1, t1a;  // offsets in floats, after the doubles
+  int w, g[3], t1, t1a, u, ua;
   int bytes;
 };
 
-__host__ __device__ inline ExpandTiles expand_tiles(int nrem, int rest, const int16_t* g_dim, const int16_t* mb) {
+__host__ __device__ inline ExpandTiles expand_tiles(int nrem, int rest, const int16_t* g_dim, const int16_t* mb,
+                                                    bool lane_sums) {
   ExpandTiles t{};
-  int d = 0;
-  t.w64 = d;
-  d += rest * mb[0];
+  int f = 0;
+  t.w = f;
+  f += rest * (mb[0] | 1);
   for (int r = 0; r < 3; ++r) {
-    t.g64[r] = d;
-    if (r < nrem) d += g_dim[r] * mb[r + 1];
-  }
-  d += d & 1;  // float part starts on an even double
-  int f = 2 * d;
-  t.w32 = f;
-  f += rest * mb[0];
-  for (int r = 0; r < 3; ++r) {
-    t.g32[r] = f;
+    f = (f + 3) & ~3;
+    t.g[r] = f;
     if (r < nrem) f += g_dim[r] * mb[r + 1];
   }
-  const int jlp = nrem >= 2 ? (rest / g_dim[0]) * mb[0] * mb[1] : 0;
+  const int jl = lane_sums && nrem >= 2 ? rest / g_dim[0] : 0;
+  const int d2 = lane_sums && nrem >= 3 ? g_dim[2] : 0;
   t.t1 = f;
-  f += jlp;
+  f += 32 * jl;
   t.t1a = f;
-  f += jlp;
-  t.bytes = 4 * f;
+  f += 32 * jl;
+  t.u = f;
+  f += 32 * d2;
+  t.ua = f;
+  f += 32 * d2;
+  t.bytes = 4 * ((f + 3) & ~3);
   return t;
 }
 
@@ -223,224 +226,329 @@ __device__ __forceinline__ double exact_x(int nrem, int d0, int d1, int d2, cons
   return x;
 }
 
-// one contribution: threshold, bra key, accumulation of x * c_ket
-__device__ __forceinline__ void expand_emit(const OpenParams& p, double x, double tc, const double* crow,
-                                            unsigned long long keybase, int64_t idx, unsigned long long* keys,
-                                            double* vals, unsigned long long cap_mask,
-                                            unsigned long long* counters) {
-  if (!(fabs(x) > tc)) return;
-  double add[kOpenMaxR];
-  for (int r = 0; r < p.R; ++r) add[r] = x * crow[r];
-  table_add(keys, vals, cap_mask, keybase | (unsigned long long)idx, add, p.R, counters + 2);
+// What a warp needs of its current job to evaluate and store one contribution.
+struct ExpandJob {
+  int nrem, rest, d0, d1, d2;
+  int mb[4];
+  int64_t sa[4];  // key stride of each active cluster's bra state
+  int64_t base;   // key of the ket's other clusters
+  unsigned long long keybase;
+  double tc;      // contributions of |x| <= tc are dropped
+  const double* w;
+  const double* g[3];
+  const double* crow;  // the ket's coefficients times the term's sign (shared memory)
+};
+
+struct ExpandTable {
+  unsigned long long* keys;
+  double* vals;
+  unsigned long long cap_mask;
+  unsigned long long* counters;
+};
+
+// exact value, threshold, accumulation of x * c_ket of the bra tuple (b0, b1, b2, b3)
+__device__ __forceinline__ void expand_exact(const ExpandJob& J, const ExpandTable& H, int R, int b0, int b1, int b2,
+                                             int b3) {
+  const double x = exact_x(J.nrem, J.d0, J.d1, J.d2, J.w + int64_t(J.rest) * b0, J.g[0] + int64_t(J.d0) * b1,
+                           J.g[1] + int64_t(J.d1) * b2, J.g[2] + int64_t(J.d2) * b3);
+  if (!(fabs(x) > J.tc)) return;
+  const int64_t idx = J.base + b0 * J.sa[0] + b1 * J.sa[1] + b2 * J.sa[2] + b3 * J.sa[3];
+  table_add(H.keys, H.vals, H.cap_mask, J.keybase | (unsigned long long)idx, x, J.crow, R, H.counters + 2);
 }
 
-// One (b0, b1, b2) unit of a four-cluster job: float sums over the third remaining cluster's
-// index l < D2 for every b3, screened; survivors evaluated exactly.  D2 = 16 serves any
-// d2 <= 16 with the run-time length `d2`.
-template <int D2>
-__device__ __forceinline__ void unit4(const OpenParams& p, const float* T1, const float* T1a, int P, int pr, int d1,
-                                      const float* g1, const float* G2f, int mb3, float tcf, double tc,
-                                      int d0, const double* wc, const double* g0d, const double* g1d,
-                                      const double* G2d, const double* crow, unsigned long long keybase,
-                                      int64_t idx3, int64_t sa3, unsigned long long* keys, double* vals,
-                                      unsigned long long cap_mask, unsigned long long* counters, int d2 = D2) {
-  float ul[D2], ua[D2];
-#pragma unroll
-  for (int l = 0; l < D2; ++l) {
-    ul[l] = 0.f;
-    ua[l] = 0.f;
-    if (D2 != 16 || l < d2)
-      for (int j = 0; j < d1; ++j) {
-        ul[l] = fmaf(T1[pr + P * (j + d1 * l)], g1[j], ul[l]);
-        ua[l] = fmaf(T1a[pr + P * (j + d1 * l)], fabsf(g1[j]), ua[l]);
-      }
-  }
-  for (int b3 = 0; b3 < mb3; ++b3) {
-    const float* g2 = G2f + d2 * b3;
-    float x32 = 0.f, s32 = 0.f;
-#pragma unroll
-    for (int l = 0; l < D2; ++l)
-      if (D2 != 16 || l < d2) {
-        x32 = fmaf(ul[l], g2[l], x32);
-        s32 = fmaf(ua[l], fabsf(g2[l]), s32);
-      }
-    if (fabsf(x32) + kFilterMargin * s32 > tcf) {
-      const double x = exact_x(3, d0, d1, d2, wc, g0d, g1d, G2d + d2 * b3);
-      expand_emit(p, x, tc, crow, keybase, idx3 + b3 * sa3, keys, vals, cap_mask, counters);
-    }
+// A warp's candidates: those of one step are appended, and every 32 are evaluated by the whole
+// warp, one per lane (few lanes pass the screen at a time, and an FP64 instruction costs the
+// same for one lane as for 32).  Entry: b3 | b2 << 8 | (b0 + mb0 * b1) << 16.
+struct ExpandQueue {
+  unsigned* q;
+  int n;
+};
+
+__device__ __forceinline__ void queue_run(const ExpandQueue& Q, int at, const ExpandJob& J, const ExpandTable& H, int R) {
+  const unsigned e = Q.q[at];
+  const int pr = int(e >> 16), b1 = pr / J.mb[0];
+  expand_exact(J, H, R, pr - b1 * J.mb[0], b1, int((e >> 8) & 255u), int(e & 255u));
+}
+
+__device__ __forceinline__ void queue_push(ExpandQueue& Q, bool keep, unsigned entry, const ExpandJob& J,
+                                           const ExpandTable& H, int R) {
+  const unsigned m = __ballot_sync(0xffffffffu, keep);
+  if (m == 0) return;
+  const int lane = threadIdx.x & 31;
+  if (keep) Q.q[Q.n + __popc(m & ((1u << lane) - 1u))] = entry;
+  Q.n += __popc(m);
+  __syncwarp();
+  if (Q.n >= 32) {
+    Q.n -= 32;
+    queue_run(Q, Q.n + lane, J, H, R);
+    __syncwarp();  // the entries are read before the next push overwrites them
   }
 }
 
-// Persistent CTAs take kept (ket, term) jobs from a counter.  Per job the W block and the
-// TDM columns for all bra states are staged in shared memory (double and float copies) and,
-// for three- and four-cluster terms, W is contracted with the first remaining cluster's
-// TDM once in float (T1, with its absolute-value twin).  Every bra tuple is then screened
-// in float (value and the sum of |products|); the tuples that can pass the threshold are
-// evaluated exactly with the per-element double formula (exact_x) and thresholded as the
-// reference does.  Jobs whose tiles exceed the shared-memory budget are evaluated per
+constexpr int kExpMaxD = 6;  // longest orbital index of the register sums
+
+// One warp per kept (ket, term) job, taken from a counter.  The job's W block and TDM columns
+// are staged in the warp's shared-memory slice (the float copies the library keeps of both);
+// each lane owns one (b0, b1) pair at a time and keeps
+//   T1[j, l] = sum_i W[i, j, l, b0] G0[i, b1]
+// and its absolute-value twin in registers (D: bound of the two index lengths; 0: in shared
+// memory), from which every (b2, b3) is screened in float.  Pairs and (pair, b2) units that no
+// lane's bound can lift over the threshold are skipped whole.  What passes the screen is
+// queued and evaluated exactly, 32 at a time, with the per-element double formula, and
+// thresholded as the reference does.  Jobs whose tiles exceed a slice are evaluated per
 // element, exactly, from global memory.
-__global__ void __launch_bounds__(kExpThreads) expand_jobs_kernel(
+//
+// What bounds it: the screen's instructions (about 10 per surviving contribution) and the
+// latency of a job's first loads, which 16 or more warps per SM cover; contributions over the
+// threshold are rare (0.4 % at 1e-3), so neither the FP64 pipe nor the table's atomics are.
+// A CTA per job (two resident per SM, five barriers per job) and a divergent exact evaluation
+// took 57 ms longer on 3 001 configurations of the 24-orbital problem at 1e-3, 4 roots (1.09e6
+// kept jobs, 9.7e9 contributions): whole call 126.8 -> 69.4 ms.
+template <int D>
+__global__ void __launch_bounds__(32 * kExpWarps, D == 3 || D == 4 ? 2 : 1) expand_jobs_kernel(
     OpenParams p, const int2* __restrict__ kept, int64_t n_kept, const double* __restrict__ w,
-    const double* __restrict__ op, unsigned long long* __restrict__ keys, double* __restrict__ vals,
-    unsigned long long cap_mask, unsigned long long* __restrict__ counters, int smem_bytes) {
-  extern __shared__ __align__(16) double xs[];
-  float* xf = reinterpret_cast<float*>(xs);
-  __shared__ unsigned long long s_job;
-  __shared__ double s_cs[kOpenMaxR];
+    const double* __restrict__ op, const float* __restrict__ w32, const float* __restrict__ op32,
+    const double* __restrict__ gmax, ExpandTable H, int slice) {
+  extern __shared__ __align__(16) unsigned char xsm[];
+  __shared__ double s_cs[kExpWarps][kOpenMaxR];
+  __shared__ unsigned s_queue[kExpWarps][kQueue];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  float* xf = reinterpret_cast<float*>(xsm + size_t(wid) * slice);
+  ExpandQueue Q{s_queue[wid], 0};
+  const int R = p.R;
   for (;;) {
-    if (threadIdx.x == 0) s_job = atomicAdd(counters + 4, 1ull);
-    __syncthreads();
-    const int64_t jn = int64_t(s_job);
-    if (jn >= n_kept) break;  // uniform over the CTA
+    unsigned long long jn = 0;
+    if (lane == 0) jn = atomicAdd(H.counters + 4, 1ull);
+    jn = __shfl_sync(0xffffffffu, jn, 0);
+    if (int64_t(jn) >= n_kept) break;
     const int2 job = kept[jn];
     const OpenTerm& o = p.ot[job.y];
     const TermSector& ts = o.ts;
     const int16_t* ck = p.cfg + int64_t(job.x) * kCfgStride;
-    const double* c_ket = p.c + int64_t(job.x) * p.R;
-    const double tc = p.thresh / row_maxabs(c_ket, p.R);
-    const float tcf = float(tc * (1.0 - 1e-6));
+    const double* c_ket = p.c + int64_t(job.x) * R;
+    ExpandJob J{};
+    J.tc = p.thresh / row_maxabs(c_ket, R);
+    const float tcf = float(J.tc * (1.0 - 1e-6));
     const int nrem = ts.nrem, rest = ts.rest_len;
     const int d0 = nrem >= 1 ? ts.g_dim[0] : 1, d1 = nrem >= 2 ? ts.g_dim[1] : 1, d2 = nrem >= 3 ? ts.g_dim[2] : 1;
-    int mb[4] = {1, 1, 1, 1};
-    int64_t sa[4] = {0, 0, 0, 0};
+    J.nrem = nrem, J.rest = rest, J.d0 = d0, J.d1 = d1, J.d2 = d2;
     // bra key of (b0, .., b3) = keybase | (base + sum_a b_a * st[c_a])
     const int64_t* st = p.strides + int64_t(o.bsec) * p.N;
-    int64_t base = 0;
-    for (int c = 0; c < p.N; ++c) base += int64_t(ck[c]) * st[c];
-    for (int a = 0; a < o.n_act; ++a) {
-      mb[a] = o.mb_act[a];
-      sa[a] = st[o.c_act[a]];
-      base -= int64_t(ck[o.c_act[a]]) * sa[a];
+    for (int c = 0; c < p.N; ++c) J.base += int64_t(ck[c]) * st[c];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+      J.mb[a] = 1;
+      if (a < o.n_act) {
+        J.mb[a] = o.mb_act[a];
+        J.sa[a] = st[o.c_act[a]];
+        J.base -= int64_t(ck[o.c_act[a]]) * J.sa[a];
+      }
     }
-    const unsigned long long keybase = (unsigned long long)(o.bsec) << kKeyIdxBits;
+    J.keybase = (unsigned long long)(o.bsec) << kKeyIdxBits;
+    // a kept value x contributes x * (sg * c) = (sg * x) * c to every root
     const double sg = ts.sign < 0 ? -1.0 : 1.0;
-    // the ket's coefficients times the term's sign (exact): a kept value x contributes
-    // x * (sg * c) = (sg * x) * c to every root
-    if (threadIdx.x < p.R) s_cs[threadIdx.x] = sg * c_ket[threadIdx.x];
-    __syncthreads();
-    const double* crow = s_cs;
-    const double* wblk = w + ts.w_off + int64_t(rest) * ts.w_mb * ck[ts.cw];  // [rest][mb0] for the ket state
-    const double* gblk[3] = {nullptr, nullptr, nullptr};
-    for (int r = 0; r < nrem; ++r) gblk[r] = op + ts.g_off[r] + int64_t(ts.g_dim[r]) * ts.g_mb[r] * ck[ts.cr[r]];
-    const ExpandTiles t = expand_tiles(nrem, rest, ts.g_dim, o.mb_act);
-    if (t.bytes <= smem_bytes && d2 <= 16) {
-      for (int i = threadIdx.x; i < rest * mb[0]; i += kExpThreads) {
-        const double v = wblk[i];
-        xs[t.w64 + i] = v;
-        xf[t.w32 + i] = float(v);
+    if (lane < R) s_cs[wid][lane] = sg * c_ket[lane];
+    J.crow = s_cs[wid];
+    const int64_t w_at = ts.w_off + int64_t(rest) * ts.w_mb * ck[ts.cw];  // [rest][mb0] for the ket state
+    J.w = w + w_at;
+    int64_t g_at[3] = {0, 0, 0};
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      J.g[r] = op;
+      if (r < nrem) {
+        g_at[r] = ts.g_off[r] + int64_t(ts.g_dim[r]) * ts.g_mb[r] * ck[ts.cr[r]];
+        J.g[r] = op + g_at[r];
       }
-      for (int r = 0; r < nrem; ++r) {
-        const int n = ts.g_dim[r] * mb[r + 1];
-        for (int i = threadIdx.x; i < n; i += kExpThreads) {
-          const double v = gblk[r][i];
-          xs[t.g64[r] + i] = v;
-          xf[t.g32[r] + i] = float(v);
+    }
+    const int mb0 = J.mb[0], mbp = mb0 | 1, P = mb0 * J.mb[1];
+    const ExpandTiles t = expand_tiles(nrem, rest, ts.g_dim, o.mb_act, D == 0);
+    if (nrem == 0) {
+      __syncwarp();
+      for (int b0 = lane; b0 < mb0; b0 += 32) expand_exact(J, H, R, b0, 0, 0, 0);
+    } else if (t.bytes <= slice) {
+      for (int i = lane; i < rest * mb0; i += 32) {
+        const int b0 = i / rest;
+        xf[t.w + (i - b0 * rest) * mbp + b0] = __ldg(w32 + w_at + i);
+      }
+#pragma unroll
+      for (int r = 0; r < 3; ++r)
+        if (r < nrem) {
+          const int n = ts.g_dim[r] * J.mb[r + 1];
+          for (int i = lane; i < n; i += 32) xf[t.g[r] + i] = __ldg(op32 + g_at[r] + i);
         }
-      }
-      __syncthreads();
-      const double* W = xs + t.w64;
-      const float* Wf = xf + t.w32;
-      const float* G0f = xf + t.g32[0];
-      const int P = mb[0] * mb[1];
-      if (nrem == 0) {
-        for (int b0 = threadIdx.x; b0 < mb[0]; b0 += kExpThreads)
-          expand_emit(p, W[b0], tc, crow, keybase, base + b0 * sa[0], keys, vals, cap_mask, counters);
-      } else if (nrem == 1) {
-        for (int pr = threadIdx.x; pr < P; pr += kExpThreads) {
-          const int b1 = pr / mb[0], b0 = pr - b1 * mb[0];
-          const float* wc = Wf + rest * b0;
-          const float* g0 = G0f + d0 * b1;
-          float x32 = 0.f, s32 = 0.f;
-          for (int i = 0; i < d0; ++i) {
-            x32 = fmaf(wc[i], g0[i], x32);
-            s32 = fmaf(fabsf(wc[i]), fabsf(g0[i]), s32);
+      __syncwarp();
+      const float* W = xf + t.w;
+      const float* G0 = xf + t.g[0];
+      if (nrem == 1) {
+        for (int p0 = 0; p0 < P; p0 += 32) {
+          const int pr = p0 + lane;
+          bool keep = false;
+          if (pr < P) {
+            const int b1 = pr / mb0, b0 = pr - b1 * mb0;
+            float x32 = 0.f, s32 = 0.f;
+            for (int i = 0; i < d0; ++i) {
+              const float wv = W[i * mbp + b0], gv = G0[i + d0 * b1];
+              x32 = fmaf(wv, gv, x32);
+              s32 = fmaf(fabsf(wv), fabsf(gv), s32);
+            }
+            keep = fabsf(x32) + kFilterMargin * s32 > tcf;
           }
-          if (fabsf(x32) + kFilterMargin * s32 > tcf) {
-            const double x = exact_x(1, d0, 1, 1, W + rest * b0, xs + t.g64[0] + d0 * b1, nullptr, nullptr);
-            expand_emit(p, x, tc, crow, keybase, base + b0 * sa[0] + b1 * sa[1], keys, vals, cap_mask, counters);
-          }
+          queue_push(Q, keep, unsigned(pr) << 16, J, H, R);
         }
       } else {
-        const int JL = rest / d0;
-        float* T1 = xf + t.t1;
-        float* T1a = xf + t.t1a;
-        for (int e = threadIdx.x; e < JL * P; e += kExpThreads) {
-          const int jl = e / P, pr = e - jl * P;
-          const int b1 = pr / mb[0], b0 = pr - b1 * mb[0];
-          const float* wc = Wf + d0 * jl + rest * b0;
-          const float* g0 = G0f + d0 * b1;
-          float acc = 0.f, aa = 0.f;
-          for (int i = 0; i < d0; ++i) {
-            acc = fmaf(wc[i], g0[i], acc);
-            aa = fmaf(fabsf(wc[i]), fabsf(g0[i]), aa);
+        constexpr int E = D > 0 ? D : 1;
+        // column maxima of the second and third remaining clusters for the ket's states
+        const double* gm1 = gmax + o.gmax_off[1] + int64_t(d1) * ck[ts.cr[1]];
+        const double* gm2 = nrem == 3 ? gmax + o.gmax_off[2] + int64_t(d2) * ck[ts.cr[2]] : nullptr;
+        float m1[E], m2[E];
+        if (D > 0) {
+#pragma unroll
+          for (int j = 0; j < E; ++j) {
+            m1[j] = j < d1 ? __double2float_ru(gm1[j]) : 0.f;
+            m2[j] = nrem == 3 ? (j < d2 ? __double2float_ru(gm2[j]) : 0.f) : (j == 0 ? 1.f : 0.f);
           }
-          T1[pr + P * jl] = acc;
-          T1a[pr + P * jl] = aa;
         }
-        __syncthreads();
-        const float* G1f = xf + t.g32[1];
-        const int units = P * mb[2];
-        for (int u = threadIdx.x; u < units; u += kExpThreads) {
-          const int b2 = u / P, pr = u - b2 * P;
-          const int b1 = pr / mb[0], b0 = pr - b1 * mb[0];
-          const int64_t idx3 = base + b0 * sa[0] + b1 * sa[1] + b2 * sa[2];
-          const float* g1 = G1f + d1 * b2;
-          const double* wc = W + rest * b0;
-          const double* g0d = xs + t.g64[0] + d0 * b1;
-          const double* g1d = xs + t.g64[1] + d1 * b2;
-          if (nrem == 2) {
-            float x32 = 0.f, s32 = 0.f;
-            for (int j = 0; j < d1; ++j) {
-              x32 = fmaf(T1[pr + P * j], g1[j], x32);
-              s32 = fmaf(T1a[pr + P * j], fabsf(g1[j]), s32);
+        const float* G1 = xf + t.g[1];
+        const float* G2 = xf + t.g[2];
+        for (int p0 = 0; p0 < P; p0 += 32) {
+          const int pr = p0 + lane;
+          const bool live = pr < P;
+          const int b1 = live ? pr / mb0 : 0, b0 = live ? pr - b1 * mb0 : 0;
+          const float* g0 = G0 + d0 * b1;
+          if constexpr (D > 0) {
+            float t1[E * E], ta[E * E];  // [j + E * l]
+#pragma unroll
+            for (int e = 0; e < E * E; ++e) t1[e] = ta[e] = 0.f;
+            for (int i = 0; i < d0; ++i) {
+              const float gv = live ? g0[i] : 0.f, ga = fabsf(gv);
+              const float* wi = W + i * mbp + b0;
+#pragma unroll
+              for (int l = 0; l < E; ++l) {
+                if (l < d2) {
+#pragma unroll
+                  for (int j = 0; j < E; ++j)
+                    if (j < d1) {
+                      const float wv = wi[d0 * (j + d1 * l) * mbp];
+                      t1[j + E * l] = fmaf(wv, gv, t1[j + E * l]);
+                      ta[j + E * l] = fmaf(fabsf(wv), ga, ta[j + E * l]);
+                    }
+                }
+              }
             }
-            if (fabsf(x32) + kFilterMargin * s32 > tcf) {
-              const double x = exact_x(2, d0, d1, 1, wc, g0d, g1d, nullptr);
-              expand_emit(p, x, tc, crow, keybase, idx3, keys, vals, cap_mask, counters);
+            float top = 0.f;  // bound of s32 over every (b2, b3) of this pair
+#pragma unroll
+            for (int l = 0; l < E; ++l) {
+              float a = 0.f;
+#pragma unroll
+              for (int j = 0; j < E; ++j) a = fmaf(ta[j + E * l], m1[j], a);
+              top = fmaf(a, m2[l], top);
+            }
+            if (!__any_sync(0xffffffffu, top * kBoundSlack > tcf)) continue;
+            for (int b2 = 0; b2 < J.mb[2]; ++b2) {
+              const float* g1 = G1 + d1 * b2;
+              float g1v[E];
+#pragma unroll
+              for (int j = 0; j < E; ++j) g1v[j] = j < d1 ? g1[j] : 0.f;
+              float ul[E], ua[E];
+#pragma unroll
+              for (int l = 0; l < E; ++l) {
+                ul[l] = ua[l] = 0.f;
+#pragma unroll
+                for (int j = 0; j < E; ++j) {
+                  ul[l] = fmaf(t1[j + E * l], g1v[j], ul[l]);
+                  ua[l] = fmaf(ta[j + E * l], fabsf(g1v[j]), ua[l]);
+                }
+                if (nrem == 2) break;
+              }
+              if (nrem == 2) {
+                queue_push(Q, fabsf(ul[0]) + kFilterMargin * ua[0] > tcf, unsigned(pr) << 16 | unsigned(b2) << 8, J, H, R);
+                continue;
+              }
+              float bnd = 0.f;
+#pragma unroll
+              for (int l = 0; l < E; ++l) bnd = fmaf(ua[l], m2[l], bnd);
+              if (!__any_sync(0xffffffffu, bnd * kBoundSlack > tcf)) continue;
+              for (int b3 = 0; b3 < J.mb[3]; ++b3) {
+                const float* g2 = G2 + d2 * b3;
+                float x32 = 0.f, s32 = 0.f;
+#pragma unroll
+                for (int l = 0; l < E; ++l) {
+                  const float gv = l < d2 ? g2[l] : 0.f;
+                  x32 = fmaf(ul[l], gv, x32);
+                  s32 = fmaf(ua[l], fabsf(gv), s32);
+                }
+                queue_push(Q, fabsf(x32) + kFilterMargin * s32 > tcf,
+                           unsigned(pr) << 16 | unsigned(b2) << 8 | unsigned(b3), J, H, R);
+              }
             }
           } else {
-            switch (d2) {
-              case 1: unit4<1>(p, T1, T1a, P, pr, d1, g1, xf + t.g32[2], mb[3], tcf, tc, d0, wc, g0d, g1d,
-                               xs + t.g64[2], crow, keybase, idx3, sa[3], keys, vals, cap_mask, counters); break;
-              case 2: unit4<2>(p, T1, T1a, P, pr, d1, g1, xf + t.g32[2], mb[3], tcf, tc, d0, wc, g0d, g1d,
-                               xs + t.g64[2], crow, keybase, idx3, sa[3], keys, vals, cap_mask, counters); break;
-              case 3: unit4<3>(p, T1, T1a, P, pr, d1, g1, xf + t.g32[2], mb[3], tcf, tc, d0, wc, g0d, g1d,
-                               xs + t.g64[2], crow, keybase, idx3, sa[3], keys, vals, cap_mask, counters); break;
-              case 4: unit4<4>(p, T1, T1a, P, pr, d1, g1, xf + t.g32[2], mb[3], tcf, tc, d0, wc, g0d, g1d,
-                               xs + t.g64[2], crow, keybase, idx3, sa[3], keys, vals, cap_mask, counters); break;
-              case 5: unit4<5>(p, T1, T1a, P, pr, d1, g1, xf + t.g32[2], mb[3], tcf, tc, d0, wc, g0d, g1d,
-                               xs + t.g64[2], crow, keybase, idx3, sa[3], keys, vals, cap_mask, counters); break;
-              case 6: unit4<6>(p, T1, T1a, P, pr, d1, g1, xf + t.g32[2], mb[3], tcf, tc, d0, wc, g0d, g1d,
-                               xs + t.g64[2], crow, keybase, idx3, sa[3], keys, vals, cap_mask, counters); break;
-              case 8: unit4<8>(p, T1, T1a, P, pr, d1, g1, xf + t.g32[2], mb[3], tcf, tc, d0, wc, g0d, g1d,
-                               xs + t.g64[2], crow, keybase, idx3, sa[3], keys, vals, cap_mask, counters); break;
-              default: unit4<16>(p, T1, T1a, P, pr, d1, g1, xf + t.g32[2], mb[3], tcf, tc, d0, wc, g0d, g1d,
-                                 xs + t.g64[2], crow, keybase, idx3, sa[3], keys, vals, cap_mask, counters, d2); break;
+            // index lengths over kExpMaxD: the lane's sums in its column of shared memory
+            const int JL = d1 * d2;
+            float* t1 = xf + t.t1 + lane;
+            float* ta = xf + t.t1a + lane;
+            float* us = xf + t.u + lane;
+            float* ua = xf + t.ua + lane;
+            for (int jl = 0; jl < JL; ++jl) {
+              float a = 0.f, b = 0.f;
+              for (int i = 0; i < d0; ++i) {
+                const float gv = live ? g0[i] : 0.f, wv = W[(i + d0 * jl) * mbp + b0];
+                a = fmaf(wv, gv, a);
+                b = fmaf(fabsf(wv), fabsf(gv), b);
+              }
+              t1[32 * jl] = a;
+              ta[32 * jl] = b;
+            }
+            for (int b2 = 0; b2 < J.mb[2]; ++b2) {
+              const float* g1 = G1 + d1 * b2;
+              float x0 = 0.f, s0 = 0.f;
+              for (int l = 0; l < d2; ++l) {
+                float a = 0.f, b = 0.f;
+                for (int j = 0; j < d1; ++j) {
+                  a = fmaf(t1[32 * (j + d1 * l)], g1[j], a);
+                  b = fmaf(ta[32 * (j + d1 * l)], fabsf(g1[j]), b);
+                }
+                if (nrem == 2) {
+                  x0 = a, s0 = b;
+                } else {
+                  us[32 * l] = a;
+                  ua[32 * l] = b;
+                }
+              }
+              if (nrem == 2) {
+                queue_push(Q, fabsf(x0) + kFilterMargin * s0 > tcf, unsigned(pr) << 16 | unsigned(b2) << 8, J, H, R);
+                continue;
+              }
+              for (int b3 = 0; b3 < J.mb[3]; ++b3) {
+                const float* g2 = G2 + d2 * b3;
+                float x32 = 0.f, s32 = 0.f;
+                for (int l = 0; l < d2; ++l) {
+                  x32 = fmaf(us[32 * l], g2[l], x32);
+                  s32 = fmaf(ua[32 * l], fabsf(g2[l]), s32);
+                }
+                queue_push(Q, fabsf(x32) + kFilterMargin * s32 > tcf,
+                           unsigned(pr) << 16 | unsigned(b2) << 8 | unsigned(b3), J, H, R);
+              }
             }
           }
         }
       }
+      if (lane < Q.n) queue_run(Q, lane, J, H, R);  // the job's last candidates
+      Q.n = 0;
     } else {
       // tiles too large: every element exactly, from global memory
-      const int64_t n_el = o.out_count;
-      for (int64_t e = threadIdx.x; e < n_el; e += kExpThreads) {
+      __syncwarp();
+      for (int64_t e = lane; e < o.out_count; e += 32) {
         int64_t loc = e;
-        int b[4] = {0, 0, 0, 0};
-        for (int a = 0; a < o.n_act; ++a) {
-          b[a] = int(loc % mb[a]);
-          loc /= mb[a];
+        int b[4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+          b[a] = int(loc % J.mb[a]);
+          loc /= J.mb[a];
         }
-        const double xr = exact_x(nrem, d0, d1, d2, wblk + int64_t(rest) * b[0],
-                                  nrem >= 1 ? gblk[0] + int64_t(d0) * b[1] : nullptr,
-                                  nrem >= 2 ? gblk[1] + int64_t(d1) * b[2] : nullptr,
-                                  nrem >= 3 ? gblk[2] + int64_t(d2) * b[3] : nullptr);
-        const double x = xr;
-        int64_t idx = base;
-        for (int a = 0; a < o.n_act; ++a) idx += b[a] * sa[a];
-        expand_emit(p, x, tc, crow, keybase, idx, keys, vals, cap_mask, counters);
+        expand_exact(J, H, R, b[0], b[1], b[2], b[3]);
       }
     }
-    __syncthreads();  // tiles and s_job are rewritten for the next job
+    __syncwarp();  // tiles, coefficients and queue are rewritten for the next job
   }
 }
 
@@ -672,17 +780,26 @@ int fcg_sigma_open(fcg_ctx* ctx, int R, const double* c, double thresh, int nbod
   const int64_t n_elem = int64_t(cnt[1]);
   int launches = 2;
   if (n_kept > 0) {
-    // shared memory of the expand CTAs: the largest job tiles, up to the budget
-    int smem_bytes = 0;
+    // a warp's slice: the largest job tiles, up to kExpSlice; as many warps to a CTA as fit.
+    // The register sums serve index lengths up to kExpMaxD (the second and third remaining
+    // clusters of the longest term), the shared-memory sums anything longer.
+    int d_max = 1, slice = 16;
     for (const OpenTerm& o : ots)
-      smem_bytes = std::max(smem_bytes, expand_tiles(o.ts.nrem, o.ts.rest_len, o.ts.g_dim, o.mb_act).bytes);
-    smem_bytes = std::min(smem_bytes, kExpSmemBytes);
-    const size_t smem = size_t(smem_bytes);
-    FCG_CUDA(cudaFuncSetAttribute(expand_jobs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kExpSmemBytes));
+      for (int r = 1; r < o.ts.nrem; ++r) d_max = std::max<int>(d_max, o.ts.g_dim[r]);
+    for (const OpenTerm& o : ots)
+      slice = std::max(slice, expand_tiles(o.ts.nrem, o.ts.rest_len, o.ts.g_dim, o.mb_act, d_max > kExpMaxD).bytes);
+    slice = std::min(slice, kExpSlice);
+    const int warps = std::min(kExpWarps, kExpCtaBytes / slice), threads = 32 * warps;
+    const size_t smem = size_t(warps) * size_t(slice);
+    auto kernel = d_max <= 3 ? expand_jobs_kernel<3>
+                  : d_max == 4 ? expand_jobs_kernel<4>
+                  : d_max <= kExpMaxD ? expand_jobs_kernel<kExpMaxD> : expand_jobs_kernel<0>;
+    FCG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kExpCtaBytes));
     int per_sm = 0, n_sm = 0;
-    FCG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, expand_jobs_kernel, kExpThreads, smem));
+    FCG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
     FCG_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, ctx->device));
-    const int64_t grid = std::max<int64_t>(1, std::min<int64_t>(int64_t(std::max(per_sm, 1)) * n_sm, n_kept));
+    const int64_t grid =
+        std::max<int64_t>(1, std::min<int64_t>(int64_t(std::max(per_sm, 1)) * n_sm, (n_kept + warps - 1) / warps));
     // table: twice the contributions, power of two, at least 4096 slots; doubled on overflow
     unsigned long long cap = 4096;
     while (cap < 2ull * (unsigned long long)n_elem && cap < (1ull << 28)) cap <<= 1;
@@ -693,9 +810,9 @@ int fcg_sigma_open(fcg_ctx* ctx, int R, const double* c, double thresh, int nbod
       FCG_CUDA(cudaMemsetAsync(ctx->d_hvals.p, 0, cap * R * sizeof(double), s));
       FCG_CUDA(cudaMemsetAsync(ctx->d_counters.p + 2, 0, 3 * sizeof(unsigned long long), s));
       FCG_CUDA(cudaEventRecord(ctx->ev2, s));
-      expand_jobs_kernel<<<unsigned(grid), kExpThreads, smem, s>>>(p, ctx->d_ojobs.p, n_kept, ctx->d_w64.p,
-                                                                   ctx->d_op64.p, ctx->d_hkeys.p, ctx->d_hvals.p,
-                                                                   cap - 1, ctx->d_counters.p, smem_bytes);
+      kernel<<<unsigned(grid), threads, smem, s>>>(
+          p, ctx->d_ojobs.p, n_kept, ctx->d_w64.p, ctx->d_op64.p, ctx->d_w32.p, ctx->d_op32.p, ctx->d_gmax.p,
+          ExpandTable{ctx->d_hkeys.p, ctx->d_hvals.p, cap - 1, ctx->d_counters.p}, slice);
       FCG_CUDA(cudaGetLastError());
       FCG_CUDA(cudaEventRecord(ctx->ev3, s));
       FCG_CUDA(cudaMemcpyAsync(cnt, ctx->d_counters.p, sizeof(cnt), cudaMemcpyDeviceToHost, s));
