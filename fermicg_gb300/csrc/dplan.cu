@@ -17,7 +17,7 @@
 //     thread per pair, compacted in order;
 //  4. join: every bra group of a pair looks its key up among the ket sector's groups (binary
 //     search); each match is a work item;
-//  5. lane jobs: each bra row of an item with up to 32 of its kets, then a stable radix sort
+//  5. lane jobs: each bra row of an item with up to lane_kets of its kets, then a stable radix sort
 //     by (window of 8 bra sectors, term shape, decreasing cost): the host's window sort;
 //  6. warp tasks (32 lane jobs), the prefix sums of their cost and stored values, and the
 //     warp chunks.
@@ -31,6 +31,7 @@ namespace fcg {
 namespace {
 
 constexpr int kThreads = 256;
+constexpr int kCounters = 18;  // device counters of a plan (see where they are read)
 constexpr int kWindow = 8;  // bra sectors per lane-job sort window
 constexpr uint8_t kActive = 255;  // spectator bit offset of a cluster inside the active set
 
@@ -441,16 +442,20 @@ struct ItemOut {
   int32_t* nk;    // kets
   int32_t* pair;  // (bra sector, term list) pair
   int64_t* jobs;  // lane jobs (E + 1 entries, zero past the last item)
+  int32_t* nb;    // bras
+  int32_t* blk;   // block jobs (E + 1 entries; 0: not a block item)
 };
 
-// counters: 0 triples, 1 reference flops, 2 executed flops, 3 largest lane-job cost
+// counters: 0 triples, 1 reference flops, 2 executed flops, 3 largest ket step of a lane job, 9 block
+// jobs, 10-13 lane jobs with each kLaneKets, 14-17 those of the block items
 __global__ void items_kernel(PairParams p, int64_t E, const int64_t* __restrict__ pt_e, const int64_t* __restrict__ pt_nt,
                              const int64_t* __restrict__ pt_flop, const int64_t* __restrict__ pt_flopd,
                              const int32_t* __restrict__ g_start, const int32_t* __restrict__ g_cnt,
                              const int32_t* __restrict__ item_of, const int32_t* __restrict__ m_ket,
-                             const int32_t* __restrict__ m_pair, ItemOut out, unsigned long long* __restrict__ counters) {
+                             const int32_t* __restrict__ m_pair, const uint8_t* __restrict__ tl_block, ItemOut out,
+                             unsigned long long* __restrict__ counters) {
   const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  unsigned long long tri = 0, fl = 0, fld = 0, cmax = 0;
+  unsigned long long tri = 0, fl = 0, fld = 0, cmax = 0, bj = 0, jobs[4] = {0, 0, 0, 0};
   if (e < E && item_of[e + 1] != item_of[e]) {
     const int32_t it = item_of[e];
     const int64_t w = m_pair[e];
@@ -464,18 +469,38 @@ __global__ void items_kernel(PairParams p, int64_t E, const int64_t* __restrict_
     out.ket[it] = g_start[gk];
     out.nk[it] = int32_t(nk);
     out.pair[it] = int32_t(w);
-    out.jobs[it] = nb * ((nk + kLaneKets - 1) / kLaneKets);
+    for (int i = 0; i < 4; ++i)  // 32, 16, 8, 4 kets
+      jobs[i] = (unsigned long long)(nb * ((nk + (32 >> i) - 1) >> (5 - i)));
+    out.nb[it] = int32_t(nb);
+    if (block_item(tl_block[j] != 0, nb, nk)) bj = (unsigned long long)block_jobs_of(nb, nk);
+    out.blk[it] = int32_t(bj);
     tri = (unsigned long long)(nb * nk * nt);
     fl = (unsigned long long)(nb * nk * pt_flop[w]);
     fld = (unsigned long long)(nb * nk * pt_flopd[w]);
     const int64_t step = pt_flopd[w] / 2 + 8 * nt + 4;
-    cmax = (unsigned long long)min64(step * min64(kLaneKets, nk), int64_t(1) << 30);
+    cmax = (unsigned long long)min64(step, int64_t(1) << 30);
   }
   tri = warp_sum(tri);
   fl = warp_sum(fl);
   fld = warp_sum(fld);
+  unsigned long long bjobs[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    bjobs[i] = warp_sum(bj ? jobs[i] : 0ull);
+    jobs[i] = warp_sum(jobs[i]);
+  }
+  bj = warp_sum(bj);
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) cmax = max(cmax, __shfl_xor_sync(0xffffffffu, cmax, d));
+  if ((threadIdx.x & 31) == 0 && bj) {
+    atomicAdd(counters + 9, bj);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) atomicAdd(counters + 14 + i, bjobs[i]);
+  }
+  if ((threadIdx.x & 31) == 0 && jobs[0]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) atomicAdd(counters + 10 + i, jobs[i]);
+  }
   if ((threadIdx.x & 31) == 0 && (tri | fl | fld | cmax)) {
     atomicAdd(counters + 0, tri);
     atomicAdd(counters + 1, fl);
@@ -489,11 +514,17 @@ __global__ void rows_collect_kernel(const int32_t* __restrict__ n_sec_at, unsign
   counters[1] = (unsigned long long)*n_sec_at;
 }
 
-// the sizes the next phase needs, in one place for one copy
-__global__ void collect_kernel(const int32_t* __restrict__ n_items_at, const int64_t* __restrict__ n_jobs_at,
-                               unsigned long long* __restrict__ counters) {
+// the item count, for the host
+__global__ void collect_kernel(const int32_t* __restrict__ n_items_at, unsigned long long* __restrict__ counters) {
   counters[4] = (unsigned long long)*n_items_at;
-  counters[5] = (unsigned long long)*n_jobs_at;
+}
+
+// lane jobs of every item with lane_kets kets each (0 past the last item)
+__global__ void job_counts_kernel(int64_t n_items, int lane_kets, const int32_t* __restrict__ nb,
+                                  const int32_t* __restrict__ nk, int64_t* __restrict__ jobs) {
+  const int64_t it = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (it > n_items) return;
+  jobs[it] = it < n_items ? nb[it] * int64_t((nk[it] + lane_kets - 1) / lane_kets) : 0;
 }
 
 // ---- 5. lane jobs -----------------------------------------------------------------------
@@ -502,6 +533,7 @@ struct JobParams {
   const int32_t* bra;
   const int32_t* ket;
   const int32_t* nk;
+  const int32_t* blk;
   const int32_t* pair;
   const int64_t* pt_ts;    // record offset of each pair (scanned)
   const int64_t* pt_flopd;
@@ -510,6 +542,9 @@ struct JobParams {
   int64_t n_items, n_jobs;
   int n_tl;
   int cost_bits;
+  int lane_kets;           // kets of a lane job at most
+  int blocks;              // 1: block items' jobs go after the others'
+  int block_bit;           // the sort-key bit for that, above the others
 };
 
 __global__ void __launch_bounds__(kThreads) jobs_kernel(JobParams p, LaneJob* __restrict__ jobs,
@@ -534,9 +569,9 @@ __global__ void __launch_bounds__(kThreads) jobs_kernel(JobParams p, LaneJob* __
   const int64_t it = lo + loc;
   const int64_t q = job - s_off[loc];
   const int nk = p.nk[it];
-  const int nkc = (nk + kLaneKets - 1) / kLaneKets;
+  const int nkc = (nk + p.lane_kets - 1) / p.lane_kets;
   const int64_t bj = q / nkc;
-  const int k0 = int(q - bj * nkc) * kLaneKets;
+  const int k0 = int(q - bj * nkc) * p.lane_kets;
   const int64_t w = p.pair[it];
   const int64_t sb = w / p.n_tl;
   const int j = int(w - sb * p.n_tl);
@@ -545,7 +580,7 @@ __global__ void __launch_bounds__(kThreads) jobs_kernel(JobParams p, LaneJob* __
   L.b = p.perm[p.bra[it] + bj];
   L.kp = p.ket[it] + k0;
   L.ts_off = int32_t(p.pt_ts[w]);
-  L.len = uint16_t(min(kLaneKets, nk - k0));
+  L.len = uint16_t(min(p.lane_kets, nk - k0));
   L.nt = uint16_t(nt);
   const int64_t step = p.pt_flopd[w] / 2 + 8 * nt + 4;
   const int32_t c = int32_t(min64(step * L.len, int64_t(1) << 30));
@@ -553,7 +588,8 @@ __global__ void __launch_bounds__(kThreads) jobs_kernel(JobParams p, LaneJob* __
   const uint64_t cc = uint64_t(min(c, (1 << 26) - 1));
   jobs[job] = L;
   cost[job] = c;
-  keys[job] = (uint64_t(sb / kWindow) << (p.cost_bits + 3)) | (uint64_t(p.tl_nbody[j]) << p.cost_bits) | (cmask - cc);
+  keys[job] = (uint64_t(p.blocks && p.blk[it] != 0) << p.block_bit) | (uint64_t(sb / kWindow) << (p.cost_bits + 3)) |
+              (uint64_t(p.tl_nbody[j]) << p.cost_bits) | (cmask - cc);
   vals[job] = uint32_t(job);
 }
 
@@ -570,6 +606,29 @@ __global__ void gather_jobs_kernel(int64_t n_jobs, int64_t n_slots, const uint32
   } else {
     dst[x] = LaneJob{0, 0, 0, 0, 0};
   }
+}
+
+// ---- block jobs -----------------------------------------------------------------------------
+// Every block item cut into its block jobs (bra rows in steps of kBlockBras, kets of kBlockKets),
+// at the item's offset; a few per item, one thread each.
+__global__ void block_jobs_kernel(JobParams p, const int32_t* __restrict__ nb, const int32_t* __restrict__ off,
+                                  BlockJob* __restrict__ out) {
+  const int64_t it = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (it >= p.n_items) return;
+  int64_t o = off[it];
+  if (int64_t(off[it + 1]) == o) return;
+  const int64_t w = p.pair[it];
+  BlockJob J;
+  J.ts_off = int32_t(p.pt_ts[w]);
+  J.nt = uint16_t(p.pt_ts[w + 1] - p.pt_ts[w]);
+  for (int b0 = 0; b0 < nb[it]; b0 += kBlockBras)
+    for (int k0 = 0; k0 < p.nk[it]; k0 += kBlockKets) {
+      J.bra = p.bra[it] + b0;
+      J.ket = p.ket[it] + k0;
+      J.nb = uint8_t(min(kBlockBras, nb[it] - b0));
+      J.nk = uint8_t(min(kBlockKets, p.nk[it] - k0));
+      out[o++] = J;
+    }
 }
 
 // ---- 6. warp tasks and chunks -------------------------------------------------------------
@@ -608,7 +667,7 @@ __global__ void chunks_kernel(int64_t n_wt, int64_t n_chunks, int64_t chunk_cost
     lo = a;
   }
   lo_out[c] = lo;
-  val_out[c] = wt_vals[lo];
+  if (val_out) val_out[c] = wt_vals[lo];
 }
 
 }  // namespace
@@ -662,8 +721,9 @@ static int upload_term_tables(fcg_ctx* ctx) {
   FCG_CUDA(D.d_tl_terms.upload(L.terms.data(), L.terms.size(), s));
   FCG_CUDA(D.d_tl_nbody.upload(nbody.data(), nbody.size(), s));
   FCG_CUDA(D.d_spec_off.upload(spec_off.data(), spec_off.size(), s));
-  FCG_CUDA(D.d_cnt.alloc(8));
-  FCG_CUDA(D.h_cnt.alloc(8));
+  FCG_CUDA(D.d_tl_block.upload(L.block.data(), L.block.size(), s));
+  FCG_CUDA(D.d_cnt.alloc(kCounters));
+  FCG_CUDA(D.h_cnt.alloc(kCounters));
   D.ready = true;
   return FCG_OK;
 }
@@ -703,8 +763,8 @@ int state_rows_device(fcg_ctx* ctx, int64_t n_cfg, const int16_t* fock, const in
   FCG_REQUIRE(N <= kMaxClusters, FCG_EINVAL, "more than 8 clusters");
   FCG_REQUIRE(n_cfg < (int64_t(1) << 31), FCG_EINVAL, "too many configurations");
   cudaStream_t s = ctx->stream;
-  FCG_CUDA(D.d_cnt.alloc(8));
-  FCG_CUDA(D.h_cnt.alloc(8));
+  FCG_CUDA(D.d_cnt.alloc(kCounters));
+  FCG_CUDA(D.h_cnt.alloc(kCounters));
   FCG_CUDA(D.d_fock_in.upload(fock, size_t(n_cfg) * 2 * N, s));
   FCG_CUDA(D.d_cfg_in.upload(cfg, size_t(n_cfg) * N, s));
   FCG_CUDA(ctx->d_cfg.alloc(size_t(n_cfg) * kCfgStride));
@@ -768,15 +828,24 @@ int state_rows_device(fcg_ctx* ctx, int64_t n_cfg, const int16_t* fock, const in
   return FCG_OK;
 }
 
-int device_chunks(fcg_ctx* ctx, int64_t target, DevBuf<int64_t>& lo, DevBuf<int64_t>& val, int64_t* n_chunks) {
-  const int64_t total = ctx->plan_total_cost, n_wt = ctx->plan_wt;
-  const int64_t chunk_cost =
-      std::max<int64_t>(kMinChunkCost, std::min<int64_t>(kChunkCost, total / std::max<int64_t>(target, 1)));
-  const int64_t nc = (total + chunk_cost - 1) / chunk_cost;
+static int64_t chunk_cost_of(int64_t total, int64_t target) {
+  return std::max<int64_t>(kMinChunkCost, std::min<int64_t>(kChunkCost, total / std::max<int64_t>(target, 1)));
+}
+
+static int64_t n_chunks_of(int64_t total, int64_t target) {
+  const int64_t c = chunk_cost_of(total, target);
+  return (total + c - 1) / c;
+}
+
+int device_chunks(fcg_ctx* ctx, int64_t target, DevBuf<int64_t>& lo, DevBuf<int64_t>* val, int64_t* n_chunks,
+                  bool direct) {
+  const int64_t total = direct ? ctx->direct_cost : ctx->plan_total_cost;
+  const int64_t n_wt = direct ? (ctx->plan.n_direct + 31) / 32 : ctx->plan_wt;
+  const int64_t chunk_cost = chunk_cost_of(total, target), nc = n_chunks_of(total, target);
   FCG_CUDA(lo.alloc(size_t(nc + 1)));
-  FCG_CUDA(val.alloc(size_t(nc + 1)));
+  if (val) FCG_CUDA(val->alloc(size_t(nc + 1)));
   chunks_kernel<<<grid_for(nc + 1), kThreads, 0, ctx->stream>>>(n_wt, nc, chunk_cost, ctx->d_wt_cum.p,
-                                                                 ctx->d_wt_vals.p, lo.p, val.p);
+                                                                 ctx->d_wt_vals.p, lo.p, val ? val->p : nullptr);
   FCG_CUDA(cudaGetLastError());
   *n_chunks = nc;
   return FCG_OK;
@@ -804,10 +873,10 @@ int build_join_device(fcg_ctx* ctx) {
   P.prefix.clear();
   P.ts_pool.clear();
   P.perm_pool.clear();
-  P.n_triples = P.flops_ref = P.flops_dressed = P.task_values = 0;
+  P.n_triples = P.flops_ref = P.flops_dressed = P.task_values = P.n_direct = 0;
   FCG_CUDA(D.d_sec_start.upload(P.sec_start.data(), P.sec_start.size(), s));
   FCG_CUDA(D.d_sec_count.upload(P.sec_count.data(), P.sec_count.size(), s));
-  FCG_CUDA(cudaMemsetAsync(D.d_cnt.p, 0, 8 * sizeof(unsigned long long), s));
+  FCG_CUDA(cudaMemsetAsync(D.d_cnt.p, 0, kCounters * sizeof(unsigned long long), s));
 
   // ---- 1. spectator keys, sort, groups --------------------------------------------------
   uint64_t* gk[2];
@@ -925,29 +994,36 @@ int build_join_device(fcg_ctx* ctx) {
     io.nk = b.take<int32_t>(E);
     io.pair = b.take<int32_t>(E);
     io.jobs = b.take<int64_t>(E + 1);
+    io.nb = b.take<int32_t>(E);
+    io.blk = b.take<int32_t>(E + 1);
     j_tmp = b.take<int64_t>(dprim::scan_scratch(E + 1));
   }));
   match_kernel<<<grid_for(E + 1), kThreads, 0, s>>>(pp, E, pt_ng, g_key, m_flag, m_ket, m_pair);
   FCG_CUDA(cudaGetLastError());
   FCG_CUDA(dprim::exclusive_scan<int32_t>(m_flag, E + 1, m_tmp, s));
-  FCG_CUDA(cudaMemsetAsync(io.jobs, 0, sizeof(int64_t) * (E + 1), s));
   if (E > 0) {
     items_kernel<<<grid_for(E), kThreads, 0, s>>>(pp, E, pt_ng, pt_nt, pt_flop, pt_flopd, g_start, g_cnt, m_flag,
-                                                  m_ket, m_pair, io, D.d_cnt.p);
+                                                  m_ket, m_pair, D.d_tl_block.p, io, D.d_cnt.p);
     FCG_CUDA(cudaGetLastError());
   }
-  FCG_CUDA(dprim::exclusive_scan<int64_t>(io.jobs, E + 1, j_tmp, s));
-  collect_kernel<<<1, 1, 0, s>>>(m_flag + E, io.jobs + E, D.d_cnt.p);
+  collect_kernel<<<1, 1, 0, s>>>(m_flag + E, D.d_cnt.p);
   FCG_CUDA(cudaGetLastError());
   {
-    const int rc = read_counters(ctx, 6);
+    const int rc = read_counters(ctx, kCounters);
     if (rc) return rc;
   }
-  const int64_t n_items = int64_t(D.h_cnt.p[4]), n_jobs = int64_t(D.h_cnt.p[5]);
   P.n_triples = int64_t(D.h_cnt.p[0]);
   P.flops_ref = int64_t(D.h_cnt.p[1]);
   P.flops_dressed = int64_t(D.h_cnt.p[2]);
-  const int64_t cmax = std::min<int64_t>(int64_t(D.h_cnt.p[3]), (int64_t(1) << 26) - 1);
+  const bool with_blocks = P.flops_dressed / 2 >= kBlockMinFma;
+  int64_t n_lane[4];
+  for (int i = 0; i < 4; ++i) n_lane[i] = int64_t(D.h_cnt.p[10 + i]);
+  const int lk = lane_kets(n_lane);
+  P.lane_kets = kLaneKets[lk];
+  const int64_t n_items = int64_t(D.h_cnt.p[4]), n_jobs = n_lane[lk];
+  P.n_direct = with_blocks ? n_jobs - int64_t(D.h_cnt.p[14 + lk]) : n_jobs;
+  ctx->n_block_jobs = with_blocks ? int64_t(D.h_cnt.p[9]) : 0;
+  const int64_t cmax = std::min<int64_t>(int64_t(D.h_cnt.p[3]) * P.lane_kets, (int64_t(1) << 26) - 1);
   FCG_REQUIRE(n_jobs < (int64_t(1) << 31) - 32, FCG_ELIMIT, "lane jobs exceed 2^31");
 
   // ---- 5. lane jobs, window sort -------------------------------------------------------
@@ -972,6 +1048,9 @@ int build_join_device(fcg_ctx* ctx) {
   FCG_CUDA(ctx->d_wt_cum.alloc(size_t(n_wt + 1)));
   FCG_CUDA(ctx->d_wt_vals.alloc(size_t(n_wt + 1)));
   if (n_jobs > 0) {
+    job_counts_kernel<<<grid_for(n_items + 1), kThreads, 0, s>>>(n_items, P.lane_kets, io.nb, io.nk, io.jobs);
+    FCG_CUDA(cudaGetLastError());
+    FCG_CUDA(dprim::exclusive_scan<int64_t>(io.jobs, n_items + 1, j_tmp, s));
     JobParams jp{};
     jp.job_off = io.jobs;
     jp.bra = io.bra;
@@ -985,12 +1064,16 @@ int build_join_device(fcg_ctx* ctx) {
     jp.n_items = n_items;
     jp.n_jobs = n_jobs;
     jp.n_tl = n_tl;
+    jp.lane_kets = P.lane_kets;
+    jp.blocks = ctx->n_block_jobs > 0 ? 1 : 0;
+    jp.blk = io.blk;
     jp.cost_bits = bit_width(uint64_t(cmax));
+    jp.block_bit = jp.cost_bits + 3 + bit_width(uint64_t(std::max<int64_t>(n_sec - 1, 0) / kWindow));
     jobs_kernel<<<grid_for(n_jobs), kThreads, 0, s>>>(jp, jobs_tmp, cost, jk[0], jv[0]);
     FCG_CUDA(cudaGetLastError());
     dprim::Digit passes[16];
     int np = 0;
-    const int bits = jp.cost_bits + 3 + bit_width(uint64_t(std::max<int64_t>(n_sec - 1, 0) / kWindow));
+    const int bits = jp.block_bit + (ctx->n_block_jobs > 0 ? 1 : 0);
     for (int sh = 0; sh < bits; sh += 8) passes[np++] = dprim::Digit{sh, 0, nullptr};
     int which = 0;
     FCG_CUDA(dprim::radix_sort(jk, jv, n_jobs, passes, np, js_tmp, &which, s));
@@ -1007,11 +1090,15 @@ int build_join_device(fcg_ctx* ctx) {
   FCG_CUDA(dprim::exclusive_scan<int64_t>(ctx->d_wt_vals.p, n_wt + 1, wt_tmp, s));
   FCG_CUDA(cudaMemcpyAsync(D.d_cnt.p + 0, ctx->d_wt_cum.p + n_wt, sizeof(int64_t), cudaMemcpyDeviceToDevice, s));
   FCG_CUDA(cudaMemcpyAsync(D.d_cnt.p + 1, ctx->d_wt_vals.p + n_wt, sizeof(int64_t), cudaMemcpyDeviceToDevice, s));
+  FCG_CUDA(cudaMemcpyAsync(D.d_cnt.p + 2, ctx->d_wt_cum.p + (P.n_direct + 31) / 32, sizeof(int64_t),
+                           cudaMemcpyDeviceToDevice, s));
   {
-    const int rc = read_counters(ctx, 2);
+    const int rc = read_counters(ctx, 3);
     if (rc) return rc;
   }
   ctx->plan_total_cost = int64_t(D.h_cnt.p[0]);
+  ctx->direct_cost = int64_t(D.h_cnt.p[2]);
+  ctx->direct_ready = false;  // the block jobs and the other lane jobs' chunks: on the first direct sigma
   P.task_values = int64_t(D.h_cnt.p[1]);
   ctx->plan_wt = n_wt;
   ctx->plan_jobs = n_wt * 32;
@@ -1019,9 +1106,49 @@ int build_join_device(fcg_ctx* ctx) {
   ctx->plan_ts = n_ts;
   ctx->plan_perm = n_el;
   {
-    const int rc = device_chunks(ctx, kTargetChunks, ctx->d_chunk_lo, ctx->d_chunk_val, &ctx->n_chunks);
+    const int rc = device_chunks(ctx, kTargetChunks, ctx->d_chunk_lo, &ctx->d_chunk_val, &ctx->n_chunks, false);
     if (rc) return rc;
   }
+  // what the first direct sigma fills, allocated here (fcg_sigma_closed_noalloc may come first)
+  FCG_REQUIRE(ctx->n_block_jobs < (int64_t(1) << 31), FCG_ELIMIT, "block jobs exceed 2^31");
+  FCG_CUDA(ctx->d_block_jobs.alloc(size_t(ctx->n_block_jobs)));
+  FCG_CUDA(ctx->d_block_next.alloc(1));
+  FCG_CUDA(ctx->d_chunk_lo_direct.alloc(size_t(n_chunks_of(ctx->direct_cost, kTargetChunks) + 1)));
+  D.join.bra = io.bra;
+  D.join.ket = io.ket;
+  D.join.nk = io.nk;
+  D.join.nb = io.nb;
+  D.join.blk = io.blk;
+  D.join.pair = io.pair;
+  D.join.pt_ts = pt_nt;
+  D.join.scan_tmp = m_tmp;
+  D.join.n_items = n_items;
   FCG_CUDA(cudaStreamSynchronize(s));
+  return FCG_OK;
+}
+
+int build_block_jobs(fcg_ctx* ctx) {
+  if (ctx->direct_ready) return FCG_OK;
+  auto& D = ctx->dj;
+  cudaStream_t s = ctx->stream;
+  if (ctx->n_block_jobs > 0) {
+    JobParams jp{};
+    jp.bra = D.join.bra;
+    jp.ket = D.join.ket;
+    jp.nk = D.join.nk;
+    jp.pair = D.join.pair;
+    jp.pt_ts = D.join.pt_ts;
+    jp.n_items = D.join.n_items;
+    FCG_CUDA(cudaMemsetAsync(D.join.blk + jp.n_items, 0, sizeof(int32_t), s));
+    FCG_CUDA(dprim::exclusive_scan<int32_t>(D.join.blk, jp.n_items + 1, D.join.scan_tmp, s));
+    block_jobs_kernel<<<grid_for(jp.n_items), kThreads, 0, s>>>(jp, D.join.nb, D.join.blk, ctx->d_block_jobs.p);
+    FCG_CUDA(cudaGetLastError());
+  }
+  ctx->n_chunks_direct = 0;
+  if (ctx->direct_cost > 0) {
+    const int rc = device_chunks(ctx, kTargetChunks, ctx->d_chunk_lo_direct, nullptr, &ctx->n_chunks_direct, true);
+    if (rc) return rc;
+  }
+  ctx->direct_ready = true;
   return FCG_OK;
 }

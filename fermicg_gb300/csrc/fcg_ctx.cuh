@@ -133,6 +133,13 @@ struct fcg_ctx {
   // items, term-sector records, permutation-pool entries
   int64_t n_chunks = 0, plan_jobs = 0, plan_wt = 0, plan_total_cost = 0, plan_items = 0, plan_ts = 0,
           plan_perm = 0;
+  // the direct (not stored) double sigma of a device plan: the block items as block jobs, the lane
+  // jobs of the others (the first plan.n_direct) in chunks of their own; built by its first use
+  bool direct_ready = false;
+  int64_t n_block_jobs = 0, n_chunks_direct = 0, direct_cost = 0;
+  DevBuf<BlockJob> d_block_jobs;
+  DevBuf<unsigned> d_block_next;        // work counter of the block-job launch
+  DevBuf<int64_t> d_chunk_lo_direct;
   bool plan_on_device = true;           // the join runs on the device (dplan.cu), else plan.cpp
   DevBuf<int64_t> d_wt_cum, d_wt_vals;  // exclusive prefix of warp-task cost / stored values (device planner)
   // device planner: the term set's tables on the device (uploaded at the first plan after
@@ -146,7 +153,7 @@ struct fcg_ctx {
     DevBuf<int64_t> d_w_index;
     DevBuf<int16_t> d_trans;
     DevBuf<int32_t> d_first_of_tr, d_tl_tr, d_tl_set, d_tl_off, d_tl_terms, d_tl_nbody;
-    DevBuf<uint8_t> d_spec_off;
+    DevBuf<uint8_t> d_spec_off, d_tl_block;
     DevBuf<int64_t> d_sec_start, d_sec_count;
     DevBuf<unsigned long long> d_cnt;
     PinnedBuf<unsigned long long> h_cnt;
@@ -158,14 +165,21 @@ struct fcg_ctx {
     DevBuf<int32_t> d_tvals;
     int64_t table_cap = 0;
     bool table_ready = false;
+    // the work items of the last join (in the arenas), for the block jobs of the direct sigma
+    struct {
+      int32_t *bra = nullptr, *ket = nullptr, *nk = nullptr, *nb = nullptr, *blk = nullptr, *pair = nullptr,
+              *scan_tmp = nullptr;
+      int64_t* pt_ts = nullptr;
+      int64_t n_items = 0;
+    } join;
   } dj;
   // closed-sigma kernel tuning: candidate per precision (0 fp64, 1 fp32; -1 not yet tuned),
   // forced candidate (-1: auto), the finer chunk table of candidates 2-3, candidate timings
   int tuned[2] = {-1, -1};
   int tune_mode = -1;
-  bool fine_built = false;
-  DevBuf<int64_t> d_chunk_lo_fine, d_chunk_val_fine;
-  int64_t n_chunks_fine = 0;
+  bool fine_built[2] = {false, false};  // all lane jobs / those of the direct double sigma
+  DevBuf<int64_t> d_chunk_lo_fine[2];
+  int64_t n_chunks_fine[2] = {0, 0};
   float tune_ms[2][4] = {};
   DevBuf<int32_t> d_perm;
   DevBuf<TermSector> d_ts;
@@ -290,14 +304,17 @@ ProblemInfo problem_info(fcg_ctx* ctx);
 int term_norms(fcg_ctx* ctx);
 
 // The closed-sigma join of the state on the device (dplan.cu): fills d_perm, d_ts, d_jobs,
-// d_chunk_lo / d_chunk_val, d_wt_cum / d_wt_vals and the plan sizes; and a chunk table of
-// about `target` warp chunks over its warp tasks.
+// d_chunk_lo / d_chunk_val, d_wt_cum / d_wt_vals and the plan sizes; the block jobs and chunks of
+// the direct double sigma on such a plan; and a chunk table of about `target` warp chunks over its
+// warp tasks (val: with each chunk's first stored value) or over those of that sigma (direct).
 int build_join_device(fcg_ctx* ctx);
+int build_block_jobs(fcg_ctx* ctx);
 
 // The rows of a state checked, their sectors found and the sector table built on the device
 // (dplan.cu); same results and messages as build_sectors.
 int state_rows_device(fcg_ctx* ctx, int64_t n_cfg, const int16_t* fock, const int16_t* cfg);
-int device_chunks(fcg_ctx* ctx, int64_t target, DevBuf<int64_t>& lo, DevBuf<int64_t>& val, int64_t* n_chunks);
+int device_chunks(fcg_ctx* ctx, int64_t target, DevBuf<int64_t>& lo, DevBuf<int64_t>* val, int64_t* n_chunks,
+                  bool direct);
 
 // BST sigma on device vectors [R][core_total] queued on ctx->stream without the host wait
 // (timed: CUDA events around the kernels), and the check of the tensor-core error flag (one

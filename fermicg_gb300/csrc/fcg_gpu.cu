@@ -8,19 +8,18 @@
 //                1-body terms store their "H" block here
 //   block index  dense int32 table (cluster, op, fb_a, fb_b, fk_a, fk_b) -> block id
 //   state        local states int16 [n_cfg][N]
-//   plan         work items (bra group x ket group x term-sector list), their triple
-//                prefix sum, the grouping permutation pool and the term-sector records
+//   plan         the grouping permutation pool, term-sector records, lane jobs in warp chunks and
+//                (for the double sigma of larger states) block jobs
 //   vectors      coefficients / sigma row-major [n_cfg][R] in the compute precision
 //
 // Kernels:
 //   dress_kernel         W blocks, once per problem (fcg_set_terms)
-//   closed_sigma_kernel  one pass over the flattened (work item, bra, ket, term) triple
-//                        space; each CTA takes a fixed chunk (exact load balance), each
-//                        warp 32 consecutive triples; a matrix element is the W column of
-//                        the dressed cluster contracted with the TDM columns of the other
-//                        active clusters (contract_matrix_element, src/tpsci_inner.jl:10-216,
-//                        re-associated); sigma is scattered with warp-segmented sums and
-//                        one atomic per run of equal bra rows.
+//   closed_sigma_lane_kernel  a bra row and up to 32 kets per lane; a matrix element is the W
+//                        column of the dressed cluster contracted with the TDM columns of the
+//                        other active clusters (contract_matrix_element,
+//                        src/tpsci_inner.jl:10-216, re-associated)
+//   block_sigma_kernel   a block of bras x kets per warp, the partly contracted W columns shared
+//   cached_sigma_lane_kernel  the same product from stored Hamiltonian blocks
 //   diag kernels         compute_diagonal (src/tpsci_outer.jl:694-757).
 //   pack / unpack        column-major float64 <-> row-major compute precision.
 #include <cuda_runtime.h>
@@ -283,6 +282,7 @@ struct LaneParams {
   const int32_t* perm;
   const TermSector* ts;
   const int16_t* cfg;  // [n_cfg][kCfgStride]
+  int64_t n_jobs;      // lane jobs to run: the ones past it are left to the block jobs
   int R;
 };
 
@@ -342,7 +342,7 @@ __device__ __forceinline__ void closed_lane_warp(const LaneParams& p, const T* _
   const uint4* cfg = reinterpret_cast<const uint4*>(p.cfg);
   for (int64_t wt = t_lo; wt < t_hi; ++wt) {
     const LaneJob j = p.jobs[wt * 32 + lane];
-    if (j.len == 0) continue;
+    if (j.len == 0 || wt * 32 + lane >= p.n_jobs) continue;
     const uint4 rb = __ldg(cfg + j.b);
     const TermSector* tsl = p.ts + j.ts_off;
     T acc[RV];
@@ -370,6 +370,299 @@ __global__ void __launch_bounds__(kSigmaThreads, MINB)
   const int64_t chunk = int64_t(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5);
   if (chunk >= p.n_chunks) return;
   closed_lane_warp<T, RR>(p, w, op, cin, sig, chunk);
+}
+
+// ---- block jobs --------------------------------------------------------------------------------
+// A warp per block job: up to 32 bras x 128 kets of one work item of three or four active clusters.
+// An element of such an item is W (the dressed cluster's column) contracted with the TDM columns of
+// the other active clusters.  W contracted with one of them,
+//   U[rest] = sum_i W[.. i .., bw, kw] G_q[i, b_q, k_q],
+// depends only on the states of the dressed cluster and cluster q, and a block of bras and kets has
+// few distinct ones (on the 24-orbital problem at 1e5 configurations a quarter to a half of the
+// bras, and of the kets).  The warp finds them by matching (the cluster q with the fewest (bra, ket)
+// combinations), forms U once for each combination into shared memory, and a (bra, ket) pair then
+// costs the contraction with what is left: 4 multiply-adds in place of 20 (three clusters), 20 in
+// place of 84 (four).  Pairs run with a bra per lane; a block of fewer bras gives the other lanes a
+// slice of the kets.  Kets are taken in order of their U index, in passes of as many as fit.
+//
+// Bound: the FP64 pipe (2 multiply-adds a clock per SM; 84 % busy).  24 orbitals, 1e5
+// configurations, 4 roots: 3.9 ms for work that took the lane kernel 7.0 ms; whole sigma 9.78 ->
+// 6.58 ms; 32 orbitals, 2e4 configurations, 2 roots: 6.53 -> 4.10 ms.
+constexpr int kBlockWarps = 4;
+constexpr int kBlockTerms = 2;  // terms of one shape whose U are held together
+
+template <typename T>
+struct alignas(16) BlockSmem {
+  // at least kBlockBras U columns of the longest length
+  static constexpr int kU = 1408;
+  T u[kU];
+  int2 ket[32];       // kets of the batch by U index: row, U index | states of the clusters left
+  uint32_t bst[32];   // (bw | b_q << 8) of every distinct bra pair
+  uint32_t kst[32];   // (kw | k_q << 8) of every distinct ket pair
+  int32_t kpos[33];   // first ket of every distinct ket pair
+};
+static_assert(BlockSmem<double>::kU >= kBlockBras * kBlockU, "one U column per bra of a block");
+
+struct BlockParams {
+  const BlockJob* jobs;
+  int64_t n_jobs;
+  const int32_t* perm;
+  const TermSector* ts;
+  const int16_t* cfg;
+  unsigned* next;
+  int R;
+};
+
+__device__ __forceinline__ bool same_shape(const TermSector& a, const TermSector& b) {
+  bool ok = a.cw == b.cw && a.nrem == b.nrem && a.rest_len == b.rest_len && a.w_mb == b.w_mb;
+  for (int q = 0; q < 3; ++q)
+    if (q < a.nrem) ok = ok && a.cr[q] == b.cr[q] && a.g_dim[q] == b.g_dim[q] && a.g_mb[q] == b.g_mb[q];
+  return ok;
+}
+
+// exclusive prefix sum over the warp
+__device__ __forceinline__ int warp_exclusive(int v) {
+  const int lane = threadIdx.x & 31;
+  int x = v;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, d);
+    if (lane >= d) x += y;
+  }
+  return x - v;
+}
+
+// -x without the floating-point pipe
+__device__ __forceinline__ float flip(float x) { return __int_as_float(__float_as_int(x) ^ int(0x80000000)); }
+__device__ __forceinline__ double flip(double x) {
+  return __longlong_as_double(__double_as_longlong(x) ^ (long long)(0x8000000000000000ull));
+}
+
+// x / n for x * n < 65536, n <= 65535, with m = div_magic(n)
+__device__ __forceinline__ unsigned div_magic(unsigned n) { return (65535u + n) / n; }
+__device__ __forceinline__ unsigned div_by(unsigned x, unsigned m) { return (x * m) >> 16; }
+
+// 4 consecutive elements of shared memory (16-byte aligned)
+__device__ __forceinline__ void load_u4(const float* p, float* v) {
+  const float4 q = *reinterpret_cast<const float4*>(p);
+  v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+}
+__device__ __forceinline__ void load_u4(const double* p, double* v) {
+  const double2 a = *reinterpret_cast<const double2*>(p), b = *reinterpret_cast<const double2*>(p + 2);
+  v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
+}
+
+// U contracted with the columns of the clusters left (one: ga; two: ga, gb)
+template <typename T>
+__device__ __forceinline__ T block_pair(const T* u, int da, int db, const T* __restrict__ ga, const T* __restrict__ gb) {
+  if (da == 4) {
+    Vec4<T> av;
+    av.load(ga);
+    T x[4];
+    if (db == 1) {
+      load_u4(u, x);
+      T me = x[0] * av.v[0];
+#pragma unroll
+      for (int i = 1; i < 4; ++i) me = fma(x[i], av.v[i], me);
+      return me;
+    }
+    T me = T(0);
+    for (int b = 0; b < db; ++b) {
+      load_u4(u + 4 * b, x);
+      T acc = x[0] * av.v[0];
+#pragma unroll
+      for (int i = 1; i < 4; ++i) acc = fma(x[i], av.v[i], acc);
+      me = fma(acc, __ldg(gb + b), me);
+    }
+    return me;
+  }
+  T me = T(0);
+  for (int b = 0; b < db; ++b) {
+    T acc = T(0);
+    for (int i = 0; i < da; ++i) acc = fma(u[da * b + i], __ldg(ga + i), acc);
+    me = db == 1 ? acc : fma(acc, __ldg(gb + b), me);
+  }
+  return me;
+}
+
+template <typename T, int RR>
+__global__ void __launch_bounds__(32 * kBlockWarps)
+    block_sigma_kernel(BlockParams p, const T* __restrict__ w, const T* __restrict__ op, const T* __restrict__ cin,
+                       T* __restrict__ sig) {
+  constexpr int RV = RR > 0 ? RR : kMaxR;
+  __shared__ BlockSmem<T> smem[kBlockWarps];
+  BlockSmem<T>& S = smem[threadIdx.x >> 5];
+  const int R = RR > 0 ? RR : p.R;
+  const int lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1u;
+  const uint4* cfg = reinterpret_cast<const uint4*>(p.cfg);
+  constexpr unsigned kTake = 4;  // jobs taken from the counter at a time
+  for (;;) {
+    unsigned first = 0;
+    if (lane == 0) first = atomicAdd(p.next, kTake);
+    first = __shfl_sync(0xffffffffu, first, 0);
+    if (int64_t(first) >= p.n_jobs) break;
+    const int64_t last = min(int64_t(first) + kTake, p.n_jobs);
+    for (int64_t jn = first; jn < last; ++jn) {
+      const BlockJob J = p.jobs[jn];
+      const int nb = J.nb;
+      const int brow = lane < nb ? p.perm[J.bra + lane] : 0;
+      uint4 rb = make_uint4(0, 0, 0, 0);
+      if (lane < nb) rb = __ldg(cfg + brow);
+      // pair phase: lane = slice * nb + bra
+      const int slices = min(32 / nb, int(J.nk)), sl = lane / nb, bl = lane - sl * nb;
+      const bool on = sl < slices;
+      uint4 mine;  // the states of this lane's bra
+      mine.x = __shfl_sync(0xffffffffu, rb.x, bl);
+      mine.y = __shfl_sync(0xffffffffu, rb.y, bl);
+      mine.z = __shfl_sync(0xffffffffu, rb.z, bl);
+      mine.w = __shfl_sync(0xffffffffu, rb.w, bl);
+      T acc[RV];
+#pragma unroll
+      for (int r = 0; r < RV; ++r) acc[r] = T(0);
+      for (int k0 = 0; k0 < J.nk; k0 += 32) {
+        const int nkb = min(32, int(J.nk) - k0);
+        const int krow = lane < nkb ? p.perm[J.ket + k0 + lane] : 0;
+        uint4 rk = make_uint4(0, 0, 0, 0);
+        if (lane < nkb) rk = __ldg(cfg + krow);
+        for (int t0 = 0; t0 < J.nt;) {
+          const TermSector& ts = p.ts[J.ts_off + t0];
+          int tg = 1;
+          while (tg < kBlockTerms && t0 + tg < J.nt && same_shape(ts, p.ts[J.ts_off + t0 + tg])) ++tg;
+          const int nrem = ts.nrem;
+          // distinct states of (dressed cluster, cluster q) over the bras and over the kets, for the
+          // q with the fewest combinations
+          int q = 0, n_b = 33, n_k = 33;
+          unsigned mb = 0, mk = 0;
+          const unsigned bw = unsigned(state_of(rb, ts.cw)), kw = unsigned(state_of(rk, ts.cw));
+          for (int c = 0; c < nrem; ++c) {
+            const unsigned b = lane < nb ? bw | unsigned(state_of(rb, ts.cr[c])) << 8 : 0x10000u;
+            const unsigned k = lane < nkb ? kw | unsigned(state_of(rk, ts.cr[c])) << 8 : 0x10000u;
+            const unsigned xb = __match_any_sync(0xffffffffu, b), xk = __match_any_sync(0xffffffffu, k);
+            const int db = __popc(__ballot_sync(0xffffffffu, lane < nb && !(xb & below)));
+            const int dk = __popc(__ballot_sync(0xffffffffu, lane < nkb && !(xk & below)));
+            if (db * dk < n_b * n_k) {
+              q = c, n_b = db, n_k = dk, mb = xb, mk = xk;
+            }
+          }
+          const int cq = ts.cr[q], ca = ts.cr[q == 0 ? 1 : 0], cb = ts.cr[q == 2 ? 1 : 2];
+          const int da = ts.g_dim[q == 0 ? 1 : 0], db = nrem == 3 ? ts.g_dim[q == 2 ? 1 : 2] : 1;
+          int ib;  // U index of lane bl's bra
+          {
+            const unsigned lead = __ballot_sync(0xffffffffu, lane < nb && !(mb & below));
+            const int leader = __ffs(mb) - 1;
+            const int i = __popc(lead & ((1u << leader) - 1u));
+            if (lane < nb && leader == lane) S.bst[i] = bw | unsigned(state_of(rb, cq)) << 8;
+            ib = __shfl_sync(0xffffffffu, i, bl);
+          }
+          {
+            const bool live = lane < nkb;
+            const int leader = __ffs(mk) - 1;
+            const bool lead = live && leader == lane;
+            const unsigned leads = __ballot_sync(0xffffffffu, lead);
+            const int i = __popc(leads & ((1u << leader) - 1u));
+            const int base = warp_exclusive(lead ? __popc(mk) : 0);
+            const int at = __shfl_sync(0xffffffffu, base, leader) + __popc(mk & below);
+            if (lead) {
+              S.kst[i] = kw | unsigned(state_of(rk, cq)) << 8;
+              S.kpos[i] = base;
+            }
+            if (live)
+              S.ket[at] = make_int2(krow, i | state_of(rk, ca) << 8 | (nrem == 3 ? state_of(rk, cb) : 0) << 16);
+            if (lane == 0) S.kpos[n_k] = nkb;
+          }
+          __syncwarp();
+          const int du = da * db;
+          if (n_b * du * tg > BlockSmem<T>::kU) tg = 1;  // two terms of long columns: one at a time
+          const int step = min(n_k, BlockSmem<T>::kU / (n_b * du * tg));  // ket pairs of a pass
+          const unsigned m_du = div_magic(unsigned(du)), m_nb = div_magic(unsigned(n_b)), m_da = div_magic(unsigned(da));
+          // the contracted cluster and the W columns: stride and length of its index, per-term bases
+          const int dq = ts.g_dim[q], sq = q == 0 ? 1 : (q == 1 ? ts.g_dim[0] : ts.g_dim[0] * ts.g_dim[1]);
+          const int rest = ts.rest_len, w_mb = ts.w_mb, gq_mb = ts.g_mb[q];
+          const TermSector& ts1 = p.ts[J.ts_off + t0 + tg - 1];
+          const T *w0 = w + ts.w_off, *w1 = w + ts1.w_off, *g0 = op + ts.g_off[q], *g1 = op + ts1.g_off[q];
+          const bool neg0 = ts.sign < 0, neg1 = ts1.sign < 0;
+          // the bra's columns of the clusters left, per term
+          const T* ga[kBlockTerms];
+          const T* gb[kBlockTerms];
+          int ga_mb = 0, gb_mb = 0;
+#pragma unroll
+          for (int t = 0; t < kBlockTerms; ++t) {
+            const TermSector& tt = t == 0 ? ts : ts1;
+            ga[t] = op + tt.g_off[q == 0 ? 1 : 0] + da * state_of(mine, ca);
+            gb[t] = nrem == 3 ? op + tt.g_off[q == 2 ? 1 : 2] + db * state_of(mine, cb) : op;
+          }
+          ga_mb = da * ts.g_mb[q == 0 ? 1 : 0];
+          if (nrem == 3) gb_mb = db * ts.g_mb[q == 2 ? 1 : 2];
+          for (int i0 = 0; i0 < n_k; i0 += step) {
+            const int ni = min(step, n_k - i0);
+            // one U element per lane and step: u[((ki * n_b + bi) * tg + t) * du + o]
+            const int units = n_b * ni * tg * du;
+            for (int e = lane; e < units; e += 32) {
+              const int r = int(div_by(unsigned(e), m_du)), o = e - r * du;
+              const int t = r & (tg - 1), rr = r >> (tg - 1);
+              const int ki = int(div_by(unsigned(rr), m_nb)), bi = rr - ki * n_b;
+              const unsigned b = S.bst[bi], k = S.kst[i0 + ki];
+              int x = q == 0 ? o * dq : o;
+              if (nrem == 3 && q == 1) {
+                const int l = int(div_by(unsigned(o), m_da));
+                x = o - l * da + l * da * dq;
+              }
+              const T* wx = (t ? w1 : w0) + rest * (int(b & 255u) + w_mb * int(k & 255u)) + x;
+              const T* g = (t ? g1 : g0) + dq * (int(b >> 8) + gq_mb * int(k >> 8));
+              T acc;
+              if (dq == 4) {
+                Vec4<T> gv, wv;
+                gv.load(g);
+                if (sq == 1) {
+                  wv.load(wx);
+                } else {
+#pragma unroll
+                  for (int i = 0; i < 4; ++i) wv.v[i] = __ldg(wx + sq * i);
+                }
+                acc = wv.v[0] * gv.v[0];
+#pragma unroll
+                for (int i = 1; i < 4; ++i) acc = fma(wv.v[i], gv.v[i], acc);
+              } else {
+                acc = T(0);
+                for (int i = 0; i < dq; ++i) acc = fma(__ldg(wx + sq * i), __ldg(g + i), acc);
+              }
+              S.u[e] = (t ? neg1 : neg0) ? flip(acc) : acc;
+            }
+            __syncwarp();
+            const int k_hi = S.kpos[i0 + ni];
+            if (on)
+              for (int at = S.kpos[i0] + sl; at < k_hi; at += slices) {
+                const int2 kk = S.ket[at];
+                const T* u = S.u + (((kk.y & 255) - i0) * n_b + ib) * tg * du;
+                const int oa = ga_mb * ((kk.y >> 8) & 255), ob = gb_mb * (kk.y >> 16);
+                T me = block_pair<T>(u, da, db, ga[0] + oa, gb[0] + ob);
+                if (tg == 2) me += block_pair<T>(u + du, da, db, ga[1] + oa, gb[1] + ob);
+                T c[RV];
+                load_row<T, RR, RV>(cin + int64_t(kk.x) * R, R, c);
+#pragma unroll
+                for (int r = 0; r < RV; ++r) acc[r] = fma(me, c[r], acc[r]);
+              }
+            __syncwarp();
+          }
+          t0 += tg;
+        }
+      }
+      // the slices' sums of each bra, then one row addition
+      for (int s = slices; s > 1;) {
+        const int h = (s + 1) >> 1;
+        const int src = lane + h * nb;
+#pragma unroll
+        for (int r = 0; r < RV; ++r) {
+          const T v = __shfl_sync(0xffffffffu, acc[r], src & 31);
+          if (sl + h < s) acc[r] += v;
+        }
+        s = h;
+      }
+      const int row = __shfl_sync(0xffffffffu, brow, bl);
+      if (sl == 0) add_row<T, RR, RV>(sig, row, acc, R);
+    }
+  }
 }
 
 // ---- stored Hamiltonian blocks -------------------------------------------------------------
@@ -647,6 +940,7 @@ static LaneParams make_lane_params(fcg_ctx* ctx, int R) {
   p.perm = ctx->d_perm.p;
   p.ts = ctx->d_ts.p;
   p.cfg = ctx->d_cfg.p;
+  p.n_jobs = ctx->plan_jobs;
   p.R = R;
   return p;
 }
@@ -1025,7 +1319,7 @@ static int state_rows_impl(fcg_ctx* ctx, int64_t n_cfg, const int16_t* fock, con
   ctx->stats.n_sectors = int64_t(P.sec_start.size());
   ctx->stats.plan_seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
   ctx->tuned[0] = ctx->tuned[1] = -1;  // a new shape: tune again (or find it in the shape cache)
-  ctx->fine_built = false;
+  ctx->fine_built[0] = ctx->fine_built[1] = false;
   ctx->have_state = true;
   return FCG_OK;
 }
@@ -1107,7 +1401,7 @@ int fcg_set_planner(fcg_ctx* ctx, int on_device) {
     ctx->plan_on_device = on_device == 1;
     ctx->have_plan = false;
     ctx->drop_hcache();
-    ctx->fine_built = false;
+    ctx->fine_built[0] = ctx->fine_built[1] = false;
   }
   return FCG_OK;
 }
@@ -1185,25 +1479,33 @@ std::string tune_key(const fcg_ctx* ctx, int prec, int R) {
 }
 }  // namespace
 
+// whether a direct sigma of this precision runs block jobs and the lane jobs of the other items, or
+// every lane job.  Block jobs are for double: they cut the FP64 multiply-adds that bound it by
+// more than half.  In float the lane kernel is bound by loads, and a block's set-up costs what its
+// shared columns save (24 orbitals, 1e5 configurations, 4 roots: 2.40 ms with, 2.33 ms without).
+template <typename T>
+static bool use_blocks(const fcg_ctx* ctx) {
+  return sizeof(T) == 8 && ctx->plan_on_device && ctx->n_block_jobs > 0;
+}
+
 // the finer chunk table of the tuning candidates (built on first use)
-static int fine_chunks(fcg_ctx* ctx) {
-  if (ctx->fine_built) return FCG_OK;
+static int fine_chunks(fcg_ctx* ctx, bool direct) {
+  const int which = direct ? 1 : 0;
+  if (ctx->fine_built[which]) return FCG_OK;
+  DevBuf<int64_t>& table = ctx->d_chunk_lo_fine[which];
+  int64_t nc = 0;
   if (ctx->plan_on_device) {
-    int64_t nc = 0;
-    const int rc = device_chunks(ctx, 4 * kTargetChunks, ctx->d_chunk_lo_fine, ctx->d_chunk_val_fine, &nc);
+    const int rc = device_chunks(ctx, 4 * kTargetChunks, table, nullptr, &nc, direct);
     if (rc) return rc;
-    FCG_REQUIRE(lane_ctas(nc) < (int64_t(1) << 31), FCG_ELIMIT, "too many warp chunks for one launch");
-    ctx->n_chunks_fine = nc;
-    ctx->fine_built = true;
-    return FCG_OK;
+  } else {
+    std::vector<int64_t> lo, val;
+    make_chunks(ctx->plan, 4 * kTargetChunks, lo, val);
+    FCG_CUDA(table.upload(lo.data(), lo.size(), ctx->stream));
+    nc = int64_t(lo.size()) - 1;
   }
-  std::vector<int64_t> lo, val;
-  make_chunks(ctx->plan, 4 * kTargetChunks, lo, val);
-  FCG_REQUIRE(lane_ctas(int64_t(lo.size()) - 1) < (int64_t(1) << 31), FCG_ELIMIT, "too many warp chunks for one launch");
-  FCG_CUDA(ctx->d_chunk_lo_fine.upload(lo.data(), lo.size(), ctx->stream));
-  FCG_CUDA(ctx->d_chunk_val_fine.upload(val.data(), val.size(), ctx->stream));
-  ctx->n_chunks_fine = int64_t(lo.size()) - 1;
-  ctx->fine_built = true;
+  FCG_REQUIRE(lane_ctas(nc) < (int64_t(1) << 31), FCG_ELIMIT, "too many warp chunks for one launch");
+  ctx->n_chunks_fine[which] = nc;
+  ctx->fine_built[which] = true;
   return FCG_OK;
 }
 
@@ -1213,21 +1515,28 @@ static void launch_lane(const LaneParams& p, int64_t grid, int R, const T* w, co
   switch (R) {
     case 1: closed_sigma_lane_kernel<T, 1, MINB><<<unsigned(grid), kSigmaThreads, 0, s>>>(p, w, op, cin, sig); break;
     case 2: closed_sigma_lane_kernel<T, 2, MINB><<<unsigned(grid), kSigmaThreads, 0, s>>>(p, w, op, cin, sig); break;
+    case 3: closed_sigma_lane_kernel<T, 3, MINB><<<unsigned(grid), kSigmaThreads, 0, s>>>(p, w, op, cin, sig); break;
     case 4: closed_sigma_lane_kernel<T, 4, MINB><<<unsigned(grid), kSigmaThreads, 0, s>>>(p, w, op, cin, sig); break;
     default: closed_sigma_lane_kernel<T, 0, MINB><<<unsigned(grid), kSigmaThreads, 0, s>>>(p, w, op, cin, sig); break;
   }
 }
 
-// one direct closed sigma with candidate c
+// one direct closed sigma's lane jobs with candidate c (all of them, or those of the items that do
+// not run as block jobs)
 template <typename T>
 static int launch_candidate(fcg_ctx* ctx, int c, int R, const T* w, const T* op, const T* cin, T* sig) {
   LaneParams p = make_lane_params(ctx, R);
+  const bool direct = use_blocks<T>(ctx);
+  if (direct) {
+    p.n_jobs = ctx->plan.n_direct;
+    p.chunk_lo = ctx->d_chunk_lo_direct.p;
+    p.n_chunks = ctx->n_chunks_direct;
+  }
   if (c >> 1) {
-    const int rc = fine_chunks(ctx);
+    const int rc = fine_chunks(ctx, direct);
     if (rc) return rc;
-    p.chunk_lo = ctx->d_chunk_lo_fine.p;
-    p.chunk_val = ctx->d_chunk_val_fine.p;
-    p.n_chunks = ctx->n_chunks_fine;
+    p.chunk_lo = ctx->d_chunk_lo_fine[direct].p;
+    p.n_chunks = ctx->n_chunks_fine[direct];
   }
   const int64_t grid = lane_ctas(p.n_chunks);
   if (grid == 0) return FCG_OK;
@@ -1239,7 +1548,31 @@ static int launch_candidate(fcg_ctx* ctx, int c, int R, const T* w, const T* op,
   return FCG_OK;
 }
 
-// Times every candidate once on this state (each run a complete sigma into sig), keeps the
+// the block jobs of a direct closed sigma
+static int launch_blocks(fcg_ctx* ctx, int R, const double* w, const double* op, const double* cin, double* sig) {
+  BlockParams p{};
+  p.jobs = ctx->d_block_jobs.p;
+  p.n_jobs = ctx->n_block_jobs;
+  p.perm = ctx->d_perm.p;
+  p.ts = ctx->d_ts.p;
+  p.cfg = ctx->d_cfg.p;
+  p.next = ctx->d_block_next.p;
+  p.R = R;
+  auto kernel = R == 1   ? block_sigma_kernel<double, 1>
+                : R == 2 ? block_sigma_kernel<double, 2>
+                : R == 3 ? block_sigma_kernel<double, 3>
+                : R == 4 ? block_sigma_kernel<double, 4> : block_sigma_kernel<double, 0>;
+  int per_sm = 1, n_sm = 152;
+  FCG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * kBlockWarps, 0));
+  FCG_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, ctx->device));
+  const int64_t grid = std::min<int64_t>(int64_t(std::max(per_sm, 1)) * n_sm, (p.n_jobs + kBlockWarps - 1) / kBlockWarps);
+  FCG_CUDA(cudaMemsetAsync(p.next, 0, sizeof(unsigned), ctx->stream));
+  kernel<<<unsigned(grid), 32 * kBlockWarps, 0, ctx->stream>>>(p, w, op, cin, sig);
+  FCG_CUDA(cudaGetLastError());
+  return FCG_OK;
+}
+
+// Times every candidate once on this state (each a run of its lane jobs into sig), keeps the
 // fastest for the context and for later states of the same shape in this process.
 template <typename T>
 static int tune_closed(fcg_ctx* ctx, int prec, int R, const T* w, const T* op, const T* cin, T* sig) {
@@ -1285,6 +1618,10 @@ static int launch_closed(fcg_ctx* ctx, int R, const T* w, const T* op, const T* 
                          bool timed = true) {
   const int prec = sizeof(T) == 4 ? 1 : 0;
   FCG_REQUIRE(ctx->have_plan, FCG_ESTATE, "the closed-sigma plan is missing (fcg_state_set builds it)");
+  if (!ctx->have_hcache && use_blocks<T>(ctx)) {
+    const int rc = build_block_jobs(ctx);
+    if (rc) return rc;
+  }
   if (!ctx->have_hcache && ctx->tune_mode < 0 && ctx->tuned[prec] < 0 && timed) {
     const int rc = tune_closed<T>(ctx, prec, R, w, op, cin, sig);
     if (rc) return rc;
@@ -1300,16 +1637,24 @@ static int launch_closed(fcg_ctx* ctx, int R, const T* w, const T* op, const T* 
     switch (R) {
       case 1: cached_sigma_lane_kernel<T, 1><<<unsigned(grid), kSigmaThreads, 0, ctx->stream>>>(p, hc, cin, sig); break;
       case 2: cached_sigma_lane_kernel<T, 2><<<unsigned(grid), kSigmaThreads, 0, ctx->stream>>>(p, hc, cin, sig); break;
+      case 3: cached_sigma_lane_kernel<T, 3><<<unsigned(grid), kSigmaThreads, 0, ctx->stream>>>(p, hc, cin, sig); break;
       case 4: cached_sigma_lane_kernel<T, 4><<<unsigned(grid), kSigmaThreads, 0, ctx->stream>>>(p, hc, cin, sig); break;
       default: cached_sigma_lane_kernel<T, 0><<<unsigned(grid), kSigmaThreads, 0, ctx->stream>>>(p, hc, cin, sig); break;
     }
     FCG_CUDA(cudaGetLastError());
     launches = 1;
   } else if (grid > 0) {
+    if constexpr (sizeof(T) == 8) {
+      if (use_blocks<T>(ctx)) {
+        const int rc = launch_blocks(ctx, R, w, op, cin, sig);
+        if (rc) return rc;
+        launches = 1;
+      }
+    }
     const int c = ctx->tune_mode >= 0 ? ctx->tune_mode : (ctx->tuned[prec] >= 0 ? ctx->tuned[prec] : 0);
     const int rc = launch_candidate<T>(ctx, c, R, w, op, cin, sig);
     if (rc) return rc;
-    launches = 1;
+    launches += 1;
   }
   if (timed) FCG_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
   ctx->stats.kernel_launches = launches;

@@ -100,7 +100,7 @@ struct WorkItem {
   int32_t nt;       // number of terms
 };
 
-// A closed-sigma lane job: one bra row of a work item against up to kLaneKets of the item's
+// A closed-sigma lane job: one bra row of a work item against up to lane_kets(..) of the item's
 // kets.  Warps run 32 consecutive lane jobs, one per lane; a lane sums the item's terms for
 // each of its (bra, ket) pairs, multiplies by the ket's coefficients and adds its row to
 // sigma once.  The planner orders lane jobs so that the lanes of a warp have the same term
@@ -113,7 +113,51 @@ struct LaneJob {
   uint16_t nt;     // terms
 };
 static_assert(sizeof(LaneJob) == 16, "LaneJob layout");
-constexpr int kLaneKets = 32;
+
+// Kets of a lane job at most: the largest of these that still cuts the state into kLaneTasks warp
+// tasks (eight for every warp that 152 SMs hold at 32 warps each), else the smallest.  A lane takes
+// its kets one after the other, a chain of dependent loads for each (about 1 us), so small states
+// want short jobs (12 orbitals, 2000 configurations, FP64: 76 us a sigma against 150 with 32 kets
+// always, 10 against 29 us from stored blocks); large ones want one row added for many kets.
+constexpr int kLaneKets[4] = {32, 16, 8, 4};
+constexpr int64_t kLaneTasks = 8 * 152 * 32;
+
+// A closed-sigma block job: up to kBlockBras bra rows x kBlockKets kets of a work item of three
+// or more active clusters, for one warp.  Within it the dressed cluster's W column contracted
+// with one more cluster's TDM column depends only on the two clusters' states, so it is formed
+// once per distinct (bra pair of states, ket pair of states) and not per (bra, ket).
+struct BlockJob {
+  int32_t bra, ket;  // first rows in the permutation pool
+  int32_t ts_off;    // the item's term-sector records
+  uint8_t nb, nk;
+  uint16_t nt;       // terms
+};
+static_assert(sizeof(BlockJob) == 16, "BlockJob layout");
+constexpr int kBlockBras = 32;
+constexpr int kBlockKets = 128;
+// Work items of at least this many (bra, ket) pairs run as block jobs, the others as lane jobs
+// only (the lane jobs cover every item: stored Hamiltonian blocks are laid out along them).  24
+// orbitals, 1e5 configurations, 4 roots, FP64: 6.58 ms from 32 pairs, 6.73 from 48, 6.87 from 80,
+// 8.8 from 16; 9.78 with lane jobs only.
+constexpr int kBlockPairs = 32;
+// Longest partly contracted W column (the product of the index lengths left) of a block job.
+constexpr int kBlockU = 40;
+
+FCG_HD inline bool block_item(bool eligible, int64_t nb, int64_t nk) { return eligible && nb * nk >= kBlockPairs; }
+// States of fewer multiply-adds than this (about a tenth of a millisecond of the FP64 pipe) have no
+// block items: there the lane jobs are bound by latency, and block jobs only add to it.
+constexpr int64_t kBlockMinFma = int64_t(1) << 26;
+
+// kets of a lane job from the job counts of each choice
+inline int lane_kets(const int64_t* jobs) {
+  int i = 0;
+  while (i < 3 && (jobs[i] + 31) / 32 < kLaneTasks) ++i;
+  return i;
+}
+
+FCG_HD inline int64_t block_jobs_of(int64_t nb, int64_t nk) {
+  return ((nb + kBlockBras - 1) / kBlockBras) * ((nk + kBlockKets - 1) / kBlockKets);
+}
 
 // One W block to compute (fcg_set_terms): term t dressed with TDM block g of its dressed cluster.
 struct DressJob {
@@ -226,6 +270,8 @@ struct Plan {
   std::vector<LaneJob> jobs;
   std::vector<int64_t> chunk_lo;
   std::vector<int64_t> chunk_val;
+  int lane_kets = 32;           // kets of a lane job at most
+  int64_t n_direct = 0;         // lane jobs of the items that are not block items; they come first
   int64_t task_values = 0;      // 32 x the longest lane job of every warp task, summed
   std::vector<int32_t> wt_cost;  // planner cost of every warp task (its most expensive lane)
   std::vector<int32_t> wt_len;   // longest lane job of every warp task
@@ -341,6 +387,7 @@ struct TermLists {
   std::vector<int32_t> off;          // list j holds terms[off[j], off[j+1])
   std::vector<int32_t> terms;
   std::vector<int32_t> first_of_tr;  // lists of transfer tr: [first_of_tr[tr], first_of_tr[tr+1])
+  std::vector<uint8_t> block;        // 1: items of the list may run as block jobs
 };
 std::string term_lists(const ProblemInfo& pi, TermLists& lists);
 

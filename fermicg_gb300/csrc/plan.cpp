@@ -9,7 +9,7 @@
 // transfer, active set) the bra and ket key lists are merge-joined.  Each
 // matching key gives one work item = a dense block of (bra, ket, term)
 // triples that all pass check_term.  Each bra row of a work item, with up to
-// 32 of its kets, becomes one lane job of the sigma kernel; lane jobs are
+// lane_kets of its kets, becomes one lane job of the sigma kernel; lane jobs are
 // sorted so that a warp's 32 lanes do the same kind and amount of work.
 #include <algorithm>
 #include <array>
@@ -48,6 +48,14 @@ struct PJob {
   LaneJob j;
   int32_t cost;
   int32_t nbody;
+  bool block;  // of a block item: after the jobs of the other items
+};
+
+// What an item's lane jobs need besides the item.
+struct ItemMeta {
+  int64_t step_cost;  // planner cost of one ket of a lane job
+  int32_t nbody;
+  bool block;
 };
 
 }  // namespace
@@ -102,6 +110,18 @@ std::string term_lists(const ProblemInfo& pi, TermLists& L) {
     }
   }
   L.first_of_tr[pi.n_trans] = int32_t(L.tr.size());
+  // lists that may run as block jobs: three or four active clusters, and a W column short enough
+  // once one index is contracted, whichever that is
+  L.block.assign(L.tr.size(), 0);
+  for (size_t j = 0; j < L.tr.size(); ++j) {
+    bool ok = true;
+    for (int q2 = L.off[j]; q2 < L.off[j + 1] && ok; ++q2) {
+      const TermDress& d = (*pi.dress)[size_t(L.terms[size_t(q2)])];
+      ok = d.nrem == 2 || d.nrem == 3;
+      for (int q3 = 0; ok && q3 < d.nrem; ++q3) ok = d.rest_len / d.rem_dim[q3] <= kBlockU;
+    }
+    L.block[j] = ok ? 1 : 0;
+  }
   return "";
 }
 
@@ -229,6 +249,7 @@ std::string build_join(const ProblemInfo& pi, const int16_t* fock, const int16_t
   // thread timing
   std::vector<std::vector<WorkItem>> tItems(n_sec);
   std::vector<std::vector<TermSector>> tTS(n_sec);
+  std::vector<std::vector<ItemMeta>> tMeta(n_sec);
   std::vector<std::vector<PJob>> tJobs(n_sec);
   std::vector<int64_t> tFlop(n_sec, 0), tFlopD(n_sec, 0);
   const TermTables tt = term_tables(pi);
@@ -293,18 +314,7 @@ std::string build_join(const ProblemInfo& pi, const int16_t* fock, const int16_t
               w.ts_off = ts_off;
               w.nt = int32_t(tsl.size());
               tItems[sb].push_back(w);
-              for (int bj = 0; bj < w.nb; ++bj)
-                for (int k0 = 0; k0 < w.nk; k0 += kLaneKets) {
-                  PJob pj;
-                  pj.j.b = P.perm_pool[size_t(w.bra_off) + bj];
-                  pj.j.kp = w.ket_off + k0;
-                  pj.j.ts_off = w.ts_off;  // relative; rebased at concatenation
-                  pj.j.len = uint16_t(std::min(kLaneKets, w.nk - k0));
-                  pj.j.nt = uint16_t(w.nt);
-                  pj.cost = int32_t(std::min<int64_t>(step_cost * pj.j.len, int64_t(1) << 30));
-                  pj.nbody = nbody_tl;
-                  tJobs[sb].push_back(pj);
-                }
+              tMeta[sb].push_back(ItemMeta{step_cost, nbody_tl, block_item(L.block[j] != 0, w.nb, w.nk)});
               tFlop[sb] += int64_t(w.nb) * w.nk * flop;
               tFlopD[sb] += int64_t(w.nb) * w.nk * flopd;
               ++a;
@@ -322,6 +332,35 @@ std::string build_join(const ProblemInfo& pi, const int16_t* fock, const int16_t
   }
   if (tots >= (size_t(1) << 31)) return "term-sector pool exceeds 2^31 records";
   if (tot >= (size_t(1) << 31)) return "work items exceed 2^31";
+  // lane jobs of every item, as long as the state's size allows
+  int64_t flopd_all = 0, n_lane[4] = {0, 0, 0, 0};
+  for (int64_t sb = 0; sb < n_sec; ++sb) {
+    flopd_all += tFlopD[sb];
+    for (const WorkItem& w : tItems[sb])
+      for (int i = 0; i < 4; ++i) n_lane[i] += int64_t(w.nb) * ((w.nk + kLaneKets[i] - 1) / kLaneKets[i]);
+  }
+  const int max_kets = kLaneKets[lane_kets(n_lane)];
+  const bool with_blocks = flopd_all / 2 >= kBlockMinFma;
+  P.lane_kets = max_kets;
+#pragma omp parallel for schedule(dynamic, 8)
+  for (int64_t sb = 0; sb < n_sec; ++sb)
+    for (size_t i = 0; i < tItems[sb].size(); ++i) {
+      const WorkItem& w = tItems[sb][i];
+      const ItemMeta& m = tMeta[sb][i];
+      for (int bj = 0; bj < w.nb; ++bj)
+        for (int k0 = 0; k0 < w.nk; k0 += max_kets) {
+          PJob pj;
+          pj.j.b = P.perm_pool[size_t(w.bra_off) + bj];
+          pj.j.kp = w.ket_off + k0;
+          pj.j.ts_off = w.ts_off;  // relative; rebased at concatenation
+          pj.j.len = uint16_t(std::min(max_kets, w.nk - k0));
+          pj.j.nt = uint16_t(w.nt);
+          pj.cost = int32_t(std::min<int64_t>(m.step_cost * pj.j.len, int64_t(1) << 30));
+          pj.nbody = m.nbody;
+          pj.block = m.block && with_blocks;
+          tJobs[sb].push_back(pj);
+        }
+    }
   // concatenation in sector order, each sector's part copied by one thread
   std::vector<int64_t> item_off(n_sec + 1, 0), tsp_off(n_sec + 1, 0), job_off(n_sec + 1, 0);
   for (int64_t sb = 0; sb < n_sec; ++sb) {
@@ -347,10 +386,11 @@ std::string build_join(const ProblemInfo& pi, const int16_t* fock, const int16_t
     std::vector<WorkItem>().swap(tItems[sb]);
     std::vector<TermSector>().swap(tTS[sb]);
   }
-  // Lane jobs of windows of kSortWindow bra sectors sorted by term shape, then by decreasing
-  // cost (ties in planning order: the rows of one work item stay together and share their kets), so that the
-  // 32 lanes of a warp run the same code on about the same number of kets.  The last warp task
-  // is padded with idle lanes (len 0).
+  // The lane jobs of block items come last.  Before and after that line, the lane jobs of windows
+  // of kSortWindow bra sectors are sorted by term shape, then by decreasing cost (ties in planning
+  // order: the rows of one work item stay together and share their kets), so that the 32 lanes of
+  // a warp run the same code on about the same number of kets.  The last warp task is padded with
+  // idle lanes (len 0).
   const int64_t n_jobs = job_off[n_sec];
   const int64_t n_wt = (n_jobs + 31) / 32;  // warp tasks
   P.jobs.resize(size_t(n_wt) * 32);
@@ -359,6 +399,14 @@ std::string build_join(const ProblemInfo& pi, const int16_t* fock, const int16_t
   {
     constexpr int64_t kSortWindow = 8;
     const int64_t n_win = (n_sec + kSortWindow - 1) / kSortWindow;
+    // first position of each window's jobs, of the other items and of the block items
+    std::vector<int64_t> at[2] = {std::vector<int64_t>(size_t(n_win) + 1, 0), std::vector<int64_t>(size_t(n_win) + 1, 0)};
+    for (int64_t sb = 0; sb < n_sec; ++sb)
+      for (const PJob& q : tJobs[sb]) ++at[q.block ? 1 : 0][size_t(sb / kSortWindow) + 1];
+    for (auto& a : at)
+      for (int64_t w = 0; w < n_win; ++w) a[size_t(w) + 1] += a[size_t(w)];
+    P.n_direct = at[0][size_t(n_win)];
+    for (int64_t& x : at[1]) x += P.n_direct;
 #pragma omp parallel
     {
       std::vector<uint64_t> keys;  // (nbody, decreasing cost, position in the window): one sort key
@@ -371,15 +419,16 @@ std::string build_join(const ProblemInfo& pi, const int16_t* fock, const int16_t
         for (int64_t sb = s0; sb < s1; ++sb)
           for (const PJob& q : tJobs[sb]) {
             const uint64_t c = uint64_t(std::min<int32_t>(q.cost, (1 << 26) - 1));
-            keys.push_back((uint64_t(q.nbody) << 58) | (((uint64_t(1) << 26) - 1 - c) << 32) | uint64_t(src.size()));
+            keys.push_back((uint64_t(q.block) << 63) | (uint64_t(q.nbody) << 58) | (((uint64_t(1) << 26) - 1 - c) << 32) | uint64_t(src.size()));
             src.push_back(&q);
           }
         std::sort(keys.begin(), keys.end());
-        const int64_t o = job_off[s0];
+        const int64_t n0 = at[0][size_t(wdx) + 1] - at[0][size_t(wdx)];
         for (size_t i = 0; i < keys.size(); ++i) {
           const PJob& q = *src[size_t(keys[i] & 0xFFFFFFFFu)];
-          P.jobs[size_t(o) + i] = q.j;
-          job_cost[size_t(o) + i] = q.cost;
+          const int64_t o = int64_t(i) < n0 ? at[0][size_t(wdx)] + int64_t(i) : at[1][size_t(wdx)] + int64_t(i) - n0;
+          P.jobs[size_t(o)] = q.j;
+          job_cost[size_t(o)] = q.cost;
         }
         for (int64_t sb = s0; sb < s1; ++sb) std::vector<PJob>().swap(tJobs[sb]);
       }
