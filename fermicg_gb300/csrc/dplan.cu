@@ -339,9 +339,10 @@ __device__ __forceinline__ T warp_sum(T v) {
 }
 
 // one thread per pair (a term list holds a few terms, and most pairs have no ket sector):
-// the records that exist, their flop counts, and the bra groups to join
+// the records that exist (one for a set of merged terms), the terms and their flop counts, and the
+// bra groups to join
 __global__ void pair_count_kernel(PairParams p, int64_t* __restrict__ pt_nt, int64_t* __restrict__ pt_ng,
-                                  int64_t* __restrict__ pt_flop, int64_t* __restrict__ pt_flopd) {
+                                  int64_t* __restrict__ pt_tri, int64_t* __restrict__ pt_flop, int64_t* __restrict__ pt_flopd) {
   const int64_t w = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (w > p.n_pt) return;
   if (w == p.n_pt) {  // zeros past the end for the scans
@@ -351,23 +352,27 @@ __global__ void pair_count_kernel(PairParams p, int64_t* __restrict__ pt_nt, int
   const int64_t sb = w / p.n_tl;
   const int j = int(w - sb * p.n_tl);
   const int32_t sk = p.sk_of[sb * p.n_trans + p.tl_tr[j]];
-  int64_t nt = 0, flop = 0, flopd = 0;
+  int64_t nt = 0, tri = 0, flop = 0, flopd = 0;
   if (sk >= 0) {
     const int16_t* fb = p.sec_fock + sb * 2 * p.N;
     const int16_t* fk = p.sec_fock + int64_t(sk) * 2 * p.N;
     for (int q = p.tl_off[j]; q < p.tl_off[j + 1]; ++q) {
       const int t = p.tl_terms[q];
+      if (term_exists(p.tt, t, fb, fk)) {
+        flop += term_ref_flops(p.tt.trm, t);
+        ++tri;
+      }
       TermSector ts;
       int64_t fma;
-      if (term_sector_of(p.tt, t, fb, fk, ts, &fma)) {
+      if (p.tt.rep[t] == t && term_sector_of(p.tt, t, fb, fk, ts, &fma)) {
         ++nt;
-        flop += term_ref_flops(p.tt.trm, t);
         flopd += 2 * fma;
       }
     }
   }
   const int64_t seg = sb * p.n_sets + p.tl_set[j];
   pt_nt[w] = nt;
+  pt_tri[w] = tri;
   pt_flop[w] = flop;
   pt_flopd[w] = flopd;
   pt_ng[w] = nt > 0 ? p.seg_g[seg + 1] - p.seg_g[seg] : 0;
@@ -387,7 +392,8 @@ __global__ void pair_records_kernel(PairParams p, const int64_t* __restrict__ ts
   for (int q = p.tl_off[j]; q < p.tl_off[j + 1]; ++q) {
     TermSector ts;
     int64_t fma;
-    if (term_sector_of(p.tt, p.tl_terms[q], fb, fk, ts, &fma)) pool[o++] = ts;
+    const int t = p.tl_terms[q];
+    if (p.tt.rep[t] == t && term_sector_of(p.tt, t, fb, fk, ts, &fma)) pool[o++] = ts;
   }
 }
 
@@ -449,8 +455,8 @@ struct ItemOut {
 // counters: 0 triples, 1 reference flops, 2 executed flops, 3 largest ket step of a lane job, 9 block
 // jobs, 10-13 lane jobs with each kLaneKets, 14-17 those of the block items
 __global__ void items_kernel(PairParams p, int64_t E, const int64_t* __restrict__ pt_e, const int64_t* __restrict__ pt_nt,
-                             const int64_t* __restrict__ pt_flop, const int64_t* __restrict__ pt_flopd,
-                             const int32_t* __restrict__ g_start, const int32_t* __restrict__ g_cnt,
+                             const int64_t* __restrict__ pt_tri, const int64_t* __restrict__ pt_flop,
+                             const int64_t* __restrict__ pt_flopd, const int32_t* __restrict__ g_start, const int32_t* __restrict__ g_cnt,
                              const int32_t* __restrict__ item_of, const int32_t* __restrict__ m_ket,
                              const int32_t* __restrict__ m_pair, const uint8_t* __restrict__ tl_block, ItemOut out,
                              unsigned long long* __restrict__ counters) {
@@ -474,7 +480,7 @@ __global__ void items_kernel(PairParams p, int64_t E, const int64_t* __restrict_
     out.nb[it] = int32_t(nb);
     if (block_item(tl_block[j] != 0, nb, nk)) bj = (unsigned long long)block_jobs_of(nb, nk);
     out.blk[it] = int32_t(bj);
-    tri = (unsigned long long)(nb * nk * nt);
+    tri = (unsigned long long)(nb * nk * pt_tri[w]);
     fl = (unsigned long long)(nb * nk * pt_flop[w]);
     fld = (unsigned long long)(nb * nk * pt_flopd[w]);
     const int64_t step = pt_flopd[w] / 2 + 8 * nt + 4;
@@ -712,7 +718,10 @@ static int upload_term_tables(fcg_ctx* ctx) {
   cudaStream_t s = ctx->stream;
   FCG_CUDA(D.d_trm.upload(ctx->trm.data(), ctx->trm.size(), s));
   FCG_CUDA(D.d_dress.upload(ctx->dress.data(), ctx->dress.size(), s));
-  FCG_CUDA(D.d_w_index.upload(ctx->w_index.data(), ctx->w_index.size(), s));
+  const Dressing& dz = ctx->dressing;
+  FCG_CUDA(D.d_w_index.upload(dz.w_index.data(), dz.w_index.size(), s));
+  FCG_CUDA(D.d_w_mb.upload(dz.w_mb.data(), dz.w_mb.size(), s));
+  FCG_CUDA(D.d_rep.upload(dz.rep.data(), dz.rep.size(), s));
   FCG_CUDA(D.d_trans.upload(ctx->trans.data(), ctx->trans.size(), s));
   FCG_CUDA(D.d_first_of_tr.upload(L.first_of_tr.data(), L.first_of_tr.size(), s));
   FCG_CUDA(D.d_tl_tr.upload(L.tr.data(), L.tr.size(), s));
@@ -870,7 +879,6 @@ int build_join_device(fcg_ctx* ctx) {
   P.chunk_val.clear();
   P.wt_cost.clear();
   P.wt_len.clear();
-  P.prefix.clear();
   P.ts_pool.clear();
   P.perm_pool.clear();
   P.n_triples = P.flops_ref = P.flops_dressed = P.task_values = P.n_direct = 0;
@@ -932,11 +940,12 @@ int build_join_device(fcg_ctx* ctx) {
     if (rc) return rc;
   }
   int32_t* sk_of;
-  int64_t *pt_nt, *pt_ng, *pt_flop, *pt_flopd, *pt_tmp;
+  int64_t *pt_nt, *pt_ng, *pt_tri, *pt_flop, *pt_flopd, *pt_tmp;
   FCG_CUDA(carve(D.arena[1], [&](Bump& b) {
     sk_of = b.take<int32_t>(n_sec * n_trans);
     pt_nt = b.take<int64_t>(n_pt + 1);
     pt_ng = b.take<int64_t>(n_pt + 1);
+    pt_tri = b.take<int64_t>(n_pt);
     pt_flop = b.take<int64_t>(n_pt);
     pt_flopd = b.take<int64_t>(n_pt);
     pt_tmp = b.take<int64_t>(dprim::scan_scratch(n_pt + 1));
@@ -948,7 +957,8 @@ int build_join_device(fcg_ctx* ctx) {
 
   // ---- 3. term-sector records ------------------------------------------------------------
   PairParams pp{};
-  pp.tt = TermTables{D.d_trm.p, D.d_dress.p, D.d_w_index.p, ctx->d_blk_index.p, ctx->d_blocks.p, ctx->nmax + 1};
+  pp.tt = TermTables{D.d_trm.p, D.d_dress.p, D.d_w_index.p, D.d_w_mb.p, D.d_rep.p, ctx->d_blk_index.p, ctx->d_blocks.p,
+                     ctx->nmax + 1};
   pp.sec_fock = ctx->d_sec_fock.p;
   pp.sk_of = sk_of;
   pp.tl_tr = D.d_tl_tr.p;
@@ -961,7 +971,7 @@ int build_join_device(fcg_ctx* ctx) {
   pp.n_trans = n_trans;
   pp.n_sets = n_sets;
   pp.N = N;
-  pair_count_kernel<<<grid_for(n_pt + 1), kThreads, 0, s>>>(pp, pt_nt, pt_ng, pt_flop, pt_flopd);
+  pair_count_kernel<<<grid_for(n_pt + 1), kThreads, 0, s>>>(pp, pt_nt, pt_ng, pt_tri, pt_flop, pt_flopd);
   FCG_CUDA(cudaGetLastError());
   FCG_CUDA(dprim::exclusive_scan<int64_t>(pt_nt, n_pt + 1, pt_tmp, s));
   FCG_CUDA(dprim::exclusive_scan<int64_t>(pt_ng, n_pt + 1, pt_tmp, s));
@@ -1002,7 +1012,7 @@ int build_join_device(fcg_ctx* ctx) {
   FCG_CUDA(cudaGetLastError());
   FCG_CUDA(dprim::exclusive_scan<int32_t>(m_flag, E + 1, m_tmp, s));
   if (E > 0) {
-    items_kernel<<<grid_for(E), kThreads, 0, s>>>(pp, E, pt_ng, pt_nt, pt_flop, pt_flopd, g_start, g_cnt, m_flag,
+    items_kernel<<<grid_for(E), kThreads, 0, s>>>(pp, E, pt_ng, pt_nt, pt_tri, pt_flop, pt_flopd, g_start, g_cnt, m_flag,
                                                   m_ket, m_pair, D.d_tl_block.p, io, D.d_cnt.p);
     FCG_CUDA(cudaGetLastError());
   }

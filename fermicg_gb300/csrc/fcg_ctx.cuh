@@ -107,16 +107,17 @@ struct fcg_ctx {
   std::vector<double> term_ints_norm;  // Frobenius norm of each term's integrals (0 for 1-body terms; term_norms)
   int64_t n_ints = 0;
   std::vector<TermDress> dress;
-  std::vector<int64_t> w_index;
-  int64_t n_w = 0;
+  Dressing dressing;       // merged terms: the closed sigma's W (d_w64, d_w32)
+  Dressing open_dressing;  // a W for every term: the open sigma's (d_ow64, d_ow32), built by its first use
   DevBuf<TermInfo> d_terms;
   DevBuf<double> d_ints64;
   DevBuf<float> d_ints32;
   DevBuf<double> d_w64;
   DevBuf<float> d_w32;
-  std::vector<DressJob> dress_jobs;  // W blocks to build (fcg_set_terms), built by the first fcg_state_set
-  bool dressed = false;
-  bool wmax_built = false;  // column maxima of the dressed operators (open-sigma screen)
+  bool dressed = false;      // by the first closed-sigma plan
+  bool open_dressed = false; // with the column maxima of the open sigma's screen
+  DevBuf<double> d_ow64;
+  DevBuf<float> d_ow32;
   int n_trans = 0;
   std::vector<int16_t> trans;
   // state + plan
@@ -151,6 +152,7 @@ struct fcg_ctx {
     DevBuf<int32_t> d_trm;
     DevBuf<TermDress> d_dress;
     DevBuf<int64_t> d_w_index;
+    DevBuf<int32_t> d_w_mb, d_rep;
     DevBuf<int16_t> d_trans;
     DevBuf<int32_t> d_first_of_tr, d_tl_tr, d_tl_set, d_tl_off, d_tl_terms, d_tl_nbody;
     DevBuf<uint8_t> d_spec_off, d_tl_block;
@@ -220,7 +222,7 @@ struct fcg_ctx {
   DevBuf<double> d_hd;
   // screening maxima: Gmax[i, k] = max_b |G[i, b, k]| per TDM block, Wmax likewise per W block
   std::vector<int64_t> gmax_off;   // per block
-  std::vector<int64_t> wmax_index; // parallel to w_index
+  std::vector<int64_t> wmax_index; // parallel to open_dressing.w_index
   DevBuf<double> d_gmax;
   DevBuf<double> d_wmax;
   // open sigma (FOIS) working set and last result
@@ -298,7 +300,7 @@ int sigma_closed_device_async(fcg_ctx* ctx, int R, const double* d_c, double* d_
 // The dressed operators of the term set, and the closed-sigma plan of the state, built on
 // first use (fcg_gpu.cu)
 int ensure_dressed(fcg_ctx* ctx);
-int ensure_wmax(fcg_ctx* ctx);  // the open sigma's column maxima of the dressed operators
+int ensure_open_dressed(fcg_ctx* ctx);  // the open sigma's own, with their column maxima
 int ensure_plan(fcg_ctx* ctx);
 ProblemInfo problem_info(fcg_ctx* ctx);
 int term_norms(fcg_ctx* ctx);

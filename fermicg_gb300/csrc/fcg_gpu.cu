@@ -45,8 +45,8 @@ using namespace fcg;
 namespace {
 
 // ---- dressing ----------------------------------------------------------------------------
-__global__ void dress_kernel(const DressJob* __restrict__ jobs, const double* __restrict__ op,
-                             const double* __restrict__ ints, double* __restrict__ w) {
+__global__ void dress_kernel(const DressJob* __restrict__ jobs, const DressSrc* __restrict__ src,
+                             const double* __restrict__ op, const double* __restrict__ ints, double* __restrict__ w) {
   const DressJob J = jobs[blockIdx.x];
   const int64_t n = int64_t(J.rest_len) * J.mb * J.mk;
   for (int64_t e = threadIdx.x; e < n; e += blockDim.x) {
@@ -54,19 +54,21 @@ __global__ void dress_kernel(const DressJob* __restrict__ jobs, const double* __
     const int64_t bk = e / J.rest_len;
     const int b = int(bk % J.mb);
     const int k = int(bk / J.mb);
-    double acc;
-    if (J.one_body) {
-      acc = op[J.g_off + b + int64_t(J.mb) * k];
-    } else {
-      int64_t base = J.ints_off;
+    double acc = 0.0;
+    for (int m = 0; m < J.n_src; ++m) {
+      const DressSrc& S = src[J.src0 + m];
+      const double* g = op + S.g_off + int64_t(S.nq) * (b + int64_t(J.mb) * k);
+      if (J.one_body) {
+        acc = g[0];
+        break;
+      }
+      int64_t base = S.ints_off;
       int rr = r;
       for (int o = 0; o < J.nrem; ++o) {
-        base += int64_t(rr % J.rem_dim[o]) * J.rem_stride[o];
+        base += int64_t(rr % J.rem_dim[o]) * S.rem_stride[o];
         rr /= J.rem_dim[o];
       }
-      const double* g = op + J.g_off + int64_t(J.nq) * (b + int64_t(J.mb) * k);
-      acc = 0.0;
-      for (int i = 0; i < J.nq; ++i) acc = fma(ints[base + int64_t(i) * J.stride_q], g[i], acc);
+      for (int i = 0; i < S.nq; ++i) acc = fma(ints[base + int64_t(i) * S.stride_q], g[i], acc);
     }
     w[J.w_off + e] = acc;
   }
@@ -1105,50 +1107,62 @@ int fcg_set_ops(fcg_ctx* ctx, int n_clusters, const int32_t* cluster_norb, int64
 
 }  // extern "C"
 
-// The dressed operators W of every term (and their column maxima for the open-sigma
-// screen) on the device, from the job list of fcg_set_terms; once per term set.
-int ensure_dressed(fcg_ctx* ctx) {
-  if (ctx->dressed) return FCG_OK;
-  const std::vector<DressJob>& jobs = ctx->dress_jobs;
-  const int64_t w_total = ctx->n_w;
+// The W blocks of a dressing on the device, in double and float.
+static int dress_on_device(fcg_ctx* ctx, const Dressing& dz, DevBuf<double>& w64, DevBuf<float>& w32) {
   DressJob* d_jobs = nullptr;
-  FCG_CUDA(fcg_ctx::stage(ctx->scratch_a, jobs.data(), jobs.size(), ctx->stream, &d_jobs));
-  FCG_CUDA(ctx->d_w64.alloc(std::max<int64_t>(w_total, 1)));
-  FCG_CUDA(ctx->d_w32.alloc(std::max<int64_t>(w_total, 1)));
-  if (!jobs.empty()) {
-    dress_kernel<<<unsigned(jobs.size()), 256, 0, ctx->stream>>>(d_jobs, ctx->d_op64.p, ctx->d_ints64.p,
-                                                                 ctx->d_w64.p);
+  DressSrc* d_src = nullptr;
+  FCG_CUDA(fcg_ctx::stage(ctx->scratch_a, dz.jobs.data(), dz.jobs.size(), ctx->stream, &d_jobs));
+  FCG_CUDA(fcg_ctx::stage(ctx->scratch_b, dz.src.data(), dz.src.size(), ctx->stream, &d_src));
+  FCG_CUDA(w64.alloc(std::max<int64_t>(dz.n_w, 1)));
+  FCG_CUDA(w32.alloc(std::max<int64_t>(dz.n_w, 1)));
+  if (!dz.jobs.empty()) {
+    dress_kernel<<<unsigned(dz.jobs.size()), 256, 0, ctx->stream>>>(d_jobs, d_src, ctx->d_op64.p, ctx->d_ints64.p,
+                                                                    w64.p);
     FCG_CUDA(cudaGetLastError());
-    to_float_kernel<<<1024, 256, 0, ctx->stream>>>(ctx->d_w64.p, ctx->d_w32.p, w_total);
+    to_float_kernel<<<1024, 256, 0, ctx->stream>>>(w64.p, w32.p, dz.n_w);
     FCG_CUDA(cudaGetLastError());
   }
-  FCG_CUDA(cudaStreamSynchronize(ctx->stream));  // the job list's staging buffer is reused by the next call
-  ctx->wmax_built = false;
+  FCG_CUDA(cudaStreamSynchronize(ctx->stream));  // the lists' staging buffers are reused by the next call
+  return FCG_OK;
+}
+
+// The closed sigma's dressed operators, once per term set.
+int ensure_dressed(fcg_ctx* ctx) {
+  if (ctx->dressed) return FCG_OK;
+  const int rc = dress_on_device(ctx, ctx->dressing, ctx->d_w64, ctx->d_w32);
+  if (rc) return rc;
   ctx->dressed = true;
   return FCG_OK;
 }
 
-// Column maxima of the dressed operators for the open sigma's screen: Wmax[rest, k] per W
-// block, indexed like w_index; built on the first open sigma after the dressing.
-int ensure_wmax(fcg_ctx* ctx) {
+// The open sigma's dressed operators (one W for every term) and their column maxima for its
+// screen: Wmax[rest, k] per W block, indexed like w_index; built on the first open sigma of a
+// term set.
+int ensure_open_dressed(fcg_ctx* ctx) {
+  if (ctx->open_dressed) return FCG_OK;
+  Dressing& dz = ctx->open_dressing;
   {
-    const int rc = ensure_dressed(ctx);
+    const std::string msg = build_dress(ctx->norb, ctx->nmax, ctx->trm, ctx->n_terms, ctx->h_blk_index, ctx->h_blocks,
+                                        ctx->terms, ctx->dress, false, dz);
+    FCG_REQUIRE(msg.empty(), FCG_EINVAL, msg);
+  }
+  {
+    const int rc = dress_on_device(ctx, dz, ctx->d_ow64, ctx->d_ow32);
     if (rc) return rc;
   }
-  if (ctx->wmax_built) return FCG_OK;
-  const std::vector<DressJob>& jobs = ctx->dress_jobs;
+  const std::vector<DressJob>& jobs = dz.jobs;
   std::vector<MaxJob> mj(jobs.size());
-  ctx->wmax_index.assign(ctx->w_index.size(), -1);
+  ctx->wmax_index.assign(dz.w_index.size(), -1);
   int64_t tot = 0;
   for (size_t j = 0; j < jobs.size(); ++j) {
     const DressJob& J = jobs[j];
     mj[j] = MaxJob{J.w_off, tot, J.rest_len, J.mb, J.mk, 0};
     tot += int64_t(J.rest_len) * J.mk;
   }
-  for (size_t i = 0; i < ctx->w_index.size(); ++i) {
-    if (ctx->w_index[i] < 0) continue;
+  for (size_t i = 0; i < dz.w_index.size(); ++i) {
+    if (dz.w_index[i] < 0) continue;
     // jobs are in w_off order; find the job of this W block
-    auto it = std::lower_bound(jobs.begin(), jobs.end(), ctx->w_index[i],
+    auto it = std::lower_bound(jobs.begin(), jobs.end(), dz.w_index[i],
                                [](const DressJob& J, int64_t v) { return J.w_off < v; });
     ctx->wmax_index[i] = mj[it - jobs.begin()].out_off;
   }
@@ -1156,11 +1170,11 @@ int ensure_wmax(fcg_ctx* ctx) {
   FCG_CUDA(fcg_ctx::stage(ctx->scratch_b, mj.data(), mj.size(), ctx->stream, &d_mj));
   FCG_CUDA(ctx->d_wmax.alloc(std::max<int64_t>(tot, 1)));
   if (!jobs.empty()) {
-    colmax_kernel<<<unsigned(jobs.size()), 128, 0, ctx->stream>>>(d_mj, ctx->d_w64.p, ctx->d_wmax.p);
+    colmax_kernel<<<unsigned(jobs.size()), 128, 0, ctx->stream>>>(d_mj, ctx->d_ow64.p, ctx->d_wmax.p);
     FCG_CUDA(cudaGetLastError());
   }
   FCG_CUDA(cudaStreamSynchronize(ctx->stream));  // the job list's staging buffer is reused by the next call
-  ctx->wmax_built = true;
+  ctx->open_dressed = true;
   return FCG_OK;
 }
 
@@ -1207,14 +1221,13 @@ int fcg_set_terms(fcg_ctx* ctx, int n_terms, const int32_t* term_table, int64_t 
   }
   ctx->n_ints = n_ints;
   ctx->term_ints_norm.clear();  // computed when first needed (term_norms)
-  std::vector<DressJob> jobs;
-  int64_t w_total = 0;
   {
-    std::string msg = build_dress(ctx->N, ctx->norb, ctx->nmax, ctx->trm, n_terms, ctx->h_blk_index, ctx->h_blocks,
-                                  ctx->terms, ctx->dress, ctx->w_index, jobs, w_total);
+    std::string msg = term_dress(ctx->trm, n_terms, ctx->dress);
+    FCG_REQUIRE(msg.empty(), FCG_EINVAL, msg);
+    msg = build_dress(ctx->norb, ctx->nmax, ctx->trm, n_terms, ctx->h_blk_index, ctx->h_blocks, ctx->terms, ctx->dress,
+                      true, ctx->dressing);
     FCG_REQUIRE(msg.empty(), FCG_EINVAL, msg);
   }
-  ctx->n_w = w_total;
   FCG_CUDA(ctx->d_terms.upload(ctx->terms.data(), ctx->terms.size(), ctx->stream));
   FCG_CUDA(ctx->d_ints64.upload(ints, n_ints, ctx->stream));
   FCG_CUDA(ctx->d_ints32.alloc(size_t(std::max<int64_t>(n_ints, 1))));
@@ -1223,10 +1236,10 @@ int fcg_set_terms(fcg_ctx* ctx, int n_terms, const int32_t* term_table, int64_t 
         ctx->d_ints64.p, ctx->d_ints32.p, n_ints);
     FCG_CUDA(cudaGetLastError());
   }
-  // the dressed operators themselves are built on the device by the first fcg_state_set
-  // (only the closed and open sigmas use them; a BST-only context never needs them)
-  ctx->dress_jobs.swap(jobs);
+  // the dressed operators themselves are built on the device by the first closed-sigma plan and
+  // the first open sigma (a BST-only context never needs them)
   ctx->dressed = false;
+  ctx->open_dressed = false;
   ctx->dj.ready = false;
   FCG_CUDA(cudaStreamSynchronize(ctx->stream));
   ctx->have_terms = true;
@@ -1272,7 +1285,7 @@ ProblemInfo problem_info(fcg_ctx* ctx) {
   pi.blk_index = &ctx->h_blk_index;
   pi.blocks = &ctx->h_blocks;
   pi.dress = &ctx->dress;
-  pi.w_index = &ctx->w_index;
+  pi.dressing = &ctx->dressing;
   return pi;
 }
 
@@ -1372,7 +1385,7 @@ int ensure_plan(fcg_ctx* ctx) {
   ctx->stats.n_triples = P.n_triples;
   ctx->stats.flops_reference = P.flops_ref;
   ctx->stats.flops_executed = P.flops_dressed;
-  ctx->stats.dressed_elements = ctx->n_w;
+  ctx->stats.dressed_elements = ctx->dressing.n_w;
   const double dt = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
   ctx->stats.join_seconds = dt;
   ctx->stats.join_on_device = ctx->plan_on_device ? 1 : 0;

@@ -97,7 +97,7 @@ struct WorkItem {
   int32_t nb;       // bra group size
   int32_t nk;       // ket group size
   int32_t ts_off;   // offset of the term list in the TermSector pool
-  int32_t nt;       // number of terms
+  int32_t nt;       // number of term-sector records (merged terms)
 };
 
 // A closed-sigma lane job: one bra row of a work item against up to lane_kets(..) of the item's
@@ -159,18 +159,40 @@ FCG_HD inline int64_t block_jobs_of(int64_t nb, int64_t nk) {
   return ((nb + kBlockBras - 1) / kBlockBras) * ((nk + kBlockKets - 1) / kBlockKets);
 }
 
-// One W block to compute (fcg_set_terms): term t dressed with TDM block g of its dressed cluster.
+// One W block to compute: the sum over `n_src` terms (DressSrc) of the term's integrals contracted
+// with its TDM block of the dressed cluster.
 struct DressJob {
   int64_t w_off;
-  int64_t g_off;
-  int64_t ints_off;
-  int32_t rest_len, mb, mk, nq;  // nq: dressed orbital multi-index length
-  int32_t stride_q;              // ints stride of the dressed index
+  int32_t rest_len, mb, mk;
   int32_t nrem;
   int32_t rem_dim[3];
-  int32_t rem_stride[3];
+  int32_t src0, n_src;
   int32_t one_body;  // 1: copy the H block
+};
+
+struct DressSrc {
+  int64_t g_off;
+  int64_t ints_off;
+  int32_t nq;        // dressed orbital multi-index length
+  int32_t stride_q;  // ints stride of the dressed index
+  int32_t rem_stride[3];
   int32_t pad;
+};
+
+// The dressed operators of a term set.  In the merged form (the closed sigma's), terms of one
+// transfer that differ only in the dressed cluster's operator share one W, their sum: Aa A a and
+// Bb A a of three clusters, or A a, AAa a and ABb a of two.  A matrix element is linear in W, so
+// each such set costs one contraction per (bra, ket): of the 24-orbital problem's 2.1e8 triples at
+// 1e5 configurations 1.3e8 are left, and a sigma goes from 2.33 to 1.74 ms (float) and 6.58 to
+// 4.96 ms (double).  The open sigma thresholds every term's
+// contribution by itself and takes the unmerged form.
+struct Dressing {
+  std::vector<int32_t> rep;      // per term: the term that stands for its set (itself: a W of its own)
+  std::vector<int64_t> w_index;  // [term][fb_a][fb_b] of the dressed cluster -> W offset or -1
+  std::vector<int32_t> w_mb;     // [term][fb_a][fb_b] -> bra states of that W block
+  std::vector<DressJob> jobs;    // in w_off order
+  std::vector<DressSrc> src;
+  int64_t n_w = 0;
 };
 
 // ---- block-sparse Tucker (BST) vectors ---------------------------------------------------
@@ -247,7 +269,7 @@ struct ProblemInfo {
   const std::vector<int32_t>* blk_index = nullptr;  // dense (c, op, fba, fbb, fka, fkb) -> block
   const std::vector<BlockInfo>* blocks = nullptr;
   const std::vector<TermDress>* dress = nullptr;
-  const std::vector<int64_t>* w_index = nullptr;    // [term][fb_a][fb_b] of the dressed cluster -> W offset
+  const Dressing* dressing = nullptr;
 };
 
 // Host-side plan of the closed sigma for one state.
@@ -259,8 +281,7 @@ struct Plan {
   std::vector<int32_t> perm_pool;
   std::vector<TermSector> ts_pool;
   std::vector<WorkItem> items;
-  std::vector<int64_t> prefix;  // n_items + 1
-  int64_t n_triples = 0;
+  int64_t n_triples = 0;        // (bra, ket, term) triples, every term of a set counted
   int64_t flops_ref = 0;        // sum over triples of 2*len(ints) (the reference's count)
   int64_t flops_dressed = 0;    // multiply-adds actually done per sigma (x2), excluding the R update
   std::vector<int32_t> zero_terms;
@@ -295,20 +316,33 @@ FCG_HD inline int64_t dense_block_index(int nmax1, int c, int op, int fba, int f
 }
 
 // The term tables a term-sector record is made from, as plain arrays (host vectors or their
-// device copies): term rows (kTrmCols each), dressing, W offsets [term][fb_a][fb_b] of the
-// dressed cluster, the dense TDM block index and the blocks.
+// device copies): term rows (kTrmCols each), how each is dressed, the Dressing's tables, the dense
+// TDM block index and the blocks.
 struct TermTables {
   const int32_t* trm;
   const TermDress* dress;
   const int64_t* w_index;
+  const int32_t* w_mb;
+  const int32_t* rep;
   const int32_t* blk;
   const BlockInfo* blocks;
   int nmax1;
 };
 
-// The term-sector record of term t between bra sector fb and ket sector fk (N x 2 each) and
-// its multiply-add count per (bra, ket) pair (fma); false when a TDM block the term needs does
-// not exist there.  The host and the device planner both make their records here.
+// whether every TDM block of term t exists between bra sector fb and ket sector fk
+FCG_HD inline bool term_exists(const TermTables& tt, int t, const int16_t* fb, const int16_t* fk) {
+  const int32_t* r = tt.trm + int64_t(t) * kTrmCols;
+  for (int o = 0; o < r[0]; ++o) {
+    const int c = r[2 + o];
+    if (tt.blk[dense_block_index(tt.nmax1, c, r[6 + o], fb[2 * c], fb[2 * c + 1], fk[2 * c], fk[2 * c + 1])] < 0)
+      return false;
+  }
+  return true;
+}
+
+// The term-sector record of term t (one that stands for its set) between bra sector fb and ket
+// sector fk (N x 2 each) and its multiply-add count per (bra, ket) pair (fma); false when no term of
+// the set has the TDM blocks it needs there.  The host and the device planner both make their records here.
 FCG_HD inline bool term_sector_of(const TermTables& tt, int t, const int16_t* fb, const int16_t* fk,
                                   TermSector& ts, int64_t* fma) {
   const int32_t* r = tt.trm + int64_t(t) * kTrmCols;
@@ -317,12 +351,11 @@ FCG_HD inline bool term_sector_of(const TermTables& tt, int t, const int16_t* fb
   const int nbody = r[0];
   ts = TermSector{};
   const int pos = d.pos < 0 ? 0 : d.pos;
-  const int cw = r[2 + pos], opw = r[6 + pos];
-  const int bw = tt.blk[dense_block_index(nmax1, cw, opw, fb[2 * cw], fb[2 * cw + 1], fk[2 * cw], fk[2 * cw + 1])];
-  const int64_t woff = tt.w_index[(int64_t(t) * nmax1 + fb[2 * cw]) * nmax1 + fb[2 * cw + 1]];
-  if (bw < 0 || woff < 0) return false;
-  ts.w_off = woff;
-  ts.w_mb = tt.blocks[bw].mb;
+  const int cw = r[2 + pos];
+  const int64_t wi = (int64_t(t) * nmax1 + fb[2 * cw]) * nmax1 + fb[2 * cw + 1];
+  if (tt.w_index[wi] < 0) return false;
+  ts.w_off = tt.w_index[wi];
+  ts.w_mb = tt.w_mb[wi];
   ts.cw = int8_t(cw);
   ts.rest_len = int16_t(nbody == 1 ? 1 : d.rest_len);
   ts.nrem = int8_t(nbody == 1 ? 0 : d.nrem);
@@ -391,11 +424,13 @@ struct TermLists {
 };
 std::string term_lists(const ProblemInfo& pi, TermLists& lists);
 
-// Dressing plan of every term (which cluster is dressed, the W block of each of its
-// TDM blocks); fills dress, w_index ([term][fb_a][fb_b] -> W offset or -1), jobs, w_total.
-std::string build_dress(int N, const std::vector<int>& norb, int nmax, const std::vector<int32_t>& trm, int n_terms,
+// How every term is dressed (which cluster's TDM takes its integrals).
+std::string term_dress(const std::vector<int32_t>& trm, int n_terms, std::vector<TermDress>& dress);
+
+// The W blocks of every term, or (merge) of every set of terms that share theirs.
+std::string build_dress(const std::vector<int>& norb, int nmax, const std::vector<int32_t>& trm, int n_terms,
                         const std::vector<int32_t>& blk_index, const std::vector<BlockInfo>& blocks,
-                        const std::vector<TermInfo>& terms, std::vector<TermDress>& dress,
-                        std::vector<int64_t>& w_index, std::vector<DressJob>& jobs, int64_t& w_total);
+                        const std::vector<TermInfo>& terms, const std::vector<TermDress>& dress, bool merge,
+                        Dressing& out);
 
 }  // namespace fcg

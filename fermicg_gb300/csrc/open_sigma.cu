@@ -611,7 +611,7 @@ int fcg_sigma_open(fcg_ctx* ctx, int R, const double* c, double thresh, int nbod
   FCG_REQUIRE(thresh >= 0.0, FCG_EINVAL, "thresh must be >= 0");
   FCG_CUDA(cudaSetDevice(ctx->device));
   {
-    const int rc = ensure_wmax(ctx);
+    const int rc = ensure_open_dressed(ctx);
     if (rc) return rc;
   }
   *n_out = 0;
@@ -630,7 +630,7 @@ int fcg_sigma_open(fcg_ctx* ctx, int R, const double* c, double thresh, int nbod
   pi.blk_index = &ctx->h_blk_index;
   pi.blocks = &ctx->h_blocks;
   pi.dress = &ctx->dress;
-  pi.w_index = &ctx->w_index;
+  pi.dressing = &ctx->open_dressing;
   std::vector<std::vector<int>> terms_of(ctx->n_trans);
   for (int t = 0; t < ctx->n_terms; ++t) terms_of[ctx->trm[int64_t(t) * kTrmCols + 1]].push_back(t);
   std::unordered_map<uint64_t, int32_t> bsec_of;
@@ -811,7 +811,7 @@ int fcg_sigma_open(fcg_ctx* ctx, int R, const double* c, double thresh, int nbod
       FCG_CUDA(cudaMemsetAsync(ctx->d_counters.p + 2, 0, 3 * sizeof(unsigned long long), s));
       FCG_CUDA(cudaEventRecord(ctx->ev2, s));
       kernel<<<unsigned(grid), threads, smem, s>>>(
-          p, ctx->d_ojobs.p, n_kept, ctx->d_w64.p, ctx->d_op64.p, ctx->d_w32.p, ctx->d_op32.p, ctx->d_gmax.p,
+          p, ctx->d_ojobs.p, n_kept, ctx->d_ow64.p, ctx->d_op64.p, ctx->d_ow32.p, ctx->d_op32.p, ctx->d_gmax.p,
           ExpandTable{ctx->d_hkeys.p, ctx->d_hvals.p, cap - 1, ctx->d_counters.p}, slice);
       FCG_CUDA(cudaGetLastError());
       FCG_CUDA(cudaEventRecord(ctx->ev3, s));

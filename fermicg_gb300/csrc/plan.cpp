@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <array>
 #include <cstring>
+#include <map>
 #include <unordered_map>
 
 #include "fcg_internal.h"
@@ -61,8 +62,9 @@ struct ItemMeta {
 }  // namespace
 
 TermTables term_tables(const ProblemInfo& pi) {
-  return TermTables{pi.trm->data(), pi.dress->data(), pi.w_index->data(), pi.blk_index->data(), pi.blocks->data(),
-                    pi.nmax + 1};
+  const Dressing& d = *pi.dressing;
+  return TermTables{pi.trm->data(), pi.dress->data(), d.w_index.data(), d.w_mb.data(), d.rep.data(),
+                    pi.blk_index->data(), pi.blocks->data(), pi.nmax + 1};
 }
 
 bool make_term_sector(const ProblemInfo& pi, int t, const int16_t* fb, const int16_t* fk, TermSector& ts) {
@@ -183,6 +185,7 @@ std::string build_sectors(const ProblemInfo& pi, int64_t n_cfg, const int16_t* f
 }
 
 std::string build_join(const ProblemInfo& pi, const int16_t* fock, const int16_t* cfg, Plan& P) {
+  P.n_triples = P.flops_ref = P.flops_dressed = 0;
   (void)fock;
   const int N = pi.N;
   const std::vector<int32_t>& trm = *pi.trm;
@@ -251,13 +254,12 @@ std::string build_join(const ProblemInfo& pi, const int16_t* fock, const int16_t
   std::vector<std::vector<TermSector>> tTS(n_sec);
   std::vector<std::vector<ItemMeta>> tMeta(n_sec);
   std::vector<std::vector<PJob>> tJobs(n_sec);
-  std::vector<int64_t> tFlop(n_sec, 0), tFlopD(n_sec, 0);
+  std::vector<int64_t> tTri(n_sec, 0), tFlop(n_sec, 0), tFlopD(n_sec, 0);
   const TermTables tt = term_tables(pi);
 #pragma omp parallel
   {
     std::vector<int16_t> fk(2 * N);
     std::vector<TermSector> tsl;
-    std::vector<int64_t> tflop, tflopd;
 #pragma omp for schedule(dynamic, 1)
     for (int64_t sb = 0; sb < n_sec; ++sb) {
       const int16_t* fb = &P.sec_fock[sb * 2 * N];
@@ -272,23 +274,20 @@ std::string build_join(const ProblemInfo& pi, const int16_t* fock, const int16_t
         for (int j = L.first_of_tr[tr]; j < L.first_of_tr[tr + 1]; ++j) {
           // term-sector records of this (bra sector, ket sector, term list)
           tsl.clear();
-          tflop.clear();
-          tflopd.clear();
+          int64_t flop = 0, flopd = 0, tri = 0;
           for (int q = L.off[j]; q < L.off[j + 1]; ++q) {
             const int t = L.terms[q];
+            if (term_exists(tt, t, fb, fk.data())) {  // a missing TDM block contributes nothing
+              flop += term_ref_flops(trm.data(), t);
+              ++tri;
+            }
             TermSector ts;
             int64_t fma;
-            if (!term_sector_of(tt, t, fb, fk.data(), ts, &fma)) continue;  // a missing TDM block contributes nothing
-            tflop.push_back(term_ref_flops(trm.data(), t));
-            tflopd.push_back(2 * fma);
+            if (tt.rep[t] != t || !term_sector_of(tt, t, fb, fk.data(), ts, &fma)) continue;
+            flopd += 2 * fma;
             tsl.push_back(ts);
           }
           if (tsl.empty()) continue;
-          int64_t flop = 0, flopd = 0;
-          for (size_t i = 0; i < tsl.size(); ++i) {
-            flop += tflop[i];
-            flopd += tflopd[i];
-          }
           const int32_t ts_off = int32_t(tTS[sb].size());  // relative; rebased at concatenation
           tTS[sb].insert(tTS[sb].end(), tsl.begin(), tsl.end());
           // one lane step (one ket): every term's multiply-adds, about 8 loads and index steps
@@ -315,6 +314,7 @@ std::string build_join(const ProblemInfo& pi, const int16_t* fock, const int16_t
               w.nt = int32_t(tsl.size());
               tItems[sb].push_back(w);
               tMeta[sb].push_back(ItemMeta{step_cost, nbody_tl, block_item(L.block[j] != 0, w.nb, w.nk)});
+              tTri[sb] += int64_t(w.nb) * w.nk * tri;
               tFlop[sb] += int64_t(w.nb) * w.nk * flop;
               tFlopD[sb] += int64_t(w.nb) * w.nk * flopd;
               ++a;
@@ -367,6 +367,7 @@ std::string build_join(const ProblemInfo& pi, const int16_t* fock, const int16_t
     item_off[sb + 1] = item_off[sb] + int64_t(tItems[sb].size());
     tsp_off[sb + 1] = tsp_off[sb] + int64_t(tTS[sb].size());
     job_off[sb + 1] = job_off[sb] + int64_t(tJobs[sb].size());
+    P.n_triples += tTri[sb];
     P.flops_ref += tFlop[sb];
     P.flops_dressed += tFlopD[sb];
   }
@@ -449,10 +450,6 @@ std::string build_join(const ProblemInfo& pi, const int16_t* fock, const int16_t
   P.task_values = 0;
   for (int32_t l : P.wt_len) P.task_values += 32 * int64_t(l);
   make_chunks(P, kTargetChunks, P.chunk_lo, P.chunk_val);
-  P.prefix.assign(P.items.size() + 1, 0);
-  for (size_t i = 0; i < P.items.size(); ++i)
-    P.prefix[i + 1] = P.prefix[i] + int64_t(P.items[i].nb) * P.items[i].nk * P.items[i].nt;
-  P.n_triples = P.prefix.back();
   return "";
 }
 
@@ -485,72 +482,140 @@ void make_chunks(const Plan& P, int64_t target, std::vector<int64_t>& lo, std::v
   for (; c <= n_chunks; ++c) val[size_t(c)] = vals;
 }
 
-std::string build_dress(int N, const std::vector<int>& norb, int nmax, const std::vector<int32_t>& trm, int n_terms,
-                        const std::vector<int32_t>& blk_index, const std::vector<BlockInfo>& blocks,
-                        const std::vector<TermInfo>& terms, std::vector<TermDress>& dress,
-                        std::vector<int64_t>& w_index, std::vector<DressJob>& jobs, int64_t& w_total) {
-  (void)N;
-  const int s = nmax + 1;
-  dress.assign(n_terms, TermDress{});
-  w_index.assign(size_t(n_terms) * s * s, -1);
-  jobs.clear();
-  w_total = 0;
+std::string term_dress(const std::vector<int32_t>& trm, int n_terms, std::vector<TermDress>& dress) {
+  dress.assign(size_t(n_terms), TermDress{});
   for (int t = 0; t < n_terms; ++t) {
     const int32_t* r = &trm[int64_t(t) * kTrmCols];
-    TermDress& d = dress[t];
+    TermDress& d = dress[size_t(t)];
     const int nb = r[0];
     if (nb == 1) {
       d.pos = -1;
       d.rest_len = 1;
       d.nrem = 0;
-    } else {
-      // contract the ints with the cluster of the longest orbital multi-index
-      d.pos = 0;
-      for (int o = 1; o < nb; ++o)
-        if (r[22 + o] > r[22 + d.pos]) d.pos = o;
-      d.nrem = nb - 1;
-      d.rest_len = 1;
-      for (int o = 0, q = 0; o < nb; ++o) {
-        if (o == d.pos) continue;
-        d.rem_pos[q] = o;
-        d.rem_dim[q] = r[22 + o];
-        d.rest_len *= r[22 + o];
-        ++q;
-      }
-      if (d.rest_len > 32767) return "dressed index too long";
+      continue;
     }
-    const int pos = d.pos < 0 ? 0 : d.pos;
-    const int cw = r[2 + pos], opw = r[6 + pos];
-    int stride[4];
-    stride[0] = 1;
-    for (int o = 1; o < 4; ++o) stride[o] = stride[o - 1] * r[22 + o - 1];
+    // contract the ints with the cluster of the longest orbital multi-index
+    d.pos = 0;
+    for (int o = 1; o < nb; ++o)
+      if (r[22 + o] > r[22 + d.pos]) d.pos = o;
+    d.nrem = nb - 1;
+    d.rest_len = 1;
+    for (int o = 0, q = 0; o < nb; ++o) {
+      if (o == d.pos) continue;
+      d.rem_pos[q] = o;
+      d.rem_dim[q] = r[22 + o];
+      d.rest_len *= r[22 + o];
+      ++q;
+    }
+    if (d.rest_len > 32767) return "dressed index too long";
+  }
+  return "";
+}
+
+std::string build_dress(const std::vector<int>& norb, int nmax, const std::vector<int32_t>& trm, int n_terms,
+                        const std::vector<int32_t>& blk_index, const std::vector<BlockInfo>& blocks,
+                        const std::vector<TermInfo>& terms, const std::vector<TermDress>& dress, bool merge,
+                        Dressing& out) {
+  const int s = nmax + 1;
+  out = Dressing();
+  out.rep.resize(size_t(n_terms));
+  out.w_index.assign(size_t(n_terms) * s * s, -1);
+  out.w_mb.assign(size_t(n_terms) * s * s, 0);
+  // the dressed cluster's TDM block of term t in bra sector (fba, fbb), or -1
+  auto block_at = [&](int t, int fba, int fbb) {
+    const int32_t* r = &trm[int64_t(t) * kTrmCols];
+    const int pos = dress[size_t(t)].pos < 0 ? 0 : dress[size_t(t)].pos;
+    const int cw = r[2 + pos], fka = fba - r[10 + pos], fkb = fbb - r[14 + pos];
+    if (fka < 0 || fkb < 0 || fka > norb[cw] || fkb > norb[cw]) return -1;
+    return int(blk_index[dense_block_index(s, cw, r[6 + pos], fba, fbb, fka, fkb)]);
+  };
+  std::vector<std::vector<int>> members;  // terms of each set, the one that stands for it first
+  {
+    std::map<std::vector<int32_t>, int> set_of;
+    for (int t = 0; t < n_terms; ++t) {
+      const int32_t* r = &trm[int64_t(t) * kTrmCols];
+      const TermDress& d = dress[size_t(t)];
+      int set = -1;
+      if (merge && d.pos >= 0) {
+        // everything but the dressed operator: transfer, clusters, changes of Fock sector, fermionic
+        // parities, and the other clusters' operators and index lengths
+        std::vector<int32_t> key{r[1], r[0], d.pos};
+        for (int o = 0; o < r[0]; ++o) {
+          key.insert(key.end(), {r[2 + o], r[10 + o], r[14 + o], r[18 + o]});
+          if (o != d.pos) key.insert(key.end(), {r[6 + o], r[22 + o]});
+        }
+        auto it = set_of.find(key);
+        if (it == set_of.end()) {
+          set_of.emplace(key, int(members.size()));
+        } else {
+          set = it->second;
+          // the operators' blocks must have the same local dimensions wherever several exist
+          const int cw = r[2 + d.pos];
+          for (int fba = 0; fba <= norb[cw] && set >= 0; ++fba)
+            for (int fbb = 0; fbb <= norb[cw] && set >= 0; ++fbb) {
+              const int b = block_at(t, fba, fbb);
+              if (b < 0) continue;
+              for (int m : members[size_t(set)]) {
+                const int b2 = block_at(m, fba, fbb);
+                if (b2 >= 0 && (blocks[size_t(b2)].mb != blocks[size_t(b)].mb || blocks[size_t(b2)].mk != blocks[size_t(b)].mk)) {
+                  set = -1;
+                  break;
+                }
+              }
+            }
+        }
+      }
+      if (set < 0) {
+        out.rep[size_t(t)] = t;
+        members.push_back({t});
+      } else {
+        out.rep[size_t(t)] = members[size_t(set)][0];
+        members[size_t(set)].push_back(t);
+      }
+    }
+  }
+  for (const std::vector<int>& set : members) {
+    const int t0 = set[0];
+    const int32_t* r0 = &trm[int64_t(t0) * kTrmCols];
+    const TermDress& d = dress[size_t(t0)];
+    const int nb = r0[0], cw = r0[2 + (d.pos < 0 ? 0 : d.pos)];
     for (int fba = 0; fba <= norb[cw]; ++fba)
       for (int fbb = 0; fbb <= norb[cw]; ++fbb) {
-        int fka = fba - r[10 + pos], fkb = fbb - r[14 + pos];
-        if (fka < 0 || fkb < 0 || fka > norb[cw] || fkb > norb[cw]) continue;
-        int bl = blk_index[dense_block_index(s, cw, opw, fba, fbb, fka, fkb)];
-        if (bl < 0) continue;
-        const BlockInfo& B = blocks[bl];
-        if (nb > 1 && B.nidx != r[22 + pos]) return "term dims do not match the TDM block";
-        w_total = (w_total + kAlign - 1) / kAlign * kAlign;  // vector-load alignment of W blocks
         DressJob J{};
-        J.w_off = w_total;
-        J.g_off = B.off;
-        J.ints_off = terms[t].ints_off;
-        J.rest_len = d.rest_len;
-        J.mb = B.mb;
-        J.mk = B.mk;
-        J.nq = nb == 1 ? 1 : B.nidx;
-        J.stride_q = stride[pos];
-        J.nrem = d.nrem;
-        for (int q = 0; q < d.nrem; ++q) {
-          J.rem_dim[q] = d.rem_dim[q];
-          J.rem_stride[q] = stride[d.rem_pos[q]];
+        J.src0 = int32_t(out.src.size());
+        for (int t : set) {
+          const int bl = block_at(t, fba, fbb);
+          if (bl < 0) continue;
+          const int32_t* r = &trm[int64_t(t) * kTrmCols];
+          const BlockInfo& B = blocks[size_t(bl)];
+          const int pos = d.pos < 0 ? 0 : d.pos;
+          if (nb > 1 && B.nidx != r[22 + pos]) return "term dims do not match the TDM block";
+          int stride[4];
+          stride[0] = 1;
+          for (int o = 1; o < 4; ++o) stride[o] = stride[o - 1] * r[22 + o - 1];
+          DressSrc S{};
+          S.g_off = B.off;
+          S.ints_off = terms[size_t(t)].ints_off;
+          S.nq = nb == 1 ? 1 : B.nidx;
+          S.stride_q = stride[pos];
+          for (int q = 0; q < d.nrem; ++q) S.rem_stride[q] = stride[d.rem_pos[q]];
+          out.src.push_back(S);
+          J.mb = B.mb;
+          J.mk = B.mk;
         }
+        J.n_src = int32_t(out.src.size()) - J.src0;
+        if (J.n_src == 0) continue;
+        out.n_w = (out.n_w + kAlign - 1) / kAlign * kAlign;  // vector-load alignment of W blocks
+        J.w_off = out.n_w;
+        J.rest_len = d.rest_len;
+        J.nrem = d.nrem;
+        for (int q = 0; q < d.nrem; ++q) J.rem_dim[q] = d.rem_dim[q];
         J.one_body = nb == 1;
-        jobs.push_back(J);
-        w_index[(int64_t(t) * s + fba) * s + fbb] = w_total;
-        w_total += int64_t(d.rest_len) * B.mb * B.mk;
+        out.jobs.push_back(J);
+        const size_t wi = (size_t(t0) * s + fba) * s + fbb;
+        out.w_index[wi] = out.n_w;
+        out.w_mb[wi] = J.mb;
+        out.n_w += int64_t(d.rest_len) * J.mb * J.mk;
       }
   }
   return "";

@@ -15,16 +15,18 @@ from random_operators import BODIES, random_operators, random_rows
 
 pytestmark = pytest.mark.gpu
 
-TWO = [("Aa", "A", "a"), ("Bb", "A", "a"), ("A", "a", "B", "b"), ("A", "a")]
+# merged terms (Aa A a with Bb A a; A a with AAa a), two terms of one shape (AAa Bb a, AAa Aa a)
+TWO = [("Aa", "A", "a"), ("Bb", "A", "a"), ("AAa", "Bb", "a"), ("AAa", "Aa", "a"), ("A", "a", "B", "b"), ("A", "a"),
+       ("AAa", "a")]
 MIXED = [("A", "a", "Bb"), ("AAa", "a", "Aa"), ("A", "a", "Aa"), ("B", "A", "a", "b")]
 
 
 @pytest.mark.parametrize("norb,dims,n,R,bodies", [
-    ((4, 4, 4, 4), (4, 6), 21000, 4, TWO),
+    ((4, 4, 4, 4), (4, 6), 12000, 4, TWO),
     ((4, 4, 4, 4), (9, 2), 12000, 1, MIXED),
     ((4, 4, 4), (17, 20), 8000, 2, BODIES[:5]),     # three clusters: a group is a sector, 600 rows
     ((3, 3, 3, 3), (5, 6), 18000, 3, BODIES),
-    ((2, 5, 4, 3), (5, 7), 24000, 5, TWO),
+    ((2, 5, 4, 3), (5, 7), 18000, 5, TWO),
     ((6, 5, 6, 5), (5, 3), 9000, 2, BODIES),
     ((4, 4, 4, 4), (1, 18), 14000, 7, MIXED),       # clusters of one state
     ((7, 7, 7, 7), (5, 4), 6500, 16, BODIES),       # four-cluster columns of 49: lane jobs
