@@ -34,20 +34,24 @@ namespace {
 constexpr int kBstThreads = 256;
 constexpr int kOpThreads = 64;            // threads per group of the operator-cache build
 constexpr int kGammaSmem = 6144;          // doubles of the per-p staging tile of the gamma kernel
-constexpr int kSigmaSmemBytes = 96 * 1024;  // shared-memory workspace of a CTA-per-group sigma launch
-// CTA-per-group launches by workspace size: a launch reserves its largest group's shared
-// memory for every CTA, so groups are bucketed by the bytes they need (more resident CTAs for
-// the small ones)
-constexpr int kSmemBuckets = 4;
-constexpr int kSmemBucket[kSmemBuckets] = {12 * 1024, 24 * 1024, 48 * 1024, kSigmaSmemBytes};
 // shared memory of one warp of bst_sigma_bra_kernel (description + workspace); larger groups
-// run one CTA per group.  Measured on the 32-orbital / 8-cluster vector with cores up to 12^4:
-// float builds are fastest with 4 KB (9 % faster than 8 KB once the CTA-per-group launches
+// run in CTA chunks.  Measured on the 32-orbital / 8-cluster vector with cores up to 12^4:
+// float builds are fastest with 4 KB (9 % faster than 8 KB once the larger groups
 // were bucketed by workspace size), double builds with 2 KB.
 constexpr int warp_smem_bytes(size_t elem) { return elem == 4 ? 4 * 1024 : 2 * 1024; }
 constexpr int kWarpSmemMax = 8 * 1024;
 constexpr int kAccBytes = 32 * 1024;        // shared-memory bra-core accumulator of bst_sigma_bra_kernel
-constexpr int64_t kChunkWork = int64_t(1) << 16;  // multiply-adds per bst_sigma_bra_kernel CTA, about
+// multiply-adds per bst_sigma_bra_kernel CTA, about: the work over this many CTAs, within these limits
+// and not below kChunkBraWork for each element of the bra cores (a CTA zeroes and sums its copies
+// of them).  A fixed 2^16 left warps with 40 groups in series: 32 orbitals, 7 sectors, ranks 2-8,
+// FP64 242 -> 135 us.
+constexpr int64_t kChunkWorkMin = int64_t(1) << 11, kChunkWorkMax = int64_t(1) << 16, kChunkTarget = 152 * 24;
+constexpr int64_t kChunkBraWork = 160;
+
+// groups that go to the tensor cores: at least kTcMinM bra-active rows, kTcMinK ket-active
+// columns and kTcMinN spectator columns over all roots
+constexpr int kTcMinM = 64, kTcMinK = 16, kTcMinN = 32;
+constexpr int64_t kSplitFma = int64_t(1) << 20;  // larger operator products run in column ranges of about this
 
 // ---- operator cache ----------------------------------------------------------------------
 
@@ -549,9 +553,11 @@ __device__ void bst_group_apply(const BstGroup& G, int R, const T* __restrict__ 
   const int mn = m * ns;
   const T* opg = op + G.op_off;
   const int32_t* bp = perm + G.bperm_off;
-  if (mn * R >= 16 * TEAM) {
-    bst_tile_gemm<T, TEAM, ATOMIC, 4, 4>(opg, k, m, ns, R, ws, stride, cur, bp, out, out_stride, tid);
-    return;
+  if constexpr (TEAM > 32) {  // (a warp's groups are small: the registers buy more warps instead)
+    if (mn * R >= 16 * TEAM) {
+      bst_tile_gemm<T, TEAM, ATOMIC, 4, 4>(opg, k, m, ns, R, ws, stride, cur, bp, out, out_stride, tid);
+      return;
+    }
   }
   if (mn * R >= 4 * TEAM) {
     bst_tile_gemm<T, TEAM, ATOMIC, 2, 2>(opg, k, m, ns, R, ws, stride, cur, bp, out, out_stride, tid);
@@ -611,7 +617,7 @@ __device__ void bst_group_apply(const BstGroup& G, int R, const T* __restrict__ 
 // shared-memory copies of the bra cores -- one private copy per warp when `priv` (plain
 // adds), else one shared copy (shared-memory atomics) -- and the CTA adds the sum to sigma.
 template <typename T>
-__global__ void __launch_bounds__(kBstThreads) bst_sigma_bra_kernel(const int32_t* __restrict__ chunk_bra,
+__global__ void __launch_bounds__(kBstThreads, 4) bst_sigma_bra_kernel(const int32_t* __restrict__ chunk_bra,
                                                                     const int64_t* __restrict__ chunk_ptr,
                                                                     const int32_t* __restrict__ glist,
                                                                     const BstGroup* __restrict__ groups,
@@ -655,21 +661,513 @@ __global__ void __launch_bounds__(kBstThreads) bst_sigma_bra_kernel(const int32_
   }
 }
 
-// Medium groups: one CTA per group, description and workspace in shared memory.
+// ---- chunks of one bra block and root, a CTA each ---------------------------------------------
+// Groups that do not fit a warp slice run by CTAs.  A chunk is a run of groups of one bra block
+// and one root: the CTA keeps the bra core of that root in shared memory, adds each group's
+// contribution to it without atomics and adds the sum to sigma once.  Roots apart, and column
+// ranges of large operators in entries of their own, cut the work into pieces of about the same
+// size (a CTA per group for all roots left the largest groups running 2 ms alone).
+//
+// A group: gather the ket core (actives first, the positions computed: the index tables are a
+// second read as long as the core), mode products with the spectator overlaps, product with the
+// operator.  Each mode goes to the side of the operator where it is cheaper (post), 30 % fewer
+// multiply-adds than all before it.
+//
+// Bound: instruction issue and the barriers between a group's steps (2 of 4 issue slots used).
+// 32 orbitals, 5 sectors, cores up to 12^4, 2 roots, FP32: whole sigma 16.1 -> 11.3 ms; ranks 4-10
+// of 2 sectors, FP64: 8.0 -> 5.8 ms; 9 sectors, up to three excited clusters, FP64: 12.4 -> 9.0 ms.
+struct BstEntry {
+  int32_t g;       // group
+  int32_t c0, nc;  // bra-active columns
+  int32_t pad;
+};
+
+struct BstChunk {
+  int64_t b_off;        // bra core
+  int32_t bcore, root;
+  int32_t first, last;  // entries [first, last)
+  int32_t ws;           // elements of each of the two buffers
+  int32_t acc;          // 1: the bra core in shared memory; 0: atomics to sigma
+};
+
+// shared memory of a chunk CTA: two group descriptions (this one and the next), small
+// coefficient tables, the bra core, two buffers, the tables of the bra positions
+constexpr int kChunkBuckets = 6;
+constexpr int kChunkBucket[kChunkBuckets] = {16 * 1024, 28 * 1024, 44 * 1024, 72 * 1024, 112 * 1024, 224 * 1024};
+constexpr int kChunkTeam[kChunkBuckets] = {128, 256, 256, 384, 384, 384};  // threads of a CTA
+constexpr int kChunkAccMax = 4;   // last bucket of chunks that keep the bra core
+constexpr int kPrefetchL1 = 8 * 1024;   // bytes of an operator prefetched to L1
+constexpr int kCoef = 1024;       // elements of the coefficient tables
+constexpr int kFibre = 16;        // longest input fibre of the register mode products (float)
+
 template <typename T>
-__global__ void __launch_bounds__(kBstThreads) bst_sigma_smem_kernel(const int32_t* __restrict__ list,
-                                                                     const BstGroup* __restrict__ groups, int R,
-                                                                     const T* __restrict__ op,
-                                                                     const T* __restrict__ S,
-                                                                     const int32_t* __restrict__ perm,
-                                                                     const T* __restrict__ cin, T* __restrict__ cout,
-                                                                     int64_t core_total) {
+struct ChunkHead {  // bytes before the bra core (the tables are for float)
+  static constexpr int kDesc = int(sizeof(BstGroup) + sizeof(BstLayout));
+  static constexpr int n = 2 * kDesc + (sizeof(T) == 4 ? kCoef * 4 : 0);
+};
+static_assert(ChunkHead<float>::n % 16 == 0 && ChunkHead<double>::n % 16 == 0, "16-byte aligned buffers");
+
+// x / d with d's reciprocal
+__device__ __forceinline__ int div_of(int x, int d, uint32_t mg) { return d == 1 ? x : int(__umulhi(uint32_t(x), mg)); }
+
+// Where a product element goes: a buffer, the shared bra core or sigma.  Element col + m * s of the
+// actives-first layout is bra core element ta[col] + tb[s].
+template <typename T>
+struct BstSink {
+  T* buf;              // element i to buf[i], when set
+  T* acc;              // else added to the shared bra core, when set
+  T* out;              // else atomically to sigma
+  const uint16_t* ta;  // of the bra-active columns
+  const uint16_t* tb;  // of the spectator indices
+  int m;
+  uint32_t m_mg;
+  __device__ __forceinline__ void add(int at, T v) const {
+    if (acc)
+      acc[at] += v;
+    else
+      atomicAdd(out + at, v);
+  }
+  __device__ __forceinline__ void put(int i, T v) const {
+    if (buf) {
+      buf[i] = v;
+    } else {
+      const int s = div_of(i, m, m_mg);
+      add(int(ta[i - s * m]) + int(tb[s]), v);
+    }
+  }
+  __device__ __forceinline__ void put(int col, int s, T v) const {
+    if (buf)
+      buf[col + m * s] = v;
+    else
+      add(int(ta[col]) + int(tb[s]), v);
+  }
+};
+
+// dst[a, q, o] = sum_l coef[q, l] src[a, l, o], fibres of rk <= 4 * RK4 inputs in registers; coef in
+// shared memory, rows padded with zeros to 4 * RK4.  OP: the operator product of small operators (inner = 1, q: columns).
+template <int TEAM, int RK4, bool OP>
+__device__ __forceinline__ void mode_fibres(const float* src, int inner, int rk, int rb, int outer, const float* coef,
+                                            const BstSink<float>& sink) {
+  const int n = inner * outer, ds = OP ? 0 : inner / sink.m;
+  for (int f = threadIdx.x; f < n; f += TEAM) {
+    const int o = OP ? f : f / inner, a = OP ? 0 : f - o * inner;
+    const float* s = src + a + inner * rk * o;
+    float v[4 * RK4];
+#pragma unroll
+    for (int l = 0; l < 4 * RK4; ++l) v[l] = l < rk ? s[inner * l] : 0.f;
+    // outputs: buffer element a + inner * (q + rb * o), or bra column and spectator index
+    const int at = a + inner * rb * o, sa = OP || sink.buf ? 0 : div_of(a, sink.m, sink.m_mg);
+    const int col = a - sa * sink.m, s0 = sa + ds * rb * o;
+    for (int q = 0; q < rb; ++q) {
+      float x = 0.f;
+#pragma unroll
+      for (int l4 = 0; l4 < RK4; ++l4) {
+        const float4 c = *reinterpret_cast<const float4*>(coef + 4 * (RK4 * q + l4));
+        x = fmaf(c.x, v[4 * l4], x);
+        x = fmaf(c.y, v[4 * l4 + 1], x);
+        x = fmaf(c.z, v[4 * l4 + 2], x);
+        x = fmaf(c.w, v[4 * l4 + 3], x);
+      }
+      if (sink.buf)
+        sink.buf[at + inner * q] = x;
+      else if (OP)
+        sink.put(q, o, x);
+      else
+        sink.put(col, s0 + ds * q, x);
+    }
+  }
+}
+
+// the same from coefficients coef[q + rb * l] in global memory, an output per thread
+template <typename T, int TEAM>
+__device__ __forceinline__ void mode_general(const T* src, int inner, int rk, int rb, int outer,
+                                             const T* __restrict__ coef, const BstSink<T>& sink) {
+  const int n = inner * rb * outer;
+  for (int e = threadIdx.x; e < n; e += TEAM) {
+    const int a = e % inner, q = (e / inner) % rb, o = e / (inner * rb);
+    const T* s = src + a + inner * rk * o;
+    T x = T(0);
+    for (int l = 0; l < rk; ++l) x = fma(__ldg(coef + q + rb * l), s[inner * l], x);
+    sink.put(e, x);
+  }
+}
+
+template <typename T, int TEAM, bool OP>
+__device__ __forceinline__ void mode_any(const T* src, int inner, int rk, int rb, int outer, const T* coef,
+                                         const T* __restrict__ S, const BstSink<T>& sink) {
+  if constexpr (sizeof(T) == 4) {
+    if (coef) {
+      switch ((rk + 3) >> 2) {
+        case 1: mode_fibres<TEAM, 1, OP>(src, inner, rk, rb, outer, coef, sink); return;
+        case 2: mode_fibres<TEAM, 2, OP>(src, inner, rk, rb, outer, coef, sink); return;
+        case 3: mode_fibres<TEAM, 3, OP>(src, inner, rk, rb, outer, coef, sink); return;
+        default: mode_fibres<TEAM, 4, OP>(src, inner, rk, rb, outer, coef, sink); return;
+      }
+    }
+  }
+  mode_general<T, TEAM>(src, inner, rk, rb, outer, S, sink);
+}
+
+// Operator product in register tiles of TM columns x TN spectator indices; with eight or more column
+// tiles a warp covers 8 x 4 tiles, so that a column load touches eight columns and not 32.
+template <typename T, int TEAM, int TM, int TN>
+__device__ __forceinline__ void chunk_tiles(const T* __restrict__ opg, int k, int c0, int nc, int m, int ns, const T* X,
+                                            const BstSink<T>& sink) {
+  const int tm = (nc + TM - 1) / TM, tn = (ns + TN - 1) / TN;
+  const bool vec = (k & 3) == 0, grid = tm >= 8 && tn >= 4;
+  const int wm = (tm + 7) >> 3, wn = (tn + 3) >> 2;
+  const int n_it = grid ? wm * wn * 32 : tm * tn;
+  for (int it = threadIdx.x; it < n_it; it += TEAM) {
+    int ti, tj;
+    if (grid) {
+      const int w = it >> 5, l = it & 31;
+      ti = (w % wm) * 8 + (l & 7);
+      tj = (w / wm) * 4 + (l >> 3);
+      if (ti >= tm || tj >= tn) continue;
+    } else {
+      ti = it % tm;
+      tj = it / tm;
+    }
+    const int c = ti * TM, s = tj * TN;
+    const T* a[TM];
+    const T* b[TN];
+#pragma unroll
+    for (int i = 0; i < TM; ++i) a[i] = opg + int64_t(k) * (c0 + min(c + i, nc - 1));
+#pragma unroll
+    for (int j = 0; j < TN; ++j) b[j] = X + k * min(s + j, ns - 1);
+    T acc[TM][TN];
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j) acc[i][j] = T(0);
+    if (vec) {
+      for (int kk = 0; kk < k; kk += 4) {
+        T av[TM][4], bv[TN][4];
+#pragma unroll
+        for (int i = 0; i < TM; ++i) load4(a[i] + kk, av[i]);
+#pragma unroll
+        for (int j = 0; j < TN; ++j) load4(b[j] + kk, bv[j]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+          for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < TN; ++j) acc[i][j] = fma(av[i][q], bv[j][q], acc[i][j]);
+      }
+    } else {
+      for (int kk = 0; kk < k; ++kk) {
+        T av[TM], bv[TN];
+#pragma unroll
+        for (int i = 0; i < TM; ++i) av[i] = a[i][kk];
+#pragma unroll
+        for (int j = 0; j < TN; ++j) bv[j] = b[j][kk];
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+          for (int j = 0; j < TN; ++j) acc[i][j] = fma(av[i], bv[j], acc[i][j]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j)
+        if (c + i < nc && s + j < ns) sink.put(c0 + c + i, s + j, acc[i][j]);
+  }
+}
+
+// Operator product of few outputs and long columns: a warp per 4 columns x NS spectator indices,
+// lanes along the column (coalesced operator reads).
+template <typename T, int TEAM, int NS>
+__device__ __forceinline__ void chunk_stream(const T* __restrict__ opg, int k, int c0, int nc, int m, int s0, const T* X,
+                                             const BstSink<T>& sink) {
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int c = 4 * wid; c < nc; c += 4 * (TEAM >> 5)) {
+    const T* a[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a[i] = opg + int64_t(k) * (c0 + min(c + i, nc - 1));
+    T acc[4][NS];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < NS; ++j) acc[i][j] = T(0);
+    if ((k & 3) == 0) {
+      for (int kk = 4 * lane; kk < k; kk += 128) {
+        T av[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) load4(a[i] + kk, av[i]);
+#pragma unroll
+        for (int j = 0; j < NS; ++j) {
+          T bv[4];
+          load4(X + k * (s0 + j) + kk, bv);
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) acc[i][j] = fma(av[i][q], bv[q], acc[i][j]);
+        }
+      }
+    } else {
+      for (int kk = lane; kk < k; kk += 32) {
+        T av[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) av[i] = a[i][kk];
+#pragma unroll
+        for (int j = 0; j < NS; ++j) {
+          const T b = X[k * (s0 + j) + kk];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) acc[i][j] = fma(av[i], b, acc[i][j]);
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < NS; ++j)
+#pragma unroll
+        for (int w = 16; w > 0; w >>= 1) acc[i][j] += __shfl_xor_sync(0xffffffffu, acc[i][j], w);
+    if (lane == 0) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < NS; ++j)
+          if (c + i < nc) sink.put(c0 + c + i, s0 + j, acc[i][j]);
+    }
+  }
+}
+
+// Columns from which the streaming product pays: its five shuffle steps cost additions, cheap for
+// float, a warp instruction of 16 cycles each for double.
+template <typename T>
+struct StreamK {
+  static constexpr int n = sizeof(T) == 4 ? 64 : 512;
+};
+
+template <typename T, int TEAM>
+__device__ __forceinline__ void chunk_product(const T* __restrict__ opg, int k, int c0, int nc, int m, int ns, const T* X,
+                                              const BstSink<T>& sink) {
+  if (k >= StreamK<T>::n && (ns < 4 || nc * ns < 16 * TEAM)) {
+    int s = 0;
+    for (; s + 4 <= ns; s += 4) chunk_stream<T, TEAM, 4>(opg, k, c0, nc, m, s, X, sink);
+    if (ns - s == 3) chunk_stream<T, TEAM, 3>(opg, k, c0, nc, m, s, X, sink);
+    if (ns - s == 2) chunk_stream<T, TEAM, 2>(opg, k, c0, nc, m, s, X, sink);
+    if (ns - s == 1) chunk_stream<T, TEAM, 1>(opg, k, c0, nc, m, s, X, sink);
+    return;
+  }
+  if (nc * ns >= 16 * TEAM) {
+    // tiles of four columns, or of three where that leaves fewer columns over
+    if ((nc + 2) / 3 * 3 < (nc + 3) / 4 * 4)
+      chunk_tiles<T, TEAM, 3, 4>(opg, k, c0, nc, m, ns, X, sink);
+    else
+      chunk_tiles<T, TEAM, 4, 4>(opg, k, c0, nc, m, ns, X, sink);
+  } else if (nc * ns >= 4 * TEAM) {
+    chunk_tiles<T, TEAM, 2, 2>(opg, k, c0, nc, m, ns, X, sink);
+  } else {
+    chunk_tiles<T, TEAM, 1, 1>(opg, k, c0, nc, m, ns, X, sink);
+  }
+}
+
+template <typename T, int TEAM>
+__global__ void __launch_bounds__(TEAM, (sizeof(T) == 4 ? 768 : 512) / TEAM)
+    bst_chunk_kernel(const BstChunk* __restrict__ chunks, const BstEntry* __restrict__ entries,
+                     const BstGroup* __restrict__ groups, const BstLayout* __restrict__ layouts,
+                     const T* __restrict__ op, const T* __restrict__ S, const T* __restrict__ cin,
+                     T* __restrict__ cout, int64_t core_total) {
   extern __shared__ __align__(16) unsigned char bst_smem[];
-  BstGroup* G = reinterpret_cast<BstGroup*>(bst_smem);
-  T* ws = reinterpret_cast<T*>(bst_smem + sizeof(BstGroup));
-  load_group<kBstThreads>(groups + list[blockIdx.x], G, threadIdx.x);
-  bst_group_apply<T, kBstThreads, true>(*G, R, op, S, perm, cin, core_total, ws, G->ws, cout + G->b_off,
-                                        core_total);
+  const BstChunk C = chunks[blockIdx.x];
+  const int tid = threadIdx.x;
+  constexpr int kDesc = ChunkHead<T>::kDesc;
+  T* coef = reinterpret_cast<T*>(bst_smem + 2 * kDesc);
+  T* acc = reinterpret_cast<T*>(bst_smem + ChunkHead<T>::n);
+  T* buf0 = acc + (C.acc ? (C.bcore + 3) / 4 * 4 : 0);
+  T* buf1 = buf0 + C.ws;
+  uint16_t* tab = reinterpret_cast<uint16_t*>(buf1 + C.ws);
+  T* out = cout + int64_t(C.root) * core_total + C.b_off;
+  const T* src_root = cin + int64_t(C.root) * core_total;
+  // 16-byte units of a description, one per thread
+  constexpr int kGroupUnits = int(sizeof(BstGroup) / 16), kUnits = kDesc / 16;
+  static_assert(kUnits <= TEAM, "a description is copied in one step");
+  int4* desc = reinterpret_cast<int4*>(bst_smem);
+  auto unit_of = [&](int g) {
+    return tid < kGroupUnits ? reinterpret_cast<const int4*>(groups + g)[tid]
+                             : reinterpret_cast<const int4*>(layouts + g)[tid - kGroupUnits];
+  };
+  if (C.acc)
+    for (int i = tid; i < C.bcore; i += TEAM) acc[i] = T(0);
+  if (tid < kUnits) desc[tid] = unit_of(entries[C.first].g);
+  __syncthreads();
+  int slot = 0;
+  for (int e = C.first; e < C.last; ++e, slot ^= 1) {
+    const BstGroup& G = *reinterpret_cast<const BstGroup*>(bst_smem + slot * kDesc);
+    const BstLayout& L = *reinterpret_cast<const BstLayout*>(bst_smem + slot * kDesc + sizeof(BstGroup));
+    const BstEntry E = entries[e];
+    // the next group's description and what to prefetch for it, on their way while this group runs
+    int4 next = make_int4(0, 0, 0, 0);
+    BstEntry N = E;
+    int64_t n_op = 0, n_src = 0;
+    int n_k = 0, n_core = 0;
+    if (e + 1 < C.last) {
+      N = entries[e + 1];
+      if (tid < kUnits) next = unit_of(N.g);
+      const BstGroup* nx = groups + N.g;
+      n_op = nx->op_off, n_src = nx->k_off, n_k = nx->k, n_core = nx->kcore;
+    }
+    const int k = G.k, m = G.m, nsp = G.nsp, post = G.post;
+    const T* opg = op + G.op_off;
+    // this group's operator to L1
+    prefetch_range<TEAM, true>(opg + int64_t(k) * E.c0, min(int64_t(E.nc) * k * int64_t(sizeof(T)), int64_t(kPrefetchL1)), tid);
+    // ket core, read in order and written actives first
+    {
+      const T* src = src_root + G.k_off;
+      const int n = G.kcore, ng = L.ng;
+      if (ng <= 4) {  // the description in registers
+        uint32_t mg[4];
+        int d[4], st[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          mg[c] = c < ng ? L.g_mg[c] : 0u;
+          d[c] = c < ng ? L.g_dim[c] : 0;
+          st[c] = c < ng ? L.g_st[c] : 0;
+        }
+#pragma unroll 4
+        for (int i = tid; i < n; i += TEAM) {
+          const T v = __ldg(src + i);
+          int rem = i, at = 0;
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const int x = int(__umulhi(uint32_t(rem), mg[c]));
+            at += (rem - x * d[c]) * st[c];
+            rem = x;
+          }
+          buf0[at] = v;
+        }
+      } else {
+        for (int i = tid; i < n; i += TEAM) {
+          const T v = __ldg(src + i);
+          int rem = i, at = 0;
+          for (int c = 0; c < ng; ++c) {
+            const int d = L.g_dim[c], x = int(__umulhi(uint32_t(rem), L.g_mg[c]));
+            at += (rem - x * d) * L.g_st[c];
+            rem = x;
+          }
+          buf0[at] = v;
+        }
+      }
+    }
+    // bra positions of the columns and of the spectator indices
+    uint16_t* ta = tab;
+    uint16_t* tb = tab + m;
+    {
+      const int na = G.na, ns = div_of(C.bcore, m, L.m_mg);
+      for (int i = tid; i < m + ns; i += TEAM) {
+        int at = 0, rem = i < m ? i : i - m;
+        if (i < m) {
+          for (int a = 0; a < na; ++a) {
+            const int d = G.a_br[a], x = div_of(rem, d, L.a_mg[a]);
+            at += (rem - x * d) * G.a_bs[a];
+            rem = x;
+          }
+        } else {
+          for (int j = 0; j < nsp; ++j) {
+            const int d = G.s_br[j], x = div_of(rem, d, L.s_mg[j]);
+            at += (rem - x * d) * G.s_bs[j];
+            rem = x;
+          }
+        }
+        tab[i] = uint16_t(at);
+      }
+    }
+    // small coefficient tables (float): row-padded overlaps and operator
+    int coef_op = -1;  // offset of the operator's table, -1: none
+    if constexpr (sizeof(T) == 4) {
+      int at = 0;
+      for (int j = 0; j < nsp; ++j) {
+        const int rb = G.s_br[j], rk = G.s_kr[j], rp = (rk + 3) & ~3;
+        if (G.s_off[j] < 0 || rk > kFibre || at + rb * rp > kCoef) continue;
+        const T* Sj = S + G.s_off[j];
+        for (int i = tid; i < rb * rp; i += TEAM) {
+          const int q = i / rp, l = i - q * rp;
+          coef[at + i] = l < rk ? __ldg(Sj + q + rb * l) : T(0);
+        }
+        at += rb * rp;
+      }
+      const int kp = (k + 3) & ~3;
+      if (k <= kFibre && E.nc == m && at + m * kp <= kCoef) {
+        coef_op = at;
+        for (int i = tid; i < m * kp; i += TEAM) {
+          const int q = i / kp, l = i - q * kp;
+          coef[at + i] = l < k ? __ldg(opg + l + k * q) : T(0);
+        }
+      }
+    }
+    if (e + 1 < C.last) {  // the next group's ket core and operator to L2
+      prefetch_range<TEAM, false>(src_root + n_src, int64_t(n_core) * int64_t(sizeof(T)), tid);
+      prefetch_range<TEAM, false>(op + n_op + int64_t(n_k) * N.c0, int64_t(N.nc) * n_k * int64_t(sizeof(T)), tid);
+    }
+    __syncthreads();
+    T *src = buf0, *dst = buf1;
+    BstSink<T> sink{nullptr, C.acc ? acc : nullptr, out, ta, tb, m, L.m_mg};
+    const BstSink<T> final_sink = sink;
+    int done = 0, left = 0;  // modes already in the bra bases; applied modes still to come
+    for (int j = 0; j < nsp; ++j)
+      if (G.s_off[j] < 0)
+        done |= 1 << j;
+      else
+        ++left;
+    for (int pass = 0; pass < 2; ++pass) {
+      int at = 0;
+      for (int j = 0; j < nsp; ++j) {
+        const int rb = G.s_br[j], rk = G.s_kr[j], rp = (rk + 3) & ~3;
+        if (G.s_off[j] < 0) continue;
+        const T* table = nullptr;
+        if (sizeof(T) == 4 && rk <= kFibre && at + rb * rp <= kCoef) {
+          table = coef + at;
+          at += rb * rp;
+        }
+        if (((post >> j) & 1) != pass) continue;
+        int inner = pass ? m : k, outer = 1;
+        for (int i = 0; i < nsp; ++i) {
+          const int d = (done >> i) & 1 ? G.s_br[i] : G.s_kr[i];
+          if (i < j)
+            inner *= d;
+          else if (i > j)
+            outer *= d;
+        }
+        --left;
+        if (pass && left == 0)
+          sink = final_sink;
+        else
+          sink.buf = dst;
+        mode_any<T, TEAM, false>(src, inner, rk, rb, outer, table, S + G.s_off[j], sink);
+        __syncthreads();
+        T* t = src;
+        src = dst;
+        dst = t;
+        done |= 1 << j;
+      }
+      if (pass == 0) {
+        int ns = 1;
+        for (int i = 0; i < nsp; ++i) ns *= (done >> i) & 1 ? G.s_br[i] : G.s_kr[i];
+        if (left == 0)
+          sink = final_sink;
+        else
+          sink.buf = dst;
+        if (coef_op >= 0)
+          mode_any<T, TEAM, true>(src, 1, k, m, ns, coef + coef_op, opg, sink);
+        else
+          chunk_product<T, TEAM>(opg, k, E.c0, E.nc, m, ns, src, sink);
+        __syncthreads();
+        T* t = src;
+        src = dst;
+        dst = t;
+      }
+    }
+    if (e + 1 < C.last && tid < kUnits) desc[(slot ^ 1) * kUnits + tid] = next;
+    __syncthreads();
+  }
+  if (C.acc)
+    for (int i = tid; i < C.bcore; i += TEAM) {
+      const T v = acc[i];
+      if (v != T(0)) atomicAdd(out + i, v);
+    }
 }
 
 // Large groups: resident CTAs, each with its own global-memory workspace slice, taking the
@@ -722,9 +1220,6 @@ constexpr int kTcK = 16;         // K elements staged per round: two 8-element M
 constexpr int kTcTmemCols = 256;
 constexpr int kTcSmem = 2 * (2 * kTcM * kTcK * 4 + 2 * kTcN * kTcK * 4) + 64;  // two stages
 constexpr long long kTcWaitCycles = 4000000000LL;  // about 2 s at 2 GHz: a stuck MMA becomes an error
-// groups that go to the tensor cores: at least kTcMinM bra-active rows, kTcMinK ket-active
-// columns and kTcMinN spectator columns over all roots
-constexpr int kTcMinM = 64, kTcMinK = 16, kTcMinN = 32;
 
 __global__ void __launch_bounds__(kBstThreads) bst_tc_prep_kernel(const int32_t* __restrict__ list,
                                                                   const int64_t* __restrict__ ws_off,
@@ -1050,6 +1545,7 @@ std::string finish_part(const std::vector<BstBlock>& blk, int N, BstPart& P) {
       }
     }
     int64_t size = K.core_len, ws = size, tf = 0;
+    int md[kMaxClusters], mk[kMaxClusters], mj[kMaxClusters], nm = 0;  // applied modes: bra / ket rank, mode index
     G.ntr = 0;
     for (int c = 0, j = 0; c < N; ++c) {
       if ((G.act_mask >> c) & 1) continue;
@@ -1067,10 +1563,47 @@ std::string finish_part(const std::vector<BstBlock>& blk, int N, BstPart& P) {
         it = P.overlap_at.emplace(key, P.s_total).first;
         P.s_total += align_up(int64_t(B.rank[c]) * K.rank[c]);
       }
+      md[nm] = B.rank[c];
+      mk[nm] = K.rank[c];
+      mj[nm++] = j;
       G.s_off[j++] = it->second;
       size = size / K.rank[c] * B.rank[c];
       tf += 2 * size * K.rank[c];
       ws = std::max(ws, size);
+    }
+    // the sides of the operator the modes go to: the cheapest of the 2^nm choices (all before it
+    // for groups that may run on the tensor cores, whose operand X is in the bra bases, and for
+    // operator products that are cut into column ranges)
+    G.post = 0;
+    if (nm > 0 && nm <= 4 && !(m >= kTcMinM && k >= kTcMinK) && m * k * n <= kSplitFma) {
+      int64_t best = m * k * n + tf / 2;
+      for (int set = 1; set < (1 << nm); ++set) {
+        int64_t sz = K.core_len, cost = 0, top = sz;
+        for (int pass = 0; pass < 2; ++pass) {
+          if (pass) {
+            cost += sz * m;
+            sz = sz / k * m;
+            top = std::max(top, sz);
+          }
+          for (int i = 0; i < nm; ++i)
+            if (((set >> i) & 1) == pass) {
+              cost += sz * md[i];
+              sz = sz / mk[i] * md[i];
+              top = std::max(top, sz);
+            }
+        }
+        if (cost < best) {
+          best = cost;
+          G.post = 0;
+          for (int i = 0; i < nm; ++i)
+            if ((set >> i) & 1) G.post |= 1 << mj[i];
+          G.ws = int32_t(align_up(top));  // provisional, joined with the other order's below
+        }
+      }
+      if (G.post) {
+        ws = std::max(ws, int64_t(G.ws));
+        tf = 2 * (best - m * k * n);
+      }
     }
     for (int j = G.nsp; j < kMaxClusters; ++j) G.s_off[j] = 0;
     if (ws > (int64_t(1) << 30)) return "BST: a core exceeds 2^30 elements";
@@ -1370,6 +1903,33 @@ std::string plan_bst(const fcg_ctx* ctx, int nbody, const std::vector<BstBlock>&
   return "";
 }
 
+// The chunk kernel's index arithmetic of every group.
+std::vector<BstLayout> chunk_layouts(const std::vector<BstGroup>& groups, const std::vector<BstBlock>& blk, int N) {
+  std::vector<BstLayout> out(groups.size());
+#pragma omp parallel for schedule(static)
+  for (int64_t g = 0; g < int64_t(groups.size()); ++g) {
+    const BstGroup& G = groups[size_t(g)];
+    const BstBlock& K = blk[size_t(G.ket)];
+    BstLayout& L = out[size_t(g)];
+    L = BstLayout{};
+    int act = 1, sp = G.k;  // strides of the next active cluster / spectator mode
+    for (int c = 0; c < N; ++c) {
+      const int d = K.rank[c];
+      int& st = (G.act_mask >> c) & 1 ? act : sp;
+      if (d > 1) {
+        L.g_mg[L.ng] = div_mg(uint32_t(d));
+        L.g_dim[L.ng] = d;
+        L.g_st[L.ng++] = st;
+      }
+      st *= d;
+    }
+    for (int a = 0; a < G.na; ++a) L.a_mg[a] = div_mg(uint32_t(G.a_br[a]));
+    for (int j = 0; j < G.nsp; ++j) L.s_mg[j] = div_mg(uint32_t(G.s_br[j]));
+    L.m_mg = div_mg(uint32_t(G.m));
+  }
+  return out;
+}
+
 // Every index the sigma kernels form from a group description, checked against the buffers
 // it addresses (ket / bra cores, operator cache, overlaps, workspace).
 std::string check_groups(const std::vector<BstGroup>& groups, const std::vector<BstBlock>& blk, int64_t core_total,
@@ -1410,6 +1970,21 @@ std::string check_groups(const std::vector<BstGroup>& groups, const std::vector<
     if (ka != G.k || ba != G.m) return "BST check: active products";
     if (kprod != G.kcore || bprod != G.bcore) return "BST check: mode products";
     if (kmax >= G.kcore || bmax >= G.bcore) return "BST check: core strides";
+    {
+      // the order of the chunk kernel: modes before the operator, the operator, modes after it
+      int64_t sz = G.kcore;
+      for (int pass = 0; pass < 2; ++pass) {
+        if (pass && G.post) {
+          sz = sz / G.k * G.m;
+          ws_need = std::max(ws_need, sz);
+        }
+        for (int j = 0; j < G.nsp; ++j)
+          if (G.s_off[j] >= 0 && ((G.post >> j) & 1) == pass) {
+            sz = sz / G.s_kr[j] * G.s_br[j];
+            ws_need = std::max(ws_need, sz);
+          }
+      }
+    }
     if (int64_t(G.ws) < ws_need || int64_t(G.k) * (G.bcore / std::max(G.m, 1)) > G.ws) return "BST check: workspace";
     if (G.op_off < 0 || G.op_off + int64_t(G.m) * G.k > op_total) return "BST check: operator extent";
     if (G.kperm_off < 0 || G.kperm_off + G.kcore > perm_total || G.bperm_off < 0 || G.bperm_off + G.bcore > perm_total)
@@ -1419,20 +1994,29 @@ std::string check_groups(const std::vector<BstGroup>& groups, const std::vector<
   return "";
 }
 
-// Groups by where they run.  Groups whose workspace fits a warp slice and whose bra block's
-// R cores fit kAccBytes go to bst_sigma_bra_kernel, cut per bra block into chunks of about
-// kChunkWork multiply-adds; the others run one CTA per group from shared memory, or from
-// global memory.
 // multiply-adds and element moves of one group's sigma step, about
 int64_t group_work(const BstGroup& G, int R) {
   return int64_t(R) * (int64_t(G.m) * G.k * (G.bcore / std::max(G.m, 1)) + 2 * G.kcore + 64);
 }
 
+// the same of an entry of a chunk (one root, nc columns); its chain of barriers costs about as much
+// as 2^13 of them
+int64_t entry_work(const BstGroup& G, int64_t nc) {
+  return nc * G.k * (G.bcore / std::max(G.m, 1)) + 5 * int64_t(G.kcore) + (int64_t(1) << 13);
+}
+
+// bytes of a group's bra position tables
+int64_t tab_bytes(const BstGroup& G) { return 2 * int64_t(G.m + G.bcore / std::max(G.m, 1)) + 16; }
+
+// Groups by where they run.  GEMM-shaped groups of a float build go to the tensor cores.  Groups
+// whose workspace fits a warp slice and whose bra block's R cores fit kAccBytes go to
+// bst_sigma_bra_kernel, cut per bra block into chunks; the others to bst_chunk_kernel, in chunks of
+// one bra block and root by the shared memory they need, or (larger than a CTA's) to
+// bst_sigma_global_kernel.
 void bst_lists(fcg_ctx* ctx, int R, size_t elem) {
   ctx->bst_bra_ids.clear();
   ctx->bst_bra_ptr.assign(1, 0);
   ctx->bst_bra_glist.clear();
-  ctx->bst_small.clear();
   ctx->bst_large.clear();
   ctx->bst_ws_large = 0;
   ctx->bst_bra_slice = 0;
@@ -1444,22 +2028,56 @@ void bst_lists(fcg_ctx* ctx, int R, size_t elem) {
   ctx->bst_tc_flops = 0;
   ctx->bst_tc_mma_flops = 0;
   const size_t ng = ctx->bst_groups.size();
-  std::vector<int32_t> bucket[kSmemBuckets];
-  std::vector<int64_t> chunk_work;  // per chunk of bst_sigma_bra_kernel
+  const int64_t head = elem == 4 ? ChunkHead<float>::n : ChunkHead<double>::n;
+  // where each group runs: a warp slice, a chunk bucket, global workspaces, the tensor cores
+  constexpr uint8_t kWarp = 100, kLarge = 101, kTc = 102;
+  std::vector<uint8_t> where(ng);
+  int64_t warp_work = 0, chunk_work = 0;
+  for (size_t q = 0; q < ng; ++q) {
+    const BstGroup& G = ctx->bst_groups[q];
+    const int64_t ns = G.bcore / std::max(G.m, 1);
+    if (elem == 4 && ctx->bst_tc_on && G.m >= kTcMinM && G.k >= kTcMinK && ns * R >= kTcMinN) {
+      where[q] = kTc;
+    } else if (size_t(R) * G.bcore * elem <= size_t(kAccBytes) &&
+               sizeof(BstGroup) + size_t(2) * R * G.ws * elem <= size_t(warp_smem_bytes(elem))) {
+      where[q] = kWarp;
+      warp_work += group_work(G, R);
+    } else {
+      const int64_t two = head + 2 * int64_t(G.ws) * int64_t(elem) + tab_bytes(G);
+      const int64_t all = two + (G.bcore + 3) / 4 * 4 * int64_t(elem);
+      where[q] = kLarge;
+      for (int i = 0; i < kChunkBuckets && G.bcore < 65536 && G.kcore < 65536; ++i)
+        if ((i <= kChunkAccMax ? all : two) <= kChunkBucket[i]) {
+          where[q] = uint8_t(i);
+          break;
+        }
+      if (where[q] < kChunkBuckets) chunk_work += R * entry_work(G, G.m);
+    }
+  }
+  const int64_t warp_cut = std::max(kChunkWorkMin, std::min(kChunkWorkMax, warp_work / kChunkTarget));
+  const int64_t chunk_cut = std::min<int64_t>(4 * kSplitFma, chunk_work / (4 * kChunkTarget));
+  struct Pending {  // chunks of one bucket: (work, entries) of one bra block, for every root
+    int64_t work;
+    BstChunk c;
+  };
+  std::vector<Pending> bucket[kChunkBuckets];
+  std::vector<BstEntry> entries;
+  std::vector<int32_t> of_bucket[kChunkBuckets];  // groups of the current bra block
+  std::vector<int64_t> warp_chunk_work;  // per chunk of bst_sigma_bra_kernel
   size_t g = 0;
   while (g < ng) {
     const int32_t b = ctx->bst_groups[g].bra;
     size_t g1 = g;
     while (g1 < ng && ctx->bst_groups[g1].bra == b) ++g1;  // groups of one bra are contiguous
-    const size_t acc = size_t(R) * ctx->bst_blocks[b].core_len * elem;
-    const bool own = acc <= size_t(kAccBytes);
     int64_t work = 0;
     bool open = false;
+    for (auto& v : of_bucket) v.clear();
     for (size_t q = g; q < g1; ++q) {
       const BstGroup& G = ctx->bst_groups[q];
-      const size_t need = sizeof(BstGroup) + size_t(2) * R * G.ws * elem;
       const int64_t ns = G.bcore / std::max(G.m, 1);
-      if (elem == 4 && ctx->bst_tc_on && G.m >= kTcMinM && G.k >= kTcMinK && ns * R >= kTcMinN) {
+      if (where[q] < kChunkBuckets) {
+        of_bucket[where[q]].push_back(int32_t(q));
+      } else if (where[q] == kTc) {
         // GEMM-shaped: tensor cores (its operand X in a global workspace of its own)
         const int32_t tc = int32_t(ctx->bst_tc.size());
         ctx->bst_tc.push_back(int32_t(q));
@@ -1472,32 +2090,69 @@ void bst_lists(fcg_ctx* ctx, int R, size_t elem) {
             ctx->bst_tc_mma_flops += 3 * 2 * int64_t(kTcM) * nI * ((G.k + 7) / 8 * 8);
           }
         ctx->bst_tc_flops += 2 * int64_t(G.m) * G.k * ns * R;
-        continue;
-      }
-      if (own && need <= size_t(warp_smem_bytes(elem))) {
-        if (!open || work > kChunkWork) {
+      } else if (where[q] == kWarp) {
+        // a chunk's own cost: its warps' copies of the bra core zeroed and summed
+        if (!open || work > std::max(warp_cut, std::min(kChunkWorkMax, kChunkBraWork * R * G.bcore))) {
           if (open) ctx->bst_bra_ptr.push_back(int64_t(ctx->bst_bra_glist.size()));
           ctx->bst_bra_ids.push_back(b);
-          chunk_work.push_back(0);
+          warp_chunk_work.push_back(0);
           open = true;
           work = 0;
         }
+        const size_t need = sizeof(BstGroup) + size_t(2) * R * G.ws * elem;
         ctx->bst_bra_glist.push_back(int32_t(q));
         ctx->bst_bra_slice = std::max(ctx->bst_bra_slice, int((need + 15) / 16 * 16));
         work += group_work(G, R);
-        chunk_work.back() += group_work(G, R);
-      } else if (need <= size_t(kSigmaSmemBytes)) {
-        int i = 0;
-        while (need > size_t(kSmemBucket[i])) ++i;
-        bucket[i].push_back(int32_t(q));
-      } else {
+        warp_chunk_work.back() += group_work(G, R);
+      } else if (where[q] == kLarge) {
         ctx->bst_large.push_back(int32_t(q));
         ctx->bst_ws_large = std::max(ctx->bst_ws_large, G.ws);
       }
     }
     if (open) {
       ctx->bst_bra_ptr.push_back(int64_t(ctx->bst_bra_glist.size()));
+      const size_t acc = size_t(R) * ctx->bst_blocks[b].core_len * elem;
       ctx->bst_bra_acc = std::max(ctx->bst_bra_acc, int((acc + 15) / 16 * 16));
+    }
+    for (int i = 0; i < kChunkBuckets; ++i) {
+      if (of_bucket[i].empty()) continue;
+      Pending P{};
+      int64_t tab = 0;  // largest position tables of the open chunk
+      auto flush = [&] {
+        P.c.last = int32_t(entries.size());
+        if (P.c.last > P.c.first)
+          for (int r = 0; r < R; ++r) {
+            P.c.root = r;
+            bucket[i].push_back(P);
+          }
+        P.work = 0;
+        P.c.first = int32_t(entries.size());
+        P.c.ws = 0;
+        tab = 0;
+      };
+      P.c.first = int32_t(entries.size());
+      P.c.b_off = ctx->bst_blocks[b].core_off;
+      P.c.bcore = ctx->bst_blocks[b].core_len;
+      P.c.acc = i <= kChunkAccMax ? 1 : 0;
+      for (int32_t q : of_bucket[i]) {
+        const BstGroup& G = ctx->bst_groups[q];
+        const int64_t fma = int64_t(G.m) * G.k * (G.bcore / std::max(G.m, 1));
+        // large operator products (no modes after them) in column ranges
+        const int pieces = G.post ? 1 : int(std::max<int64_t>(1, std::min<int64_t>(fma / kSplitFma, (G.m + 15) / 16)));
+        const int step = (((G.m + pieces - 1) / pieces) + 3) / 4 * 4;
+        for (int c0 = 0; c0 < G.m; c0 += step) {
+          const int nc = std::min(step, G.m - c0);
+          const int64_t bytes = head + (P.c.acc ? (P.c.bcore + 3) / 4 * 4 * int64_t(elem) : 0) +
+                                2 * int64_t(std::max(P.c.ws, G.ws)) * int64_t(elem) + std::max(tab, tab_bytes(G));
+          if (bytes > kChunkBucket[i]) flush();
+          tab = std::max(tab, tab_bytes(G));
+          entries.push_back(BstEntry{q, c0, nc, 0});
+          P.c.ws = std::max(P.c.ws, G.ws);
+          P.work += entry_work(G, nc);
+          if (P.work >= chunk_cut) flush();
+        }
+      }
+      flush();
     }
     g = g1;
   }
@@ -1506,7 +2161,8 @@ void bst_lists(fcg_ctx* ctx, int R, size_t elem) {
     const size_t nc = ctx->bst_bra_ids.size();
     std::vector<size_t> order(nc);
     for (size_t i = 0; i < nc; ++i) order[i] = i;
-    std::stable_sort(order.begin(), order.end(), [&](size_t x, size_t y) { return chunk_work[x] > chunk_work[y]; });
+    std::stable_sort(order.begin(), order.end(),
+                     [&](size_t x, size_t y) { return warp_chunk_work[x] > warp_chunk_work[y]; });
     std::vector<int32_t> ids(nc), gl;
     std::vector<int64_t> ptr(1, 0);
     gl.reserve(ctx->bst_bra_glist.size());
@@ -1525,15 +2181,18 @@ void bst_lists(fcg_ctx* ctx, int R, size_t elem) {
   std::stable_sort(ctx->bst_large.begin(), ctx->bst_large.end(), [&](int32_t x, int32_t y) {
     return group_work(ctx->bst_groups[x], R) > group_work(ctx->bst_groups[y], R);
   });
-  ctx->bst_small_ptr.assign(1, 0);
-  for (int i = 0; i < kSmemBuckets; ++i) {
-    // CTAs start in launch order: longest first keeps the tail short
-    std::stable_sort(bucket[i].begin(), bucket[i].end(), [&](int32_t x, int32_t y) {
-      return group_work(ctx->bst_groups[x], R) > group_work(ctx->bst_groups[y], R);
-    });
-    ctx->bst_small.insert(ctx->bst_small.end(), bucket[i].begin(), bucket[i].end());
-    ctx->bst_small_ptr.push_back(int64_t(ctx->bst_small.size()));
+  // chunks of every bucket longest first, in one array
+  std::vector<BstChunk> chunks;
+  ctx->bst_chunk_ptr.assign(1, 0);
+  for (int i = 0; i < kChunkBuckets; ++i) {
+    std::stable_sort(bucket[i].begin(), bucket[i].end(), [](const Pending& x, const Pending& y) { return x.work > y.work; });
+    for (const Pending& P : bucket[i]) chunks.push_back(P.c);
+    ctx->bst_chunk_ptr.push_back(int64_t(chunks.size()));
   }
+  const unsigned char* cb = reinterpret_cast<const unsigned char*>(chunks.data());
+  const unsigned char* eb = reinterpret_cast<const unsigned char*>(entries.data());
+  ctx->bst_chunks.assign(cb, cb + chunks.size() * sizeof(BstChunk));
+  ctx->bst_entries.assign(eb, eb + entries.size() * sizeof(BstEntry));
 }
 
 template <typename T>
@@ -1544,7 +2203,8 @@ int bst_launch(fcg_ctx* ctx, int R, const T* op, const T* S, const T* cin, T* co
     FCG_CUDA(ctx->d_bst_bra_ids.upload(ctx->bst_bra_ids.data(), ctx->bst_bra_ids.size(), ctx->stream));
     FCG_CUDA(ctx->d_bst_bra_ptr.upload(ctx->bst_bra_ptr.data(), ctx->bst_bra_ptr.size(), ctx->stream));
     FCG_CUDA(ctx->d_bst_bra_glist.upload(ctx->bst_bra_glist.data(), ctx->bst_bra_glist.size(), ctx->stream));
-    FCG_CUDA(ctx->d_bst_small.upload(ctx->bst_small.data(), ctx->bst_small.size(), ctx->stream));
+    FCG_CUDA(ctx->d_bst_chunks.upload(ctx->bst_chunks.data(), ctx->bst_chunks.size(), ctx->stream));
+    FCG_CUDA(ctx->d_bst_entries.upload(ctx->bst_entries.data(), ctx->bst_entries.size(), ctx->stream));
     FCG_CUDA(ctx->d_bst_large.upload(ctx->bst_large.data(), ctx->bst_large.size(), ctx->stream));
     FCG_CUDA(ctx->d_bst_tc.upload(ctx->bst_tc.data(), ctx->bst_tc.size(), ctx->stream));
     FCG_CUDA(ctx->d_bst_tc_ws_off.upload(ctx->bst_tc_ws_off.data(), ctx->bst_tc_ws_off.size(), ctx->stream));
@@ -1600,20 +2260,18 @@ int bst_launch(fcg_ctx* ctx, int R, const T* op, const T* S, const T* cin, T* co
     FCG_CUDA(cudaGetLastError());
     ++launches;
   }
-  if (!ctx->bst_small.empty()) {
-    FCG_CUDA(cudaFuncSetAttribute(bst_sigma_smem_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  int(kSigmaSmemBytes)));
-    for (int i = 0; i < kSmemBuckets; ++i) {
-      const int64_t a = ctx->bst_small_ptr[i], b = ctx->bst_small_ptr[i + 1];
-      if (a == b) continue;
-      int ws_max = 0;
-      for (int64_t q = a; q < b; ++q) ws_max = std::max(ws_max, ctx->bst_groups[ctx->bst_small[q]].ws);
-      const size_t smem = sizeof(BstGroup) + size_t(2) * R * ws_max * elem;
-      bst_sigma_smem_kernel<T><<<unsigned(b - a), kBstThreads, smem, ctx->stream>>>(
-          ctx->d_bst_small.p + a, ctx->d_bst_groups.p, R, op, S, ctx->d_bst_perm.p, cin, cout, ct);
-      FCG_CUDA(cudaGetLastError());
-      ++launches;
-    }
+  for (int i = kChunkBuckets - 1; i >= 0; --i) {  // the longest chunks first
+    const int64_t a = ctx->bst_chunk_ptr[i], b = ctx->bst_chunk_ptr[i + 1];
+    if (a == b) continue;
+    auto kernel = kChunkTeam[i] == 128   ? bst_chunk_kernel<T, 128>
+                  : kChunkTeam[i] == 256 ? bst_chunk_kernel<T, 256> : bst_chunk_kernel<T, 384>;
+    FCG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kChunkBucket[kChunkBuckets - 1]));
+    kernel<<<unsigned(b - a), unsigned(kChunkTeam[i]), size_t(kChunkBucket[i]), ctx->stream>>>(
+        reinterpret_cast<const BstChunk*>(ctx->d_bst_chunks.p) + a,
+        reinterpret_cast<const BstEntry*>(ctx->d_bst_entries.p), ctx->d_bst_groups.p, ctx->d_bst_layouts.p, op, S, cin,
+        cout, ct);
+    FCG_CUDA(cudaGetLastError());
+    ++launches;
   }
   if (!ctx->bst_large.empty()) {
     // as many CTAs as can be resident (each walks the list with the grid's stride)
@@ -1752,6 +2410,8 @@ int bst_set_impl(fcg_ctx* ctx, int nbody, int64_t n_blocks, const int16_t* fock,
   FCG_CUDA(ctx->d_bst_perm.alloc(size_t(std::max<int64_t>(P.perm_total, 1))));
   FCG_CUDA(ctx->d_bst_blocks.upload(blk.data(), blk.size(), ctx->stream));
   FCG_CUDA(ctx->d_bst_groups.upload(P.groups.data(), P.groups.size(), ctx->stream));
+  const std::vector<BstLayout> layouts = chunk_layouts(P.groups, blk, N);
+  FCG_CUDA(ctx->d_bst_layouts.upload(layouts.data(), layouts.size(), ctx->stream));
   FCG_REQUIRE(P.tables.size() < (size_t(1) << 31), FCG_ELIMIT, "BST: too many index tables");
   if (!P.tables.empty()) {
     DevBuf<BstPermTable> d_tab;

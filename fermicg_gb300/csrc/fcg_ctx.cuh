@@ -251,8 +251,9 @@ struct fcg_ctx {
   std::vector<BstBlock> bst_blocks;
   std::vector<BstGroup> bst_groups;
   std::vector<int32_t> bst_triples;     // [n][4] = {bra, ket, term, sign}
-  std::vector<int32_t> bst_small, bst_large;  // groups run one CTA per group from shared / global memory
-  std::vector<int64_t> bst_small_ptr;         // bst_small in buckets of workspace size: [ptr[i], ptr[i+1])
+  std::vector<unsigned char> bst_chunks, bst_entries;  // chunks of one bra block and root, their groups (bst.cu)
+  std::vector<int64_t> bst_chunk_ptr;         // chunks of each shared-memory bucket: [ptr[i], ptr[i+1])
+  std::vector<int32_t> bst_large;             // groups run from global workspaces
   int32_t bst_ws_large = 0;
   std::vector<int32_t> bst_bra_ids, bst_bra_glist;  // bra block of each chunk, and the chunks' groups
   std::vector<int64_t> bst_bra_ptr;                 // chunk c holds bst_bra_glist[ptr[c], ptr[c+1])
@@ -261,7 +262,9 @@ struct fcg_ctx {
   size_t bst_list_elem = 0;
   DevBuf<BstBlock> d_bst_blocks;
   DevBuf<BstGroup> d_bst_groups;
-  DevBuf<int32_t> d_bst_small, d_bst_large, d_bst_bra_ids, d_bst_bra_glist;
+  DevBuf<BstLayout> d_bst_layouts;  // per group
+  DevBuf<unsigned char> d_bst_chunks, d_bst_entries;
+  DevBuf<int32_t> d_bst_large, d_bst_bra_ids, d_bst_bra_glist;
   DevBuf<unsigned> d_bst_next;  // work counter of the global-workspace sigma launch
   DevBuf<int64_t> d_bst_bra_ptr;
   DevBuf<double> d_bst_factors;

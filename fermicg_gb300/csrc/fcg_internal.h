@@ -250,12 +250,28 @@ struct BstGroup {
   int32_t s_kr[kMaxClusters], s_br[kMaxClusters];
   int32_t s_ks[kMaxClusters], s_bs[kMaxClusters];
   int32_t ntr;                   // spectator modes with an overlap to apply (the others: U^T U = 1)
-  int32_t pad;
+  int32_t post;                  // bit j: the chunk kernel applies mode j after the operator
   // index tables (core offset of every position of the actives-first layout) of the ket and
   // the bra block for this group's active clusters
   int64_t kperm_off, bperm_off;
 };
 static_assert(sizeof(BstGroup) % 16 == 0, "BstGroup is copied to shared memory in 16-byte units");
+
+// n / d for n * d < 2^32 as the high word of n * div_mg(d) (d > 1)
+inline uint32_t div_mg(uint32_t d) { return d > 1 ? 0xFFFFFFFFu / d + 1 : 0; }
+
+// Index arithmetic of a group for the chunk kernel, which computes the actives-first positions
+// instead of reading them: the ket core's modes of rank > 1 in cluster order (reciprocal, rank,
+// stride in the actives-first layout), and the reciprocals of the bra ranks and of m.
+struct BstLayout {
+  uint32_t g_mg[kMaxClusters];
+  int32_t g_dim[kMaxClusters], g_st[kMaxClusters];
+  uint32_t a_mg[4], s_mg[kMaxClusters];
+  uint32_t m_mg;
+  int32_t ng;
+  int32_t pad[2];
+};
+static_assert(sizeof(BstLayout) % 16 == 0, "BstLayout is copied in 16-byte units");
 
 // Problem description the planner needs (host copies).
 struct ProblemInfo {
