@@ -32,8 +32,10 @@ using namespace fcg;
 namespace {
 
 constexpr int kBstThreads = 256;
-constexpr int kOpThreads = 64;            // threads per group of the operator-cache build
-constexpr int kGammaSmem = 6144;          // doubles of the per-p staging tile of the gamma kernel
+constexpr int kGammaThreads = 128;        // threads per dressed TDM
+constexpr int kOpThreads = 128;           // threads per job of the operator-cache build
+// doubles of the gamma kernel's staging tile: 24 KB (nine CTAs per SM), more where one p needs it
+constexpr int kGammaTile = 3072, kGammaTileMax = 6144;
 // shared memory of one warp of bst_sigma_bra_kernel (description + workspace); larger groups
 // run in CTA chunks.  Measured on the 32-orbital / 8-cluster vector with cores up to 12^4:
 // float builds are fastest with 4 KB (9 % faster than 8 KB once the larger groups
@@ -55,15 +57,17 @@ constexpr int64_t kSplitFma = int64_t(1) << 20;  // larger operator products run
 
 // ---- operator cache ----------------------------------------------------------------------
 
-// One CTA per gamma.  For each orbital multi-index p:  T[I, kk] = sum_J G[p, I, J] U_ket[J, kk]
-// staged in shared memory, then g[p, kb, kk] = sum_I U_bra[I, kb] T[I, kk].  Tiles that do
-// not fit the staging buffer use the direct double sum.
-__global__ void __launch_bounds__(kBstThreads) bst_gamma_kernel(const BstGamma* __restrict__ gam,
-                                                                const BstBlock* __restrict__ blocks,
-                                                                const double* __restrict__ tdm,
-                                                                const double* __restrict__ factors,
-                                                                double* __restrict__ g) {
-  __shared__ double tile[kGammaSmem];
+// One CTA per gamma.  For each orbital multi-index p:  T[p, I, kk] = sum_J G[p, I, J] U_ket[J, kk]
+// staged in shared memory for as many p as fit, then g[p, kb, kk] = sum_I U_bra[I, kb] T[p, I, kk].
+// Consecutive threads take consecutive p (the fastest index of G, of g and of the tile).  Tiles
+// that do not fit the staging buffer for one p use the direct double sum.  Bound: latency; a p at a
+// time, with two barriers each, took 3.2 ms where this takes 0.8 ms (32 orbitals, 3 sectors).
+__global__ void __launch_bounds__(kGammaThreads) bst_gamma_kernel(const BstGamma* __restrict__ gam,
+                                                                  const BstBlock* __restrict__ blocks,
+                                                                  const double* __restrict__ tdm,
+                                                                  const double* __restrict__ factors,
+                                                                  double* __restrict__ g, int tile_len) {
+  extern __shared__ double tile[];
   const BstGamma Q = gam[blockIdx.x];
   const BstBlock& B = blocks[Q.bra];
   const BstBlock& K = blocks[Q.ket];
@@ -74,21 +78,26 @@ __global__ void __launch_bounds__(kBstThreads) bst_gamma_kernel(const BstGamma* 
   const double* Uk = factors + K.factor_off[c];
   const double* G = tdm + Q.tdm_off;
   double* out = g + Q.g_off;
-  if (Lb * rk <= kGammaSmem) {
-    for (int p = 0; p < np; ++p) {
-      for (int e = threadIdx.x; e < Lb * rk; e += blockDim.x) {
-        const int I = e % Lb, kk = e / Lb;
-        const double* gcol = G + p + int64_t(np) * (sb + I);
+  const int one = Lb * rk;  // tile elements of one p
+  if (one <= tile_len) {
+    const int step = min(np, tile_len / one);
+    for (int p0 = 0; p0 < np; p0 += step) {
+      const int n = min(step, np - p0);
+      for (int e = threadIdx.x; e < one * n; e += blockDim.x) {
+        const int r = e / n, p = e - r * n;
+        const int kk = r / Lb, I = r - kk * Lb;
+        const double* gcol = G + p0 + p + int64_t(np) * (sb + I);
         double s = 0.0;
         for (int J = 0; J < Lk; ++J) s = fma(gcol[int64_t(np) * mb * (sk + J)], Uk[J + int64_t(Lk) * kk], s);
         tile[e] = s;
       }
       __syncthreads();
-      for (int e = threadIdx.x; e < rb * rk; e += blockDim.x) {
-        const int kb = e % rb, kk = e / rb;
+      for (int e = threadIdx.x; e < rb * rk * n; e += blockDim.x) {
+        const int r = e / n, p = e - r * n;
+        const int kk = r / rb, kb = r - kk * rb;
         double s = 0.0;
-        for (int I = 0; I < Lb; ++I) s = fma(Ub[I + int64_t(Lb) * kb], tile[I + Lb * kk], s);
-        out[p + int64_t(np) * e] = s;
+        for (int I = 0; I < Lb; ++I) s = fma(Ub[I + int64_t(Lb) * kb], tile[p + n * (I + Lb * kk)], s);
+        out[p0 + p + int64_t(np) * r] = s;
       }
       __syncthreads();
     }
@@ -110,122 +119,151 @@ __global__ void __launch_bounds__(kBstThreads) bst_gamma_kernel(const BstGamma* 
   }
 }
 
-// One CTA per group: the group operator, scaled by the product of the rank-1 spectator overlaps.
-// Groups of two or more active clusters are built factored on the first active cluster: for
-// each index tuple q' of the other clusters (their bra and ket ranks),
-//   u[p0] = sum_{p1..} ints[p0, p1, ..] prod_{a>0} g_a[p_a, q'_a]
-// once per term, then every element of the first cluster's (bra, ket) ranks is
-// sum_p0 g_0[p0, kb0, kk0] u[p0] -- len(p1..) + rank^2 len(p0) multiply-adds per tuple in
-// place of rank^2 len(p0..) (the successive contractions of build_dense_H_term,
-// src/tucker_build_dense_H_term.jl:5-175).  A work item is one tuple and kOpChunk of the first
-// cluster's elements; u lives in shared memory, one column per thread.
-constexpr int kOpMaxD0 = 64;  // longest orbital multi-index of the first active cluster built factored
-constexpr int kOpChunk = 16;  // operator elements per work item of the factored build
+// A range of index tuples (bra and ket ranks of the clusters after the second) of one group.
+struct BstOpJob {
+  int32_t g;
+  int32_t t0, t1;
+  int32_t pad;
+};
+constexpr int64_t kOpJob = int64_t(1) << 15;  // operator elements of a job, about
+constexpr int kOpV = 1024, kOpU = 2048, kOpG = 2304;  // largest shared tables of the factored build (doubles)
 
-__global__ void __launch_bounds__(kOpThreads) bst_op_kernel(const BstGroup* __restrict__ groups,
+// One CTA per job: operator elements, scaled by the product of the rank-1 spectator overlaps.
+// Groups of two or more active clusters are built by successive contraction (as build_dense_H_term,
+// src/tucker_build_dense_H_term.jl:5-175).  For each tuple of the clusters after the second,
+//   V[p0, p1] = sum_{p2..} ints[p0, p1, p2..] prod_{a>1} g_a[p_a, q_a]   (two clusters: the ints)
+//   u[p0, q1] = sum_p1 V[p0, p1] g_1[p1, q1]
+//   OP[q0, q1, ..] += sum_p0 g_0[p0, q0] u[p0, q1]
+// with V, u and g_0 in shared memory: every element of a step is one thread's.  The elements of OP
+// are one thread's for all terms, which it adds in term order.
+//
+// Bound: latency of the short steps.  A thread per tuple of all clusters after the first, with its
+// own u in shared memory, and recomputed u for every 16 elements of the first cluster, took 9.7 ms
+// where this takes 1.9 ms (32 orbitals, 3 sectors, up to three excited clusters, ranks 3-8: 39 150
+// groups, 5.1e6 elements, 3.9e8 multiply-adds), and 193 where this takes 24 ms (5 sectors, up to
+// four excited clusters, ranks 4-12: 3.5e8 elements).
+__global__ void __launch_bounds__(kOpThreads) bst_op_kernel(const BstOpJob* __restrict__ jobs,
+                                                             const BstGroup* __restrict__ groups,
                                                              const BstGroupTerm* __restrict__ gterms,
                                                              const BstBlock* __restrict__ blocks, int N,
                                                              const double* __restrict__ ints,
                                                              const double* __restrict__ g,
                                                              const double* __restrict__ factors,
-                                                             double* __restrict__ opc) {
-  __shared__ double scal;
-  __shared__ double u_all[kOpMaxD0 * kOpThreads];
-  const BstGroup& Gp = groups[blockIdx.x];
+                                                             double* __restrict__ opc, int v_len, int u_len, int g_len) {
+  extern __shared__ double op_smem[];
+  __shared__ double over[kMaxClusters];
+  const BstOpJob J = jobs[blockIdx.x];
+  const BstGroup& Gp = groups[J.g];
   const BstBlock& B = blocks[Gp.bra];
   const BstBlock& K = blocks[Gp.ket];
-  if (threadIdx.x == 0) {
-    double s = 1.0;
-    for (int c = 0; c < N; ++c) {
-      if ((Gp.act_mask >> c) & 1) continue;
-      if (B.rank[c] != 1 || K.rank[c] != 1) continue;
+  if (threadIdx.x < kMaxClusters) {
+    const int c = threadIdx.x;
+    double d = 1.0;
+    if (c < N && !((Gp.act_mask >> c) & 1) && B.rank[c] == 1 && K.rank[c] == 1) {
       const double* ub = factors + B.factor_off[c];
       const double* uk = factors + K.factor_off[c];
-      double d = 0.0;
+      d = 0.0;
       for (int x = 0; x < B.len[c]; ++x) d = fma(ub[x], uk[x], d);
-      s *= d;
     }
-    scal = s;
+    over[c] = d;
   }
   __syncthreads();
-  int act[4], na = 0;
+  double scal = 1.0;
+#pragma unroll
+  for (int c = 0; c < kMaxClusters; ++c) scal *= over[c];
+  int rb[4] = {1, 1, 1, 1}, rk[4] = {1, 1, 1, 1}, na = 0;
   for (int c = 0; c < N; ++c)
-    if ((Gp.act_mask >> c) & 1) act[na++] = c;
+    if ((Gp.act_mask >> c) & 1) {
+#pragma unroll
+      for (int a = 0; a < 4; ++a)  // (no dynamic register indexing)
+        if (a == na) {
+          rb[a] = B.rank[c];
+          rk[a] = K.rank[c];
+        }
+      ++na;
+    }
   bool factored = na >= 2;
   for (int t = 0; t < Gp.nt && factored; ++t) {
     const BstGroupTerm& T = gterms[Gp.t_off + t];
-    factored = T.ints_off >= 0 && T.nact == na && T.np[0] <= kOpMaxD0;
+    factored = T.ints_off >= 0 && T.nact == na && T.np[0] <= u_len && (na == 2 || T.np[0] * T.np[1] <= v_len);
   }
   if (factored) {
-    const int rb0 = B.rank[act[0]], rk0 = K.rank[act[0]];
-    const int q0n = rb0 * rk0;
-    const int krest = Gp.k / rk0, brest = Gp.m / rb0;
-    const int nch = (q0n + kOpChunk - 1) / kOpChunk;
-    const int64_t items = int64_t(krest) * brest * nch;
-    double* u = u_all + threadIdx.x;  // u[p] at u[p * kOpThreads]
-    for (int64_t item = threadIdx.x; item < items; item += blockDim.x) {
-      const int64_t tq = item / nch;
-      const int ch = int(item - tq * nch);
-      const int kk_rest = int(tq % krest), kb_rest = int(tq / krest);
-      int ik[4] = {0, 0, 0, 0}, ib[4] = {0, 0, 0, 0};
-      {
-        int x = kk_rest, y = kb_rest;
-        for (int a = 1; a < na; ++a) {
-          ik[a] = x % K.rank[act[a]];
-          x /= K.rank[act[a]];
-          ib[a] = y % B.rank[act[a]];
-          y /= B.rank[act[a]];
-        }
-      }
-      const int o0 = ch * kOpChunk;
-      double acc[kOpChunk];
-#pragma unroll
-      for (int o = 0; o < kOpChunk; ++o) acc[o] = 0.0;
+    double* V = op_smem;
+    double* us = V + v_len;
+    double* gs = us + u_len;
+    const int q0n = rb[0] * rk[0], q1n = rb[1] * rk[1], kt = rk[2] * rk[3];
+    for (int tq = J.t0; tq < J.t1; ++tq) {
+      const int xk = tq % kt, xb = tq / kt;
+      const int ik3 = xk / rk[2], ik2 = xk - ik3 * rk[2], ib3 = xb / rb[2], ib2 = xb - ib3 * rb[2];
+      // OP element (ik0, ib0, q1 = ib1 + rb1 * ik1): ket index kk0 + ik0 + rk0 * ik1, bra likewise
+      const int64_t kk0 = int64_t(rk[0]) * rk[1] * xk, kb0 = int64_t(rb[0]) * rb[1] * xb;
       for (int t = 0; t < Gp.nt; ++t) {
-        const BstGroupTerm T = gterms[Gp.t_off + t];
-        const double* v = ints + T.ints_off;
+        const BstGroupTerm& T = gterms[Gp.t_off + t];
         const int d0 = T.np[0], d1 = T.np[1];
-        const int d2 = T.nact > 2 ? T.np[2] : 1, d3 = T.nact > 3 ? T.np[3] : 1;
-        const double* ga[4];
-        for (int a = 1; a < T.nact; ++a)
-          ga[a] = g + T.g_off[a] + int64_t(T.np[a]) * (ib[a] + int64_t(B.rank[act[a]]) * ik[a]);
-        for (int p = 0; p < d0; ++p) u[p * kOpThreads] = 0.0;
-        for (int l = 0; l < d3; ++l) {
-          const double x3 = T.nact > 3 ? ga[3][l] : 1.0;
-          for (int r = 0; r < d2; ++r) {
-            const double x2 = (T.nact > 2 ? ga[2][r] : 1.0) * x3;
-            for (int j = 0; j < d1; ++j) {
-              const double x1 = ga[1][j] * x2;
-              const double* vj = v + int64_t(d0) * (j + int64_t(d1) * (r + int64_t(d2) * l));
-              for (int p = 0; p < d0; ++p) u[p * kOpThreads] = fma(vj[p], x1, u[p * kOpThreads]);
-            }
-          }
-        }
-        const double sg = double(T.sign);
+        const double* v = ints + T.ints_off;
         const double* g0 = g + T.g_off[0];
-#pragma unroll
-        for (int o = 0; o < kOpChunk; ++o) {
-          const int q = o0 + o;
-          if (q < q0n) {
-            const double* g0q = g0 + int64_t(d0) * q;  // (ib0 + rb0 * ik0) = q
-            double sacc = 0.0;
-            for (int p = 0; p < d0; ++p) sacc = fma(g0q[p], u[p * kOpThreads], sacc);
-            acc[o] = fma(sg, sacc, acc[o]);
+        const double* g1 = g + T.g_off[1];
+        const double sg = T.sign < 0 ? -scal : scal;
+        const bool staged = q0n * d0 <= g_len;
+        if (staged && (Gp.nt > 1 || tq == J.t0))  // g_0 with the ket index fastest, as OP is written
+          for (int e = threadIdx.x; e < q0n * d0; e += blockDim.x) {
+            const int q = e / d0, p = e - q * d0, k0 = q / rb[0], b0 = q - k0 * rb[0];
+            gs[p * q0n + k0 + rk[0] * b0] = g0[e];
+          }
+        if (na > 2) {
+          const int d2 = T.np[2], d3 = na > 3 ? T.np[3] : 1;
+          const double* g2 = g + T.g_off[2] + int64_t(d2) * (ib2 + int64_t(rb[2]) * ik2);
+          const double* g3 = na > 3 ? g + T.g_off[3] + int64_t(d3) * (ib3 + int64_t(rb[3]) * ik3) : nullptr;
+          for (int e = threadIdx.x; e < d0 * d1; e += blockDim.x) {
+            double x = 0.0;
+            for (int l = 0; l < d3; ++l) {
+              double y = 0.0;
+              for (int r = 0; r < d2; ++r) y = fma(v[e + int64_t(d0) * d1 * (r + int64_t(d2) * l)], g2[r], y);
+              x = na > 3 ? fma(y, g3[l], x) : y;
+            }
+            V[e] = x;
+          }
+        } else {
+          V = const_cast<double*>(v);  // read only
+        }
+        const int step = min(q1n, u_len / d0);
+        for (int q1 = 0; q1 < q1n; q1 += step) {
+          const int nq = min(step, q1n - q1);
+          __syncthreads();
+          for (int e = threadIdx.x; e < nq * d0; e += blockDim.x) {
+            const int q = e / d0, p = e - q * d0;
+            const double* g1q = g1 + int64_t(d1) * (q1 + q);
+            double x = 0.0;
+            for (int j = 0; j < d1; ++j) x = fma(V[p + d0 * j], g1q[j], x);
+            us[e] = sg * x;
+          }
+          __syncthreads();
+          for (int e = threadIdx.x; e < nq * q0n; e += blockDim.x) {
+            const int q = e / q0n, z = e - q * q0n;  // z = ik0 + rk0 * ib0
+            const int b0 = z / rk[0], k0 = z - b0 * rk[0];
+            const double* u = us + q * d0;
+            double x = 0.0;
+            if (staged) {
+              for (int p = 0; p < d0; ++p) x = fma(gs[p * q0n + z], u[p], x);
+            } else {
+              const double* gq = g0 + int64_t(d0) * (b0 + rb[0] * k0);
+              for (int p = 0; p < d0; ++p) x = fma(gq[p], u[p], x);
+            }
+            const int k1 = (q1 + q) / rb[1], b1 = q1 + q - k1 * rb[1];
+            double* dst = opc + Gp.op_off + (kk0 + k0 + rk[0] * k1) + int64_t(Gp.k) * (kb0 + b0 + rb[0] * b1);
+            *dst = t ? *dst + x : x;
           }
         }
-      }
-#pragma unroll
-      for (int o = 0; o < kOpChunk; ++o) {
-        const int q = o0 + o;
-        if (q < q0n) {
-          const int ib0 = q % rb0, ik0 = q / rb0;
-          const int64_t kk = ik0 + int64_t(rk0) * kk_rest, kb = ib0 + int64_t(rb0) * kb_rest;
-          opc[Gp.op_off + kk + int64_t(Gp.k) * kb] = scal * acc[o];
-        }
+        __syncthreads();
       }
     }
     return;
   }
+  if (J.t0 > 0) return;  // (element by element: the first job takes the whole group)
+  int act[4];
+  na = 0;
+  for (int c = 0; c < N; ++c)
+    if ((Gp.act_mask >> c) & 1) act[na++] = c;
   const int64_t n = int64_t(Gp.m) * Gp.k;
   for (int64_t e = threadIdx.x; e < n; e += blockDim.x) {
     int64_t kk = e % Gp.k, kb = e / Gp.k;
@@ -2421,6 +2459,7 @@ int bst_set_impl(fcg_ctx* ctx, int nbody, int64_t n_blocks, const int16_t* fock,
     FCG_CUDA(cudaGetLastError());
     FCG_CUDA(cudaStreamSynchronize(ctx->stream));  // before d_tab goes
   }
+  DevBuf<BstOpJob> d_jobs;
   DevBuf<BstGamma> d_gam;
   DevBuf<BstGroupTerm> d_gt;
   DevBuf<BstOverlapJob> d_ov;
@@ -2436,14 +2475,46 @@ int bst_set_impl(fcg_ctx* ctx, int nbody, int64_t n_blocks, const int16_t* fock,
   FCG_REQUIRE(P.gammas.size() < (size_t(1) << 31) && P.overlaps.size() < (size_t(1) << 31), FCG_ELIMIT,
               "BST: too many cache jobs");
   if (!P.gammas.empty()) {
-    bst_gamma_kernel<<<unsigned(P.gammas.size()), kBstThreads, 0, ctx->stream>>>(
-        d_gam.p, ctx->d_bst_blocks.p, ctx->d_op64.p, ctx->d_bst_factors.p, d_g.p);
+    int tile = kGammaTile;
+    for (const BstGamma& Q : P.gammas) {
+      const int one = blk[Q.bra].len[Q.c] * blk[Q.ket].rank[Q.c];
+      if (one > tile && one <= kGammaTileMax) tile = one;
+    }
+    bst_gamma_kernel<<<unsigned(P.gammas.size()), kGammaThreads, size_t(tile) * sizeof(double), ctx->stream>>>(
+        d_gam.p, ctx->d_bst_blocks.p, ctx->d_op64.p, ctx->d_bst_factors.p, d_g.p, tile);
     FCG_CUDA(cudaGetLastError());
   }
   if (!P.groups.empty()) {
-    bst_op_kernel<<<unsigned(P.groups.size()), kOpThreads, 0, ctx->stream>>>(
-        ctx->d_bst_groups.p, d_gt.p, ctx->d_bst_blocks.p, N, ctx->d_ints64.p, d_g.p, ctx->d_bst_factors.p,
-        ctx->d_bst_op64.p);
+    // jobs of about kOpJob elements; shared tables as long as any group needs, up to their limits
+    std::vector<BstOpJob> jobs;
+    jobs.reserve(P.groups.size());
+    int v_len = 1, u_len = 1, g_len = 1;
+    for (size_t q = 0; q < P.groups.size(); ++q) {
+      const BstGroup& G = P.groups[q];
+      int64_t tuples = 1, q0n = 1, q1n = 1;
+      int a = 0;
+      for (int c = 0; c < N; ++c)
+        if ((G.act_mask >> c) & 1) {
+          const int64_t r = int64_t(blk[G.bra].rank[c]) * blk[G.ket].rank[c];
+          (a == 0 ? q0n : a == 1 ? q1n : tuples) *= r;
+          ++a;
+        }
+      for (int t = 0; t < G.nt; ++t) {
+        const BstGroupTerm& T = P.gterms[size_t(G.t_off) + t];
+        if (a > 2 && T.np[0] * T.np[1] <= kOpV) v_len = std::max(v_len, T.np[0] * T.np[1]);
+        if (a > 1 && T.np[0] <= kOpU) u_len = std::max(u_len, int(std::min<int64_t>(kOpU, q1n * T.np[0])));
+        if (a > 1 && q0n * T.np[0] <= kOpG) g_len = std::max(g_len, int(q0n * T.np[0]));
+      }
+      const int64_t pieces = std::max<int64_t>(1, std::min<int64_t>(tuples, int64_t(G.m) * G.k / kOpJob));
+      const int64_t step = (tuples + pieces - 1) / pieces;
+      for (int64_t t0 = 0; t0 < tuples; t0 += step)
+        jobs.push_back(BstOpJob{int32_t(q), int32_t(t0), int32_t(std::min(tuples, t0 + step)), 0});
+    }
+    FCG_REQUIRE(jobs.size() < (size_t(1) << 31), FCG_ELIMIT, "BST: too many operator jobs");
+    FCG_CUDA(d_jobs.upload(jobs.data(), jobs.size(), ctx->stream));
+    bst_op_kernel<<<unsigned(jobs.size()), kOpThreads, sizeof(double) * size_t(v_len + u_len + g_len), ctx->stream>>>(
+        d_jobs.p, ctx->d_bst_groups.p, d_gt.p, ctx->d_bst_blocks.p, N, ctx->d_ints64.p, d_g.p, ctx->d_bst_factors.p,
+        ctx->d_bst_op64.p, v_len, u_len, g_len);
     FCG_CUDA(cudaGetLastError());
     bst_convert_kernel<<<1024, 256, 0, ctx->stream>>>(ctx->d_bst_op64.p, ctx->d_bst_op32.p, P.op_total);
     FCG_CUDA(cudaGetLastError());
