@@ -138,7 +138,7 @@ constexpr int kOpV = 1024, kOpU = 2048, kOpG = 2304;  // largest shared tables o
 // are one thread's for all terms, which it adds in term order.
 //
 // Bound: latency of the short steps.  A thread per tuple of all clusters after the first, with its
-// own u in shared memory, and recomputed u for every 16 elements of the first cluster, took 9.7 ms
+// own u in shared memory and recomputed u for every 16 elements of the first cluster, took 9.7 ms
 // where this takes 1.9 ms (32 orbitals, 3 sectors, up to three excited clusters, ranks 3-8: 39 150
 // groups, 5.1e6 elements, 3.9e8 multiply-adds), and 193 where this takes 24 ms (5 sectors, up to
 // four excited clusters, ranks 4-12: 3.5e8 elements).
@@ -1751,18 +1751,22 @@ std::string plan_bst(const fcg_ctx* ctx, int nbody, const std::vector<BstBlock>&
     std::unordered_map<int, std::unordered_map<uint64_t, std::vector<int32_t>>> lookup;
     {
       std::vector<int> sides = split > 0 ? std::vector<int>{0, 1} : std::vector<int>{2};
+      std::vector<int> keys;
       for (int t = 0; t < ctx->n_terms; ++t) {
         const int32_t* r = &ctx->trm[int64_t(t) * kTrmCols];
         if (r[0] > nbody) continue;
         int mask = 0;
         for (int o = 0; o < r[0]; ++o) mask |= 1 << r[2 + o];
-        for (int side : sides) {
-          const int key = mask * 4 + side;
-          if (lookup.count(key)) continue;
-          auto& m = lookup[key];
-          for (int64_t k = 0; k < nb; ++k)
-            if (in_side(k, side)) m[hash_of(k, fock + 2 * N * k, mask)].push_back(int32_t(k));
-        }
+        for (int side : sides)
+          if (lookup.emplace(mask * 4 + side, std::unordered_map<uint64_t, std::vector<int32_t>>()).second)
+            keys.push_back(mask * 4 + side);
+      }
+#pragma omp parallel for schedule(dynamic, 1)
+      for (int64_t i = 0; i < int64_t(keys.size()); ++i) {
+        auto& m = lookup.find(keys[size_t(i)])->second;
+        const int mask = keys[size_t(i)] >> 2, side = keys[size_t(i)] & 3;
+        for (int64_t k = 0; k < nb; ++k)
+          if (in_side(k, side)) m[hash_of(k, fock + 2 * N * k, mask)].push_back(int32_t(k));
       }
     }
     // the transfers with terms whose ket sector exists, once per distinct bra sector (and ket
@@ -1819,7 +1823,9 @@ std::string plan_bst(const fcg_ctx* ctx, int nbody, const std::vector<BstBlock>&
       list_worker();
       for (auto& th : lpool) th.join();
     }
-    constexpr int64_t kBrasPerPart = 16;
+    // parts small enough that the threads' last ones are short (16 parts a thread), at most 16 bras
+    const int64_t n_cpu = std::max(1u, std::thread::hardware_concurrency());
+    const int64_t kBrasPerPart = std::max<int64_t>(1, std::min<int64_t>(16, nb / (16 * n_cpu)));
     const int64_t n_parts = (nb + kBrasPerPart - 1) / kBrasPerPart;
     parts.resize(size_t(n_parts));
     std::atomic<int64_t> next{0};
@@ -1879,65 +1885,76 @@ std::string plan_bst(const fcg_ctx* ctx, int nbody, const std::vector<BstBlock>&
     for (const BstPart& part : parts)
       if (!part.err.empty()) return part.err;
   }
-  // concatenation in bra order; the index tables are shared: each (block, active mask) gets
-  // its table where it is first used, as a serial walk over the groups would place it
-  {
-    size_t n_groups = 0, n_gterms = 0, n_triples = 0, n_gammas = 0, n_ov = 0;
-    for (const BstPart& part : parts) {
-      n_groups += part.groups.size();
-      n_gterms += part.gterms.size();
-      n_triples += part.triples.size();
-      n_gammas += part.gammas.size();
-      n_ov += part.overlaps.size();
-    }
-    P.groups.reserve(n_groups);
-    P.gterms.reserve(n_gterms);
-    P.triples.reserve(n_triples);
-    P.gammas.reserve(n_gammas);
-    P.overlaps.reserve(n_ov);
-  }
-  std::unordered_map<uint64_t, int64_t> perm_at;  // (block, active mask) -> index table offset
-  for (BstPart& part : parts) {
-    const int64_t g0 = P.g_total, op0 = P.op_total, s0 = P.s_total, t0 = int64_t(P.gterms.size());
-    if (t0 + int64_t(part.gterms.size()) >= (int64_t(1) << 31)) return "BST: more than 2^31 group terms";
-    for (BstGamma Q : part.gammas) {
-      Q.g_off += g0;
-      P.gammas.push_back(Q);
-    }
-    for (BstGroupTerm T : part.gterms) {
-      for (int o = 0; o < T.nact; ++o) T.g_off[o] += g0;
-      P.gterms.push_back(T);
-    }
-    for (BstOverlapJob J : part.overlaps) {
-      J.s_off += s0;
-      P.overlaps.push_back(J);
-    }
-    P.triples.insert(P.triples.end(), part.triples.begin(), part.triples.end());
-    for (BstGroup G : part.groups) {
-      G.op_off += op0;
-      G.t_off += int32_t(t0);
-      for (int j = 0; j < G.nsp; ++j)
-        if (G.s_off[j] >= 0) G.s_off[j] += s0;
-      for (int side = 0; side < 2; ++side) {
-        const int32_t b = side == 0 ? G.ket : G.bra;
-        const uint64_t key = uint64_t(b) * 256 + uint64_t(G.act_mask);
-        auto it = perm_at.find(key);
-        if (it == perm_at.end()) {
-          it = perm_at.emplace(key, P.perm_total).first;
-          P.tables.push_back(BstPermTable{P.perm_total, b, G.act_mask});
-          P.perm_total += blk[b].core_len;
-        }
-        (side == 0 ? G.kperm_off : G.bperm_off) = it->second;
-      }
-      P.groups.push_back(G);
-    }
-    P.g_total += part.g_total;
-    P.op_total += part.op_total;
-    P.s_total += part.s_total;
+  // concatenation in bra order, the parts copied side by side; the index tables are shared: each
+  // (block, active mask) gets its table where it is first used, as a serial walk over the groups
+  // would place it
+  const size_t np = parts.size();
+  struct At {  // where a part's entries start
+    int64_t groups, gterms, triples, gammas, overlaps, g, op, s;
+  };
+  std::vector<At> at(np + 1, At{});
+  for (size_t q = 0; q < np; ++q) {
+    const BstPart& part = parts[q];
+    const At& a = at[q];
+    at[q + 1] = At{a.groups + int64_t(part.groups.size()),     a.gterms + int64_t(part.gterms.size()),
+                   a.triples + int64_t(part.triples.size()),   a.gammas + int64_t(part.gammas.size()),
+                   a.overlaps + int64_t(part.overlaps.size()), a.g + part.g_total,
+                   a.op + part.op_total,                       a.s + part.s_total};
     P.flops_exec += part.flops_exec;
     P.flops_ref += part.flops_ref;
+  }
+  if (at[np].gterms >= (int64_t(1) << 31)) return "BST: more than 2^31 group terms";
+  P.groups.resize(size_t(at[np].groups));
+  P.gterms.resize(size_t(at[np].gterms));
+  P.triples.resize(size_t(at[np].triples));
+  P.gammas.resize(size_t(at[np].gammas));
+  P.overlaps.resize(size_t(at[np].overlaps));
+  P.g_total = at[np].g;
+  P.op_total = at[np].op;
+  P.s_total = at[np].s;
+#pragma omp parallel for schedule(dynamic, 1)
+  for (int64_t q = 0; q < int64_t(np); ++q) {
+    BstPart& part = parts[size_t(q)];
+    const At& a = at[size_t(q)];
+    for (size_t i = 0; i < part.gammas.size(); ++i) {
+      part.gammas[i].g_off += a.g;
+      P.gammas[size_t(a.gammas) + i] = part.gammas[i];
+    }
+    for (size_t i = 0; i < part.gterms.size(); ++i) {
+      for (int o = 0; o < part.gterms[i].nact; ++o) part.gterms[i].g_off[o] += a.g;
+      P.gterms[size_t(a.gterms) + i] = part.gterms[i];
+    }
+    for (size_t i = 0; i < part.overlaps.size(); ++i) {
+      part.overlaps[i].s_off += a.s;
+      P.overlaps[size_t(a.overlaps) + i] = part.overlaps[i];
+    }
+    std::copy(part.triples.begin(), part.triples.end(), P.triples.begin() + a.triples);
+    for (size_t i = 0; i < part.groups.size(); ++i) {
+      BstGroup& G = part.groups[i];
+      G.op_off += a.op;
+      G.t_off += int32_t(a.gterms);
+      for (int j = 0; j < G.nsp; ++j)
+        if (G.s_off[j] >= 0) G.s_off[j] += a.s;
+      P.groups[size_t(a.groups) + i] = G;
+    }
     part = BstPart();  // free the part as it is consumed
   }
+  // (block, active mask) -> index table offset: an array while that is a few MB
+  const bool flat = nb <= 2048;
+  std::vector<int64_t> perm_flat(flat ? size_t(nb) << kMaxClusters : 0, -1);
+  std::unordered_map<uint64_t, int64_t> perm_map;
+  for (BstGroup& G : P.groups)
+    for (int side = 0; side < 2; ++side) {
+      const int32_t b = side == 0 ? G.ket : G.bra;
+      const size_t key = (size_t(b) << kMaxClusters) | size_t(G.act_mask);
+      int64_t& off = flat ? perm_flat[key] : perm_map.emplace(key, -1).first->second;
+      if (off < 0) {
+        off = P.perm_total;
+        P.tables.push_back(BstPermTable{off, b, G.act_mask});
+        P.perm_total += blk[size_t(b)].core_len;
+      }
+      (side == 0 ? G.kperm_off : G.bperm_off) = off;
+    }
   return "";
 }
 
