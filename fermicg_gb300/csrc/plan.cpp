@@ -14,7 +14,6 @@
 #include <algorithm>
 #include <array>
 #include <cstring>
-#include <map>
 #include <unordered_map>
 
 #include "fcg_internal.h"
@@ -517,106 +516,139 @@ std::string build_dress(const std::vector<int>& norb, int nmax, const std::vecto
                         const std::vector<TermInfo>& terms, const std::vector<TermDress>& dress, bool merge,
                         Dressing& out) {
   const int s = nmax + 1;
-  out = Dressing();
+  out.jobs.clear();  // (the vectors keep their memory for the next term set)
+  out.src.clear();
+  out.n_w = 0;
   out.rep.resize(size_t(n_terms));
   out.w_index.assign(size_t(n_terms) * s * s, -1);
   out.w_mb.assign(size_t(n_terms) * s * s, 0);
-  // the dressed cluster's TDM block of term t in bra sector (fba, fbb), or -1
-  auto block_at = [&](int t, int fba, int fbb) {
+  // the TDM blocks of every (cluster, operator), and from them those of a term's dressed cluster:
+  // calls f(bra sector cell, block) in cell order
+  const int ss = s * s;
+  struct Cell {
+    int32_t fb, fk, block;
+  };
+  std::vector<std::vector<Cell>> cells(norb.size() * kNumOps);
+  for (size_t i = 0; i < blk_index.size(); ++i)
+    if (blk_index[i] >= 0) {
+      const size_t fk = i % ss, fb = i / ss % ss;
+      cells[i / ss / ss].push_back(Cell{int32_t(fb), int32_t(fk), blk_index[i]});
+    }
+  auto each_block = [&](int t, auto&& f) {
     const int32_t* r = &trm[int64_t(t) * kTrmCols];
     const int pos = dress[size_t(t)].pos < 0 ? 0 : dress[size_t(t)].pos;
-    const int cw = r[2 + pos], fka = fba - r[10 + pos], fkb = fbb - r[14 + pos];
-    if (fka < 0 || fkb < 0 || fka > norb[cw] || fkb > norb[cw]) return -1;
-    return int(blk_index[dense_block_index(s, cw, r[6 + pos], fba, fbb, fka, fkb)]);
+    for (const Cell& c : cells[size_t(r[2 + pos]) * kNumOps + r[6 + pos]])
+      if (c.fb / s - r[10 + pos] == c.fk / s && c.fb % s - r[14 + pos] == c.fk % s) f(c.fb, c.block);
   };
-  std::vector<std::vector<int>> members;  // terms of each set, the one that stands for it first
-  {
-    std::map<std::vector<int32_t>, int> set_of;
-    for (int t = 0; t < n_terms; ++t) {
+  // sets of terms that share a W: term by term, next[t] the next one of t's set (or -1)
+  std::vector<int32_t> next(size_t(n_terms), -1);
+  if (!merge) {
+    for (int t = 0; t < n_terms; ++t) out.rep[size_t(t)] = t;
+  } else {
+    // by a hash of everything but the dressed operator: transfer, clusters, changes of Fock sector,
+    // fermionic parities, and the other clusters' operators and index lengths
+    auto hash_of = [&](int t) {
       const int32_t* r = &trm[int64_t(t) * kTrmCols];
-      const TermDress& d = dress[size_t(t)];
-      int set = -1;
-      if (merge && d.pos >= 0) {
-        // everything but the dressed operator: transfer, clusters, changes of Fock sector, fermionic
-        // parities, and the other clusters' operators and index lengths
-        std::vector<int32_t> key{r[1], r[0], d.pos};
-        for (int o = 0; o < r[0]; ++o) {
-          key.insert(key.end(), {r[2 + o], r[10 + o], r[14 + o], r[18 + o]});
-          if (o != d.pos) key.insert(key.end(), {r[6 + o], r[22 + o]});
-        }
-        auto it = set_of.find(key);
-        if (it == set_of.end()) {
-          set_of.emplace(key, int(members.size()));
-        } else {
-          set = it->second;
-          // the operators' blocks must have the same local dimensions wherever several exist
-          const int cw = r[2 + d.pos];
-          for (int fba = 0; fba <= norb[cw] && set >= 0; ++fba)
-            for (int fbb = 0; fbb <= norb[cw] && set >= 0; ++fbb) {
-              const int b = block_at(t, fba, fbb);
-              if (b < 0) continue;
-              for (int m : members[size_t(set)]) {
-                const int b2 = block_at(m, fba, fbb);
-                if (b2 >= 0 && (blocks[size_t(b2)].mb != blocks[size_t(b)].mb || blocks[size_t(b2)].mk != blocks[size_t(b)].mk)) {
-                  set = -1;
-                  break;
-                }
-              }
-            }
-        }
+      const int pos = dress[size_t(t)].pos;
+      uint64_t h = 1469598103934665603ull;
+      auto f = [&](int32_t v) { h = (h ^ uint64_t(uint32_t(v))) * 1099511628211ull; };
+      f(r[1]), f(r[0]), f(pos);
+      for (int o = 0; o < r[0]; ++o) {
+        f(r[2 + o]), f(r[10 + o]), f(r[14 + o]), f(r[18 + o]);
+        if (o != pos) f(r[6 + o]), f(r[22 + o]);
       }
-      if (set < 0) {
-        out.rep[size_t(t)] = t;
-        members.push_back({t});
-      } else {
-        out.rep[size_t(t)] = members[size_t(set)][0];
-        members[size_t(set)].push_back(t);
+      return h ^ (h >> 29);
+    };
+    auto same = [&](int t, int t2) {
+      const int32_t *r = &trm[int64_t(t) * kTrmCols], *r2 = &trm[int64_t(t2) * kTrmCols];
+      const int pos = dress[size_t(t)].pos;
+      if (r[1] != r2[1] || r[0] != r2[0] || pos != dress[size_t(t2)].pos) return false;
+      for (int o = 0; o < r[0]; ++o) {
+        if (r[2 + o] != r2[2 + o] || r[10 + o] != r2[10 + o] || r[14 + o] != r2[14 + o] || r[18 + o] != r2[18 + o])
+          return false;
+        if (o != pos && (r[6 + o] != r2[6 + o] || r[22 + o] != r2[22 + o])) return false;
       }
+      return true;
+    };
+    size_t cap = 64;
+    while (cap < 2 * size_t(n_terms)) cap <<= 1;
+    std::vector<int32_t> table(cap, -1);           // open addressing: the first term of a set
+    std::vector<int32_t> last(size_t(n_terms), -1);  // by first term: the set's last term so far
+    for (int t = 0; t < n_terms; ++t) {
+      out.rep[size_t(t)] = t;
+      if (dress[size_t(t)].pos < 0) continue;
+      size_t at = size_t(hash_of(t)) & (cap - 1);
+      while (table[at] >= 0 && !same(t, table[at])) at = (at + 1) & (cap - 1);
+      const int t0 = table[at] >= 0 ? table[at] : t;
+      // the operators' blocks must have the same local dimensions wherever several exist
+      bool fits = true;
+      for (int m = t0; m >= 0 && m != t; m = next[size_t(m)])
+        each_block(t, [&](int cell, int b) {
+          each_block(m, [&](int cell2, int b2) {
+            if (cell == cell2 && (blocks[size_t(b)].mb != blocks[size_t(b2)].mb || blocks[size_t(b)].mk != blocks[size_t(b2)].mk))
+              fits = false;
+          });
+        });
+      if (!fits) continue;
+      table[at] = t0;
+      if (t0 != t) {
+        out.rep[size_t(t)] = t0;
+        next[size_t(last[size_t(t0)])] = t;
+      }
+      last[size_t(t0)] = t;
     }
   }
-  for (const std::vector<int>& set : members) {
-    const int t0 = set[0];
+  struct Source {
+    int32_t cell, order, term, block;
+  };
+  std::vector<Source> sources;  // of one set
+  for (int t0 = 0; t0 < n_terms; ++t0) {
+    if (out.rep[size_t(t0)] != t0) continue;
     const int32_t* r0 = &trm[int64_t(t0) * kTrmCols];
     const TermDress& d = dress[size_t(t0)];
-    const int nb = r0[0], cw = r0[2 + (d.pos < 0 ? 0 : d.pos)];
-    for (int fba = 0; fba <= norb[cw]; ++fba)
-      for (int fbb = 0; fbb <= norb[cw]; ++fbb) {
-        DressJob J{};
-        J.src0 = int32_t(out.src.size());
-        for (int t : set) {
-          const int bl = block_at(t, fba, fbb);
-          if (bl < 0) continue;
-          const int32_t* r = &trm[int64_t(t) * kTrmCols];
-          const BlockInfo& B = blocks[size_t(bl)];
-          const int pos = d.pos < 0 ? 0 : d.pos;
-          if (nb > 1 && B.nidx != r[22 + pos]) return "term dims do not match the TDM block";
-          int stride[4];
-          stride[0] = 1;
-          for (int o = 1; o < 4; ++o) stride[o] = stride[o - 1] * r[22 + o - 1];
-          DressSrc S{};
-          S.g_off = B.off;
-          S.ints_off = terms[size_t(t)].ints_off;
-          S.nq = nb == 1 ? 1 : B.nidx;
-          S.stride_q = stride[pos];
-          for (int q = 0; q < d.nrem; ++q) S.rem_stride[q] = stride[d.rem_pos[q]];
-          out.src.push_back(S);
-          J.mb = B.mb;
-          J.mk = B.mk;
-        }
-        J.n_src = int32_t(out.src.size()) - J.src0;
-        if (J.n_src == 0) continue;
-        out.n_w = (out.n_w + kAlign - 1) / kAlign * kAlign;  // vector-load alignment of W blocks
-        J.w_off = out.n_w;
-        J.rest_len = d.rest_len;
-        J.nrem = d.nrem;
-        for (int q = 0; q < d.nrem; ++q) J.rem_dim[q] = d.rem_dim[q];
-        J.one_body = nb == 1;
-        out.jobs.push_back(J);
-        const size_t wi = (size_t(t0) * s + fba) * s + fbb;
-        out.w_index[wi] = out.n_w;
-        out.w_mb[wi] = J.mb;
-        out.n_w += int64_t(d.rest_len) * J.mb * J.mk;
+    const int nb = r0[0], pos = d.pos < 0 ? 0 : d.pos;
+    sources.clear();
+    for (int t = t0, i = 0; t >= 0; t = next[size_t(t)], ++i)
+      each_block(t, [&](int cell, int b) { sources.push_back(Source{cell, i, t, b}); });
+    if (next[size_t(t0)] >= 0)
+      std::sort(sources.begin(), sources.end(), [](const Source& x, const Source& y) {
+        return x.cell != y.cell ? x.cell < y.cell : x.order < y.order;
+      });
+    for (size_t i = 0; i < sources.size();) {
+      DressJob J{};
+      J.src0 = int32_t(out.src.size());
+      const int cell = sources[i].cell;
+      for (; i < sources.size() && sources[i].cell == cell; ++i) {
+        const int t = sources[i].term;
+        const int32_t* r = &trm[int64_t(t) * kTrmCols];
+        const BlockInfo& B = blocks[size_t(sources[i].block)];
+        if (nb > 1 && B.nidx != r[22 + pos]) return "term dims do not match the TDM block";
+        int stride[4];
+        stride[0] = 1;
+        for (int o = 1; o < 4; ++o) stride[o] = stride[o - 1] * r[22 + o - 1];
+        DressSrc S{};
+        S.g_off = B.off;
+        S.ints_off = terms[size_t(t)].ints_off;
+        S.nq = nb == 1 ? 1 : B.nidx;
+        S.stride_q = stride[pos];
+        for (int q = 0; q < d.nrem; ++q) S.rem_stride[q] = stride[d.rem_pos[q]];
+        out.src.push_back(S);
+        J.mb = B.mb;
+        J.mk = B.mk;
       }
+      J.n_src = int32_t(out.src.size()) - J.src0;
+      out.n_w = (out.n_w + kAlign - 1) / kAlign * kAlign;  // vector-load alignment of W blocks
+      J.w_off = out.n_w;
+      J.rest_len = d.rest_len;
+      J.nrem = d.nrem;
+      for (int q = 0; q < d.nrem; ++q) J.rem_dim[q] = d.rem_dim[q];
+      J.one_body = nb == 1;
+      out.jobs.push_back(J);
+      const size_t wi = size_t(t0) * ss + cell;
+      out.w_index[wi] = out.n_w;
+      out.w_mb[wi] = J.mb;
+      out.n_w += int64_t(d.rest_len) * J.mb * J.mk;
+    }
   }
   return "";
 }
