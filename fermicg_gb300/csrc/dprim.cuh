@@ -116,10 +116,10 @@ struct Digit {
 };
 
 // digit counts of every tile, digit-major: cnt[d * n_tiles + tile]
-__global__ void __launch_bounds__(kSortThreads) radix_hist_kernel(const uint64_t* __restrict__ keys,
-                                                                  const uint32_t* __restrict__ vals, int64_t n,
-                                                                  Digit dg, int32_t* __restrict__ cnt,
-                                                                  int64_t n_tiles) {
+static __global__ void __launch_bounds__(kSortThreads) radix_hist_kernel(const uint64_t* __restrict__ keys,
+                                                                         const uint32_t* __restrict__ vals, int64_t n,
+                                                                         Digit dg, int32_t* __restrict__ cnt,
+                                                                         int64_t n_tiles) {
   __shared__ int h[kRadix];
   const int tid = threadIdx.x;
   h[tid] = 0;
@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(kSortThreads) radix_hist_kernel(const uint64_t
 }
 
 // stable scatter of every tile to its scanned digit offsets
-__global__ void __launch_bounds__(kSortThreads) radix_scatter_kernel(
+static __global__ void __launch_bounds__(kSortThreads) radix_scatter_kernel(
     const uint64_t* __restrict__ kin, const uint32_t* __restrict__ vin, uint64_t* __restrict__ kout,
     uint32_t* __restrict__ vout, int64_t n, Digit dg, const int32_t* __restrict__ offs, int64_t n_tiles) {
   constexpr int kWarps = kSortThreads / 32;

@@ -225,6 +225,16 @@ struct fcg_ctx {
   std::vector<int64_t> wmax_index; // parallel to open_dressing.w_index
   DevBuf<double> d_gmax;
   DevBuf<double> d_wmax;
+  // open sigma: the term set's tables on the device (with open_dressing), the plan's working arrays,
+  // and how far its hash table is empty
+  struct {
+    DevBuf<int32_t> d_trm, d_w_mb, d_rep, d_first_of_tr, d_tr_terms, d_rows, d_nt, d_used;
+    DevBuf<TermDress> d_dress;
+    DevBuf<int64_t> d_w_index, d_wmax_index, d_gmax_off, d_i64, d_bra_dims;
+    DevBuf<int16_t> d_trans, d_bra_fock;
+    DevBuf<uint64_t> d_key;
+    size_t clean_keys = 0, clean_vals = 0;
+  } oplan;
   // open sigma (FOIS) working set and last result
   DevBuf<OpenTerm> d_oterms;
   DevBuf<OpenItem> d_oitems;
@@ -239,7 +249,6 @@ struct fcg_ctx {
   DevBuf<unsigned long long> d_counters;
   DevBuf<unsigned char> d_scan_tmp;
   std::vector<int16_t> open_bra_fock;   // [n_bra_sectors][N][2]
-  std::vector<int64_t> open_strides;    // [n_bra_sectors][N]
   std::vector<int64_t> open_dims;       // [n_bra_sectors][N]
   PinnedBuf<unsigned long long> open_keys;  // keys of the last open sigma, open_rows of them
   PinnedBuf<double> open_vals;              // [open_rows][R] row-major

@@ -1173,6 +1173,25 @@ int ensure_open_dressed(fcg_ctx* ctx) {
     colmax_kernel<<<unsigned(jobs.size()), 128, 0, ctx->stream>>>(d_mj, ctx->d_ow64.p, ctx->d_wmax.p);
     FCG_CUDA(cudaGetLastError());
   }
+  // the tables its plan kernels read; terms by transfer, ascending
+  auto& O = ctx->oplan;
+  std::vector<int32_t> first(size_t(ctx->n_trans) + 1, 0), terms(size_t(ctx->n_terms));
+  for (int t = 0; t < ctx->n_terms; ++t) ++first[size_t(ctx->trm[int64_t(t) * kTrmCols + 1]) + 1];
+  for (int tr = 0; tr < ctx->n_trans; ++tr) first[size_t(tr) + 1] += first[size_t(tr)];
+  {
+    std::vector<int32_t> at(first.begin(), first.end() - 1);
+    for (int t = 0; t < ctx->n_terms; ++t) terms[size_t(at[size_t(ctx->trm[int64_t(t) * kTrmCols + 1])]++)] = t;
+  }
+  FCG_CUDA(O.d_trm.upload(ctx->trm.data(), ctx->trm.size(), ctx->stream));
+  FCG_CUDA(O.d_dress.upload(ctx->dress.data(), ctx->dress.size(), ctx->stream));
+  FCG_CUDA(O.d_w_index.upload(dz.w_index.data(), dz.w_index.size(), ctx->stream));
+  FCG_CUDA(O.d_w_mb.upload(dz.w_mb.data(), dz.w_mb.size(), ctx->stream));
+  FCG_CUDA(O.d_rep.upload(dz.rep.data(), dz.rep.size(), ctx->stream));
+  FCG_CUDA(O.d_wmax_index.upload(ctx->wmax_index.data(), ctx->wmax_index.size(), ctx->stream));
+  FCG_CUDA(O.d_gmax_off.upload(ctx->gmax_off.data(), ctx->gmax_off.size(), ctx->stream));
+  FCG_CUDA(O.d_trans.upload(ctx->trans.data(), ctx->trans.size(), ctx->stream));
+  FCG_CUDA(O.d_first_of_tr.upload(first.data(), first.size(), ctx->stream));
+  FCG_CUDA(O.d_tr_terms.upload(terms.data(), terms.size(), ctx->stream));
   FCG_CUDA(cudaStreamSynchronize(ctx->stream));  // the job list's staging buffer is reused by the next call
   ctx->open_dressed = true;
   return FCG_OK;

@@ -419,9 +419,6 @@ std::string build_sectors(const ProblemInfo& pi, int64_t n_cfg, const int16_t* f
 std::string build_join(const ProblemInfo& pi, const int16_t* fock, const int16_t* cfg, Plan& plan);
 std::string build_plan(const ProblemInfo& pi, int64_t n_cfg, const int16_t* fock, const int16_t* cfg, Plan& plan);
 
-// The term-sector record of term t between bra sector fb and ket sector fk (N x 2 each);
-// false when a TDM block the term needs does not exist there.
-bool make_term_sector(const ProblemInfo& pi, int t, const int16_t* fb, const int16_t* fk, TermSector& ts);
 TermTables term_tables(const ProblemInfo& pi);
 
 // the terms of the zero transfer (the diagonal's terms), in term order

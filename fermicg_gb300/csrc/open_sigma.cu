@@ -8,6 +8,7 @@
 // the per-contribution test of _collect_significant_thread! (:830-885).
 //
 // Pipeline (one stream):
+//   plan kernels    bra sectors and one OpenTerm record per (ket sector, term) whose target exists
 //   screen_kernel   one thread per (ket row, term) job: a rigorous max-norm bound
 //                   sum_rest Wmax * prod Gmax skips jobs whose every contribution would
 //                   fail the threshold (the role of upper_bound_thread, :897-1023; skipping
@@ -18,14 +19,13 @@
 //                   exactly (threshold per contribution, as the reference), and insert into
 //                   an open-addressed table keyed by (bra sector, mixed-radix local-state
 //                   index) with atomic accumulation of the R values;
-//   compact_kernel  occupied slots -> (key, values).
+//   compact_kernel  occupied slots -> (key, values); the slots are emptied for the next call.
 // A table that overflows its probe limit sets a flag and the call is repeated with a
 // table twice as large.
 #include <cmath>
 #include <cstring>
-#include <unordered_map>
-#include <unordered_set>
 
+#include "dprim.cuh"
 #include "fcg_ctx.cuh"
 
 using namespace fcg;
@@ -37,7 +37,10 @@ constexpr int kMaxProbe = 1 << 16;
 constexpr int kKeyIdxBits = 40;
 
 // counters: [0] kept jobs, [1] elements of kept jobs, [2] table overflow, [3] output rows,
-// [4] next job of the expand warps
+// [4] next job of the expand warps; of the plan: [5] bra sectors, [6] records, [7] items, [8] jobs,
+// [9] reference flops, [10] error, [11] longest index of the register sums, [12] largest tiles with
+// register sums, [13] with shared-memory sums, [14] bytes of the TDM blocks in use
+constexpr int kCounters = 15;
 struct OpenParams {
   const OpenTerm* ot;
   const OpenItem* items;
@@ -552,16 +555,276 @@ __global__ void __launch_bounds__(32 * kExpWarps, D == 3 || D == 4 ? 2 : 1) expa
   }
 }
 
-__global__ void compact_kernel(const unsigned long long* __restrict__ keys, const double* __restrict__ vals,
-                               unsigned long long cap, int R, unsigned long long* __restrict__ okeys,
-                               double* __restrict__ ovals, unsigned long long* __restrict__ counters) {
-  const unsigned long long s = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= cap) return;
-  const unsigned long long k = keys[s];
-  if (k == kEmpty) return;
-  const unsigned long long pos = atomicAdd(counters + 3, 1ull);
-  okeys[pos] = k;
-  for (int r = 0; r < R; ++r) ovals[pos * R + r] = vals[s * R + r];
+// A block per kCompactSlots table slots: the occupied ones to the output (one place reserved per
+// block), each emptied as it is read, so that the next call finds the table as new and a call
+// fills (10.7 GB, 1.6 ms at 2^28 slots of 4 roots) only what it adds.  Bound: the read of the keys:
+// 1.26 ms for 2^28 slots and 4.9e6 rows (a thread and an atomic per slot: 3.3 ms).
+constexpr int kCompactThreads = 256, kCompactKeys = 16, kCompactSlots = kCompactThreads * kCompactKeys;
+__global__ void __launch_bounds__(kCompactThreads) compact_kernel(unsigned long long* __restrict__ keys,
+                                                                  double* __restrict__ vals, int R,
+                                                                  unsigned long long* __restrict__ okeys,
+                                                                  double* __restrict__ ovals,
+                                                                  unsigned long long* __restrict__ counters) {
+  __shared__ unsigned warp_n[kCompactThreads / 32];
+  __shared__ unsigned long long first;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const unsigned long long base = (unsigned long long)blockIdx.x * kCompactSlots + 2 * threadIdx.x;
+  ulonglong2 k[kCompactKeys / 2];
+  int n = 0;
+#pragma unroll
+  for (int i = 0; i < kCompactKeys / 2; ++i) {
+    k[i] = *reinterpret_cast<const ulonglong2*>(keys + base + 2 * kCompactThreads * i);
+    n += (k[i].x != kEmpty) + (k[i].y != kEmpty);
+  }
+  int before = n;  // inclusive, then exclusive, over the warp
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, before, d);
+    if (lane >= d) before += y;
+  }
+  if (lane == 31) warp_n[wid] = unsigned(before);
+  before -= n;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned sum = 0;
+    for (int w = 0; w < kCompactThreads / 32; ++w) {
+      const unsigned c = warp_n[w];
+      warp_n[w] = sum;
+      sum += c;
+    }
+    first = sum ? atomicAdd(counters + 3, (unsigned long long)sum) : 0ull;
+  }
+  __syncthreads();
+  unsigned long long pos = first + warp_n[wid] + (unsigned long long)before;
+  auto take = [&](unsigned long long key, unsigned long long slot) {
+    if (key == kEmpty) return;
+    okeys[pos] = key;
+    keys[slot] = kEmpty;
+    for (int r = 0; r < R; ++r) {
+      ovals[pos * R + r] = vals[slot * R + r];
+      vals[slot * R + r] = 0.0;
+    }
+    ++pos;
+  };
+#pragma unroll
+  for (int i = 0; i < kCompactKeys / 2; ++i) {
+    const unsigned long long slot = base + 2 * kCompactThreads * i;
+    take(k[i].x, slot);
+    take(k[i].y, slot + 1);
+  }
+}
+
+// ---- plan ------------------------------------------------------------------------------------
+// A thread per pair (ket sector, transfer), ket sector major: count, number the bra sectors and
+// scan, write.  Bound: the table reads of term_sector_of, a serial chain per term.  Host loops with
+// hash maps took 29 ms for 193 sectors x 1441 transfers (194,496 records) and their upload 1 ms;
+// the kernels take under 1 ms, and the call 28 ms instead of 69 with the emptied table below.
+struct OpenPlan {
+  TermTables tt;  // the open dressing's
+  const int16_t* sec_fock;
+  const int32_t* sec_start;  // rows of the ket sectors
+  const int32_t* sec_count;
+  const int16_t* trans;
+  const int32_t* first_of_tr;  // terms of each transfer
+  const int32_t* tr_terms;
+  const int32_t* norb;
+  const int64_t* wmax_index;
+  const int64_t* gmax_off;
+  int64_t n_pairs;
+  int n_trans, N, nbody;
+  uint64_t* key;    // bra sector of each pair (4 bits per entry)
+  int32_t* nt;      // its terms with at most nbody clusters whose TDM blocks exist; -1: no target
+  int64_t* ot;      // the same for the scan (0 without a target)
+  int64_t* has;     // 1: an item (some terms)
+  int64_t* jobs;    // (row, term) jobs
+};
+
+__device__ __forceinline__ bool open_target(const OpenPlan& p, int64_t i, int16_t* fb, int64_t* dims) {
+  const int64_t sk = i / p.n_trans;
+  const int tr = int(i - sk * p.n_trans);
+  if (p.first_of_tr[tr] == p.first_of_tr[tr + 1]) return false;
+  const int16_t* fk = p.sec_fock + sk * 2 * p.N;
+  for (int c = 0; c < 2 * p.N; ++c) {
+    const int f = fk[c] + p.trans[int64_t(tr) * 2 * p.N + c];
+    if (f < 0 || f > p.norb[c / 2]) return false;
+    fb[c] = int16_t(f);
+  }
+  // every cluster must have a local basis in its bra sector (:39-46)
+  for (int c = 0; c < p.N; ++c) {
+    const int bl = p.tt.blk[dense_block_index(p.tt.nmax1, c, kOpH, fb[2 * c], fb[2 * c + 1], fb[2 * c], fb[2 * c + 1])];
+    if (bl < 0) return false;
+    dims[c] = p.tt.blocks[bl].mb;
+  }
+  return true;
+}
+
+__global__ void open_count_kernel(OpenPlan p) {
+  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i > p.n_pairs) return;
+  int32_t nt = -1;
+  int64_t rows = 0;
+  if (i < p.n_pairs) {
+    int16_t fb[2 * kMaxClusters];
+    int64_t dims[kMaxClusters];
+    if (open_target(p, i, fb, dims)) {
+      uint64_t key = 0;
+      for (int c = 0; c < 2 * p.N; ++c) key |= uint64_t(fb[c]) << (4 * c);
+      p.key[i] = key;
+      const int64_t sk = i / p.n_trans;
+      const int tr = int(i - sk * p.n_trans);
+      const int16_t* fk = p.sec_fock + sk * 2 * p.N;
+      nt = 0;
+      for (int q = p.first_of_tr[tr]; q < p.first_of_tr[tr + 1]; ++q) {
+        const int t = p.tr_terms[q];
+        TermSector ts;
+        int64_t fma;
+        if (p.tt.trm[int64_t(t) * kTrmCols] <= p.nbody && term_sector_of(p.tt, t, fb, fk, ts, &fma)) ++nt;
+      }
+      rows = p.sec_count[sk];
+    }
+    p.nt[i] = nt;
+  }
+  p.ot[i] = max(nt, 0);
+  p.has[i] = nt > 0 ? 1 : 0;
+  p.jobs[i] = nt > 0 ? int64_t(nt) * rows : 0;
+}
+
+// bra sectors numbered by their first pair: an open-addressed table of pairs (kEmpty: none)
+__global__ void open_sectors_kernel(OpenPlan p, unsigned long long* __restrict__ table, int64_t mask,
+                                    int64_t* __restrict__ slot_of) {
+  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= p.n_pairs || p.nt[i] < 0) return;
+  const uint64_t key = p.key[i];
+  uint64_t h = key * 0x9E3779B97F4A7C15ull;
+  h ^= h >> 29;
+  for (int64_t at = int64_t(h & uint64_t(mask));; at = (at + 1) & mask) {  // at most half full
+    const unsigned long long cur = atomicCAS(table + at, kEmpty, (unsigned long long)i);
+    if (cur == kEmpty || p.key[cur] == key) {
+      if (cur > (unsigned long long)i) atomicMin(table + at, (unsigned long long)i);
+      slot_of[i] = at;
+      return;
+    }
+  }
+}
+
+__global__ void open_first_kernel(OpenPlan p, const unsigned long long* __restrict__ table,
+                                  const int64_t* __restrict__ slot_of, int64_t* __restrict__ rep,
+                                  int64_t* __restrict__ flag) {
+  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i > p.n_pairs) return;
+  const int64_t r = i < p.n_pairs && p.nt[i] >= 0 ? int64_t(table[slot_of[i]]) : -1;
+  if (i < p.n_pairs) rep[i] = r;
+  flag[i] = r == i ? 1 : 0;
+}
+
+// sizes after the scans, for the host
+__global__ void open_sizes_kernel(int64_t n_pairs, const int64_t* __restrict__ flag, const int64_t* __restrict__ ot,
+                                  const int64_t* __restrict__ has, const int64_t* __restrict__ jobs,
+                                  unsigned long long* __restrict__ counters) {
+  counters[5] = (unsigned long long)flag[n_pairs];
+  counters[6] = (unsigned long long)ot[n_pairs];
+  counters[7] = (unsigned long long)has[n_pairs];
+  counters[8] = (unsigned long long)jobs[n_pairs];
+}
+
+// the records, items and bra sectors; counters [9] .. [13]; used[block] = 1 for every TDM block read.
+// Scanned: flag (bra sector ids), ot, has, jobs.
+__global__ void open_records_kernel(OpenPlan p, const int64_t* __restrict__ rep, const int64_t* __restrict__ id,
+                                    OpenTerm* __restrict__ ots, OpenItem* __restrict__ items,
+                                    int64_t* __restrict__ prefix, int16_t* __restrict__ bra_fock,
+                                    int64_t* __restrict__ strides, int64_t* __restrict__ bra_dims,
+                                    int32_t* __restrict__ used, unsigned long long* __restrict__ counters) {
+  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= p.n_pairs) return;
+  if (i == 0) prefix[p.has[p.n_pairs]] = p.jobs[p.n_pairs];
+  if (rep[i] < 0) return;
+  int16_t fb[2 * kMaxClusters];
+  int64_t dims[kMaxClusters];
+  open_target(p, i, fb, dims);
+  const int64_t sk = i / p.n_trans;
+  const int tr = int(i - sk * p.n_trans);
+  const int16_t* fk = p.sec_fock + sk * 2 * p.N;
+  const int32_t bs = int32_t(id[rep[i]]);
+  if (rep[i] == i) {
+    int64_t stride = 1;
+    for (int c = 0; c < p.N; ++c) {
+      bra_fock[(int64_t(bs) * p.N + c) * 2] = fb[2 * c];
+      bra_fock[(int64_t(bs) * p.N + c) * 2 + 1] = fb[2 * c + 1];
+      strides[int64_t(bs) * p.N + c] = stride;
+      bra_dims[int64_t(bs) * p.N + c] = dims[c];
+      stride = min(stride * dims[c], int64_t(1) << kKeyIdxBits);
+    }
+    if (stride >= (int64_t(1) << kKeyIdxBits)) atomicMax(counters + 10, 1ull);
+  }
+  if (p.has[i] == p.has[i + 1]) return;
+  const int64_t it = p.has[i];
+  prefix[it] = p.jobs[i];
+  int64_t at = p.ot[i];
+  items[it] = OpenItem{p.sec_start[sk], p.sec_count[sk], int32_t(at), int32_t(p.ot[i + 1] - at)};
+  const int nmax1 = p.tt.nmax1;
+  auto block_of = [&](int c, int op) {
+    return p.tt.blk[dense_block_index(nmax1, c, op, fb[2 * c], fb[2 * c + 1], fk[2 * c], fk[2 * c + 1])];
+  };
+  unsigned long long flops = 0, d_max = 1, reg = 0, shared = 0;
+  for (int q = p.first_of_tr[tr]; q < p.first_of_tr[tr + 1]; ++q) {
+    const int t = p.tr_terms[q];
+    const int32_t* r = p.tt.trm + int64_t(t) * kTrmCols;
+    OpenTerm o{};
+    int64_t fma;
+    if (r[0] > p.nbody || !term_sector_of(p.tt, t, fb, fk, o.ts, &fma)) continue;
+    const TermDress& dr = p.tt.dress[t];
+    const int cw = r[2 + (dr.pos < 0 ? 0 : dr.pos)];
+    o.wmax_off = p.wmax_index[(int64_t(t) * nmax1 + fb[2 * cw]) * nmax1 + fb[2 * cw + 1]];
+    o.bsec = bs;
+    o.n_act = int8_t(1 + o.ts.nrem);
+    o.c_act[0] = int8_t(cw);
+    o.mb_act[0] = int16_t(o.ts.w_mb);
+    int64_t cnt = o.ts.w_mb;
+    for (int a = 0; a < o.ts.nrem; ++a) {
+      o.gmax_off[a] = p.gmax_off[block_of(o.ts.cr[a], r[6 + dr.rem_pos[a]])];
+      o.c_act[1 + a] = o.ts.cr[a];
+      o.mb_act[1 + a] = int16_t(o.ts.g_mb[a]);
+      cnt *= o.ts.g_mb[a];
+      if (a > 0) d_max = max(d_max, (unsigned long long)o.ts.g_dim[a]);
+    }
+    if (cnt >= (int64_t(1) << 31)) atomicMax(counters + 10, 2ull);
+    o.out_count = int32_t(cnt);
+    reg = max(reg, (unsigned long long)expand_tiles(o.ts.nrem, o.ts.rest_len, o.ts.g_dim, o.mb_act, false).bytes);
+    shared = max(shared, (unsigned long long)expand_tiles(o.ts.nrem, o.ts.rest_len, o.ts.g_dim, o.mb_act, true).bytes);
+    // the reference's GEMM flops of this (ket, term) job (contract_matvec_thread,
+    // src/tpsci_matvec_thread.jl:279-818, no prescreen): bra dims M and orbital index
+    // lengths n in term order
+    int64_t M[4] = {1, 1, 1, 1}, n[4] = {1, 1, 1, 1};
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+      if (a < r[0]) {
+        const int bl = block_of(r[2 + a], r[6 + a]);
+        M[a] = p.tt.blocks[bl].mb;
+        n[a] = r[22 + a];
+        used[bl] = 1;
+      }
+    int64_t f = 0;
+    if (r[0] == 2) f = n[0] * n[1] * M[0] + n[1] * M[0] * M[1];
+    if (r[0] == 3) f = M[2] * (n[0] * n[1] * n[2] + n[0] * n[1] * M[1] + n[0] * M[0] * M[1]);
+    if (r[0] == 4)
+      f = M[3] * (n[0] * n[1] * n[2] * n[3] + M[2] * (n[0] * n[1] * n[2] + n[0] * n[1] * M[1] + n[0] * M[0] * M[1]));
+    flops += (unsigned long long)(2 * f * p.sec_count[sk]);
+    ots[at++] = o;
+  }
+  if (flops) atomicAdd(counters + 9, flops);
+  auto raise = [&](int k, unsigned long long v) {  // a stale read only costs an atomic
+    if (*reinterpret_cast<volatile unsigned long long*>(counters + k) < v) atomicMax(counters + k, v);
+  };
+  raise(11, d_max);
+  raise(12, reg);
+  raise(13, shared);
+}
+
+__global__ void open_bytes_kernel(int64_t n_blocks, const int32_t* __restrict__ used, const BlockInfo* __restrict__ blocks,
+                                  unsigned long long* __restrict__ counters) {
+  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i < n_blocks && used[i])
+    atomicAdd(counters + 14, (unsigned long long)(int64_t(blocks[i].nidx) * blocks[i].mb * blocks[i].mk * 8));
 }
 
 __global__ void pack_rows_kernel(const double* __restrict__ c, double* __restrict__ out, int64_t n, int R) {
@@ -570,16 +833,6 @@ __global__ void pack_rows_kernel(const double* __restrict__ c, double* __restric
   int64_t row = i / R;
   int r = int(i - row * R);
   out[i] = c[row + n * r];
-}
-
-inline bool fock_key(const int16_t* f, int N, uint64_t* key) {
-  uint64_t k = 0;
-  for (int i = 0; i < 2 * N; ++i) {
-    if (f[i] < 0 || f[i] > 15) return false;
-    k |= uint64_t(f[i]) << (4 * i);
-  }
-  *key = k;
-  return true;
 }
 
 }  // namespace
@@ -616,152 +869,111 @@ int fcg_sigma_open(fcg_ctx* ctx, int R, const double* c, double thresh, int nbod
   }
   *n_out = 0;
   const int N = ctx->N;
-  const int nmax1 = ctx->nmax + 1;
   const Plan& P = ctx->plan;
-  // ---- host plan: bra sectors and open term records per (ket sector, transfer) -------
-  ProblemInfo pi;
-  pi.N = N;
-  pi.norb = ctx->norb;
-  pi.nmax = ctx->nmax;
-  pi.trm = &ctx->trm;
-  pi.n_terms = ctx->n_terms;
-  pi.trans = &ctx->trans;
-  pi.n_trans = ctx->n_trans;
-  pi.blk_index = &ctx->h_blk_index;
-  pi.blocks = &ctx->h_blocks;
-  pi.dress = &ctx->dress;
-  pi.dressing = &ctx->open_dressing;
-  std::vector<std::vector<int>> terms_of(ctx->n_trans);
-  for (int t = 0; t < ctx->n_terms; ++t) terms_of[ctx->trm[int64_t(t) * kTrmCols + 1]].push_back(t);
-  std::unordered_map<uint64_t, int32_t> bsec_of;
-  ctx->open_bra_fock.clear();
-  ctx->open_strides.clear();
-  ctx->open_dims.clear();
-  std::vector<OpenTerm> ots;
-  std::vector<OpenItem> items;
-  std::vector<int16_t> fb(2 * N);
-  int64_t flops_ref = 0;
-  std::unordered_set<int32_t> tdm_used;  // TDM blocks the jobs read
-  for (size_t sk = 0; sk < P.sec_start.size(); ++sk) {
-    const int16_t* fk = &P.sec_fock[sk * 2 * N];
-    for (int tr = 0; tr < ctx->n_trans; ++tr) {
-      if (terms_of[tr].empty()) continue;
-      bool ok = true;
-      for (int i = 0; i < 2 * N; ++i) {
-        fb[i] = int16_t(fk[i] + ctx->trans[size_t(tr) * 2 * N + i]);
-        if (fb[i] < 0 || fb[i] > ctx->norb[i / 2]) ok = false;
-      }
-      if (!ok) continue;
-      // every cluster must have a local basis in its bra sector (:39-46)
-      int64_t dims[kMaxClusters];
-      for (int ci = 0; ci < N && ok; ++ci) {
-        int bl = ctx->h_blk_index[dense_block_index(nmax1, ci, kOpH, fb[2 * ci], fb[2 * ci + 1], fb[2 * ci],
-                                                    fb[2 * ci + 1])];
-        if (bl < 0)
-          ok = false;
-        else
-          dims[ci] = ctx->h_blocks[bl].mb;
-      }
-      if (!ok) continue;
-      uint64_t key;
-      fock_key(fb.data(), N, &key);
-      int32_t bs;
-      auto it = bsec_of.find(key);
-      if (it == bsec_of.end()) {
-        bs = int32_t(ctx->open_bra_fock.size() / (2 * N));
-        FCG_REQUIRE(bs < (1 << 23), FCG_ELIMIT, "too many bra sectors for the open sigma key");
-        bsec_of[key] = bs;
-        ctx->open_bra_fock.insert(ctx->open_bra_fock.end(), fb.begin(), fb.end());
-        int64_t stride = 1;
-        for (int ci = 0; ci < N; ++ci) {
-          ctx->open_strides.push_back(stride);
-          ctx->open_dims.push_back(dims[ci]);
-          stride *= dims[ci];
-        }
-        FCG_REQUIRE(stride < (int64_t(1) << kKeyIdxBits), FCG_ELIMIT, "bra sector product space exceeds 2^40");
-      } else {
-        bs = it->second;
-      }
-      const int32_t ot_off = int32_t(ots.size());
-      for (int t : terms_of[tr]) {
-        const int32_t* r = &ctx->trm[int64_t(t) * kTrmCols];
-        if (r[0] > nbody) continue;
-        OpenTerm o{};
-        if (!make_term_sector(pi, t, fb.data(), fk, o.ts)) continue;
-        const int pos = ctx->dress[t].pos < 0 ? 0 : ctx->dress[t].pos;
-        const int cw = r[2 + pos];
-        o.wmax_off = ctx->wmax_index[(int64_t(t) * nmax1 + fb[2 * cw]) * nmax1 + fb[2 * cw + 1]];
-        o.bsec = bs;
-        o.n_act = int8_t(1 + o.ts.nrem);
-        o.c_act[0] = int8_t(cw);
-        o.mb_act[0] = int16_t(o.ts.w_mb);
-        int64_t cnt = o.ts.w_mb;
-        for (int q = 0; q < o.ts.nrem; ++q) {
-          const int cq = o.ts.cr[q];
-          const int op = r[6 + ctx->dress[t].rem_pos[q]];
-          const int bl = ctx->h_blk_index[dense_block_index(nmax1, cq, op, fb[2 * cq], fb[2 * cq + 1], fk[2 * cq],
-                                                            fk[2 * cq + 1])];
-          o.gmax_off[q] = ctx->gmax_off[bl];
-          o.c_act[1 + q] = int8_t(cq);
-          o.mb_act[1 + q] = int16_t(o.ts.g_mb[q]);
-          cnt *= o.ts.g_mb[q];
-        }
-        FCG_REQUIRE(cnt < (int64_t(1) << 31), FCG_ELIMIT, "bra tuples of one term exceed 2^31");
-        o.out_count = int32_t(cnt);
-        // the reference's GEMM flops of this (ket, term) job (contract_matvec_thread,
-        // src/tpsci_matvec_thread.jl:279-818, no prescreen): bra dims M and orbital index
-        // lengths n in term order
-        {
-          const int nbd = r[0];
-          int64_t M[4] = {1, 1, 1, 1}, nn[4] = {1, 1, 1, 1};
-          for (int o2 = 0; o2 < nbd; ++o2) {
-            const int cq = r[2 + o2];
-            const int bl = ctx->h_blk_index[dense_block_index(nmax1, cq, r[6 + o2], fb[2 * cq], fb[2 * cq + 1],
-                                                              fk[2 * cq], fk[2 * cq + 1])];
-            M[o2] = ctx->h_blocks[bl].mb;
-            nn[o2] = r[22 + o2];
-            tdm_used.insert(bl);
-          }
-          int64_t f = 0;
-          if (nbd == 2) f = nn[0] * nn[1] * M[0] + nn[1] * M[0] * M[1];
-          if (nbd == 3) f = M[2] * (nn[0] * nn[1] * nn[2] + nn[0] * nn[1] * M[1] + nn[0] * M[0] * M[1]);
-          if (nbd == 4)
-            f = M[3] * (nn[0] * nn[1] * nn[2] * nn[3] +
-                        M[2] * (nn[0] * nn[1] * nn[2] + nn[0] * nn[1] * M[1] + nn[0] * M[0] * M[1]));
-          flops_ref += 2 * f * int64_t(P.sec_count[sk]);
-        }
-        ots.push_back(o);
-      }
-      const int32_t nt = int32_t(ots.size()) - ot_off;
-      if (nt > 0) items.push_back(OpenItem{int32_t(P.sec_start[sk]), int32_t(P.sec_count[sk]), ot_off, nt});
-    }
+  cudaStream_t s = ctx->stream;
+  auto& O = ctx->oplan;
+  constexpr int kT = 256;
+  auto grid_of = [](int64_t n) { return unsigned(std::max<int64_t>((n + kT - 1) / kT, 1)); };
+  // ---- plan: bra sectors and open term records per (ket sector, transfer) -----------------
+  const int64_t n_sec = int64_t(P.sec_start.size()), n_pairs = n_sec * ctx->n_trans;
+  int64_t cap_tab = 64;
+  while (cap_tab < 2 * n_pairs) cap_tab <<= 1;
+  std::vector<int32_t> rows(size_t(2 * n_sec));  // first rows, then row counts
+  for (int64_t i = 0; i < n_sec; ++i) {
+    rows[size_t(i)] = int32_t(P.sec_start[size_t(i)]);
+    rows[size_t(n_sec + i)] = int32_t(P.sec_count[size_t(i)]);
   }
+  FCG_CUDA(O.d_rows.upload(rows.data(), rows.size(), s));
+  FCG_CUDA(O.d_key.alloc(size_t(n_pairs)));
+  // table, ot, has, jobs, slot, rep, flag, scratch of the scans
+  const int64_t n1 = n_pairs + 1, scr = dprim::scan_scratch(n1) + 1;
+  FCG_CUDA(O.d_nt.alloc(size_t(n1)));
+  FCG_CUDA(O.d_i64.alloc(size_t(cap_tab + 6 * n1 + scr)));
+  FCG_CUDA(O.d_used.alloc(ctx->h_blocks.size()));
+  FCG_CUDA(ctx->d_counters.alloc(kCounters));
+  FCG_CUDA(cudaMemsetAsync(ctx->d_counters.p, 0, kCounters * sizeof(unsigned long long), s));
+  FCG_CUDA(cudaMemsetAsync(O.d_used.p, 0, ctx->h_blocks.size() * sizeof(int32_t), s));
+  OpenPlan op{};
+  op.tt = TermTables{O.d_trm.p, O.d_dress.p, O.d_w_index.p, O.d_w_mb.p, O.d_rep.p, ctx->d_blk_index.p, ctx->d_blocks.p,
+                     ctx->nmax + 1};
+  op.sec_fock = ctx->d_sec_fock.p;
+  op.sec_start = O.d_rows.p;
+  op.sec_count = O.d_rows.p + n_sec;
+  op.trans = O.d_trans.p;
+  op.first_of_tr = O.d_first_of_tr.p;
+  op.tr_terms = O.d_tr_terms.p;
+  op.norb = ctx->d_norb.p;
+  op.wmax_index = O.d_wmax_index.p;
+  op.gmax_off = O.d_gmax_off.p;
+  op.n_pairs = n_pairs;
+  op.n_trans = ctx->n_trans;
+  op.N = N;
+  op.nbody = nbody;
+  op.key = O.d_key.p;
+  op.nt = O.d_nt.p;
+  auto* table = reinterpret_cast<unsigned long long*>(O.d_i64.p);
+  op.ot = O.d_i64.p + cap_tab;
+  op.has = op.ot + n1;
+  op.jobs = op.has + n1;
+  int64_t *slot = op.jobs + n1, *rep = slot + n1, *flag = rep + n1, *scratch = flag + n1;
+  FCG_CUDA(cudaMemsetAsync(table, 0xFF, size_t(cap_tab) * sizeof(int64_t), s));
+  open_count_kernel<<<grid_of(n1), kT, 0, s>>>(op);
+  FCG_CUDA(cudaGetLastError());
+  open_sectors_kernel<<<grid_of(n_pairs), kT, 0, s>>>(op, table, cap_tab - 1, slot);
+  FCG_CUDA(cudaGetLastError());
+  open_first_kernel<<<grid_of(n1), kT, 0, s>>>(op, table, slot, rep, flag);
+  FCG_CUDA(cudaGetLastError());
+  for (int64_t* a : {flag, op.ot, op.has, op.jobs}) FCG_CUDA(dprim::exclusive_scan<int64_t>(a, n1, scratch, s));
+  open_sizes_kernel<<<1, 1, 0, s>>>(n_pairs, flag, op.ot, op.has, op.jobs, ctx->d_counters.p);
+  FCG_CUDA(cudaGetLastError());
+  unsigned long long cnt[kCounters];
+  FCG_CUDA(cudaMemcpyAsync(cnt, ctx->d_counters.p, sizeof(cnt), cudaMemcpyDeviceToHost, s));
+  FCG_CUDA(cudaStreamSynchronize(s));
+  const int64_t n_bra = int64_t(cnt[5]), n_ots = int64_t(cnt[6]), n_items = int64_t(cnt[7]), n_jobs = int64_t(cnt[8]);
+  FCG_REQUIRE(n_bra < (1 << 23), FCG_ELIMIT, "too many bra sectors for the open sigma key");
+  FCG_REQUIRE(n_ots < (int64_t(1) << 31), FCG_ELIMIT, "too many term records for the open sigma");
   ctx->open_R = R;
   ctx->open_rows = 0;
-  if (items.empty()) return FCG_OK;
-  std::vector<int64_t> prefix(items.size() + 1, 0);
-  for (size_t i = 0; i < items.size(); ++i) prefix[i + 1] = prefix[i] + int64_t(items[i].nrow) * items[i].nt;
-  const int64_t n_jobs = prefix.back();
-  // ---- device ---------------------------------------------------------------------------
-  cudaStream_t s = ctx->stream;
+  FCG_CUDA(ctx->d_oterms.alloc(size_t(n_ots)));
+  FCG_CUDA(ctx->d_oitems.alloc(size_t(n_items)));
+  FCG_CUDA(ctx->d_oprefix.alloc(size_t(n_items + 1)));
+  FCG_CUDA(ctx->d_ostrides.alloc(size_t(n_bra * N)));
+  FCG_CUDA(O.d_bra_fock.alloc(size_t(n_bra * N * 2)));
+  FCG_CUDA(O.d_bra_dims.alloc(size_t(n_bra * N)));
+  open_records_kernel<<<grid_of(n_pairs), kT, 0, s>>>(op, rep, flag, ctx->d_oterms.p, ctx->d_oitems.p, ctx->d_oprefix.p,
+                                                      O.d_bra_fock.p, ctx->d_ostrides.p, O.d_bra_dims.p, O.d_used.p,
+                                                      ctx->d_counters.p);
+  FCG_CUDA(cudaGetLastError());
+  open_bytes_kernel<<<grid_of(int64_t(ctx->h_blocks.size())), kT, 0, s>>>(int64_t(ctx->h_blocks.size()), O.d_used.p,
+                                                                         ctx->d_blocks.p, ctx->d_counters.p);
+  FCG_CUDA(cudaGetLastError());
+  ctx->open_bra_fock.resize(size_t(n_bra * N * 2));
+  ctx->open_dims.resize(size_t(n_bra * N));
+  if (n_bra > 0) {
+    FCG_CUDA(cudaMemcpyAsync(ctx->open_bra_fock.data(), O.d_bra_fock.p, sizeof(int16_t) * size_t(n_bra * N * 2),
+                             cudaMemcpyDeviceToHost, s));
+    FCG_CUDA(cudaMemcpyAsync(ctx->open_dims.data(), O.d_bra_dims.p, sizeof(int64_t) * size_t(n_bra * N),
+                             cudaMemcpyDeviceToHost, s));
+  }
   const int64_t n = ctx->n_cfg;
-  FCG_CUDA(ctx->d_oterms.upload(ots.data(), ots.size(), s));
-  FCG_CUDA(ctx->d_oitems.upload(items.data(), items.size(), s));
-  FCG_CUDA(ctx->d_oprefix.upload(prefix.data(), prefix.size(), s));
-  FCG_CUDA(ctx->d_ostrides.upload(ctx->open_strides.data(), ctx->open_strides.size(), s));
+  if (n_items == 0) {  // no term reaches a sector with a basis
+    FCG_CUDA(cudaMemcpyAsync(cnt, ctx->d_counters.p, sizeof(cnt), cudaMemcpyDeviceToHost, s));
+    FCG_CUDA(cudaStreamSynchronize(s));
+    FCG_REQUIRE(cnt[10] == 0, FCG_ELIMIT, "bra sector product space exceeds 2^40");
+    return FCG_OK;
+  }
+  // ---- device ---------------------------------------------------------------------------
   FCG_CUDA(ctx->d_in64.alloc(size_t(n) * R));
   FCG_CUDA(ctx->d_c64.alloc(size_t(n) * R));
   FCG_CUDA(cudaMemcpyAsync(ctx->d_in64.p, c, sizeof(double) * n * R, cudaMemcpyHostToDevice, s));
   pack_rows_kernel<<<unsigned((n * R + 255) / 256), 256, 0, s>>>(ctx->d_in64.p, ctx->d_c64.p, n, R);
   FCG_CUDA(cudaGetLastError());
-  FCG_CUDA(ctx->d_counters.alloc(5));
-  FCG_CUDA(cudaMemsetAsync(ctx->d_counters.p, 0, 4 * sizeof(unsigned long long), s));
   FCG_CUDA(ctx->d_ojobs.alloc(size_t(n_jobs)));
   OpenParams p{};
   p.ot = ctx->d_oterms.p;
   p.items = ctx->d_oitems.p;
   p.prefix = ctx->d_oprefix.p;
-  p.n_items = int64_t(items.size());
+  p.n_items = n_items;
   p.n_jobs = n_jobs;
   p.cfg = ctx->d_cfg.p;
   p.c = ctx->d_c64.p;
@@ -773,22 +985,20 @@ int fcg_sigma_open(fcg_ctx* ctx, int R, const double* c, double thresh, int nbod
   screen_kernel<<<unsigned((n_jobs + 255) / 256), 256, 0, s>>>(p, ctx->d_wmax.p, ctx->d_gmax.p, ctx->d_ojobs.p,
                                                               ctx->d_counters.p);
   FCG_CUDA(cudaGetLastError());
-  unsigned long long cnt[4];
   FCG_CUDA(cudaMemcpyAsync(cnt, ctx->d_counters.p, sizeof(cnt), cudaMemcpyDeviceToHost, s));
   FCG_CUDA(cudaStreamSynchronize(s));
+  FCG_REQUIRE(cnt[10] == 0, FCG_ELIMIT, cnt[10] == 1 ? "bra sector product space exceeds 2^40"
+                                                        : "bra tuples of one term exceed 2^31");
   const int64_t n_kept = int64_t(cnt[0]);
   const int64_t n_elem = int64_t(cnt[1]);
-  int launches = 2;
+  const int64_t flops_ref = int64_t(cnt[9]), tdm_bytes = int64_t(cnt[14]);
+  int launches = 8;
   if (n_kept > 0) {
     // a warp's slice: the largest job tiles, up to kExpSlice; as many warps to a CTA as fit.
     // The register sums serve index lengths up to kExpMaxD (the second and third remaining
     // clusters of the longest term), the shared-memory sums anything longer.
-    int d_max = 1, slice = 16;
-    for (const OpenTerm& o : ots)
-      for (int r = 1; r < o.ts.nrem; ++r) d_max = std::max<int>(d_max, o.ts.g_dim[r]);
-    for (const OpenTerm& o : ots)
-      slice = std::max(slice, expand_tiles(o.ts.nrem, o.ts.rest_len, o.ts.g_dim, o.mb_act, d_max > kExpMaxD).bytes);
-    slice = std::min(slice, kExpSlice);
+    const int d_max = int(cnt[11]);
+    const int slice = std::min(kExpSlice, std::max(16, int(d_max > kExpMaxD ? cnt[13] : cnt[12])));
     const int warps = std::min(kExpWarps, kExpCtaBytes / slice), threads = 32 * warps;
     const size_t smem = size_t(warps) * size_t(slice);
     auto kernel = d_max <= 3 ? expand_jobs_kernel<3>
@@ -803,11 +1013,19 @@ int fcg_sigma_open(fcg_ctx* ctx, int R, const double* c, double thresh, int nbod
     // table: twice the contributions, power of two, at least 4096 slots; doubled on overflow
     unsigned long long cap = 4096;
     while (cap < 2ull * (unsigned long long)n_elem && cap < (1ull << 28)) cap <<= 1;
+    size_t keys_after = 0, vals_after = 0;
     for (int attempt = 0;; ++attempt) {
+      // the table is empty up to clean_keys / clean_vals: every call empties the slots it used
+      if (cap > ctx->d_hkeys.n) O.clean_keys = 0;
+      if (cap * R > ctx->d_hvals.n) O.clean_vals = 0;
       FCG_CUDA(ctx->d_hkeys.alloc(cap));
       FCG_CUDA(ctx->d_hvals.alloc(cap * R));
-      FCG_CUDA(cudaMemsetAsync(ctx->d_hkeys.p, 0xFF, cap * sizeof(unsigned long long), s));
-      FCG_CUDA(cudaMemsetAsync(ctx->d_hvals.p, 0, cap * R * sizeof(double), s));
+      if (O.clean_keys < cap)
+        FCG_CUDA(cudaMemsetAsync(ctx->d_hkeys.p + O.clean_keys, 0xFF, (cap - O.clean_keys) * sizeof(unsigned long long), s));
+      if (O.clean_vals < cap * R)
+        FCG_CUDA(cudaMemsetAsync(ctx->d_hvals.p + O.clean_vals, 0, (cap * R - O.clean_vals) * sizeof(double), s));
+      const size_t clean_keys = std::max<size_t>(O.clean_keys, cap), clean_vals = std::max<size_t>(O.clean_vals, cap * R);
+      O.clean_keys = O.clean_vals = 0;  // until this call's slots are emptied
       FCG_CUDA(cudaMemsetAsync(ctx->d_counters.p + 2, 0, 3 * sizeof(unsigned long long), s));
       FCG_CUDA(cudaEventRecord(ctx->ev2, s));
       kernel<<<unsigned(grid), threads, smem, s>>>(
@@ -818,19 +1036,26 @@ int fcg_sigma_open(fcg_ctx* ctx, int R, const double* c, double thresh, int nbod
       FCG_CUDA(cudaMemcpyAsync(cnt, ctx->d_counters.p, sizeof(cnt), cudaMemcpyDeviceToHost, s));
       FCG_CUDA(cudaStreamSynchronize(s));
       launches += 2;
-      if (cnt[2] == 0) break;
+      if (cnt[2] == 0) {
+        keys_after = clean_keys;
+        vals_after = clean_vals;
+        break;
+      }
       FCG_REQUIRE(attempt < 3 && cap < (1ull << 31), FCG_ENOMEM, "open sigma hash table overflow");
       cap <<= 1;
     }
     FCG_CUDA(ctx->d_okeys.alloc(cap));
     FCG_CUDA(ctx->d_ovals.alloc(cap * R));
-    compact_kernel<<<unsigned((cap + 255) / 256), 256, 0, s>>>(ctx->d_hkeys.p, ctx->d_hvals.p, cap, R,
-                                                               ctx->d_okeys.p, ctx->d_ovals.p, ctx->d_counters.p);
+    compact_kernel<<<unsigned(cap / kCompactSlots), kCompactThreads, 0, s>>>(ctx->d_hkeys.p, ctx->d_hvals.p, R,
+                                                                           ctx->d_okeys.p, ctx->d_ovals.p,
+                                                                           ctx->d_counters.p);
     FCG_CUDA(cudaGetLastError());
     FCG_CUDA(cudaEventRecord(ctx->ev1, s));
     FCG_CUDA(cudaMemcpyAsync(cnt, ctx->d_counters.p, sizeof(cnt), cudaMemcpyDeviceToHost, s));
     FCG_CUDA(cudaStreamSynchronize(s));
     launches += 1;
+    O.clean_keys = keys_after;
+    O.clean_vals = vals_after;
     const int64_t n_rows = int64_t(cnt[3]);
     FCG_CUDA(ctx->open_keys.alloc(size_t(n_rows)));
     FCG_CUDA(ctx->open_vals.alloc(size_t(n_rows) * R));
@@ -847,11 +1072,6 @@ int fcg_sigma_open(fcg_ctx* ctx, int R, const double* c, double thresh, int nbod
     ctx->stats.open_expand_ms = ms;
   }
   // compulsory bytes: the TDM blocks the jobs touch, C, and one key + row per output
-  int64_t tdm_bytes = 0;
-  for (int32_t bl : tdm_used) {
-    const BlockInfo& B = ctx->h_blocks[bl];
-    tdm_bytes += int64_t(B.nidx) * B.mb * B.mk * 8;
-  }
   ctx->stats.open_flops_reference = flops_ref;
   ctx->stats.open_bytes = tdm_bytes + 8 * n * R + ctx->open_rows * (6 * int64_t(N) + 8 * int64_t(R));
   ctx->stats.kernel_launches = launches;

@@ -66,11 +66,6 @@ TermTables term_tables(const ProblemInfo& pi) {
                     pi.blk_index->data(), pi.blocks->data(), pi.nmax + 1};
 }
 
-bool make_term_sector(const ProblemInfo& pi, int t, const int16_t* fb, const int16_t* fk, TermSector& ts) {
-  int64_t fma;
-  return term_sector_of(term_tables(pi), t, fb, fk, ts, &fma);
-}
-
 std::string term_lists(const ProblemInfo& pi, TermLists& L) {
   const std::vector<int32_t>& trm = *pi.trm;
   L = TermLists();
