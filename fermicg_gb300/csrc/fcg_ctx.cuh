@@ -215,6 +215,8 @@ struct fcg_ctx {
   DevBuf<double> dav_V, dav_AV, dav_X, dav_tmp, dav_hd, dav_part, dav_rn, dav_out, dav_up;
   DevBuf<unsigned> dav_counters;
   PinnedBuf<double> dav_h_out, dav_h_up;
+  PinnedBuf<unsigned long long> dav_flag;  // number of the last finished Gram product, of dav_seq queued
+  unsigned long long dav_seq = 0;
   // vectors
   DevBuf<double> d_in64, d_out64;  // column-major staging for host calls
   DevBuf<double> d_c64, d_s64;     // row-major fp64
