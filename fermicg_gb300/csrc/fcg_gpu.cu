@@ -289,7 +289,8 @@ struct LaneParams {
 };
 
 // R coefficients of one row of a row-major [n][R] array (RR > 0: R == RR, known at compile
-// time), with vector loads when exactly 2 or 4 roots; out[r] = 0 for r >= R
+// time), with vector loads when exactly 2 or 4 roots or a row is whole 16-byte pieces; out[r] = 0
+// for r >= R
 template <typename T, int RR, int RV>
 __device__ __forceinline__ void load_row(const T* __restrict__ p, int R, T* out) {
   if (RR == 4 && sizeof(T) == 4) {
@@ -306,14 +307,39 @@ __device__ __forceinline__ void load_row(const T* __restrict__ p, int R, T* out)
   } else if (RR == 2) {
     const double2 q = __ldg(reinterpret_cast<const double2*>(p));
     out[0] = T(q.x), out[1] = T(q.y);
+  } else if (RV >= 4 && (RR * sizeof(T)) % 16 == 0 && (R * sizeof(T)) % 16 == 0 &&
+             reinterpret_cast<uintptr_t>(p) % 16 == 0) {
+    constexpr int kV = 16 / int(sizeof(T));
+#pragma unroll
+    for (int r = 0; r < RV; r += kV)
+      if (r < R) {
+        if constexpr (sizeof(T) == 4) {
+          const float4 q = __ldg(reinterpret_cast<const float4*>(p + r));
+          out[r] = q.x, out[r + 1] = q.y, out[r + 2] = q.z, out[r + 3] = q.w;
+        } else {
+          const double2 q = __ldg(reinterpret_cast<const double2*>(p + r));
+          out[r] = q.x, out[r + 1] = q.y;
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < kV; ++i) out[r + i] = T(0);
+      }
   } else {
 #pragma unroll
     for (int r = 0; r < RV; ++r) out[r] = r < R ? __ldg(p + r) : T(0);
   }
 }
 
-// sig[row] += acc for R roots: one vector reduction for exactly four float roots, else
-// scalar atomics
+// acc += x * c.  Every root of the width costs float64 pipe, used or not (guards become predicates,
+// which cost the same): hence the widths.  50,021 rows of 24 orbitals, float64, 6 roots: direct 2471 us
+// at a width of 16, 1693 at 6; stored blocks 982 and 424.
+template <typename T, int RV>
+__device__ __forceinline__ void add_scaled(T* acc, T x, const T* c) {
+#pragma unroll
+  for (int r = 0; r < RV; ++r) acc[r] = fma(x, c[r], acc[r]);
+}
+
+// sig[row] += acc for R roots: vector reductions for fours of float roots, else scalar atomics
 template <typename T, int RR, int RV>
 __device__ __forceinline__ void add_row(T* __restrict__ sig, int b, const T* acc, int R) {
   T* dst = sig + int64_t(b) * R;
@@ -321,6 +347,13 @@ __device__ __forceinline__ void add_row(T* __restrict__ sig, int b, const T* acc
     asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(float(acc[0])), "f"(float(acc[1])),
                  "f"(float(acc[2])), "f"(float(acc[3]))
                  : "memory");
+  } else if (RV >= 4 && RR % 4 == 0 && sizeof(T) == 4 && R % 4 == 0 && reinterpret_cast<uintptr_t>(dst) % 16 == 0) {
+#pragma unroll
+    for (int r = 0; r < RV; r += 4)
+      if (r < R)
+        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + r), "f"(float(acc[r])),
+                     "f"(float(acc[r + 1])), "f"(float(acc[r + 2])), "f"(float(acc[r + 3]))
+                     : "memory");
   } else {
 #pragma unroll
     for (int r = 0; r < RV; ++r)
@@ -357,21 +390,20 @@ __device__ __forceinline__ void closed_lane_warp(const LaneParams& p, const T* _
       for (int t = 0; t < int(j.nt); ++t) me += dressed_element<T>(tsl[t], w, op, rb, rk);
       T c[RV];
       load_row<T, RR, RV>(cin + int64_t(k) * R, R, c);
-#pragma unroll
-      for (int r = 0; r < RV; ++r) acc[r] = fma(me, c[r], acc[r]);
+      add_scaled<T, RV>(acc, me, c);
     }
     add_row<T, RR, RV>(sig, j.b, acc, R);
   }
 }
 
 // MINB: resident CTAs per SM the register allocation is sized for (a tuning candidate)
-template <typename T, int RR, int MINB>
+template <typename T, int RR, int MINB, int RMAX = kMaxR>
 __global__ void __launch_bounds__(kSigmaThreads, MINB)
     closed_sigma_lane_kernel(LaneParams p, const T* __restrict__ w, const T* __restrict__ op,
                              const T* __restrict__ cin, T* __restrict__ sig) {
   const int64_t chunk = int64_t(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5);
   if (chunk >= p.n_chunks) return;
-  closed_lane_warp<T, RR>(p, w, op, cin, sig, chunk);
+  closed_lane_warp<T, RR, RMAX>(p, w, op, cin, sig, chunk);
 }
 
 // ---- block jobs --------------------------------------------------------------------------------
@@ -487,11 +519,11 @@ __device__ __forceinline__ T block_pair(const T* u, int da, int db, const T* __r
   return me;
 }
 
-template <typename T, int RR>
+template <typename T, int RR, int RMAX = kMaxR>
 __global__ void __launch_bounds__(32 * kBlockWarps)
     block_sigma_kernel(BlockParams p, const T* __restrict__ w, const T* __restrict__ op, const T* __restrict__ cin,
                        T* __restrict__ sig) {
-  constexpr int RV = RR > 0 ? RR : kMaxR;
+  constexpr int RV = RR > 0 ? RR : RMAX;
   __shared__ BlockSmem<T> smem[kBlockWarps];
   BlockSmem<T>& S = smem[threadIdx.x >> 5];
   const int R = RR > 0 ? RR : p.R;
@@ -642,8 +674,7 @@ __global__ void __launch_bounds__(32 * kBlockWarps)
                 if (tg == 2) me += block_pair<T>(u + du, da, db, ga[1] + oa, gb[1] + ob);
                 T c[RV];
                 load_row<T, RR, RV>(cin + int64_t(kk.x) * R, R, c);
-#pragma unroll
-                for (int r = 0; r < RV; ++r) acc[r] = fma(me, c[r], acc[r]);
+                add_scaled<T, RV>(acc, me, c);
               }
             __syncwarp();
           }
@@ -656,6 +687,7 @@ __global__ void __launch_bounds__(32 * kBlockWarps)
         const int src = lane + h * nb;
 #pragma unroll
         for (int r = 0; r < RV; ++r) {
+          if (RR == 0 && r >= R) break;
           const T v = __shfl_sync(0xffffffffu, acc[r], src & 31);
           if (sl + h < s) acc[r] += v;
         }
@@ -722,8 +754,7 @@ __device__ __forceinline__ void cached_lane_warp(const LaneParams& p, const T* _
         const T v = __ldg(hv + 32 * s);
         T c[RV];
         load_row<T, RR, RV>(cin + int64_t(__ldg(p.perm + j.kp + s)) * R, R, c);
-#pragma unroll
-        for (int r = 0; r < RV; ++r) acc[r] = fma(v, c[r], acc[r]);
+        add_scaled<T, RV>(acc, v, c);
       }
       add_row<T, RR, RV>(sig, j.b, acc, R);
     }
@@ -731,13 +762,13 @@ __device__ __forceinline__ void cached_lane_warp(const LaneParams& p, const T* _
   }
 }
 
-template <typename T, int RR>
+template <typename T, int RR, int RMAX = kMaxR>
 __global__ void __launch_bounds__(kSigmaThreads) cached_sigma_lane_kernel(LaneParams p, const T* __restrict__ hc,
                                                                           const T* __restrict__ cin,
                                                                           T* __restrict__ sig) {
   const int64_t chunk = int64_t(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5);
   if (chunk >= p.n_chunks) return;
-  cached_lane_warp<T, RR>(p, hc, cin, sig, chunk);
+  cached_lane_warp<T, RR, RMAX>(p, hc, cin, sig, chunk);
 }
 
 // Many independent problems in one launch: problem q owns CTAs [cta0, cta0 + ceil(its chunks
@@ -1550,13 +1581,21 @@ static int fine_chunks(fcg_ctx* ctx, bool direct) {
 template <typename T, int MINB>
 static void launch_lane(const LaneParams& p, int64_t grid, int R, const T* w, const T* op, const T* cin, T* sig,
                         cudaStream_t s) {
+  const auto run = [&](auto kernel) { kernel<<<unsigned(grid), kSigmaThreads, 0, s>>>(p, w, op, cin, sig); };
   switch (R) {
-    case 1: closed_sigma_lane_kernel<T, 1, MINB><<<unsigned(grid), kSigmaThreads, 0, s>>>(p, w, op, cin, sig); break;
-    case 2: closed_sigma_lane_kernel<T, 2, MINB><<<unsigned(grid), kSigmaThreads, 0, s>>>(p, w, op, cin, sig); break;
-    case 3: closed_sigma_lane_kernel<T, 3, MINB><<<unsigned(grid), kSigmaThreads, 0, s>>>(p, w, op, cin, sig); break;
-    case 4: closed_sigma_lane_kernel<T, 4, MINB><<<unsigned(grid), kSigmaThreads, 0, s>>>(p, w, op, cin, sig); break;
-    default: closed_sigma_lane_kernel<T, 0, MINB><<<unsigned(grid), kSigmaThreads, 0, s>>>(p, w, op, cin, sig); break;
+    case 1: return run(closed_sigma_lane_kernel<T, 1, MINB>);
+    case 2: return run(closed_sigma_lane_kernel<T, 2, MINB>);
+    case 3: return run(closed_sigma_lane_kernel<T, 3, MINB>);
+    case 4: return run(closed_sigma_lane_kernel<T, 4, MINB>);
+    case 5: return run(closed_sigma_lane_kernel<T, 5, MINB>);
+    case 6: return run(closed_sigma_lane_kernel<T, 6, MINB>);
+    case 7: return run(closed_sigma_lane_kernel<T, 7, MINB>);
+    case 8: return run(closed_sigma_lane_kernel<T, 8, MINB>);
   }
+  if constexpr (sizeof(T) == 8) {
+    if (R <= 12) return run(closed_sigma_lane_kernel<T, 0, MINB, 12>);
+  }
+  run(closed_sigma_lane_kernel<T, 0, MINB>);
 }
 
 // one direct closed sigma's lane jobs with candidate c (all of them, or those of the items that do
@@ -1599,7 +1638,12 @@ static int launch_blocks(fcg_ctx* ctx, int R, const double* w, const double* op,
   auto kernel = R == 1   ? block_sigma_kernel<double, 1>
                 : R == 2 ? block_sigma_kernel<double, 2>
                 : R == 3 ? block_sigma_kernel<double, 3>
-                : R == 4 ? block_sigma_kernel<double, 4> : block_sigma_kernel<double, 0>;
+                : R == 4 ? block_sigma_kernel<double, 4>
+                : R == 5 ? block_sigma_kernel<double, 5>
+                : R == 6 ? block_sigma_kernel<double, 6>
+                : R == 7 ? block_sigma_kernel<double, 7>
+                : R == 8 ? block_sigma_kernel<double, 8>
+                : R <= 12 ? block_sigma_kernel<double, 0, 12> : block_sigma_kernel<double, 0>;
   int per_sm = 1, n_sm = 152;
   FCG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * kBlockWarps, 0));
   FCG_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, ctx->device));
@@ -1651,6 +1695,31 @@ static int tune_closed(fcg_ctx* ctx, int prec, int R, const T* w, const T* op, c
   return FCG_OK;
 }
 
+// Exact widths to 8 in float64.  In float the width of 8 with whole vector loads is as fast or faster
+// (stored blocks of 50,021 rows of 24 orbitals, 6 and 8 roots: 252 and 186 us, exact 267 and 226).
+template <typename T>
+static void launch_cached(const LaneParams& p, int64_t grid, int R, const T* hc, const T* cin, T* sig, cudaStream_t s) {
+  const auto run = [&](auto kernel) { kernel<<<unsigned(grid), kSigmaThreads, 0, s>>>(p, hc, cin, sig); };
+  switch (R) {
+    case 1: return run(cached_sigma_lane_kernel<T, 1>);
+    case 2: return run(cached_sigma_lane_kernel<T, 2>);
+    case 3: return run(cached_sigma_lane_kernel<T, 3>);
+    case 4: return run(cached_sigma_lane_kernel<T, 4>);
+  }
+  if constexpr (sizeof(T) == 8) {
+    switch (R) {
+      case 5: return run(cached_sigma_lane_kernel<T, 5>);
+      case 6: return run(cached_sigma_lane_kernel<T, 6>);
+      case 7: return run(cached_sigma_lane_kernel<T, 7>);
+      case 8: return run(cached_sigma_lane_kernel<T, 8>);
+    }
+    if (R <= 12) return run(cached_sigma_lane_kernel<T, 0, 12>);
+  } else {
+    if (R <= 8) return run(cached_sigma_lane_kernel<T, 0, 8>);
+  }
+  run(cached_sigma_lane_kernel<T, 0>);
+}
+
 template <typename T>
 static int launch_closed(fcg_ctx* ctx, int R, const T* w, const T* op, const T* cin, T* sig, bool zero_sig = true,
                          bool timed = true) {
@@ -1672,13 +1741,7 @@ static int launch_closed(fcg_ctx* ctx, int R, const T* w, const T* op, const T* 
   if (timed) FCG_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));
   if (grid > 0 && ctx->have_hcache) {  // from the stored Hamiltonian blocks
     const T* hc = sizeof(T) == 4 ? reinterpret_cast<const T*>(ctx->d_hc32.p) : reinterpret_cast<const T*>(ctx->d_hc64.p);
-    switch (R) {
-      case 1: cached_sigma_lane_kernel<T, 1><<<unsigned(grid), kSigmaThreads, 0, ctx->stream>>>(p, hc, cin, sig); break;
-      case 2: cached_sigma_lane_kernel<T, 2><<<unsigned(grid), kSigmaThreads, 0, ctx->stream>>>(p, hc, cin, sig); break;
-      case 3: cached_sigma_lane_kernel<T, 3><<<unsigned(grid), kSigmaThreads, 0, ctx->stream>>>(p, hc, cin, sig); break;
-      case 4: cached_sigma_lane_kernel<T, 4><<<unsigned(grid), kSigmaThreads, 0, ctx->stream>>>(p, hc, cin, sig); break;
-      default: cached_sigma_lane_kernel<T, 0><<<unsigned(grid), kSigmaThreads, 0, ctx->stream>>>(p, hc, cin, sig); break;
-    }
+    launch_cached<T>(p, grid, R, hc, cin, sig, ctx->stream);
     FCG_CUDA(cudaGetLastError());
     launches = 1;
   } else if (grid > 0) {
@@ -1867,8 +1930,12 @@ static int grouped_impl(int n, fcg_ctx* const* ctxs, const int* R, const double*
   if (cta > 0) {
     int rmax = 0;
     for (int q = 0; q < n; ++q) rmax = std::max(rmax, R[q]);
-    if (rmax <= 4)
+    if (rmax <= 1)
+      closed_sigma_grouped_kernel<T, 1><<<unsigned(cta), kSigmaThreads, 0, ctx->stream>>>(dg, ctx->d_group_cta.p);
+    else if (rmax <= 4)
       closed_sigma_grouped_kernel<T, 4><<<unsigned(cta), kSigmaThreads, 0, ctx->stream>>>(dg, ctx->d_group_cta.p);
+    else if (rmax <= 8)
+      closed_sigma_grouped_kernel<T, 8><<<unsigned(cta), kSigmaThreads, 0, ctx->stream>>>(dg, ctx->d_group_cta.p);
     else
       closed_sigma_grouped_kernel<T, kMaxR><<<unsigned(cta), kSigmaThreads, 0, ctx->stream>>>(dg, ctx->d_group_cta.p);
     FCG_CUDA(cudaGetLastError());
@@ -1877,8 +1944,12 @@ static int grouped_impl(int n, fcg_ctx* const* ctxs, const int* R, const double*
     int rmax = 0;
     for (int q = 0; q < n; ++q) rmax = std::max(rmax, R[q]);
     const int32_t* tab = ctx->d_group_cta.p + cta;
-    if (rmax <= 4)
+    if (rmax <= 1)
+      cached_sigma_grouped_kernel<T, 1><<<unsigned(cta_hc), kSigmaThreads, 0, ctx->stream>>>(dg, tab);
+    else if (rmax <= 4)
       cached_sigma_grouped_kernel<T, 4><<<unsigned(cta_hc), kSigmaThreads, 0, ctx->stream>>>(dg, tab);
+    else if (rmax <= 8)
+      cached_sigma_grouped_kernel<T, 8><<<unsigned(cta_hc), kSigmaThreads, 0, ctx->stream>>>(dg, tab);
     else
       cached_sigma_grouped_kernel<T, kMaxR><<<unsigned(cta_hc), kSigmaThreads, 0, ctx->stream>>>(dg, tab);
     FCG_CUDA(cudaGetLastError());
