@@ -219,8 +219,8 @@ struct fcg_ctx {
   unsigned long long dav_seq = 0;
   // vectors
   DevBuf<double> d_in64, d_out64;  // column-major staging for host calls
-  DevBuf<double> d_c64, d_s64;     // row-major fp64
-  DevBuf<float> d_c32, d_s32;      // row-major fp32
+  DevBuf<double> d_c64, d_s64;     // row-major fp64; d_s64 the sigma of either precision
+  DevBuf<float> d_c32;             // row-major fp32
   DevBuf<double> d_hd;
   // screening maxima: Gmax[i, k] = max_b |G[i, b, k]| per TDM block, Wmax likewise per W block
   std::vector<int64_t> gmax_off;   // per block

@@ -339,25 +339,43 @@ __device__ __forceinline__ void add_scaled(T* acc, T x, const T* c) {
   for (int r = 0; r < RV; ++r) acc[r] = fma(x, c[r], acc[r]);
 }
 
-// sig[row] += acc for R roots: vector reductions for fours of float roots, else scalar atomics
+// sig[row] += acc for R roots.  Sigma is float64 in both precisions: a row takes hundreds of jobs'
+// sums, whose roundings in float are larger than the products' (50,021 rows of 24 orbitals, 4 roots,
+// float: error 1.9e-7 and 510 us with float additions of whole rows, 3.3e-8 and 520 us so; from stored
+// blocks 1.4e-7 and 178 us, 3.0e-8 and 209 us, 237 us without the transposition below).
+template <typename T, int RV>
+__device__ __forceinline__ void add_row(double* __restrict__ sig, int b, const T* acc, int R) {
+  double* dst = sig + int64_t(b) * R;
+#pragma unroll
+  for (int r = 0; r < RV; ++r)
+    if (r < R) atomicAdd(dst + r, double(acc[r]));
+}
+
+// The same for the 32 lanes' rows (row < 0: none).  Fours of roots: four lanes add a row's four
+// together, a 32-byte sector at once, after a 4 x 4 transposition.
+template <typename T>
+__device__ __forceinline__ T pick4(const T* v, int i) {
+  const T a = i & 1 ? v[1] : v[0], b = i & 1 ? v[3] : v[2];
+  return i & 2 ? b : a;
+}
 template <typename T, int RR, int RV>
-__device__ __forceinline__ void add_row(T* __restrict__ sig, int b, const T* acc, int R) {
-  T* dst = sig + int64_t(b) * R;
-  if (RR == 4 && sizeof(T) == 4) {
-    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(float(acc[0])), "f"(float(acc[1])),
-                 "f"(float(acc[2])), "f"(float(acc[3]))
-                 : "memory");
-  } else if (RV >= 4 && RR % 4 == 0 && sizeof(T) == 4 && R % 4 == 0 && reinterpret_cast<uintptr_t>(dst) % 16 == 0) {
+__device__ __forceinline__ void add_rows(double* __restrict__ sig, int row, const T* acc, int R) {
+  if (RV % 4 == 0 && R % 4 == 0) {
+    const int lane = threadIdx.x & 31, i = lane & 3;
 #pragma unroll
-    for (int r = 0; r < RV; r += 4)
-      if (r < R)
-        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + r), "f"(float(acc[r])),
-                     "f"(float(acc[r + 1])), "f"(float(acc[r + 2])), "f"(float(acc[r + 3]))
-                     : "memory");
+    for (int q = 0; q + 4 <= RV; q += 4) {
+      if (q >= R) break;
+      T m[4];  // m[t]: root q + i of lane ^ t
+#pragma unroll
+      for (int t = 0; t < 4; ++t) m[t] = __shfl_xor_sync(0xffffffffu, pick4(acc + q, i ^ t), t);
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const int to = __shfl_sync(0xffffffffu, row, (lane & ~3) + t);
+        if (to >= 0) atomicAdd(sig + int64_t(R) * to + q + i, double(pick4(m, i ^ t)));
+      }
+    }
   } else {
-#pragma unroll
-    for (int r = 0; r < RV; ++r)
-      if (r < R) atomicAdd(dst + r, acc[r]);
+    if (row >= 0) add_row<T, RV>(sig, row, acc, R);
   }
 }
 
@@ -369,7 +387,7 @@ __device__ __forceinline__ void add_row(T* __restrict__ sig, int b, const T* acc
 template <typename T, int RR, int RMAX = kMaxR>
 __device__ __forceinline__ void closed_lane_warp(const LaneParams& p, const T* __restrict__ w,
                                                  const T* __restrict__ op, const T* __restrict__ cin,
-                                                 T* __restrict__ sig, int64_t chunk) {
+                                                 double* __restrict__ sig, int64_t chunk) {
   constexpr int RV = RR > 0 ? RR : RMAX;
   const int R = RR > 0 ? RR : p.R;
   const int lane = threadIdx.x & 31;
@@ -377,13 +395,13 @@ __device__ __forceinline__ void closed_lane_warp(const LaneParams& p, const T* _
   const uint4* cfg = reinterpret_cast<const uint4*>(p.cfg);
   for (int64_t wt = t_lo; wt < t_hi; ++wt) {
     const LaneJob j = p.jobs[wt * 32 + lane];
-    if (j.len == 0 || wt * 32 + lane >= p.n_jobs) continue;
-    const uint4 rb = __ldg(cfg + j.b);
+    const int len = wt * 32 + lane < p.n_jobs ? int(j.len) : 0;
+    const uint4 rb = len > 0 ? __ldg(cfg + j.b) : make_uint4(0, 0, 0, 0);
     const TermSector* tsl = p.ts + j.ts_off;
     T acc[RV];
 #pragma unroll
     for (int r = 0; r < RV; ++r) acc[r] = T(0);
-    for (int kk = 0; kk < int(j.len); ++kk) {
+    for (int kk = 0; kk < len; ++kk) {
       const int k = __ldg(p.perm + j.kp + kk);
       const uint4 rk = __ldg(cfg + k);
       T me = T(0);
@@ -392,7 +410,7 @@ __device__ __forceinline__ void closed_lane_warp(const LaneParams& p, const T* _
       load_row<T, RR, RV>(cin + int64_t(k) * R, R, c);
       add_scaled<T, RV>(acc, me, c);
     }
-    add_row<T, RR, RV>(sig, j.b, acc, R);
+    add_rows<T, RR, RV>(sig, len > 0 ? j.b : -1, acc, R);
   }
 }
 
@@ -400,7 +418,7 @@ __device__ __forceinline__ void closed_lane_warp(const LaneParams& p, const T* _
 template <typename T, int RR, int MINB, int RMAX = kMaxR>
 __global__ void __launch_bounds__(kSigmaThreads, MINB)
     closed_sigma_lane_kernel(LaneParams p, const T* __restrict__ w, const T* __restrict__ op,
-                             const T* __restrict__ cin, T* __restrict__ sig) {
+                             const T* __restrict__ cin, double* __restrict__ sig) {
   const int64_t chunk = int64_t(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5);
   if (chunk >= p.n_chunks) return;
   closed_lane_warp<T, RR, RMAX>(p, w, op, cin, sig, chunk);
@@ -522,7 +540,7 @@ __device__ __forceinline__ T block_pair(const T* u, int da, int db, const T* __r
 template <typename T, int RR, int RMAX = kMaxR>
 __global__ void __launch_bounds__(32 * kBlockWarps)
     block_sigma_kernel(BlockParams p, const T* __restrict__ w, const T* __restrict__ op, const T* __restrict__ cin,
-                       T* __restrict__ sig) {
+                       double* __restrict__ sig) {
   constexpr int RV = RR > 0 ? RR : RMAX;
   __shared__ BlockSmem<T> smem[kBlockWarps];
   BlockSmem<T>& S = smem[threadIdx.x >> 5];
@@ -694,7 +712,7 @@ __global__ void __launch_bounds__(32 * kBlockWarps)
         s = h;
       }
       const int row = __shfl_sync(0xffffffffu, brow, bl);
-      if (sl == 0) add_row<T, RR, RV>(sig, row, acc, R);
+      if (sl == 0) add_row<T, RV>(sig, row, acc, R);
     }
   }
 }
@@ -736,7 +754,7 @@ __global__ void __launch_bounds__(kSigmaThreads) hcache_lane_build_kernel(LanePa
 // per lane and ket in place of the term loop
 template <typename T, int RR, int RMAX = kMaxR>
 __device__ __forceinline__ void cached_lane_warp(const LaneParams& p, const T* __restrict__ hc,
-                                                 const T* __restrict__ cin, T* __restrict__ sig, int64_t chunk) {
+                                                 const T* __restrict__ cin, double* __restrict__ sig, int64_t chunk) {
   constexpr int RV = RR > 0 ? RR : RMAX;
   const int R = RR > 0 ? RR : p.R;
   const int lane = threadIdx.x & 31;
@@ -745,19 +763,17 @@ __device__ __forceinline__ void cached_lane_warp(const LaneParams& p, const T* _
   for (int64_t wt = t_lo; wt < t_hi; ++wt) {
     const LaneJob j = p.jobs[wt * 32 + lane];
     const int steps = task_len(j.len);
-    if (j.len > 0) {
-      const T* hv = hc + val + lane;
-      T acc[RV];
+    const T* hv = hc + val + lane;
+    T acc[RV];
 #pragma unroll
-      for (int r = 0; r < RV; ++r) acc[r] = T(0);
-      for (int s = 0; s < int(j.len); ++s) {
-        const T v = __ldg(hv + 32 * s);
-        T c[RV];
-        load_row<T, RR, RV>(cin + int64_t(__ldg(p.perm + j.kp + s)) * R, R, c);
-        add_scaled<T, RV>(acc, v, c);
-      }
-      add_row<T, RR, RV>(sig, j.b, acc, R);
+    for (int r = 0; r < RV; ++r) acc[r] = T(0);
+    for (int s = 0; s < int(j.len); ++s) {
+      const T v = __ldg(hv + 32 * s);
+      T c[RV];
+      load_row<T, RR, RV>(cin + int64_t(__ldg(p.perm + j.kp + s)) * R, R, c);
+      add_scaled<T, RV>(acc, v, c);
     }
+    add_rows<T, RR, RV>(sig, j.len > 0 ? j.b : -1, acc, R);
     val += 32 * int64_t(steps);
   }
 }
@@ -765,7 +781,7 @@ __device__ __forceinline__ void cached_lane_warp(const LaneParams& p, const T* _
 template <typename T, int RR, int RMAX = kMaxR>
 __global__ void __launch_bounds__(kSigmaThreads) cached_sigma_lane_kernel(LaneParams p, const T* __restrict__ hc,
                                                                           const T* __restrict__ cin,
-                                                                          T* __restrict__ sig) {
+                                                                          double* __restrict__ sig) {
   const int64_t chunk = int64_t(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5);
   if (chunk >= p.n_chunks) return;
   cached_lane_warp<T, RR, RMAX>(p, hc, cin, sig, chunk);
@@ -781,7 +797,7 @@ struct GroupEntry {
   const T* op;
   const T* hc;       // stored Hamiltonian blocks, or null
   T* cin;            // row-major [n_cfg][R] working copy of C
-  T* sig;            // row-major [n_cfg][R] sigma
+  double* sig;       // row-major [n_cfg][R] sigma
   const double* src; // caller's column-major C
   double* dst;       // caller's column-major sigma
   int64_t cta0;
@@ -818,7 +834,7 @@ __global__ void grouped_pack_kernel(const GroupEntry<T>* __restrict__ g) {
     const int64_t row = i / R;
     const int r = int(i - row * R);
     e.cin[i] = T(e.src[row + n * r]);
-    e.sig[i] = T(0);
+    e.sig[i] = 0.0;
   }
 }
 
@@ -830,28 +846,27 @@ __global__ void grouped_unpack_kernel(const GroupEntry<T>* __restrict__ g) {
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n * R; i += int64_t(gridDim.x) * blockDim.x) {
     const int64_t row = i % n;
     const int r = int(i / n);
-    e.dst[i] = double(e.sig[row * R + r]);
+    e.dst[i] = e.sig[row * R + r];
   }
 }
 
 template <typename T>
 __global__ void pack_in_kernel(const double* __restrict__ c, T* __restrict__ out, int64_t n, int R,
-                               T* __restrict__ zero) {
+                               double* __restrict__ zero) {
   int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n * R) return;
   int64_t row = i / R;
   int r = int(i - row * R);
   out[i] = T(c[row + n * r]);
-  if (zero) zero[i] = T(0);  // the sigma accumulator of the same shape, when given
+  if (zero) zero[i] = 0.0;  // the sigma accumulator of the same shape, when given
 }
 
-template <typename T>
-__global__ void unpack_out_kernel(const T* __restrict__ s, double* __restrict__ out, int64_t n, int R) {
+__global__ void unpack_out_kernel(const double* __restrict__ s, double* __restrict__ out, int64_t n, int R) {
   int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n * R) return;
   int64_t row = i % n;
   int r = int(i / n);
-  out[i] = double(s[row * R + r]);
+  out[i] = s[row * R + r];
 }
 
 // ---- diagonal ------------------------------------------------------------------------------
@@ -1579,7 +1594,7 @@ static int fine_chunks(fcg_ctx* ctx, bool direct) {
 }
 
 template <typename T, int MINB>
-static void launch_lane(const LaneParams& p, int64_t grid, int R, const T* w, const T* op, const T* cin, T* sig,
+static void launch_lane(const LaneParams& p, int64_t grid, int R, const T* w, const T* op, const T* cin, double* sig,
                         cudaStream_t s) {
   const auto run = [&](auto kernel) { kernel<<<unsigned(grid), kSigmaThreads, 0, s>>>(p, w, op, cin, sig); };
   switch (R) {
@@ -1601,7 +1616,7 @@ static void launch_lane(const LaneParams& p, int64_t grid, int R, const T* w, co
 // one direct closed sigma's lane jobs with candidate c (all of them, or those of the items that do
 // not run as block jobs)
 template <typename T>
-static int launch_candidate(fcg_ctx* ctx, int c, int R, const T* w, const T* op, const T* cin, T* sig) {
+static int launch_candidate(fcg_ctx* ctx, int c, int R, const T* w, const T* op, const T* cin, double* sig) {
   LaneParams p = make_lane_params(ctx, R);
   const bool direct = use_blocks<T>(ctx);
   if (direct) {
@@ -1657,7 +1672,7 @@ static int launch_blocks(fcg_ctx* ctx, int R, const double* w, const double* op,
 // Times every candidate once on this state (each a run of its lane jobs into sig), keeps the
 // fastest for the context and for later states of the same shape in this process.
 template <typename T>
-static int tune_closed(fcg_ctx* ctx, int prec, int R, const T* w, const T* op, const T* cin, T* sig) {
+static int tune_closed(fcg_ctx* ctx, int prec, int R, const T* w, const T* op, const T* cin, double* sig) {
   const auto t0 = std::chrono::steady_clock::now();
   const std::string key = tune_key(ctx, prec, R);
   {
@@ -1672,7 +1687,7 @@ static int tune_closed(fcg_ctx* ctx, int prec, int R, const T* w, const T* op, c
   float best = 0.f;
   int best_c = 0;
   for (int c = 0; c < kTuneCandidates; ++c) {
-    FCG_CUDA(cudaMemsetAsync(sig, 0, sizeof(T) * size_t(ctx->n_cfg) * R, ctx->stream));
+    FCG_CUDA(cudaMemsetAsync(sig, 0, sizeof(double) * size_t(ctx->n_cfg) * R, ctx->stream));
     FCG_CUDA(cudaEventRecord(ctx->ev2, ctx->stream));
     const int rc = launch_candidate<T>(ctx, c, R, w, op, cin, sig);
     if (rc) return rc;
@@ -1696,9 +1711,10 @@ static int tune_closed(fcg_ctx* ctx, int prec, int R, const T* w, const T* op, c
 }
 
 // Exact widths to 8 in float64.  In float the width of 8 with whole vector loads is as fast or faster
-// (stored blocks of 50,021 rows of 24 orbitals, 6 and 8 roots: 252 and 186 us, exact 267 and 226).
+// (stored blocks of 50,021 rows of 24 orbitals, 6 and 8 roots, while sums were added in float: 252 and
+// 186 us, exact 267 and 226).
 template <typename T>
-static void launch_cached(const LaneParams& p, int64_t grid, int R, const T* hc, const T* cin, T* sig, cudaStream_t s) {
+static void launch_cached(const LaneParams& p, int64_t grid, int R, const T* hc, const T* cin, double* sig, cudaStream_t s) {
   const auto run = [&](auto kernel) { kernel<<<unsigned(grid), kSigmaThreads, 0, s>>>(p, hc, cin, sig); };
   switch (R) {
     case 1: return run(cached_sigma_lane_kernel<T, 1>);
@@ -1721,7 +1737,7 @@ static void launch_cached(const LaneParams& p, int64_t grid, int R, const T* hc,
 }
 
 template <typename T>
-static int launch_closed(fcg_ctx* ctx, int R, const T* w, const T* op, const T* cin, T* sig, bool zero_sig = true,
+static int launch_closed(fcg_ctx* ctx, int R, const T* w, const T* op, const T* cin, double* sig, bool zero_sig = true,
                          bool timed = true) {
   const int prec = sizeof(T) == 4 ? 1 : 0;
   FCG_REQUIRE(ctx->have_plan, FCG_ESTATE, "the closed-sigma plan is missing (fcg_state_set builds it)");
@@ -1735,7 +1751,7 @@ static int launch_closed(fcg_ctx* ctx, int R, const T* w, const T* op, const T* 
     zero_sig = true;  // the tuning runs left a sigma behind
   }
   const LaneParams p = make_lane_params(ctx, R);
-  if (zero_sig) FCG_CUDA(cudaMemsetAsync(sig, 0, sizeof(T) * size_t(ctx->n_cfg) * R, ctx->stream));
+  if (zero_sig) FCG_CUDA(cudaMemsetAsync(sig, 0, sizeof(double) * size_t(ctx->n_cfg) * R, ctx->stream));
   const int64_t grid = lane_ctas(p.n_chunks);
   int launches = 0;
   if (timed) FCG_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));
@@ -1784,14 +1800,14 @@ static int sigma_device_impl(fcg_ctx* ctx, int R, const double* d_c, double* d_s
     pack_in_kernel<double><<<g, 256, 0, ctx->stream>>>(d_c, ctx->d_c64.p, n, R, ctx->d_s64.p);
     rc = launch_closed<double>(ctx, R, ctx->d_w64.p, ctx->d_op64.p, ctx->d_c64.p, ctx->d_s64.p, false, wait);
     if (rc) return rc;
-    unpack_out_kernel<double><<<g, 256, 0, ctx->stream>>>(ctx->d_s64.p, d_sigma, n, R);
+    unpack_out_kernel<<<g, 256, 0, ctx->stream>>>(ctx->d_s64.p, d_sigma, n, R);
   } else {
     FCG_CUDA(ctx->d_c32.alloc(nR));
-    FCG_CUDA(ctx->d_s32.alloc(nR));
-    pack_in_kernel<float><<<g, 256, 0, ctx->stream>>>(d_c, ctx->d_c32.p, n, R, ctx->d_s32.p);
-    rc = launch_closed<float>(ctx, R, ctx->d_w32.p, ctx->d_op32.p, ctx->d_c32.p, ctx->d_s32.p, false, wait);
+    FCG_CUDA(ctx->d_s64.alloc(nR));
+    pack_in_kernel<float><<<g, 256, 0, ctx->stream>>>(d_c, ctx->d_c32.p, n, R, ctx->d_s64.p);
+    rc = launch_closed<float>(ctx, R, ctx->d_w32.p, ctx->d_op32.p, ctx->d_c32.p, ctx->d_s64.p, false, wait);
     if (rc) return rc;
-    unpack_out_kernel<float><<<g, 256, 0, ctx->stream>>>(ctx->d_s32.p, d_sigma, n, R);
+    unpack_out_kernel<<<g, 256, 0, ctx->stream>>>(ctx->d_s64.p, d_sigma, n, R);
   }
   FCG_CUDA(cudaGetLastError());
   ctx->stats.kernel_launches += 2;
@@ -1883,18 +1899,18 @@ static int grouped_impl(int n, fcg_ctx* const* ctxs, const int* R, const double*
     e.p = make_lane_params(c, R[q]);
     if (sizeof(T) == 4) {
       FCG_CUDA(c->d_c32.alloc(size_t(nr)));
-      FCG_CUDA(c->d_s32.alloc(size_t(nr)));
+      FCG_CUDA(c->d_s64.alloc(size_t(nr)));
       e.w = reinterpret_cast<const T*>(c->d_w32.p);
       e.op = reinterpret_cast<const T*>(c->d_op32.p);
       e.cin = reinterpret_cast<T*>(c->d_c32.p);
-      e.sig = reinterpret_cast<T*>(c->d_s32.p);
+      e.sig = c->d_s64.p;
     } else {
       FCG_CUDA(c->d_c64.alloc(size_t(nr)));
       FCG_CUDA(c->d_s64.alloc(size_t(nr)));
       e.w = reinterpret_cast<const T*>(c->d_w64.p);
       e.op = reinterpret_cast<const T*>(c->d_op64.p);
       e.cin = reinterpret_cast<T*>(c->d_c64.p);
-      e.sig = reinterpret_cast<T*>(c->d_s64.p);
+      e.sig = c->d_s64.p;
     }
     e.src = d_c[q];
     e.dst = d_sigma[q];
@@ -2144,14 +2160,14 @@ extern "C" int fcg_sigma_closed_noalloc(fcg_ctx* ctx, int R, const double* d_c, 
     pack_in_kernel<double><<<g, 256, 0, ctx->stream>>>(d_c, cbuf, n, R, nullptr);
     rc = launch_closed<double>(ctx, R, ctx->d_w64.p, ctx->d_op64.p, cbuf, sbuf);  // zeroes sbuf first
     if (rc) return rc;
-    unpack_out_kernel<double><<<g, 256, 0, ctx->stream>>>(sbuf, d_sigma, n, R);
+    unpack_out_kernel<<<g, 256, 0, ctx->stream>>>(sbuf, d_sigma, n, R);
   } else {
     float* cbuf = reinterpret_cast<float*>(scratch);
-    float* sbuf = reinterpret_cast<float*>(scratch + kNoAllocMaxElems);
+    double* sbuf = scratch + kNoAllocMaxElems;
     pack_in_kernel<float><<<g, 256, 0, ctx->stream>>>(d_c, cbuf, n, R, nullptr);
     rc = launch_closed<float>(ctx, R, ctx->d_w32.p, ctx->d_op32.p, cbuf, sbuf);
     if (rc) return rc;
-    unpack_out_kernel<float><<<g, 256, 0, ctx->stream>>>(sbuf, d_sigma, n, R);
+    unpack_out_kernel<<<g, 256, 0, ctx->stream>>>(sbuf, d_sigma, n, R);
   }
   FCG_CUDA(cudaGetLastError());
   ctx->stats.kernel_launches += 2;
