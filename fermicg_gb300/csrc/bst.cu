@@ -335,11 +335,6 @@ __global__ void bst_convert_kernel(const double* __restrict__ a, float* __restri
     b[i] = float(a[i]);
 }
 
-__global__ void bst_widen_kernel(const float* __restrict__ a, double* __restrict__ b, int64_t n) {
-  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
-    b[i] = double(a[i]);
-}
-
 // One actives-first index table: block `block`'s positions for the active clusters `mask`,
 // at perm[off, off + core_len).
 struct BstPermTable {
@@ -511,9 +506,9 @@ __device__ __forceinline__ void load4(const T* p, T* v) {
 // feeds TN (or TM) multiply-adds; columns of length k % 4 == 0 are read 4 elements at a time
 // (operator and workspace columns then start on 16-byte boundaries).  Edge tiles repeat the
 // last column and drop the extra results.
-template <typename T, int TEAM, bool ATOMIC, int TM, int TN>
+template <typename T, int TEAM, bool ATOMIC, int TM, int TN, typename O>
 __device__ __forceinline__ void bst_tile_gemm(const T* __restrict__ opg, int k, int m, int ns, int R, const T* ws,
-                                              int stride, int cur, const int32_t* __restrict__ bp, T* out,
+                                              int stride, int cur, const int32_t* __restrict__ bp, O* out,
                                               int64_t out_stride, int tid) {
   const int tm = (m + TM - 1) / TM, tn = (ns + TN - 1) / TN, tiles = tm * tn;
   const bool vec = (k & 3) == 0;
@@ -559,16 +554,16 @@ __device__ __forceinline__ void bst_tile_gemm(const T* __restrict__ opg, int k, 
           for (int j = 0; j < TN; ++j) acc[i][j] = fma(av[i], bv[j], acc[i][j]);
       }
     }
-    T* outr = out + int64_t(r) * out_stride;
+    O* outr = out + int64_t(r) * out_stride;
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
       for (int j = 0; j < TN; ++j) {
         const int col = c0 + i, sp = s0 + j;
         if (col < m && sp < ns) {
-          T* dst = outr + __ldg(bp + col + m * sp);
+          O* dst = outr + __ldg(bp + col + m * sp);
           if (ATOMIC)
-            atomicAdd(dst, acc[i][j]);
+            atomicAdd(dst, O(acc[i][j]));
           else
             *dst += acc[i][j];
         }
@@ -576,10 +571,10 @@ __device__ __forceinline__ void bst_tile_gemm(const T* __restrict__ opg, int k, 
   }
 }
 
-template <typename T, int TEAM, bool ATOMIC>
+template <typename T, int TEAM, bool ATOMIC, typename O>
 __device__ void bst_group_apply(const BstGroup& G, int R, const T* __restrict__ op, const T* __restrict__ S,
                                 const int32_t* __restrict__ perm, const T* __restrict__ cin, int64_t core_total,
-                                T* ws, int stride, T* out, int64_t out_stride) {
+                                T* ws, int stride, O* out, int64_t out_stride) {
   const int tid = TEAM == 32 ? int(threadIdx.x & 31) : int(threadIdx.x);
   const int k = G.k, m = G.m, nsp = G.nsp;
   prefetch_range<TEAM, true>(op + G.op_off, int64_t(m) * k * int64_t(sizeof(T)), tid);
@@ -605,7 +600,7 @@ __device__ void bst_group_apply(const BstGroup& G, int R, const T* __restrict__ 
     // short columns: one thread per (kb, s) and root; items of one group never share an output
     for (int r = 0; r < R; ++r) {
       const T* Xr = ws + int64_t(2 * r + cur) * stride;
-      T* outr = out + int64_t(r) * out_stride;
+      O* outr = out + int64_t(r) * out_stride;
       for (int it = tid; it < mn; it += TEAM) {
         const int s = it / m, col = it - s * m;
         const T* o = opg + int64_t(k) * col;
@@ -618,9 +613,9 @@ __device__ void bst_group_apply(const BstGroup& G, int R, const T* __restrict__ 
         }
         if (kk < k) acc = fma(o[kk], X[kk], acc);
         acc += acc2;
-        T* dst = outr + __ldg(bp + it);
+        O* dst = outr + __ldg(bp + it);
         if (ATOMIC)
-          atomicAdd(dst, acc);
+          atomicAdd(dst, O(acc));
         else
           *dst += acc;
       }
@@ -640,9 +635,9 @@ __device__ void bst_group_apply(const BstGroup& G, int R, const T* __restrict__ 
     for (int kk = lane; kk < k; kk += 32) acc = fma(o[kk], X[kk], acc);
     for (int w = 16; w > 0; w >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, w);
     if (lane == 0) {
-      T* dst = out + int64_t(r) * out_stride + __ldg(bp + rem);
+      O* dst = out + int64_t(r) * out_stride + __ldg(bp + rem);
       if (ATOMIC)
-        atomicAdd(dst, acc);
+        atomicAdd(dst, O(acc));
       else
         *dst += acc;
     }
@@ -663,7 +658,7 @@ __global__ void __launch_bounds__(kBstThreads, 4) bst_sigma_bra_kernel(const int
                                                                     const T* __restrict__ op,
                                                                     const T* __restrict__ S,
                                                                     const int32_t* __restrict__ perm,
-                                                                    const T* __restrict__ cin, T* __restrict__ cout,
+                                                                    const T* __restrict__ cin, double* __restrict__ cout,
                                                                     int64_t core_total, int slice, int priv) {
   extern __shared__ __align__(16) unsigned char bst_smem[];
   constexpr int kWarps = kBstThreads / 32;
@@ -695,7 +690,7 @@ __global__ void __launch_bounds__(kBstThreads, 4) bst_sigma_bra_kernel(const int
     T v = T(0);
     for (int c = 0; c < copies; ++c) v += acc[size_t(c) * R * n + i];
     const int r = i / n, e = i - r * n;
-    if (v != T(0)) atomicAdd(cout + int64_t(r) * core_total + B.core_off + e, v);
+    if (v != T(0)) atomicAdd(cout + int64_t(r) * core_total + B.core_off + e, double(v));
   }
 }
 
@@ -754,7 +749,7 @@ template <typename T>
 struct BstSink {
   T* buf;              // element i to buf[i], when set
   T* acc;              // else added to the shared bra core, when set
-  T* out;              // else atomically to sigma
+  double* out;         // else atomically to sigma (float64 in both precisions, see bst_launch)
   const uint16_t* ta;  // of the bra-active columns
   const uint16_t* tb;  // of the spectator indices
   int m;
@@ -763,7 +758,7 @@ struct BstSink {
     if (acc)
       acc[at] += v;
     else
-      atomicAdd(out + at, v);
+      atomicAdd(out + at, double(v));
   }
   __device__ __forceinline__ void put(int i, T v) const {
     if (buf) {
@@ -1008,7 +1003,7 @@ __global__ void __launch_bounds__(TEAM, (sizeof(T) == 4 ? 768 : 512) / TEAM)
     bst_chunk_kernel(const BstChunk* __restrict__ chunks, const BstEntry* __restrict__ entries,
                      const BstGroup* __restrict__ groups, const BstLayout* __restrict__ layouts,
                      const T* __restrict__ op, const T* __restrict__ S, const T* __restrict__ cin,
-                     T* __restrict__ cout, int64_t core_total) {
+                     double* __restrict__ cout, int64_t core_total) {
   extern __shared__ __align__(16) unsigned char bst_smem[];
   const BstChunk C = chunks[blockIdx.x];
   const int tid = threadIdx.x;
@@ -1018,7 +1013,7 @@ __global__ void __launch_bounds__(TEAM, (sizeof(T) == 4 ? 768 : 512) / TEAM)
   T* buf0 = acc + (C.acc ? (C.bcore + 3) / 4 * 4 : 0);
   T* buf1 = buf0 + C.ws;
   uint16_t* tab = reinterpret_cast<uint16_t*>(buf1 + C.ws);
-  T* out = cout + int64_t(C.root) * core_total + C.b_off;
+  double* out = cout + int64_t(C.root) * core_total + C.b_off;
   const T* src_root = cin + int64_t(C.root) * core_total;
   // 16-byte units of a description, one per thread
   constexpr int kGroupUnits = int(sizeof(BstGroup) / 16), kUnits = kDesc / 16;
@@ -1204,7 +1199,7 @@ __global__ void __launch_bounds__(TEAM, (sizeof(T) == 4 ? 768 : 512) / TEAM)
   if (C.acc)
     for (int i = tid; i < C.bcore; i += TEAM) {
       const T v = acc[i];
-      if (v != T(0)) atomicAdd(out + i, v);
+      if (v != T(0)) atomicAdd(out + i, double(v));
     }
 }
 
@@ -1217,7 +1212,7 @@ __global__ void __launch_bounds__(kBstThreads) bst_sigma_global_kernel(const int
                                                                        const T* __restrict__ S,
                                                                        const int32_t* __restrict__ perm,
                                                                        const T* __restrict__ cin,
-                                                                       T* __restrict__ cout, int64_t core_total,
+                                                                       double* __restrict__ cout, int64_t core_total,
                                                                        T* __restrict__ ws_all, int stride,
                                                                        unsigned* __restrict__ next) {
   __shared__ __align__(16) BstGroup G;
@@ -1281,7 +1276,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) bst_tc_gemm_kernel(const BstTcJ
                                                                    const float* __restrict__ ws_all,
                                                                    const int64_t* __restrict__ ws_off,
                                                                    const int32_t* __restrict__ perm,
-                                                                   float* __restrict__ cout, int64_t core_total,
+                                                                   double* __restrict__ cout, int64_t core_total,
                                                                    unsigned* __restrict__ err) {
   extern __shared__ __align__(1024) unsigned char tc_smem[];
   constexpr int kAB = kTcM * kTcK * 4;  // bytes of one A operand copy (hi or lo) of a stage
@@ -1397,7 +1392,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) bst_tc_gemm_kernel(const BstTcJ
     // epilogue: thread tid holds tile row tid; columns in runs of 16
     const int i = J.m0 + tid;
     const int32_t* bp = perm + G.bperm_off;
-    float* outb = cout + G.b_off;
+    double* outb = cout + G.b_off;
     for (int c0 = 0; c0 < nI; c0 += 16) {
       float v[16];
       tc::tmem_ld16(taddr + (uint32_t(32 * warp) << 16) + uint32_t(c0), v);
@@ -1408,7 +1403,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) bst_tc_gemm_kernel(const BstTcJ
           if (col < cols) {
             const int jp = J.n0 + col;
             const int r = jp / ns, sidx = jp - r * ns;
-            atomicAdd(outb + int64_t(r) * core_total + __ldg(bp + i + m * sidx), v[q]);
+            atomicAdd(outb + int64_t(r) * core_total + __ldg(bp + i + m * sidx), double(v[q]));
           }
         }
       }
@@ -2250,8 +2245,11 @@ void bst_lists(fcg_ctx* ctx, int R, size_t elem) {
   ctx->bst_entries.assign(eb, eb + entries.size() * sizeof(BstEntry));
 }
 
+// cout is float64 in both precisions: a bra core takes the sums of many chunks, and float additions
+// there round at its full size (1 sector, q 2: error 6.9e-8 with float, 5.8e-8 so; 5 sectors, q 4:
+// 1.2e-7 and 8.5e-8, 11.3 and 11.5 ms).
 template <typename T>
-int bst_launch(fcg_ctx* ctx, int R, const T* op, const T* S, const T* cin, T* cout, DevBuf<T>& ws) {
+int bst_launch(fcg_ctx* ctx, int R, const T* op, const T* S, const T* cin, double* cout, DevBuf<T>& ws) {
   const size_t elem = sizeof(T);
   if (ctx->bst_list_R != R || ctx->bst_list_elem != elem) {
     bst_lists(ctx, R, elem);
@@ -2270,7 +2268,7 @@ int bst_launch(fcg_ctx* ctx, int R, const T* op, const T* S, const T* cin, T* co
     ctx->bst_list_elem = elem;
   }
   const int64_t ct = ctx->bst_core_total;
-  FCG_CUDA(cudaMemsetAsync(cout, 0, elem * size_t(ct) * R, ctx->stream));
+  FCG_CUDA(cudaMemsetAsync(cout, 0, sizeof(double) * size_t(ct) * R, ctx->stream));
   int launches = 1;
   // tensor-core groups (float builds) on the second stream, overlapping the CUDA-core
   // launches below: every kernel adds into the bra cores atomically
@@ -2369,17 +2367,16 @@ int bst_sigma_device_async(fcg_ctx* ctx, int R, const double* d_cores, double* d
     if (timed) FCG_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
   } else {
     FCG_CUDA(ctx->d_bst_in32.alloc(size_t(n)));
-    FCG_CUDA(ctx->d_bst_out32.alloc(size_t(n)));
+    FCG_CUDA(ctx->d_bst_acc.alloc(size_t(n)));
     bst_convert_kernel<<<512, 256, 0, ctx->stream>>>(d_cores, ctx->d_bst_in32.p, n);
     FCG_CUDA(cudaGetLastError());
     if (timed) FCG_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));
-    rc = bst_launch<float>(ctx, R, ctx->d_bst_op32.p, ctx->d_bst_s32.p, ctx->d_bst_in32.p, ctx->d_bst_out32.p,
+    rc = bst_launch<float>(ctx, R, ctx->d_bst_op32.p, ctx->d_bst_s32.p, ctx->d_bst_in32.p, ctx->d_bst_acc.p,
                            ctx->d_bst_ws32);
     if (rc) return rc;
     if (timed) FCG_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
-    bst_widen_kernel<<<512, 256, 0, ctx->stream>>>(ctx->d_bst_out32.p, d_sigma, n);
-    FCG_CUDA(cudaGetLastError());
-    ctx->stats.kernel_launches += 2;
+    FCG_CUDA(cudaMemcpyAsync(d_sigma, ctx->d_bst_acc.p, sizeof(double) * size_t(n), cudaMemcpyDefault, ctx->stream));
+    ctx->stats.kernel_launches += 1;
   }
   return FCG_OK;
 }

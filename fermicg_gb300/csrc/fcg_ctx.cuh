@@ -283,7 +283,8 @@ struct fcg_ctx {
   DevBuf<double> d_bst_op64, d_bst_s64;
   DevBuf<float> d_bst_op32, d_bst_s32;
   DevBuf<double> d_bst_in64, d_bst_out64, d_bst_ws64;
-  DevBuf<float> d_bst_in32, d_bst_out32, d_bst_ws32;
+  DevBuf<float> d_bst_in32, d_bst_ws32;
+  DevBuf<double> d_bst_acc;  // sigma of a float build
   // tensor-core groups of the float sigma: group ids, their X workspace offsets, the 128 x N
   // tile jobs {tc index, group, m0, n0}, algorithmic and executed MMA flops per sigma
   bool bst_tc_on = true;
