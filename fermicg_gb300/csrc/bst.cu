@@ -728,6 +728,7 @@ struct BstChunk {
 constexpr int kChunkBuckets = 6;
 constexpr int kChunkBucket[kChunkBuckets] = {16 * 1024, 28 * 1024, 44 * 1024, 72 * 1024, 112 * 1024, 224 * 1024};
 constexpr int kChunkTeam[kChunkBuckets] = {128, 256, 256, 384, 384, 384};  // threads of a CTA
+constexpr int64_t kLargeEnough = 152;  // groups that give the global-workspace kernel one per SM
 constexpr int kChunkAccMax = 4;   // last bucket of chunks that keep the bra core
 constexpr int kPrefetchL1 = 8 * 1024;   // bytes of an operator prefetched to L1
 constexpr int kCoef = 1024;       // elements of the coefficient tables
@@ -2083,6 +2084,7 @@ void bst_lists(fcg_ctx* ctx, int R, size_t elem) {
   constexpr uint8_t kWarp = 100, kLarge = 101, kTc = 102;
   std::vector<uint8_t> where(ng);
   int64_t warp_work = 0, chunk_work = 0;
+  int64_t n_large = 0;  // groups larger than a CTA's memory
   for (size_t q = 0; q < ng; ++q) {
     const BstGroup& G = ctx->bst_groups[q];
     const int64_t ns = G.bcore / std::max(G.m, 1);
@@ -2102,8 +2104,20 @@ void bst_lists(fcg_ctx* ctx, int R, size_t elem) {
           break;
         }
       if (where[q] < kChunkBuckets) chunk_work += R * entry_work(G, G.m);
+      n_large += where[q] == kLarge;
     }
   }
+  // Double groups of more than 72 KB go to the global-workspace kernel too where it has a group for
+  // every SM anyway: a chunk of 384 threads per SM leaves the float64 pipe half idle, but few groups
+  // leave SMs idle there.  32 orbitals, 4 excited clusters, 2 roots: ranks 4-12, 5 / 2 sectors, chunks
+  // 56.2 / 17.0 ms, global 47.3 / 14.4; ranks 4-10, 1 sector, chunks 1.8, global 2.0.
+  if (elem == 8 && n_large >= kLargeEnough)
+    for (size_t q = 0; q < ng; ++q)
+      if (where[q] < kChunkBuckets && where[q] > kChunkAccMax - 1) {
+        const BstGroup& G = ctx->bst_groups[q];
+        chunk_work -= R * entry_work(G, G.m);
+        where[q] = kLarge;
+      }
   const int64_t warp_cut = std::max(kChunkWorkMin, std::min(kChunkWorkMax, warp_work / kChunkTarget));
   const int64_t chunk_cut = std::min<int64_t>(4 * kSplitFma, chunk_work / (4 * kChunkTarget));
   struct Pending {  // chunks of one bucket: (work, entries) of one bra block, for every root
