@@ -831,10 +831,11 @@ struct DavidsonWork {
         return FCG_OK;
       }
       if (i % 2048) continue;
+      std::this_thread::yield();
+      if (i % (1 << 17)) continue;  // seldom: a query takes the driver's lock from the solves beside this one
       const cudaError_t e = cudaStreamQuery(ctx->stream);
       if (e != cudaErrorNotReady) break;
       cudaGetLastError();  // not an error
-      std::this_thread::yield();
     }
     await = 0;
     FCG_CUDA(cudaStreamSynchronize(ctx->stream));
