@@ -10,7 +10,7 @@
 //   state        local states int16 [n_cfg][N]
 //   plan         the grouping permutation pool, term-sector records, lane jobs in warp chunks and
 //                (for the double sigma of larger states) block jobs
-//   vectors      coefficients / sigma row-major [n_cfg][R] in the compute precision
+//   vectors      row-major [n_cfg][R]: coefficients in the compute precision, sigma float64
 //
 // Kernels:
 //   dress_kernel         W blocks, once per problem (fcg_set_terms)
@@ -21,7 +21,7 @@
 //   block_sigma_kernel   a block of bras x kets per warp, the partly contracted W columns shared
 //   cached_sigma_lane_kernel  the same product from stored Hamiltonian blocks
 //   diag kernels         compute_diagonal (src/tpsci_outer.jl:694-757).
-//   pack / unpack        column-major float64 <-> row-major compute precision.
+//   pack / unpack        column-major float64 -> row-major compute precision, row-major sigma back.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -1606,6 +1606,7 @@ static void launch_lane(const LaneParams& p, int64_t grid, int R, const T* w, co
     case 6: return run(closed_sigma_lane_kernel<T, 6, MINB>);
     case 7: return run(closed_sigma_lane_kernel<T, 7, MINB>);
     case 8: return run(closed_sigma_lane_kernel<T, 8, MINB>);
+    default: break;
   }
   if constexpr (sizeof(T) == 8) {
     if (R <= 12) return run(closed_sigma_lane_kernel<T, 0, MINB, 12>);
@@ -1721,6 +1722,7 @@ static void launch_cached(const LaneParams& p, int64_t grid, int R, const T* hc,
     case 2: return run(cached_sigma_lane_kernel<T, 2>);
     case 3: return run(cached_sigma_lane_kernel<T, 3>);
     case 4: return run(cached_sigma_lane_kernel<T, 4>);
+    default: break;
   }
   if constexpr (sizeof(T) == 8) {
     switch (R) {
@@ -1728,6 +1730,7 @@ static void launch_cached(const LaneParams& p, int64_t grid, int R, const T* hc,
       case 6: return run(cached_sigma_lane_kernel<T, 6>);
       case 7: return run(cached_sigma_lane_kernel<T, 7>);
       case 8: return run(cached_sigma_lane_kernel<T, 8>);
+      default: break;
     }
     if (R <= 12) return run(cached_sigma_lane_kernel<T, 0, 12>);
   } else {
