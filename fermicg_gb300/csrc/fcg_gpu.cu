@@ -25,6 +25,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <chrono>
 #include <map>
 #include <mutex>
@@ -944,21 +945,34 @@ __device__ double diag_element(const DiagParams& p, const TermInfo& tm, const do
   return s ? -me : me;
 }
 
-// A warp per row, a term per lane (a thread per row took 155 us for 2000 rows of 12 orbitals: a serial
-// chain of gathers and 16 CTAs); the lanes' sums are added in a fixed order.
+// 2^sh lanes per row, each a share of the terms; neighbouring rows (mostly of one sector) run the same
+// term side by side and so read the same records and integrals.  The lanes' sums are added in a fixed
+// order.
 __global__ void diag_terms_kernel(DiagParams p, const double* __restrict__ op, const double* __restrict__ ints,
-                                  const int32_t* __restrict__ zero_terms, int n_zero, int64_t n,
+                                  const int32_t* __restrict__ zero_terms, int n_zero, int64_t n, int sh,
                                   double* __restrict__ hd) {
-  const int64_t i = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (i >= n) return;
-  const int16_t* f = p.sec_fock + int64_t(p.row_sector[i]) * 2 * p.N;
+  const int lane = threadIdx.x & 31, rows = 32 >> sh;  // rows of a warp
+  const int64_t i = ((int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * rows + (lane & (rows - 1));
   double s = 0.0;
-  for (int z = lane; z < n_zero; z += 32)
-    s += diag_element(p, p.terms[zero_terms[z]], op, ints, f, p.cfg + i * kCfgStride);
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-  if (lane == 0) hd[i] = s;
+  if (i < n) {
+    const int16_t* f = p.sec_fock + int64_t(p.row_sector[i]) * 2 * p.N;
+    for (int z = lane >> (5 - sh); z < n_zero; z += 1 << sh)
+      s += diag_element(p, p.terms[zero_terms[z]], op, ints, f, p.cfg + i * kCfgStride);
+  }
+  for (int off = 16; off >= rows; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+  if (i < n && lane < rows) hd[i] = s;
+}
+
+// Lanes of a row: the power of two nearest to 64,000 / rows, from 2 to 32.  A row alone is a serial chain of
+// gathers, so few rows want many lanes; many rows fill the chip by themselves, and more lanes of a row
+// only spread a warp's loads over more records.  Whole call, by lanes 1 / 2 / 4 / 8 / 16 / 32 (us):
+// 12 orbitals, 500 rows 178 / 104 / 66 / 54 / 41 / 30; 24 orbitals, 3 000 rows 906 / 464 / 265 / 218 / 202 / 239,
+// 10 007 rows 910 / 648 / 451 / 450 / 513 / 726, 100 000 rows 3238 / 2905 / 2974 / 3452 / 4364 / 6681;
+// 32 orbitals, 5 000 rows 1673 / 850 / 597 / 400 / 474 / 660, 20 011 rows 2340 / 1588 / 1254 / 1144 / 1506 / 2352.
+constexpr double kDiagLanes = 64000.0;
+inline int diag_lane_bits(int64_t rows) {
+  const double x = std::log2(kDiagLanes / double(std::max<int64_t>(rows, 1)));
+  return std::max(1, std::min(5, int(std::lround(x))));
 }
 
 __global__ void diag_op_kernel(DiagParams p, const double* __restrict__ op, int opid, int64_t n,
@@ -2078,8 +2092,10 @@ int fcg_diagonal(fcg_ctx* ctx, int op_id, double* hd) {
   DiagParams p = make_diag_params(ctx);
   const unsigned g = unsigned((n + 127) / 128);
   if (op_id < 0) {
-    diag_terms_kernel<<<unsigned((32 * n + 127) / 128), 128, 0, ctx->stream>>>(p, ctx->d_op64.p, ctx->d_ints64.p, ctx->d_zero_terms.p,
-                                                  int(ctx->plan.zero_terms.size()), n, ctx->d_hd.p);
+    const int sh = diag_lane_bits(n);
+    const int64_t warps = (n + (32 >> sh) - 1) / (32 >> sh);
+    diag_terms_kernel<<<unsigned((warps + 3) / 4), 128, 0, ctx->stream>>>(p, ctx->d_op64.p, ctx->d_ints64.p, ctx->d_zero_terms.p,
+                                                                          int(ctx->plan.zero_terms.size()), n, sh, ctx->d_hd.p);
     FCG_CUDA(cudaGetLastError());
   } else {
     DevBuf<int> missing;
