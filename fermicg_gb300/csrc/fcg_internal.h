@@ -356,6 +356,34 @@ FCG_HD inline bool term_exists(const TermTables& tt, int t, const int16_t* fb, c
   return true;
 }
 
+// What term_exists and, for a term that stands for its set, term_sector_of say, in one walk over the
+// clusters that is the same for every term (threads of a warp take different terms): whether t exists,
+// whether it has a record, and the record's multiply-add count.
+FCG_HD inline void term_count(const TermTables& tt, int t, const int16_t* fb, const int16_t* fk, bool* exists,
+                              bool* record, int64_t* fma) {
+  const int32_t* r = tt.trm + int64_t(t) * kTrmCols;
+  const int nbody = r[0], pos = tt.dress[t].pos < 0 ? 0 : tt.dress[t].pos;
+  bool rem = true, dressed = true;
+  int d1 = 1, d2 = 1;  // index lengths of the second and third cluster besides the dressed one
+  for (int o = 0, q = 0; o < nbody; ++o) {
+    const int c = r[2 + o];
+    const int bl = tt.blk[dense_block_index(tt.nmax1, c, r[6 + o], fb[2 * c], fb[2 * c + 1], fk[2 * c], fk[2 * c + 1])];
+    if (o == pos) {
+      dressed = bl >= 0;
+    } else {
+      rem = rem && bl >= 0;
+      if (q == 1) d1 = r[22 + o];
+      if (q == 2) d2 = r[22 + o];
+      ++q;
+    }
+  }
+  *exists = rem && dressed;
+  const int cw = r[2 + pos];
+  *record = rem && tt.rep[t] == t && tt.w_index[(int64_t(t) * tt.nmax1 + fb[2 * cw]) * tt.nmax1 + fb[2 * cw + 1]] >= 0;
+  const int64_t rest = tt.dress[t].rest_len;
+  *fma = nbody <= 1 ? 0 : nbody == 2 ? rest : nbody == 3 ? rest + d1 : rest + int64_t(d1) * d2 + d2;
+}
+
 // The term-sector record of term t (one that stands for its set) between bra sector fb and ket
 // sector fk (N x 2 each) and its multiply-add count per (bra, ket) pair (fma); false when no term of
 // the set has the TDM blocks it needs there.  The host and the device planner both make their records here.
