@@ -1118,6 +1118,7 @@ int fcg_set_ops(fcg_ctx* ctx, int n_clusters, const int32_t* cluster_norb, int64
     ctx->h_blocks[b] = BlockInfo{cursor, int32_t(r[6]), int32_t(r[7]), int32_t(r[8]), 0};
     cursor += r[6] * r[7] * r[8];
   }
+  ctx->cells = op_cells(ctx->norb, ctx->nmax, ctx->opb, ctx->h_blk_index, ctx->h_blocks);
   // the caller's blob goes up once; a kernel places every block at its aligned offset and
   // writes the float copy (the gaps between blocks are zero)
   {
@@ -1208,8 +1209,8 @@ int ensure_open_dressed(fcg_ctx* ctx) {
   if (ctx->open_dressed) return FCG_OK;
   Dressing& dz = ctx->open_dressing;
   {
-    const std::string msg = build_dress(ctx->norb, ctx->nmax, ctx->trm, ctx->n_terms, ctx->h_blk_index, ctx->h_blocks,
-                                        ctx->terms, ctx->dress, false, dz);
+    const std::string msg = build_dress(ctx->nmax, ctx->trm, ctx->n_terms, ctx->cells, ctx->h_blocks, ctx->terms,
+                                        ctx->dress, false, dz);
     FCG_REQUIRE(msg.empty(), FCG_EINVAL, msg);
   }
   {
@@ -1309,8 +1310,7 @@ int fcg_set_terms(fcg_ctx* ctx, int n_terms, const int32_t* term_table, int64_t 
   {
     std::string msg = term_dress(ctx->trm, n_terms, ctx->dress);
     FCG_REQUIRE(msg.empty(), FCG_EINVAL, msg);
-    msg = build_dress(ctx->norb, ctx->nmax, ctx->trm, n_terms, ctx->h_blk_index, ctx->h_blocks, ctx->terms, ctx->dress,
-                      true, ctx->dressing);
+    msg = build_dress(ctx->nmax, ctx->trm, n_terms, ctx->cells, ctx->h_blocks, ctx->terms, ctx->dress, true, ctx->dressing);
     FCG_REQUIRE(msg.empty(), FCG_EINVAL, msg);
   }
   FCG_CUDA(ctx->d_terms.upload(ctx->terms.data(), ctx->terms.size(), ctx->stream));

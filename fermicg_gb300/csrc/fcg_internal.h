@@ -468,10 +468,27 @@ std::string term_lists(const ProblemInfo& pi, TermLists& lists);
 // How every term is dressed (which cluster's TDM takes its integrals).
 std::string term_dress(const std::vector<int32_t>& trm, int n_terms, std::vector<TermDress>& dress);
 
+// The TDM blocks of every (cluster, operator) by change of Fock sector and then bra sector: what the
+// dressing walks over, made once per operator set.
+struct OpCells {
+  struct Cell {
+    int32_t fb;  // bra sector: alpha x (nmax + 1) + beta
+    int32_t block;
+  };
+  struct Run {
+    int32_t da, db, first, last;  // cells [first, last)
+  };
+  std::vector<Cell> cells;
+  std::vector<Run> runs;
+  std::vector<int32_t> first_run;  // per cluster x kNumOps + operator
+  bool uniform = true;  // the blocks of a cluster agree on the local dimensions of every sector
+};
+OpCells op_cells(const std::vector<int>& norb, int nmax, const std::vector<int64_t>& opb,
+                 const std::vector<int32_t>& blk_index, const std::vector<BlockInfo>& blocks);
+
 // The W blocks of every term, or (merge) of every set of terms that share theirs.
-std::string build_dress(const std::vector<int>& norb, int nmax, const std::vector<int32_t>& trm, int n_terms,
-                        const std::vector<int32_t>& blk_index, const std::vector<BlockInfo>& blocks,
-                        const std::vector<TermInfo>& terms, const std::vector<TermDress>& dress, bool merge,
-                        Dressing& out);
+std::string build_dress(int nmax, const std::vector<int32_t>& trm, int n_terms, const OpCells& cells,
+                        const std::vector<BlockInfo>& blocks, const std::vector<TermInfo>& terms,
+                        const std::vector<TermDress>& dress, bool merge, Dressing& out);
 
 }  // namespace fcg

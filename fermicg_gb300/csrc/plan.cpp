@@ -506,34 +506,76 @@ std::string term_dress(const std::vector<int32_t>& trm, int n_terms, std::vector
   return "";
 }
 
-std::string build_dress(const std::vector<int>& norb, int nmax, const std::vector<int32_t>& trm, int n_terms,
-                        const std::vector<int32_t>& blk_index, const std::vector<BlockInfo>& blocks,
-                        const std::vector<TermInfo>& terms, const std::vector<TermDress>& dress, bool merge,
-                        Dressing& out) {
-  const int s = nmax + 1;
-  out.jobs.clear();  // (the vectors keep their memory for the next term set)
-  out.src.clear();
-  out.n_w = 0;
-  out.rep.resize(size_t(n_terms));
-  out.w_index.assign(size_t(n_terms) * s * s, -1);
-  out.w_mb.assign(size_t(n_terms) * s * s, 0);
-  // the TDM blocks of every (cluster, operator), and from them those of a term's dressed cluster:
-  // calls f(bra sector cell, block) in cell order
-  const int ss = s * s;
-  struct Cell {
-    int32_t fb, fk, block;
+OpCells op_cells(const std::vector<int>& norb, int nmax, const std::vector<int64_t>& opb,
+                 const std::vector<int32_t>& blk_index, const std::vector<BlockInfo>& blocks) {
+  const int s = nmax + 1, ss = s * s;
+  struct At {
+    int64_t key;  // dense block index: cluster, operator, bra sector, ket sector
+    int32_t block;
   };
-  std::vector<std::vector<Cell>> cells(norb.size() * kNumOps);
-  for (size_t i = 0; i < blk_index.size(); ++i)
-    if (blk_index[i] >= 0) {
-      const size_t fk = i % ss, fb = i / ss % ss;
-      cells[i / ss / ss].push_back(Cell{int32_t(fb), int32_t(fk), blk_index[i]});
+  std::vector<At> at;
+  at.reserve(blocks.size());
+  for (size_t b = 0; b < blocks.size(); ++b) {
+    const int64_t* r = &opb[b * kOpbCols];
+    const int64_t key = dense_block_index(s, int(r[0]), int(r[1]), int(r[2]), int(r[3]), int(r[4]), int(r[5]));
+    if (blk_index[size_t(key)] == int32_t(b)) at.push_back(At{key, int32_t(b)});  // (the last of equal entries)
+  }
+  const auto before = [](const At& x, const At& y) { return x.key < y.key; };
+  if (!std::is_sorted(at.begin(), at.end(), before)) std::sort(at.begin(), at.end(), before);
+  OpCells C;
+  C.cells.reserve(at.size());
+  C.first_run.assign(norb.size() * kNumOps + 1, 0);
+  std::vector<int32_t> mb(norb.size() * size_t(ss), 0), mk(norb.size() * size_t(ss), 0);
+  const auto row = [&](size_t q) { return &opb[size_t(at[q].block) * kOpbCols]; };
+  size_t i = 0;
+  for (size_t op = 0; op < norb.size() * kNumOps; ++op) {
+    C.first_run[op] = int32_t(C.runs.size());
+    const size_t i0 = i;
+    while (i < at.size() && size_t(row(i)[0]) * kNumOps + size_t(row(i)[1]) == op) ++i;
+    // one run per change of sector (an operator has one)
+    for (size_t q = i0; q < i; ++q) {
+      const int64_t* r = row(q);
+      const int32_t da = int32_t(r[2] - r[4]), db = int32_t(r[3] - r[5]);
+      const BlockInfo& B = blocks[size_t(at[q].block)];
+      int32_t &b = mb[size_t(r[0] * ss + r[2] * s + r[3])], &k = mk[size_t(r[0] * ss + r[4] * s + r[5])];
+      C.uniform = C.uniform && (b == 0 || b == B.mb) && (k == 0 || k == B.mk);
+      b = B.mb, k = B.mk;
+      bool known = false;
+      for (size_t z = size_t(C.first_run[op]); z < C.runs.size(); ++z) known = known || (C.runs[z].da == da && C.runs[z].db == db);
+      if (known) continue;
+      OpCells::Run R{da, db, int32_t(C.cells.size()), 0};
+      for (size_t z = q; z < i; ++z) {
+        const int64_t* rz = row(z);
+        if (rz[2] - rz[4] == da && rz[3] - rz[5] == db) C.cells.push_back(OpCells::Cell{int32_t(rz[2] * s + rz[3]), at[z].block});
+      }
+      R.last = int32_t(C.cells.size());
+      C.runs.push_back(R);
     }
-  auto each_block = [&](int t, auto&& f) {
+  }
+  C.first_run.back() = int32_t(C.runs.size());
+  return C;
+}
+
+std::string build_dress(int nmax, const std::vector<int32_t>& trm, int n_terms, const OpCells& cells,
+                        const std::vector<BlockInfo>& blocks, const std::vector<TermInfo>& terms,
+                        const std::vector<TermDress>& dress, bool merge, Dressing& out) {
+  const int s = nmax + 1, ss = s * s;
+  out.rep.resize(size_t(n_terms));  // (the vectors keep their memory for the next term set)
+  out.w_index.assign(size_t(n_terms) * ss, -1);
+  out.w_mb.assign(size_t(n_terms) * ss, 0);
+  // the blocks of a term's dressed cluster and operator, in order of the bra sector
+  struct List {
+    const OpCells::Cell *p = nullptr, *end = nullptr;
+  };
+  auto blocks_of = [&](int t) {
     const int32_t* r = &trm[int64_t(t) * kTrmCols];
     const int pos = dress[size_t(t)].pos < 0 ? 0 : dress[size_t(t)].pos;
-    for (const Cell& c : cells[size_t(r[2 + pos]) * kNumOps + r[6 + pos]])
-      if (c.fb / s - r[10 + pos] == c.fk / s && c.fb % s - r[14 + pos] == c.fk % s) f(c.fb, c.block);
+    const size_t op = size_t(r[2 + pos]) * kNumOps + r[6 + pos];
+    for (int32_t i = cells.first_run[op]; i < cells.first_run[op + 1]; ++i) {
+      const OpCells::Run& R = cells.runs[size_t(i)];
+      if (R.da == r[10 + pos] && R.db == r[14 + pos]) return List{&cells.cells[0] + R.first, &cells.cells[0] + R.last};
+    }
+    return List{};
   };
   // sets of terms that share a W: term by term, next[t] the next one of t's set (or -1)
   std::vector<int32_t> next(size_t(n_terms), -1);
@@ -565,6 +607,20 @@ std::string build_dress(const std::vector<int>& norb, int nmax, const std::vecto
       }
       return true;
     };
+    // the operators' blocks must have the same local dimensions wherever several exist
+    auto fits = [&](int t, int t0) {
+      if (cells.uniform) return true;
+      for (int m = t0; m >= 0 && m != t; m = next[size_t(m)])
+        for (List x = blocks_of(t), y = blocks_of(m); x.p != x.end && y.p != y.end;) {
+          if (x.p->fb != y.p->fb) {
+            ++(x.p->fb < y.p->fb ? x : y).p;
+            continue;
+          }
+          const BlockInfo &B = blocks[size_t(x.p++->block)], &B2 = blocks[size_t(y.p++->block)];
+          if (B.mb != B2.mb || B.mk != B2.mk) return false;
+        }
+      return true;
+    };
     size_t cap = 64;
     while (cap < 2 * size_t(n_terms)) cap <<= 1;
     std::vector<int32_t> table(cap, -1);           // open addressing: the first term of a set
@@ -575,16 +631,7 @@ std::string build_dress(const std::vector<int>& norb, int nmax, const std::vecto
       size_t at = size_t(hash_of(t)) & (cap - 1);
       while (table[at] >= 0 && !same(t, table[at])) at = (at + 1) & (cap - 1);
       const int t0 = table[at] >= 0 ? table[at] : t;
-      // the operators' blocks must have the same local dimensions wherever several exist
-      bool fits = true;
-      for (int m = t0; m >= 0 && m != t; m = next[size_t(m)])
-        each_block(t, [&](int cell, int b) {
-          each_block(m, [&](int cell2, int b2) {
-            if (cell == cell2 && (blocks[size_t(b)].mb != blocks[size_t(b2)].mb || blocks[size_t(b)].mk != blocks[size_t(b2)].mk))
-              fits = false;
-          });
-        });
-      if (!fits) continue;
+      if (!fits(t, t0)) continue;
       table[at] = t0;
       if (t0 != t) {
         out.rep[size_t(t)] = t0;
@@ -593,58 +640,71 @@ std::string build_dress(const std::vector<int>& norb, int nmax, const std::vecto
       last[size_t(t0)] = t;
     }
   }
-  struct Source {
-    int32_t cell, order, term, block;
+  // the jobs of a set, bra sector by bra sector: its terms' lists merged, the terms of a sector in order
+  struct Member {
+    List list;
+    DressSrc src;
+    int nidx;  // index length of the dressed operator
   };
-  std::vector<Source> sources;  // of one set
+  std::vector<Member> set;
+  std::vector<DressJob>& jobs = out.jobs;
+  std::vector<DressSrc>& src = out.src;
+  size_t n_src = 0, n_jobs = 0;
+  for (int t = 0; t < n_terms; ++t) n_src += size_t(blocks_of(t).end - blocks_of(t).p);
+  jobs.resize(n_src);
+  src.resize(n_src);
+  n_src = 0;
+  int64_t n_w = 0;
   for (int t0 = 0; t0 < n_terms; ++t0) {
     if (out.rep[size_t(t0)] != t0) continue;
-    const int32_t* r0 = &trm[int64_t(t0) * kTrmCols];
     const TermDress& d = dress[size_t(t0)];
-    const int nb = r0[0], pos = d.pos < 0 ? 0 : d.pos;
-    sources.clear();
-    for (int t = t0, i = 0; t >= 0; t = next[size_t(t)], ++i)
-      each_block(t, [&](int cell, int b) { sources.push_back(Source{cell, i, t, b}); });
-    if (next[size_t(t0)] >= 0)
-      std::sort(sources.begin(), sources.end(), [](const Source& x, const Source& y) {
-        return x.cell != y.cell ? x.cell < y.cell : x.order < y.order;
-      });
-    for (size_t i = 0; i < sources.size();) {
-      DressJob J{};
-      J.src0 = int32_t(out.src.size());
-      const int cell = sources[i].cell;
-      for (; i < sources.size() && sources[i].cell == cell; ++i) {
-        const int t = sources[i].term;
-        const int32_t* r = &trm[int64_t(t) * kTrmCols];
-        const BlockInfo& B = blocks[size_t(sources[i].block)];
-        if (nb > 1 && B.nidx != r[22 + pos]) return "term dims do not match the TDM block";
-        int stride[4];
-        stride[0] = 1;
-        for (int o = 1; o < 4; ++o) stride[o] = stride[o - 1] * r[22 + o - 1];
-        DressSrc S{};
-        S.g_off = B.off;
-        S.ints_off = terms[size_t(t)].ints_off;
-        S.nq = nb == 1 ? 1 : B.nidx;
-        S.stride_q = stride[pos];
-        for (int q = 0; q < d.nrem; ++q) S.rem_stride[q] = stride[d.rem_pos[q]];
-        out.src.push_back(S);
+    const int nb = trm[int64_t(t0) * kTrmCols], pos = d.pos < 0 ? 0 : d.pos;
+    set.clear();
+    for (int t = t0; t >= 0; t = next[size_t(t)]) {
+      const int32_t* r = &trm[int64_t(t) * kTrmCols];
+      int stride[4];
+      stride[0] = 1;
+      for (int o = 1; o < 4; ++o) stride[o] = stride[o - 1] * r[22 + o - 1];
+      Member M{blocks_of(t), DressSrc{}, r[22 + pos]};
+      M.src.ints_off = terms[size_t(t)].ints_off;
+      M.src.nq = nb == 1 ? 1 : r[22 + pos];
+      M.src.stride_q = stride[pos];
+      for (int q = 0; q < d.nrem; ++q) M.src.rem_stride[q] = stride[d.rem_pos[q]];
+      if (M.list.p != M.list.end) set.push_back(M);
+    }
+    DressJob J{};
+    J.rest_len = d.rest_len;
+    J.nrem = d.nrem;
+    for (int q = 0; q < d.nrem; ++q) J.rem_dim[q] = d.rem_dim[q];
+    J.one_body = nb == 1;
+    int64_t* w_index = &out.w_index[size_t(t0) * ss];
+    int32_t* w_mb = &out.w_mb[size_t(t0) * ss];
+    for (;;) {
+      int cell = ss;
+      for (const Member& M : set)
+        if (M.list.p != M.list.end) cell = std::min(cell, M.list.p->fb);
+      if (cell == ss) break;
+      J.src0 = int32_t(n_src);
+      for (Member& M : set) {
+        if (M.list.p == M.list.end || M.list.p->fb != cell) continue;
+        const BlockInfo& B = blocks[size_t(M.list.p++->block)];
+        if (nb > 1 && B.nidx != M.nidx) return "term dims do not match the TDM block";
+        M.src.g_off = B.off;
+        src[n_src++] = M.src;
         J.mb = B.mb;
         J.mk = B.mk;
       }
-      J.n_src = int32_t(out.src.size()) - J.src0;
-      out.n_w = (out.n_w + kAlign - 1) / kAlign * kAlign;  // vector-load alignment of W blocks
-      J.w_off = out.n_w;
-      J.rest_len = d.rest_len;
-      J.nrem = d.nrem;
-      for (int q = 0; q < d.nrem; ++q) J.rem_dim[q] = d.rem_dim[q];
-      J.one_body = nb == 1;
-      out.jobs.push_back(J);
-      const size_t wi = size_t(t0) * ss + cell;
-      out.w_index[wi] = out.n_w;
-      out.w_mb[wi] = J.mb;
-      out.n_w += int64_t(d.rest_len) * J.mb * J.mk;
+      J.n_src = int32_t(n_src) - J.src0;
+      n_w = (n_w + kAlign - 1) / kAlign * kAlign;  // vector-load alignment of W blocks
+      J.w_off = n_w;
+      jobs[n_jobs++] = J;
+      w_index[cell] = n_w;
+      w_mb[cell] = J.mb;
+      n_w += int64_t(d.rest_len) * J.mb * J.mk;
     }
   }
+  jobs.resize(n_jobs);
+  out.n_w = n_w;
   return "";
 }
 
