@@ -231,11 +231,15 @@ struct fcg_ctx {
   // open sigma: the term set's tables on the device (with open_dressing), the plan's working arrays,
   // and how far its hash table is empty
   struct {
-    DevBuf<int32_t> d_trm, d_w_mb, d_rep, d_first_of_tr, d_tr_terms, d_rows, d_nt, d_used;
-    DevBuf<TermDress> d_dress;
-    DevBuf<int64_t> d_w_index, d_wmax_index, d_gmax_off, d_i64, d_bra_dims;
-    DevBuf<int16_t> d_trans, d_bra_fock;
-    DevBuf<uint64_t> d_key;
+    DevBuf<unsigned char> d_tables;
+    const int32_t *trm = nullptr, *w_mb = nullptr, *rep = nullptr, *first_of_tr = nullptr, *tr_terms = nullptr;
+    const TermDress* dress = nullptr;
+    const int64_t *w_index = nullptr, *wmax_index = nullptr, *gmax_off = nullptr;
+    const int16_t* trans = nullptr;
+    DevBuf<int32_t> d_rows, d_used;
+    DevBuf<int64_t> d_i64;
+    DevBuf<unsigned char> d_bra;
+    PinnedBuf<unsigned long long> h_cnt;
     size_t clean_keys = 0, clean_vals = 0;
   } oplan;
   // open sigma (FOIS) working set and last result
@@ -251,8 +255,8 @@ struct fcg_ctx {
   DevBuf<double> d_ovals;
   DevBuf<unsigned long long> d_counters;
   DevBuf<unsigned char> d_scan_tmp;
-  std::vector<int16_t> open_bra_fock;   // [n_bra_sectors][N][2]
-  std::vector<int64_t> open_dims;       // [n_bra_sectors][N]
+  std::vector<unsigned char> open_bra;  // bra sectors: local dimensions [n][N] (int64), Fock sectors [n][N][2] (int16)
+  int64_t open_sectors = 0;
   PinnedBuf<unsigned long long> open_keys;  // keys of the last open sigma, open_rows of them
   PinnedBuf<double> open_vals;              // [open_rows][R] row-major
   int64_t open_rows = 0;

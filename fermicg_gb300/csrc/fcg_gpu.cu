@@ -32,6 +32,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/fcg_gpu.h"
@@ -1249,16 +1250,21 @@ int ensure_open_dressed(fcg_ctx* ctx) {
     std::vector<int32_t> at(first.begin(), first.end() - 1);
     for (int t = 0; t < ctx->n_terms; ++t) terms[size_t(at[size_t(ctx->trm[int64_t(t) * kTrmCols + 1])]++)] = t;
   }
-  FCG_CUDA(O.d_trm.upload(ctx->trm.data(), ctx->trm.size(), ctx->stream));
-  FCG_CUDA(O.d_dress.upload(ctx->dress.data(), ctx->dress.size(), ctx->stream));
-  FCG_CUDA(O.d_w_index.upload(dz.w_index.data(), dz.w_index.size(), ctx->stream));
-  FCG_CUDA(O.d_w_mb.upload(dz.w_mb.data(), dz.w_mb.size(), ctx->stream));
-  FCG_CUDA(O.d_rep.upload(dz.rep.data(), dz.rep.size(), ctx->stream));
-  FCG_CUDA(O.d_wmax_index.upload(ctx->wmax_index.data(), ctx->wmax_index.size(), ctx->stream));
-  FCG_CUDA(O.d_gmax_off.upload(ctx->gmax_off.data(), ctx->gmax_off.size(), ctx->stream));
-  FCG_CUDA(O.d_trans.upload(ctx->trans.data(), ctx->trans.size(), ctx->stream));
-  FCG_CUDA(O.d_first_of_tr.upload(first.data(), first.size(), ctx->stream));
-  FCG_CUDA(O.d_tr_terms.upload(terms.data(), terms.size(), ctx->stream));
+  // one buffer and one copy for all of them
+  std::vector<unsigned char> blob;
+  std::vector<size_t> at;
+  auto put = [&](const auto& v) {
+    at.push_back((blob.size() + 15) / 16 * 16);
+    blob.resize(at.back() + v.size() * sizeof(v[0]));
+    if (!v.empty()) std::memcpy(&blob[at.back()], v.data(), v.size() * sizeof(v[0]));
+  };
+  put(ctx->trm), put(ctx->dress), put(dz.w_index), put(dz.w_mb), put(dz.rep), put(ctx->wmax_index), put(ctx->gmax_off);
+  put(ctx->trans), put(first), put(terms);
+  FCG_CUDA(O.d_tables.upload(blob.data(), blob.size(), ctx->stream));
+  size_t k = 0;
+  auto take = [&](auto*& p) { p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(O.d_tables.p + at[k++]); };
+  take(O.trm), take(O.dress), take(O.w_index), take(O.w_mb), take(O.rep), take(O.wmax_index), take(O.gmax_off);
+  take(O.trans), take(O.first_of_tr), take(O.tr_terms);
   FCG_CUDA(cudaStreamSynchronize(ctx->stream));  // the job list's staging buffer is reused by the next call
   ctx->open_dressed = true;
   return FCG_OK;

@@ -614,9 +614,11 @@ __global__ void __launch_bounds__(kCompactThreads) compact_kernel(unsigned long 
   }
 }
 
+constexpr int64_t kOpenWarps = 152 * 32;
+
 // ---- plan ------------------------------------------------------------------------------------
-// A thread per pair (ket sector, transfer), ket sector major: count, number the bra sectors and
-// scan, write.  Bound: the table reads of term_sector_of, a serial chain per term.  Host loops with
+// Over the pairs (ket sector, transfer), ket sector major: count, number the bra sectors and scan,
+// write.  Bound: the table reads of term_sector_of, a serial chain per term.  Host loops with
 // hash maps took 29 ms for 193 sectors x 1441 transfers (194,496 records) and their upload 1 ms;
 // the kernels take under 1 ms, and the call 28 ms instead of 69 with the emptied table below.
 struct OpenPlan {
@@ -632,6 +634,7 @@ struct OpenPlan {
   const int64_t* gmax_off;
   int64_t n_pairs;
   int n_trans, N, nbody;
+  int warp_pairs;  // pairs of a warp of the count and records kernels
   uint64_t* key;    // bra sector of each pair (4 bits per entry)
   int32_t* nt;      // its terms with at most nbody clusters whose TDM blocks exist; -1: no target
   int64_t* ot;      // the same for the scan (0 without a target)
@@ -639,54 +642,113 @@ struct OpenPlan {
   int64_t* jobs;    // (row, term) jobs
 };
 
-__device__ __forceinline__ bool open_target(const OpenPlan& p, int64_t i, int16_t* fb, int64_t* dims) {
+// the bra sector of pair i (4 bits per entry), false: none
+__device__ __forceinline__ bool open_target(const OpenPlan& p, int64_t i, uint64_t* key) {
   const int64_t sk = i / p.n_trans;
   const int tr = int(i - sk * p.n_trans);
   if (p.first_of_tr[tr] == p.first_of_tr[tr + 1]) return false;
   const int16_t* fk = p.sec_fock + sk * 2 * p.N;
-  for (int c = 0; c < 2 * p.N; ++c) {
-    const int f = fk[c] + p.trans[int64_t(tr) * 2 * p.N + c];
-    if (f < 0 || f > p.norb[c / 2]) return false;
-    fb[c] = int16_t(f);
-  }
-  // every cluster must have a local basis in its bra sector (:39-46)
+  uint64_t k = 0;
   for (int c = 0; c < p.N; ++c) {
-    const int bl = p.tt.blk[dense_block_index(p.tt.nmax1, c, kOpH, fb[2 * c], fb[2 * c + 1], fb[2 * c], fb[2 * c + 1])];
-    if (bl < 0) return false;
-    dims[c] = p.tt.blocks[bl].mb;
+    const int fa = fk[2 * c] + p.trans[(int64_t(tr) * p.N + c) * 2], fb = fk[2 * c + 1] + p.trans[(int64_t(tr) * p.N + c) * 2 + 1];
+    if (fa < 0 || fa > p.norb[c] || fb < 0 || fb > p.norb[c]) return false;
+    // every cluster must have a local basis in its bra sector (:39-46)
+    if (p.tt.blk[dense_block_index(p.tt.nmax1, c, kOpH, fa, fb, fa, fb)] < 0) return false;
+    k |= uint64_t(fa | fb << 4) << (8 * c);
   }
+  *key = k;
   return true;
 }
 
-__global__ void open_count_kernel(OpenPlan p) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i > p.n_pairs) return;
-  int32_t nt = -1;
-  int64_t rows = 0;
-  if (i < p.n_pairs) {
-    int16_t fb[2 * kMaxClusters];
-    int64_t dims[kMaxClusters];
-    if (open_target(p, i, fb, dims)) {
-      uint64_t key = 0;
-      for (int c = 0; c < 2 * p.N; ++c) key |= uint64_t(fb[c]) << (4 * c);
-      p.key[i] = key;
-      const int64_t sk = i / p.n_trans;
-      const int tr = int(i - sk * p.n_trans);
-      const int16_t* fk = p.sec_fock + sk * 2 * p.N;
-      nt = 0;
-      for (int q = p.first_of_tr[tr]; q < p.first_of_tr[tr + 1]; ++q) {
-        const int t = p.tr_terms[q];
-        TermSector ts;
-        int64_t fma;
-        if (p.tt.trm[int64_t(t) * kTrmCols] <= p.nbody && term_sector_of(p.tt, t, fb, fk, ts, &fma)) ++nt;
-      }
-      rows = p.sec_count[sk];
-    }
-    p.nt[i] = nt;
+// The (pair, term) combinations of a warp's pairs, side by side over its lanes.  A warp has p.warp_pairs
+// pairs, lane l the l-th; the terms of a pair are checked in order, 32 combinations a step.  Bound: the
+// chain of table reads of one term (about 7 us with its record), so few pairs are spread over many warps:
+// 12 orbitals, one row, count and records 96 us with a thread for every pair's list, 19 so.
+struct OpenLanes {
+  uint64_t key = 0;        // of this lane's pair: bra sector,
+  int first = 0;           // first term,
+  int begin = 0, end = 0;  // and its combinations [begin, end)
+  int total = 0;           // of the warp
+};
+__device__ __forceinline__ int64_t open_pair_of(const OpenPlan& p) {  // this thread's pair (n_pairs: past the last)
+  const int64_t thread = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  return lane < p.warp_pairs ? min((thread >> 5) * p.warp_pairs + lane, p.n_pairs + 1) : p.n_pairs + 1;
+}
+__device__ __forceinline__ OpenLanes open_lanes(const OpenPlan& p, bool target, int64_t i, uint64_t key) {
+  OpenLanes L;
+  int n = 0;
+  if (target) {
+    const int tr = int(i % p.n_trans);
+    L.key = key;
+    L.first = p.first_of_tr[tr];
+    n = p.first_of_tr[tr + 1] - L.first;
   }
-  p.ot[i] = max(nt, 0);
+  L.end = n;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, L.end, d);
+    if (int(threadIdx.x & 31) >= d) L.end += y;
+  }
+  L.begin = L.end - n;
+  L.total = __shfl_sync(0xffffffffu, L.end, 31);
+  return L;
+}
+
+// one combination: ket sector, term, bra sector
+struct OpenPair {
+  int64_t i;  // pair
+  int lane;   // whose pair
+  int t;
+  const int16_t* fk;
+  int64_t rows;
+  int16_t fb[2 * kMaxClusters];
+};
+// combination x of the warp (all lanes take part; x >= total: none, t < 0)
+__device__ __forceinline__ OpenPair open_pair(const OpenPlan& p, const OpenLanes& L, int x) {
+  int lane = 0;  // pairs that end at or before x
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1)
+    if (__shfl_sync(0xffffffffu, L.end, lane + d - 1) <= x) lane += d;
+  OpenPair P;
+  P.lane = lane;
+  const uint64_t key = __shfl_sync(0xffffffffu, L.key, lane);
+  const int q = __shfl_sync(0xffffffffu, L.first, lane) + x - __shfl_sync(0xffffffffu, L.begin, lane);
+  P.i = ((int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * p.warp_pairs + lane;
+  P.t = -1;
+  if (x >= L.total) return P;
+  const int64_t sk = P.i / p.n_trans;
+  P.t = p.tr_terms[q];
+  P.fk = p.sec_fock + sk * 2 * p.N;
+  P.rows = p.sec_count[sk];
+#pragma unroll
+  for (int c = 0; c < 2 * kMaxClusters; ++c) P.fb[c] = int16_t((key >> (4 * c)) & 15);
+  return P;
+}
+
+__global__ void open_count_kernel(OpenPlan p) {
+  const int64_t i = open_pair_of(p);
+  const int lane = threadIdx.x & 31;
+  uint64_t key = 0;
+  const bool target = i < p.n_pairs && open_target(p, i, &key);
+  const OpenLanes L = open_lanes(p, target, i, key);
+  int nt = 0;
+  for (int x0 = 0; x0 < L.total; x0 += 32) {
+    const OpenPair P = open_pair(p, L, x0 + lane);
+    bool exists, record = false;
+    int64_t fma;
+    if (P.t >= 0 && p.tt.trm[int64_t(P.t) * kTrmCols] <= p.nbody)
+      term_count(p.tt, P.t, P.fb, P.fk, &exists, &record, &fma);
+    const unsigned has = __ballot_sync(0xffffffffu, record);
+    const int lo = max(L.begin - x0, 0), hi = min(L.end - x0, 32);  // this lane's pair in the step
+    if (lo < hi) nt += __popc(has & ((hi < 32 ? 1u << hi : 0u) - 1u) & ~((1u << lo) - 1u));
+  }
+  if (i > p.n_pairs) return;
+  if (i < p.n_pairs) p.nt[i] = target ? nt : -1;
+  if (target) p.key[i] = key;
+  p.ot[i] = nt;
   p.has[i] = nt > 0 ? 1 : 0;
-  p.jobs[i] = nt > 0 ? int64_t(nt) * rows : 0;
+  p.jobs[i] = nt > 0 ? int64_t(nt) * p.sec_count[i / p.n_trans] : 0;
 }
 
 // bra sectors numbered by their first pair: an open-addressed table of pairs (kEmpty: none)
@@ -717,107 +779,161 @@ __global__ void open_first_kernel(OpenPlan p, const unsigned long long* __restri
   flag[i] = r == i ? 1 : 0;
 }
 
-// sizes after the scans, for the host
-__global__ void open_sizes_kernel(int64_t n_pairs, const int64_t* __restrict__ flag, const int64_t* __restrict__ ot,
-                                  const int64_t* __restrict__ has, const int64_t* __restrict__ jobs,
-                                  unsigned long long* __restrict__ counters) {
-  counters[5] = (unsigned long long)flag[n_pairs];
-  counters[6] = (unsigned long long)ot[n_pairs];
-  counters[7] = (unsigned long long)has[n_pairs];
-  counters[8] = (unsigned long long)jobs[n_pairs];
+// the last elements of four scanned arrays of n behind one another, for the host
+__global__ void open_sizes_kernel(const int64_t* __restrict__ a, int64_t n, unsigned long long* __restrict__ out) {
+  out[threadIdx.x] = (unsigned long long)a[(threadIdx.x + 1) * n - 1];
 }
 
-// the records, items and bra sectors; counters [9] .. [13]; used[block] = 1 for every TDM block read.
-// Scanned: flag (bra sector ids), ot, has, jobs.
+// The same with the scans, a CTA (1024 threads) per array: spaces of few sectors, whose call is some
+// twenty launches of a few microseconds (12 orbitals, one row: 3 us for five kernels' 9).
+constexpr int64_t kOpenScan = 8192;
+__global__ void __launch_bounds__(1024) open_scan_kernel(int64_t* __restrict__ a, int64_t n, unsigned long long* __restrict__ out) {
+  __shared__ int64_t sums[32];
+  int64_t* v = a + blockIdx.x * n;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  int64_t before = 0;  // of the earlier rounds
+  for (int64_t i0 = 0; i0 < n; i0 += 1024) {
+    const int64_t i = i0 + threadIdx.x;
+    const int64_t own = i < n ? v[i] : 0;
+    int64_t x = own;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int64_t y = __shfl_up_sync(0xffffffffu, x, d);
+      if (lane >= d) x += y;
+    }
+    if (lane == 31) sums[wid] = x;
+    __syncthreads();
+    int64_t all = 0, below = 0;
+    for (int w = 0; w < 32; ++w) {
+      const int64_t y = sums[w];
+      all += y;
+      if (w < wid) below += y;
+    }
+    if (i < n) v[i] = before + below + x - own;
+    before += all;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) out[blockIdx.x] = (unsigned long long)v[n - 1];
+}
+
+// what the records of a thread add to the counters
+struct OpenSums {
+  unsigned long long flops = 0, d_max = 1, reg = 0, shared = 0, err = 0;
+};
+
+// the record of a combination (false: none); used[block] = 1 for every TDM block read
+__device__ __forceinline__ bool open_record(const OpenPlan& p, const OpenPair& P, int32_t bs, OpenTerm& o,
+                                            int32_t* __restrict__ used, OpenSums& S) {
+  const int t = P.t;
+  const int32_t* r = p.tt.trm + int64_t(t) * kTrmCols;
+  int64_t fma;
+  o = OpenTerm{};
+  if (r[0] > p.nbody || !term_sector_of(p.tt, t, P.fb, P.fk, o.ts, &fma)) return false;
+  const int nmax1 = p.tt.nmax1;
+  auto block_of = [&](int c, int op) {
+    return p.tt.blk[dense_block_index(nmax1, c, op, P.fb[2 * c], P.fb[2 * c + 1], P.fk[2 * c], P.fk[2 * c + 1])];
+  };
+  const TermDress& dr = p.tt.dress[t];
+  const int cw = r[2 + (dr.pos < 0 ? 0 : dr.pos)];
+  o.wmax_off = p.wmax_index[(int64_t(t) * nmax1 + P.fb[2 * cw]) * nmax1 + P.fb[2 * cw + 1]];
+  o.bsec = bs;
+  o.n_act = int8_t(1 + o.ts.nrem);
+  o.c_act[0] = int8_t(cw);
+  o.mb_act[0] = int16_t(o.ts.w_mb);
+  int64_t cnt = o.ts.w_mb;
+  for (int a = 0; a < o.ts.nrem; ++a) {
+    o.gmax_off[a] = p.gmax_off[block_of(o.ts.cr[a], r[6 + dr.rem_pos[a]])];
+    o.c_act[1 + a] = o.ts.cr[a];
+    o.mb_act[1 + a] = int16_t(o.ts.g_mb[a]);
+    cnt *= o.ts.g_mb[a];
+    if (a > 0) S.d_max = max(S.d_max, (unsigned long long)o.ts.g_dim[a]);
+  }
+  if (cnt >= (int64_t(1) << 31)) S.err = 2;
+  o.out_count = int32_t(cnt);
+  S.reg = max(S.reg, (unsigned long long)expand_tiles(o.ts.nrem, o.ts.rest_len, o.ts.g_dim, o.mb_act, false).bytes);
+  S.shared = max(S.shared, (unsigned long long)expand_tiles(o.ts.nrem, o.ts.rest_len, o.ts.g_dim, o.mb_act, true).bytes);
+  // the reference's GEMM flops of this (ket, term) job (contract_matvec_thread,
+  // src/tpsci_matvec_thread.jl:279-818, no prescreen): bra dims M and orbital index
+  // lengths n in term order
+  int64_t M[4] = {1, 1, 1, 1}, n[4] = {1, 1, 1, 1};
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+    if (a < r[0]) {
+      const int bl = block_of(r[2 + a], r[6 + a]);
+      M[a] = p.tt.blocks[bl].mb;
+      n[a] = r[22 + a];
+      used[bl] = 1;
+    }
+  int64_t f = 0;
+  if (r[0] == 2) f = n[0] * n[1] * M[0] + n[1] * M[0] * M[1];
+  if (r[0] == 3) f = M[2] * (n[0] * n[1] * n[2] + n[0] * n[1] * M[1] + n[0] * M[0] * M[1]);
+  if (r[0] == 4)
+    f = M[3] * (n[0] * n[1] * n[2] * n[3] + M[2] * (n[0] * n[1] * n[2] + n[0] * n[1] * M[1] + n[0] * M[0] * M[1]));
+  S.flops += (unsigned long long)(2 * f * P.rows);
+  return true;
+}
+
+// the records, items and bra sectors; counters [9] .. [13].  Scanned: flag (bra sector ids), ot, has, jobs.
 __global__ void open_records_kernel(OpenPlan p, const int64_t* __restrict__ rep, const int64_t* __restrict__ id,
                                     OpenTerm* __restrict__ ots, OpenItem* __restrict__ items,
                                     int64_t* __restrict__ prefix, int16_t* __restrict__ bra_fock,
                                     int64_t* __restrict__ strides, int64_t* __restrict__ bra_dims,
                                     int32_t* __restrict__ used, unsigned long long* __restrict__ counters) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= p.n_pairs) return;
+  const int64_t i = open_pair_of(p);
+  const int lane = threadIdx.x & 31;
   if (i == 0) prefix[p.has[p.n_pairs]] = p.jobs[p.n_pairs];
-  if (rep[i] < 0) return;
-  int16_t fb[2 * kMaxClusters];
-  int64_t dims[kMaxClusters];
-  open_target(p, i, fb, dims);
-  const int64_t sk = i / p.n_trans;
-  const int tr = int(i - sk * p.n_trans);
-  const int16_t* fk = p.sec_fock + sk * 2 * p.N;
-  const int32_t bs = int32_t(id[rep[i]]);
-  if (rep[i] == i) {
+  const bool target = i < p.n_pairs && rep[i] >= 0;
+  const uint64_t key = target ? p.key[i] : 0;
+  const int32_t bs = target ? int32_t(id[rep[i]]) : 0;
+  OpenSums S;
+  if (target && rep[i] == i) {
     int64_t stride = 1;
     for (int c = 0; c < p.N; ++c) {
-      bra_fock[(int64_t(bs) * p.N + c) * 2] = fb[2 * c];
-      bra_fock[(int64_t(bs) * p.N + c) * 2 + 1] = fb[2 * c + 1];
+      const int fa = int((key >> (8 * c)) & 15), fb = int((key >> (8 * c + 4)) & 15);
+      const int64_t dim = p.tt.blocks[p.tt.blk[dense_block_index(p.tt.nmax1, c, kOpH, fa, fb, fa, fb)]].mb;
+      bra_fock[(int64_t(bs) * p.N + c) * 2] = int16_t(fa);
+      bra_fock[(int64_t(bs) * p.N + c) * 2 + 1] = int16_t(fb);
       strides[int64_t(bs) * p.N + c] = stride;
-      bra_dims[int64_t(bs) * p.N + c] = dims[c];
-      stride = min(stride * dims[c], int64_t(1) << kKeyIdxBits);
+      bra_dims[int64_t(bs) * p.N + c] = dim;
+      stride = min(stride * dim, int64_t(1) << kKeyIdxBits);
     }
-    if (stride >= (int64_t(1) << kKeyIdxBits)) atomicMax(counters + 10, 1ull);
+    if (stride >= (int64_t(1) << kKeyIdxBits)) S.err = 1;
   }
-  if (p.has[i] == p.has[i + 1]) return;
-  const int64_t it = p.has[i];
-  prefix[it] = p.jobs[i];
-  int64_t at = p.ot[i];
-  items[it] = OpenItem{p.sec_start[sk], p.sec_count[sk], int32_t(at), int32_t(p.ot[i + 1] - at)};
-  const int nmax1 = p.tt.nmax1;
-  auto block_of = [&](int c, int op) {
-    return p.tt.blk[dense_block_index(nmax1, c, op, fb[2 * c], fb[2 * c + 1], fk[2 * c], fk[2 * c + 1])];
-  };
-  unsigned long long flops = 0, d_max = 1, reg = 0, shared = 0;
-  for (int q = p.first_of_tr[tr]; q < p.first_of_tr[tr + 1]; ++q) {
-    const int t = p.tr_terms[q];
-    const int32_t* r = p.tt.trm + int64_t(t) * kTrmCols;
-    OpenTerm o{};
-    int64_t fma;
-    if (r[0] > p.nbody || !term_sector_of(p.tt, t, fb, fk, o.ts, &fma)) continue;
-    const TermDress& dr = p.tt.dress[t];
-    const int cw = r[2 + (dr.pos < 0 ? 0 : dr.pos)];
-    o.wmax_off = p.wmax_index[(int64_t(t) * nmax1 + fb[2 * cw]) * nmax1 + fb[2 * cw + 1]];
-    o.bsec = bs;
-    o.n_act = int8_t(1 + o.ts.nrem);
-    o.c_act[0] = int8_t(cw);
-    o.mb_act[0] = int16_t(o.ts.w_mb);
-    int64_t cnt = o.ts.w_mb;
-    for (int a = 0; a < o.ts.nrem; ++a) {
-      o.gmax_off[a] = p.gmax_off[block_of(o.ts.cr[a], r[6 + dr.rem_pos[a]])];
-      o.c_act[1 + a] = o.ts.cr[a];
-      o.mb_act[1 + a] = int16_t(o.ts.g_mb[a]);
-      cnt *= o.ts.g_mb[a];
-      if (a > 0) d_max = max(d_max, (unsigned long long)o.ts.g_dim[a]);
-    }
-    if (cnt >= (int64_t(1) << 31)) atomicMax(counters + 10, 2ull);
-    o.out_count = int32_t(cnt);
-    reg = max(reg, (unsigned long long)expand_tiles(o.ts.nrem, o.ts.rest_len, o.ts.g_dim, o.mb_act, false).bytes);
-    shared = max(shared, (unsigned long long)expand_tiles(o.ts.nrem, o.ts.rest_len, o.ts.g_dim, o.mb_act, true).bytes);
-    // the reference's GEMM flops of this (ket, term) job (contract_matvec_thread,
-    // src/tpsci_matvec_thread.jl:279-818, no prescreen): bra dims M and orbital index
-    // lengths n in term order
-    int64_t M[4] = {1, 1, 1, 1}, n[4] = {1, 1, 1, 1};
+  if (target && p.has[i] != p.has[i + 1]) {
+    const int64_t it = p.has[i];
+    prefix[it] = p.jobs[i];
+    items[it] = OpenItem{p.sec_start[i / p.n_trans], p.sec_count[i / p.n_trans], int32_t(p.ot[i]),
+                         int32_t(p.ot[i + 1] - p.ot[i])};
+  }
+  // the warp's records follow one another from its first pair's
+  const OpenLanes L = open_lanes(p, target, i, target ? p.key[i] : 0);
+  int64_t at = __shfl_sync(0xffffffffu, p.ot[min(i, p.n_pairs)], 0);
+  OpenTerm o;
+  for (int x0 = 0; x0 < L.total; x0 += 32) {
+    const OpenPair P = open_pair(p, L, x0 + lane);
+    const int32_t b = __shfl_sync(0xffffffffu, bs, P.lane & 31);
+    const bool has = P.t >= 0 && open_record(p, P, b, o, used, S);
+    const unsigned m = __ballot_sync(0xffffffffu, has);
+    if (has) ots[at + __popc(m & ((1u << lane) - 1u))] = o;
+    at += __popc(m);
+  }
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
-      if (a < r[0]) {
-        const int bl = block_of(r[2 + a], r[6 + a]);
-        M[a] = p.tt.blocks[bl].mb;
-        n[a] = r[22 + a];
-        used[bl] = 1;
-      }
-    int64_t f = 0;
-    if (r[0] == 2) f = n[0] * n[1] * M[0] + n[1] * M[0] * M[1];
-    if (r[0] == 3) f = M[2] * (n[0] * n[1] * n[2] + n[0] * n[1] * M[1] + n[0] * M[0] * M[1]);
-    if (r[0] == 4)
-      f = M[3] * (n[0] * n[1] * n[2] * n[3] + M[2] * (n[0] * n[1] * n[2] + n[0] * n[1] * M[1] + n[0] * M[0] * M[1]));
-    flops += (unsigned long long)(2 * f * p.sec_count[sk]);
-    ots[at++] = o;
+  for (int d = 16; d > 0; d >>= 1) {
+    S.flops += __shfl_xor_sync(0xffffffffu, S.flops, d);
+    S.d_max = max(S.d_max, __shfl_xor_sync(0xffffffffu, S.d_max, d));
+    S.reg = max(S.reg, __shfl_xor_sync(0xffffffffu, S.reg, d));
+    S.shared = max(S.shared, __shfl_xor_sync(0xffffffffu, S.shared, d));
+    S.err = max(S.err, __shfl_xor_sync(0xffffffffu, S.err, d));
   }
-  if (flops) atomicAdd(counters + 9, flops);
+  if (lane != 0) return;
+  if (S.flops) atomicAdd(counters + 9, S.flops);
   auto raise = [&](int k, unsigned long long v) {  // a stale read only costs an atomic
     if (*reinterpret_cast<volatile unsigned long long*>(counters + k) < v) atomicMax(counters + k, v);
   };
-  raise(11, d_max);
-  raise(12, reg);
-  raise(13, shared);
+  raise(10, S.err);
+  raise(11, S.d_max);
+  raise(12, S.reg);
+  raise(13, S.shared);
 }
 
 __global__ void open_bytes_kernel(int64_t n_blocks, const int32_t* __restrict__ used, const BlockInfo* __restrict__ blocks,
@@ -884,50 +1000,59 @@ int fcg_sigma_open(fcg_ctx* ctx, int R, const double* c, double thresh, int nbod
     rows[size_t(n_sec + i)] = int32_t(P.sec_count[size_t(i)]);
   }
   FCG_CUDA(O.d_rows.upload(rows.data(), rows.size(), s));
-  FCG_CUDA(O.d_key.alloc(size_t(n_pairs)));
-  // table, ot, has, jobs, slot, rep, flag, scratch of the scans
+  // table, flag, ot, has, jobs, slot, rep, keys, counts, scratch of the scans
   const int64_t n1 = n_pairs + 1, scr = dprim::scan_scratch(n1) + 1;
-  FCG_CUDA(O.d_nt.alloc(size_t(n1)));
-  FCG_CUDA(O.d_i64.alloc(size_t(cap_tab + 6 * n1 + scr)));
+  FCG_CUDA(O.d_i64.alloc(size_t(cap_tab + 8 * n1 + scr)));
   FCG_CUDA(O.d_used.alloc(ctx->h_blocks.size()));
   FCG_CUDA(ctx->d_counters.alloc(kCounters));
   FCG_CUDA(cudaMemsetAsync(ctx->d_counters.p, 0, kCounters * sizeof(unsigned long long), s));
   FCG_CUDA(cudaMemsetAsync(O.d_used.p, 0, ctx->h_blocks.size() * sizeof(int32_t), s));
   OpenPlan op{};
-  op.tt = TermTables{O.d_trm.p, O.d_dress.p, O.d_w_index.p, O.d_w_mb.p, O.d_rep.p, ctx->d_blk_index.p, ctx->d_blocks.p,
-                     ctx->nmax + 1};
+  op.tt = TermTables{O.trm, O.dress, O.w_index, O.w_mb, O.rep, ctx->d_blk_index.p, ctx->d_blocks.p, ctx->nmax + 1};
   op.sec_fock = ctx->d_sec_fock.p;
   op.sec_start = O.d_rows.p;
   op.sec_count = O.d_rows.p + n_sec;
-  op.trans = O.d_trans.p;
-  op.first_of_tr = O.d_first_of_tr.p;
-  op.tr_terms = O.d_tr_terms.p;
+  op.trans = O.trans;
+  op.first_of_tr = O.first_of_tr;
+  op.tr_terms = O.tr_terms;
   op.norb = ctx->d_norb.p;
-  op.wmax_index = O.d_wmax_index.p;
-  op.gmax_off = O.d_gmax_off.p;
+  op.wmax_index = O.wmax_index;
+  op.gmax_off = O.gmax_off;
   op.n_pairs = n_pairs;
   op.n_trans = ctx->n_trans;
   op.N = N;
   op.nbody = nbody;
-  op.key = O.d_key.p;
-  op.nt = O.d_nt.p;
+  // as few pairs to a warp as keep the chip's warps (32 an SM) busy
+  op.warp_pairs = 1;
+  while (op.warp_pairs < 32 && n_pairs > int64_t(op.warp_pairs) * kOpenWarps) op.warp_pairs *= 2;
+  const unsigned warp_grid = unsigned(((n_pairs + op.warp_pairs) / op.warp_pairs * 32 + kT - 1) / kT);
   auto* table = reinterpret_cast<unsigned long long*>(O.d_i64.p);
-  op.ot = O.d_i64.p + cap_tab;
+  int64_t* flag = O.d_i64.p + cap_tab;
+  op.ot = flag + n1;
   op.has = op.ot + n1;
   op.jobs = op.has + n1;
-  int64_t *slot = op.jobs + n1, *rep = slot + n1, *flag = rep + n1, *scratch = flag + n1;
+  int64_t *slot = op.jobs + n1, *rep = slot + n1;
+  op.key = reinterpret_cast<uint64_t*>(rep + n1);
+  op.nt = reinterpret_cast<int32_t*>(op.key + n1);
+  int64_t* scratch = O.d_i64.p + cap_tab + 8 * n1;
   FCG_CUDA(cudaMemsetAsync(table, 0xFF, size_t(cap_tab) * sizeof(int64_t), s));
-  open_count_kernel<<<grid_of(n1), kT, 0, s>>>(op);
+  open_count_kernel<<<warp_grid, kT, 0, s>>>(op);
   FCG_CUDA(cudaGetLastError());
   open_sectors_kernel<<<grid_of(n_pairs), kT, 0, s>>>(op, table, cap_tab - 1, slot);
   FCG_CUDA(cudaGetLastError());
   open_first_kernel<<<grid_of(n1), kT, 0, s>>>(op, table, slot, rep, flag);
   FCG_CUDA(cudaGetLastError());
-  for (int64_t* a : {flag, op.ot, op.has, op.jobs}) FCG_CUDA(dprim::exclusive_scan<int64_t>(a, n1, scratch, s));
-  open_sizes_kernel<<<1, 1, 0, s>>>(n_pairs, flag, op.ot, op.has, op.jobs, ctx->d_counters.p);
+  if (n1 <= kOpenScan) {
+    open_scan_kernel<<<4, 1024, 0, s>>>(flag, n1, ctx->d_counters.p + 5);
+  } else {
+    for (int k = 0; k < 4; ++k) FCG_CUDA(dprim::exclusive_scan<int64_t>(flag + k * n1, n1, scratch, s));
+    open_sizes_kernel<<<1, 4, 0, s>>>(flag, n1, ctx->d_counters.p + 5);
+  }
   FCG_CUDA(cudaGetLastError());
-  unsigned long long cnt[kCounters];
-  FCG_CUDA(cudaMemcpyAsync(cnt, ctx->d_counters.p, sizeof(cnt), cudaMemcpyDeviceToHost, s));
+  FCG_CUDA(O.h_cnt.alloc(kCounters));
+  const unsigned long long* cnt = O.h_cnt.p;  // page-locked: three or four waits of a call end with this copy
+  constexpr size_t kCntBytes = kCounters * sizeof(unsigned long long);
+  FCG_CUDA(cudaMemcpyAsync(O.h_cnt.p, ctx->d_counters.p, kCntBytes, cudaMemcpyDeviceToHost, s));
   FCG_CUDA(cudaStreamSynchronize(s));
   const int64_t n_bra = int64_t(cnt[5]), n_ots = int64_t(cnt[6]), n_items = int64_t(cnt[7]), n_jobs = int64_t(cnt[8]);
   FCG_REQUIRE(n_bra < (1 << 23), FCG_ELIMIT, "too many bra sectors for the open sigma key");
@@ -938,26 +1063,23 @@ int fcg_sigma_open(fcg_ctx* ctx, int R, const double* c, double thresh, int nbod
   FCG_CUDA(ctx->d_oitems.alloc(size_t(n_items)));
   FCG_CUDA(ctx->d_oprefix.alloc(size_t(n_items + 1)));
   FCG_CUDA(ctx->d_ostrides.alloc(size_t(n_bra * N)));
-  FCG_CUDA(O.d_bra_fock.alloc(size_t(n_bra * N * 2)));
-  FCG_CUDA(O.d_bra_dims.alloc(size_t(n_bra * N)));
-  open_records_kernel<<<grid_of(n_pairs), kT, 0, s>>>(op, rep, flag, ctx->d_oterms.p, ctx->d_oitems.p, ctx->d_oprefix.p,
-                                                      O.d_bra_fock.p, ctx->d_ostrides.p, O.d_bra_dims.p, O.d_used.p,
-                                                      ctx->d_counters.p);
+  // local dimensions of the bra sectors, then their Fock sectors
+  const size_t bra_bytes = size_t(n_bra * N) * (sizeof(int64_t) + 2 * sizeof(int16_t));
+  FCG_CUDA(O.d_bra.alloc(bra_bytes));
+  int64_t* d_dims = reinterpret_cast<int64_t*>(O.d_bra.p);
+  int16_t* d_fock = reinterpret_cast<int16_t*>(d_dims + n_bra * N);
+  open_records_kernel<<<warp_grid, kT, 0, s>>>(op, rep, flag, ctx->d_oterms.p, ctx->d_oitems.p, ctx->d_oprefix.p, d_fock,
+                                               ctx->d_ostrides.p, d_dims, O.d_used.p, ctx->d_counters.p);
   FCG_CUDA(cudaGetLastError());
   open_bytes_kernel<<<grid_of(int64_t(ctx->h_blocks.size())), kT, 0, s>>>(int64_t(ctx->h_blocks.size()), O.d_used.p,
                                                                          ctx->d_blocks.p, ctx->d_counters.p);
   FCG_CUDA(cudaGetLastError());
-  ctx->open_bra_fock.resize(size_t(n_bra * N * 2));
-  ctx->open_dims.resize(size_t(n_bra * N));
-  if (n_bra > 0) {
-    FCG_CUDA(cudaMemcpyAsync(ctx->open_bra_fock.data(), O.d_bra_fock.p, sizeof(int16_t) * size_t(n_bra * N * 2),
-                             cudaMemcpyDeviceToHost, s));
-    FCG_CUDA(cudaMemcpyAsync(ctx->open_dims.data(), O.d_bra_dims.p, sizeof(int64_t) * size_t(n_bra * N),
-                             cudaMemcpyDeviceToHost, s));
-  }
+  ctx->open_bra.resize(bra_bytes);
+  ctx->open_sectors = n_bra;
+  if (n_bra > 0) FCG_CUDA(cudaMemcpyAsync(ctx->open_bra.data(), O.d_bra.p, bra_bytes, cudaMemcpyDeviceToHost, s));
   const int64_t n = ctx->n_cfg;
   if (n_items == 0) {  // no term reaches a sector with a basis
-    FCG_CUDA(cudaMemcpyAsync(cnt, ctx->d_counters.p, sizeof(cnt), cudaMemcpyDeviceToHost, s));
+    FCG_CUDA(cudaMemcpyAsync(O.h_cnt.p, ctx->d_counters.p, kCntBytes, cudaMemcpyDeviceToHost, s));
     FCG_CUDA(cudaStreamSynchronize(s));
     FCG_REQUIRE(cnt[10] == 0, FCG_ELIMIT, "bra sector product space exceeds 2^40");
     return FCG_OK;
@@ -985,14 +1107,14 @@ int fcg_sigma_open(fcg_ctx* ctx, int R, const double* c, double thresh, int nbod
   screen_kernel<<<unsigned((n_jobs + 255) / 256), 256, 0, s>>>(p, ctx->d_wmax.p, ctx->d_gmax.p, ctx->d_ojobs.p,
                                                               ctx->d_counters.p);
   FCG_CUDA(cudaGetLastError());
-  FCG_CUDA(cudaMemcpyAsync(cnt, ctx->d_counters.p, sizeof(cnt), cudaMemcpyDeviceToHost, s));
+  FCG_CUDA(cudaMemcpyAsync(O.h_cnt.p, ctx->d_counters.p, kCntBytes, cudaMemcpyDeviceToHost, s));
   FCG_CUDA(cudaStreamSynchronize(s));
   FCG_REQUIRE(cnt[10] == 0, FCG_ELIMIT, cnt[10] == 1 ? "bra sector product space exceeds 2^40"
                                                         : "bra tuples of one term exceed 2^31");
   const int64_t n_kept = int64_t(cnt[0]);
   const int64_t n_elem = int64_t(cnt[1]);
   const int64_t flops_ref = int64_t(cnt[9]), tdm_bytes = int64_t(cnt[14]);
-  int launches = 8;
+  int launches = 8;  // (the scans of a large plan not counted)
   if (n_kept > 0) {
     // a warp's slice: the largest job tiles, up to kExpSlice; as many warps to a CTA as fit.
     // The register sums serve index lengths up to kExpMaxD (the second and third remaining
@@ -1033,7 +1155,7 @@ int fcg_sigma_open(fcg_ctx* ctx, int R, const double* c, double thresh, int nbod
           ExpandTable{ctx->d_hkeys.p, ctx->d_hvals.p, cap - 1, ctx->d_counters.p}, slice);
       FCG_CUDA(cudaGetLastError());
       FCG_CUDA(cudaEventRecord(ctx->ev3, s));
-      FCG_CUDA(cudaMemcpyAsync(cnt, ctx->d_counters.p, sizeof(cnt), cudaMemcpyDeviceToHost, s));
+      FCG_CUDA(cudaMemcpyAsync(O.h_cnt.p, ctx->d_counters.p, kCntBytes, cudaMemcpyDeviceToHost, s));
       FCG_CUDA(cudaStreamSynchronize(s));
       launches += 2;
       if (cnt[2] == 0) {
@@ -1051,7 +1173,7 @@ int fcg_sigma_open(fcg_ctx* ctx, int R, const double* c, double thresh, int nbod
                                                                            ctx->d_counters.p);
     FCG_CUDA(cudaGetLastError());
     FCG_CUDA(cudaEventRecord(ctx->ev1, s));
-    FCG_CUDA(cudaMemcpyAsync(cnt, ctx->d_counters.p, sizeof(cnt), cudaMemcpyDeviceToHost, s));
+    FCG_CUDA(cudaMemcpyAsync(O.h_cnt.p, ctx->d_counters.p, kCntBytes, cudaMemcpyDeviceToHost, s));
     FCG_CUDA(cudaStreamSynchronize(s));
     launches += 1;
     O.clean_keys = keys_after;
@@ -1088,14 +1210,16 @@ int fcg_sigma_open_fetch(fcg_ctx* ctx, int16_t* fock, int16_t* cfg, double* coef
   const int N = ctx->N;
   const int R = ctx->open_R;
   const int64_t m = ctx->open_rows;
+  const int64_t* dims = reinterpret_cast<const int64_t*>(ctx->open_bra.data());
+  const int16_t* bra_fock = reinterpret_cast<const int16_t*>(dims + ctx->open_sectors * N);
 #pragma omp parallel for schedule(static)
   for (int64_t i = 0; i < m; ++i) {
     const unsigned long long key = ctx->open_keys.p[i];
     const int64_t bs = int64_t(key >> kKeyIdxBits);
     int64_t idx = int64_t(key & ((1ull << kKeyIdxBits) - 1));
-    std::memcpy(fock + i * 2 * N, &ctx->open_bra_fock[bs * 2 * N], sizeof(int16_t) * 2 * N);
+    std::memcpy(fock + i * 2 * N, bra_fock + bs * 2 * N, sizeof(int16_t) * 2 * N);
     for (int c = 0; c < N; ++c) {
-      const int64_t d = ctx->open_dims[bs * N + c];
+      const int64_t d = dims[bs * N + c];
       cfg[i * N + c] = int16_t(idx % d);
       idx /= d;
     }
