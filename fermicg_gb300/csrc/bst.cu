@@ -2045,19 +2045,30 @@ std::string check_groups(const std::vector<BstGroup>& groups, const std::vector<
   return "";
 }
 
+// the fields of the groups that bst_lists looks at, side by side
+std::vector<BstBrief> briefs(const std::vector<BstGroup>& groups) {
+  std::vector<BstBrief> out(groups.size());
+#pragma omp parallel for schedule(static)
+  for (int64_t g = 0; g < int64_t(groups.size()); ++g) {
+    const BstGroup& G = groups[size_t(g)];
+    out[size_t(g)] = BstBrief{G.bra, G.m, G.k, G.bcore / std::max(G.m, 1), G.bcore, G.kcore, G.ws, G.post};
+  }
+  return out;
+}
+
 // multiply-adds and element moves of one group's sigma step, about
-int64_t group_work(const BstGroup& G, int R) {
-  return int64_t(R) * (int64_t(G.m) * G.k * (G.bcore / std::max(G.m, 1)) + 2 * G.kcore + 64);
+int64_t group_work(const BstBrief& G, int R) {
+  return int64_t(R) * (int64_t(G.m) * G.k * G.ns + 2 * G.kcore + 64);
 }
 
 // the same of an entry of a chunk (one root, nc columns); its chain of barriers costs about as much
 // as 2^13 of them
-int64_t entry_work(const BstGroup& G, int64_t nc) {
-  return nc * G.k * (G.bcore / std::max(G.m, 1)) + 5 * int64_t(G.kcore) + (int64_t(1) << 13);
+int64_t entry_work(const BstBrief& G, int64_t nc) {
+  return nc * G.k * G.ns + 5 * int64_t(G.kcore) + (int64_t(1) << 13);
 }
 
 // bytes of a group's bra position tables
-int64_t tab_bytes(const BstGroup& G) { return 2 * int64_t(G.m + G.bcore / std::max(G.m, 1)) + 16; }
+int64_t tab_bytes(const BstBrief& G) { return 2 * int64_t(G.m + G.ns) + 16; }
 
 // Groups by where they run.  GEMM-shaped groups of a float build go to the tensor cores.  Groups
 // whose workspace fits a warp slice and whose bra block's R cores fit kAccBytes go to
@@ -2078,7 +2089,8 @@ void bst_lists(fcg_ctx* ctx, int R, size_t elem) {
   ctx->bst_tc_ws_total = 0;
   ctx->bst_tc_flops = 0;
   ctx->bst_tc_mma_flops = 0;
-  const size_t ng = ctx->bst_groups.size();
+  const std::vector<BstBrief>& groups = ctx->bst_brief;
+  const size_t ng = groups.size();
   const int64_t head = elem == 4 ? ChunkHead<float>::n : ChunkHead<double>::n;
   // where each group runs: a warp slice, a chunk bucket, global workspaces, the tensor cores
   constexpr uint8_t kWarp = 100, kLarge = 101, kTc = 102;
@@ -2086,8 +2098,8 @@ void bst_lists(fcg_ctx* ctx, int R, size_t elem) {
   int64_t warp_work = 0, chunk_work = 0;
   int64_t n_large = 0;  // groups larger than a CTA's memory
   for (size_t q = 0; q < ng; ++q) {
-    const BstGroup& G = ctx->bst_groups[q];
-    const int64_t ns = G.bcore / std::max(G.m, 1);
+    const BstBrief& G = groups[q];
+    const int64_t ns = G.ns;
     if (elem == 4 && ctx->bst_tc_on && G.m >= kTcMinM && G.k >= kTcMinK && ns * R >= kTcMinN) {
       where[q] = kTc;
     } else if (size_t(R) * G.bcore * elem <= size_t(kAccBytes) &&
@@ -2114,7 +2126,7 @@ void bst_lists(fcg_ctx* ctx, int R, size_t elem) {
   if (elem == 8 && n_large >= kLargeEnough)
     for (size_t q = 0; q < ng; ++q)
       if (where[q] < kChunkBuckets && where[q] > kChunkAccMax - 1) {
-        const BstGroup& G = ctx->bst_groups[q];
+        const BstBrief& G = groups[q];
         chunk_work -= R * entry_work(G, G.m);
         where[q] = kLarge;
       }
@@ -2130,18 +2142,20 @@ void bst_lists(fcg_ctx* ctx, int R, size_t elem) {
   std::vector<int64_t> warp_chunk_work;  // per chunk of bst_sigma_bra_kernel
   size_t g = 0;
   while (g < ng) {
-    const int32_t b = ctx->bst_groups[g].bra;
+    const int32_t b = groups[g].bra;
     size_t g1 = g;
-    while (g1 < ng && ctx->bst_groups[g1].bra == b) ++g1;  // groups of one bra are contiguous
+    while (g1 < ng && groups[g1].bra == b) ++g1;  // groups of one bra are contiguous
     int64_t work = 0;
     bool open = false;
     for (auto& v : of_bucket) v.clear();
     for (size_t q = g; q < g1; ++q) {
-      const BstGroup& G = ctx->bst_groups[q];
-      const int64_t ns = G.bcore / std::max(G.m, 1);
+      const BstBrief& G = groups[q];
+      const int64_t ns = G.ns;
       if (where[q] < kChunkBuckets) {
         of_bucket[where[q]].push_back(int32_t(q));
-      } else if (where[q] == kTc) {
+        continue;
+      }
+      if (where[q] == kTc) {
         // GEMM-shaped: tensor cores (its operand X in a global workspace of its own)
         const int32_t tc = int32_t(ctx->bst_tc.size());
         ctx->bst_tc.push_back(int32_t(q));
@@ -2155,6 +2169,7 @@ void bst_lists(fcg_ctx* ctx, int R, size_t elem) {
           }
         ctx->bst_tc_flops += 2 * int64_t(G.m) * G.k * ns * R;
       } else if (where[q] == kWarp) {
+        const int64_t gw = group_work(G, R);
         // a chunk's own cost: its warps' copies of the bra core zeroed and summed
         if (!open || work > std::max(warp_cut, std::min(kChunkWorkMax, kChunkBraWork * R * G.bcore))) {
           if (open) ctx->bst_bra_ptr.push_back(int64_t(ctx->bst_bra_glist.size()));
@@ -2166,8 +2181,8 @@ void bst_lists(fcg_ctx* ctx, int R, size_t elem) {
         const size_t need = sizeof(BstGroup) + size_t(2) * R * G.ws * elem;
         ctx->bst_bra_glist.push_back(int32_t(q));
         ctx->bst_bra_slice = std::max(ctx->bst_bra_slice, int((need + 15) / 16 * 16));
-        work += group_work(G, R);
-        warp_chunk_work.back() += group_work(G, R);
+        work += gw;
+        warp_chunk_work.back() += gw;
       } else if (where[q] == kLarge) {
         ctx->bst_large.push_back(int32_t(q));
         ctx->bst_ws_large = std::max(ctx->bst_ws_large, G.ws);
@@ -2199,8 +2214,8 @@ void bst_lists(fcg_ctx* ctx, int R, size_t elem) {
       P.c.bcore = ctx->bst_blocks[b].core_len;
       P.c.acc = i <= kChunkAccMax ? 1 : 0;
       for (int32_t q : of_bucket[i]) {
-        const BstGroup& G = ctx->bst_groups[q];
-        const int64_t fma = int64_t(G.m) * G.k * (G.bcore / std::max(G.m, 1));
+        const BstBrief& G = groups[size_t(q)];
+        const int64_t fma = int64_t(G.m) * G.k * G.ns;
         // large operator products (no modes after them) in column ranges
         const int pieces = G.post ? 1 : int(std::max<int64_t>(1, std::min<int64_t>(fma / kSplitFma, (G.m + 15) / 16)));
         const int step = (((G.m + pieces - 1) / pieces) + 3) / 4 * 4;
@@ -2243,14 +2258,17 @@ void bst_lists(fcg_ctx* ctx, int R, size_t elem) {
   }
   // longest first: the global-workspace CTAs take the list in order
   std::stable_sort(ctx->bst_large.begin(), ctx->bst_large.end(), [&](int32_t x, int32_t y) {
-    return group_work(ctx->bst_groups[x], R) > group_work(ctx->bst_groups[y], R);
+    return group_work(groups[x], R) > group_work(groups[y], R);
   });
   // chunks of every bucket longest first, in one array
   std::vector<BstChunk> chunks;
+  std::vector<std::pair<int64_t, int32_t>> order;  // (-work, position)
   ctx->bst_chunk_ptr.assign(1, 0);
   for (int i = 0; i < kChunkBuckets; ++i) {
-    std::stable_sort(bucket[i].begin(), bucket[i].end(), [](const Pending& x, const Pending& y) { return x.work > y.work; });
-    for (const Pending& P : bucket[i]) chunks.push_back(P.c);
+    order.clear();
+    for (const Pending& P : bucket[i]) order.emplace_back(-P.work, int32_t(order.size()));
+    std::sort(order.begin(), order.end());
+    for (const auto& o : order) chunks.push_back(bucket[i][size_t(o.second)].c);
     ctx->bst_chunk_ptr.push_back(int64_t(chunks.size()));
   }
   const unsigned char* cb = reinterpret_cast<const unsigned char*>(chunks.data());
@@ -2556,7 +2574,7 @@ int bst_set_impl(fcg_ctx* ctx, int nbody, int64_t n_blocks, const int16_t* fock,
   }
   FCG_CUDA(cudaStreamSynchronize(ctx->stream));  // before the build-only buffers are freed
   ctx->bst_blocks = std::move(blk);
-  ctx->bst_groups = std::move(P.groups);
+  ctx->bst_brief = briefs(P.groups);
   ctx->bst_triples = std::move(P.triples);
   ctx->bst_core_total = off;
   ctx->bst_list_R = 0;
@@ -2564,7 +2582,7 @@ int bst_set_impl(fcg_ctx* ctx, int nbody, int64_t n_blocks, const int16_t* fock,
   *core_total = off;
   ctx->stats.bst_blocks = n_blocks;
   ctx->stats.bst_triples = int64_t(ctx->bst_triples.size() / 4);
-  ctx->stats.bst_groups = int64_t(ctx->bst_groups.size());
+  ctx->stats.bst_groups = int64_t(ctx->bst_brief.size());
   ctx->stats.bst_cache_elements = P.op_total;
   ctx->stats.bst_flops_reference = P.flops_ref;
   ctx->stats.bst_flops_executed = P.flops_exec;

@@ -265,7 +265,7 @@ struct fcg_ctx {
   bool have_bst = false;
   int64_t bst_core_total = 0;
   std::vector<BstBlock> bst_blocks;
-  std::vector<BstGroup> bst_groups;
+  std::vector<BstBrief> bst_brief;      // per group
   std::vector<int32_t> bst_triples;     // [n][4] = {bra, ket, term, sign}
   std::vector<unsigned char> bst_chunks, bst_entries;  // chunks of one bra block and root, their groups (bst.cu)
   std::vector<int64_t> bst_chunk_ptr;         // chunks of each shared-memory bucket: [ptr[i], ptr[i+1])
