@@ -1438,6 +1438,7 @@ struct BstPlan {
   std::vector<BstGamma> gammas;
   std::vector<BstGroupTerm> gterms;
   std::vector<BstGroup> groups;
+  std::vector<BstCost> costs;  // of the groups
   std::vector<BstOverlapJob> overlaps;
   std::vector<int32_t> triples;
   std::vector<BstPermTable> tables;  // actives-first index tables, filled on the device
@@ -1453,6 +1454,7 @@ struct BstPlan {
 struct BstPart {
   std::vector<int32_t> triples;
   std::vector<BstGroup> groups;
+  std::vector<BstCost> costs;                  // of the groups, by finish_part
   std::vector<std::vector<BstGroupTerm>> gt;   // terms per group
   std::vector<BstGroupTerm> gterms;            // the same, flattened by finish_part
   std::vector<BstGamma> gammas;
@@ -1578,7 +1580,7 @@ std::string finish_part(const std::vector<BstBlock>& blk, int N, BstPart& P) {
         G.s_bs[j] = int32_t(bst[c]);
       }
     }
-    int64_t size = K.core_len, ws = size, tf = 0;
+    int64_t size = K.core_len, ws = size, tf = 0;  // tf: multiply-adds of the modes, all before the operator
     int md[kMaxClusters], mk[kMaxClusters], mj[kMaxClusters], nm = 0;  // applied modes: bra / ket rank, mode index
     G.ntr = 0;
     for (int c = 0, j = 0; c < N; ++c) {
@@ -1602,15 +1604,17 @@ std::string finish_part(const std::vector<BstBlock>& blk, int N, BstPart& P) {
       mj[nm++] = j;
       G.s_off[j++] = it->second;
       size = size / K.rank[c] * B.rank[c];
-      tf += 2 * size * K.rank[c];
+      tf += size * K.rank[c];
       ws = std::max(ws, size);
     }
+    const int64_t fma = m * k * n + tf;
+    int64_t post_fma = 0;
     // the sides of the operator the modes go to: the cheapest of the 2^nm choices (all before it
     // for groups that may run on the tensor cores, whose operand X is in the bra bases, and for
     // operator products that are cut into column ranges)
     G.post = 0;
     if (nm > 0 && nm <= 4 && !(m >= kTcMinM && k >= kTcMinK) && m * k * n <= kSplitFma) {
-      int64_t best = m * k * n + tf / 2;
+      int64_t best = fma;
       for (int set = 1; set < (1 << nm); ++set) {
         int64_t sz = K.core_len, cost = 0, top = sz;
         for (int pass = 0; pass < 2; ++pass) {
@@ -1636,15 +1640,15 @@ std::string finish_part(const std::vector<BstBlock>& blk, int N, BstPart& P) {
       }
       if (G.post) {
         ws = std::max(ws, int64_t(G.ws));
-        tf = 2 * (best - m * k * n);
+        post_fma = best;
       }
     }
     for (int j = G.nsp; j < kMaxClusters; ++j) G.s_off[j] = 0;
     if (ws > (int64_t(1) << 30)) return "BST: a core exceeds 2^30 elements";
     G.ws = int32_t(align_up(ws));
-    const int64_t f = 2 * m * k * n + tf;
-    P.flops_exec += f;
-    P.flops_ref += f * G.nt;
+    P.costs.push_back(BstCost{fma, post_fma});
+    P.flops_exec += 2 * fma;
+    P.flops_ref += 2 * fma * G.nt;
   }
   P.gt.clear();
   P.gt.shrink_to_fit();
@@ -1901,6 +1905,7 @@ std::string plan_bst(const fcg_ctx* ctx, int nbody, const std::vector<BstBlock>&
   }
   if (at[np].gterms >= (int64_t(1) << 31)) return "BST: more than 2^31 group terms";
   P.groups.resize(size_t(at[np].groups));
+  P.costs.resize(size_t(at[np].groups));
   P.gterms.resize(size_t(at[np].gterms));
   P.triples.resize(size_t(at[np].triples));
   P.gammas.resize(size_t(at[np].gammas));
@@ -1932,6 +1937,7 @@ std::string plan_bst(const fcg_ctx* ctx, int nbody, const std::vector<BstBlock>&
       for (int j = 0; j < G.nsp; ++j)
         if (G.s_off[j] >= 0) G.s_off[j] += a.s;
       P.groups[size_t(a.groups) + i] = G;
+      P.costs[size_t(a.groups) + i] = part.costs[i];
     }
     part = BstPart();  // free the part as it is consumed
   }
@@ -2046,12 +2052,12 @@ std::string check_groups(const std::vector<BstGroup>& groups, const std::vector<
 }
 
 // the fields of the groups that bst_lists looks at, side by side
-std::vector<BstBrief> briefs(const std::vector<BstGroup>& groups) {
+std::vector<BstBrief> briefs(const std::vector<BstGroup>& groups, const std::vector<BstCost>& costs) {
   std::vector<BstBrief> out(groups.size());
 #pragma omp parallel for schedule(static)
   for (int64_t g = 0; g < int64_t(groups.size()); ++g) {
     const BstGroup& G = groups[size_t(g)];
-    out[size_t(g)] = BstBrief{G.bra, G.m, G.k, G.bcore / std::max(G.m, 1), G.bcore, G.kcore, G.ws, G.post};
+    out[size_t(g)] = BstBrief{costs[size_t(g)], G.bra, G.m, G.k, G.bcore / std::max(G.m, 1), G.bcore, G.kcore, G.ws, G.post};
   }
   return out;
 }
@@ -2091,6 +2097,9 @@ void bst_lists(fcg_ctx* ctx, int R, size_t elem) {
   ctx->bst_tc_mma_flops = 0;
   const std::vector<BstBrief>& groups = ctx->bst_brief;
   const size_t ng = groups.size();
+  int64_t* const paths = ctx->bst_paths;
+  std::fill(paths, paths + kBstPaths, int64_t(0));
+  int64_t exec = 0;  // multiply-adds of a root, in the order that runs
   const int64_t head = elem == 4 ? ChunkHead<float>::n : ChunkHead<double>::n;
   // where each group runs: a warp slice, a chunk bucket, global workspaces, the tensor cores
   constexpr uint8_t kWarp = 100, kLarge = 101, kTc = 102;
@@ -2153,10 +2162,14 @@ void bst_lists(fcg_ctx* ctx, int R, size_t elem) {
       const int64_t ns = G.ns;
       if (where[q] < kChunkBuckets) {
         of_bucket[where[q]].push_back(int32_t(q));
+        exec += G.post ? G.cost.post_fma : G.cost.fma;
+        ++paths[1];
         continue;
       }
+      exec += G.cost.fma;
       if (where[q] == kTc) {
         // GEMM-shaped: tensor cores (its operand X in a global workspace of its own)
+        ++paths[5];
         const int32_t tc = int32_t(ctx->bst_tc.size());
         ctx->bst_tc.push_back(int32_t(q));
         ctx->bst_tc_ws_off.push_back(ctx->bst_tc_ws_total);
@@ -2169,6 +2182,7 @@ void bst_lists(fcg_ctx* ctx, int R, size_t elem) {
           }
         ctx->bst_tc_flops += 2 * int64_t(G.m) * G.k * ns * R;
       } else if (where[q] == kWarp) {
+        ++paths[0];
         const int64_t gw = group_work(G, R);
         // a chunk's own cost: its warps' copies of the bra core zeroed and summed
         if (!open || work > std::max(warp_cut, std::min(kChunkWorkMax, kChunkBraWork * R * G.bcore))) {
@@ -2184,6 +2198,7 @@ void bst_lists(fcg_ctx* ctx, int R, size_t elem) {
         work += gw;
         warp_chunk_work.back() += gw;
       } else if (where[q] == kLarge) {
+        ++paths[4];
         ctx->bst_large.push_back(int32_t(q));
         ctx->bst_ws_large = std::max(ctx->bst_ws_large, G.ws);
       }
@@ -2203,6 +2218,7 @@ void bst_lists(fcg_ctx* ctx, int R, size_t elem) {
           for (int r = 0; r < R; ++r) {
             P.c.root = r;
             bucket[i].push_back(P);
+            paths[3] += P.c.acc == 0;
           }
         P.work = 0;
         P.c.first = int32_t(entries.size());
@@ -2219,6 +2235,7 @@ void bst_lists(fcg_ctx* ctx, int R, size_t elem) {
         // large operator products (no modes after them) in column ranges
         const int pieces = G.post ? 1 : int(std::max<int64_t>(1, std::min<int64_t>(fma / kSplitFma, (G.m + 15) / 16)));
         const int step = (((G.m + pieces - 1) / pieces) + 3) / 4 * 4;
+        paths[2] += step < G.m;
         for (int c0 = 0; c0 < G.m; c0 += step) {
           const int nc = std::min(step, G.m - c0);
           const int64_t bytes = head + (P.c.acc ? (P.c.bcore + 3) / 4 * 4 * int64_t(elem) : 0) +
@@ -2271,6 +2288,7 @@ void bst_lists(fcg_ctx* ctx, int R, size_t elem) {
     for (const auto& o : order) chunks.push_back(bucket[i][size_t(o.second)].c);
     ctx->bst_chunk_ptr.push_back(int64_t(chunks.size()));
   }
+  ctx->stats.bst_flops_executed = 2 * exec;
   const unsigned char* cb = reinterpret_cast<const unsigned char*>(chunks.data());
   const unsigned char* eb = reinterpret_cast<const unsigned char*>(entries.data());
   ctx->bst_chunks.assign(cb, cb + chunks.size() * sizeof(BstChunk));
@@ -2574,11 +2592,12 @@ int bst_set_impl(fcg_ctx* ctx, int nbody, int64_t n_blocks, const int16_t* fock,
   }
   FCG_CUDA(cudaStreamSynchronize(ctx->stream));  // before the build-only buffers are freed
   ctx->bst_blocks = std::move(blk);
-  ctx->bst_brief = briefs(P.groups);
+  ctx->bst_brief = briefs(P.groups, P.costs);
   ctx->bst_triples = std::move(P.triples);
   ctx->bst_core_total = off;
   ctx->bst_list_R = 0;
   ctx->bst_list_elem = 0;
+  std::fill(ctx->bst_paths, ctx->bst_paths + kBstPaths, int64_t(0));
   *core_total = off;
   ctx->stats.bst_blocks = n_blocks;
   ctx->stats.bst_triples = int64_t(ctx->bst_triples.size() / 4);
@@ -2594,6 +2613,12 @@ int bst_set_impl(fcg_ctx* ctx, int nbody, int64_t n_blocks, const int16_t* fock,
 }
 
 extern "C" {
+
+int fcg_bst_paths(const fcg_ctx* ctx, int64_t* out) {
+  if (!ctx || !out) return FCG_EINVAL;
+  std::copy(ctx->bst_paths, ctx->bst_paths + kBstPaths, out);
+  return FCG_OK;
+}
 
 int fcg_bst_set(fcg_ctx* ctx, int nbody, int64_t n_blocks, const int16_t* fock, const int64_t* blocks,
                 const int64_t* factor_off, int64_t n_factors, const double* factors, int64_t* core_total) {

@@ -266,6 +266,7 @@ struct fcg_ctx {
   int64_t bst_core_total = 0;
   std::vector<BstBlock> bst_blocks;
   std::vector<BstBrief> bst_brief;      // per group
+  int64_t bst_paths[kBstPaths] = {};
   std::vector<int32_t> bst_triples;     // [n][4] = {bra, ket, term, sign}
   std::vector<unsigned char> bst_chunks, bst_entries;  // chunks of one bra block and root, their groups (bst.cu)
   std::vector<int64_t> bst_chunk_ptr;         // chunks of each shared-memory bucket: [ptr[i], ptr[i+1])

@@ -257,11 +257,18 @@ struct BstGroup {
 };
 static_assert(sizeof(BstGroup) % 16 == 0, "BstGroup is copied to shared memory in 16-byte units");
 
+// Multiply-adds of a group per root: every mode before the operator, and by its `post` (0: none after it).
+struct BstCost {
+  int64_t fma, post_fma;
+};
+
 // What the choice of a group's kernel needs of it.
 struct BstBrief {
+  BstCost cost;
   int32_t bra, m, k, ns;  // ns: spectator indices of the bra
   int32_t bcore, kcore, ws, post;
 };
+constexpr int kBstPaths = 6;  // counts of fcg_bst_paths
 
 // n / d for n * d < 2^32 as the high word of n * div_mg(d) (d > 1)
 inline uint32_t div_mg(uint32_t d) { return d > 1 ? 0xFFFFFFFFu / d + 1 : 0; }

@@ -67,6 +67,7 @@ SIGNATURES = {
     "fcg_bst_set_between": (_I, [_P, _I, _L, _L, _P, _P, _P, _L, _P, ctypes.POINTER(_L)]),
     "fcg_bst_sigma_device": (_I, [_P, _I, _P, _P, _I]),
     "fcg_bst_triples": (_I, [_P, _P]),
+    "fcg_bst_paths": (_I, [_P, _P]),
     "fcg_sigma_closed_grouped": (_I, [_I, _P, _P, _P, _P, _I]),
     "fcg_davidson_grouped": (_I, [_I, _P, _P, _P, _I, _I, ctypes.c_double, ctypes.c_double, _I, _I, _P, _P, _P,
                                   _P]),
@@ -366,6 +367,12 @@ class GpuSigma:
         out = np.zeros((n, 4), dtype=np.int32)
         self._check(self.L.fcg_bst_triples(self.h, _ptr(out)), "fcg_bst_triples")
         return out
+
+    def bst_paths(self):
+        """Groups of the last BST product by the way they ran (fcg_bst_paths)."""
+        out = np.zeros(6, dtype=np.int64)
+        self._check(self.L.fcg_bst_paths(self.h, _ptr(out)), "fcg_bst_paths")
+        return dict(zip(("warp", "chunk", "split", "atomic_chunks", "global", "tensor"), out.tolist()))
 
     def bst_fois(self, fock, blocks, factor_off, factors, cores, spaces, thresh, nbody=4, compress_twice=True):
         """build_compressed_1st_order_state on the device (fcg_bst_fois).  Inputs in the

@@ -67,7 +67,8 @@ typedef struct fcg_stats {
   int64_t bst_groups;       /* (bra block, ket block, active clusters) groups = cached operators */
   int64_t bst_cache_elements; /* elements of the cached group operators */
   int64_t bst_flops_reference; /* per root: sum over triples of 2*m*k*n + spectator transforms (reference count) */
-  int64_t bst_flops_executed;  /* per root: the same sums over groups (what one fcg_bst_sigma root does) */
+  int64_t bst_flops_executed;  /* per root: the same sums over groups, spectator transforms on the side of the
+                                  operator where the last product's kernels did them (before a product: before it) */
   double bst_cache_seconds; /* wall time of the last fcg_bst_set (planning + operator cache) */
   double bst_plan_seconds;  /* of which host planning (triples, groups, cache layout) */
   int64_t bst_fois_items;   /* (term, ket block, target TuckerConfig) contributions of the last fcg_bst_fois */
@@ -320,6 +321,12 @@ int fcg_bst_set_between(fcg_ctx* ctx, int nbody, int64_t n_first, int64_t n_bloc
 /* The triples of the last fcg_bst_set: int32 [bst_triples][4] = {bra block, ket block,
  * term index (term-table row), state sign}. */
 int fcg_bst_triples(fcg_ctx* ctx, int32_t* out);
+
+/* How the last BST product ran its groups: out[0] groups by a warp each, [1] by CTA chunks, [2] of
+ * these with the operator cut into column ranges, [3] chunks (of one root) that add straight to sigma,
+ * their bra core not fitting beside the workspaces, [4] groups from global workspaces, [5] groups on the
+ * tensor cores. */
+int fcg_bst_paths(const fcg_ctx* ctx, int64_t out[6]);
 
 /* The compressed first-order interacting space of a BST state: build_compressed_1st_order_state
  * (src/tucker_outer.jl:717-910) with form_sigma_block_expand (src/tucker_form_sigma_block_expand.jl
