@@ -288,6 +288,7 @@ struct LaneParams {
   const int16_t* cfg;  // [n_cfg][kCfgStride]
   int64_t n_jobs;      // lane jobs to run: the ones past it are left to the block jobs
   int R;
+  int short_jobs;      // 1: lane jobs of less than kLaneKets[0] kets at most
 };
 
 // R coefficients of one row of a row-major [n][R] array (RR > 0: R == RR, known at compile
@@ -379,6 +380,43 @@ __device__ __forceinline__ void add_rows(double* __restrict__ sig, int row, cons
   } else {
     if (row >= 0) add_row<T, RV>(sig, row, acc, R);
   }
+}
+
+// add_rows for float rows that go out element by element (R not a multiple of 4) where lane jobs are short:
+// neighbouring lanes of one row, the jobs of a row that has more kets than a job, sum theirs first, in pairs
+// of floats (value and rounding error) that keep what the float64 additions would.  Bound otherwise: those
+// additions, at L2 (4000 rows of 12 orbitals, 116 of a root for every row).  Eight such problems grouped,
+// from stored blocks, 3 / 6 roots: 217 / 360 us with an addition per lane, 179 / 276 so; with jobs of 32
+// kets few neighbours share a row and the test costs 6 %.
+template <int RV>
+__device__ __forceinline__ void add_runs(double* __restrict__ sig, int row, float* acc, int R) {
+  const int lane = threadIdx.x & 31;
+  const int left = __shfl_up_sync(0xffffffffu, row, 1);
+  const bool head = lane == 0 || left != row;
+  const unsigned heads = __ballot_sync(0xffffffffu, head);
+  float low[RV];
+#pragma unroll
+  for (int r = 0; r < RV; ++r) low[r] = 0.f;
+  if (heads != 0xffffffffu) {
+    const unsigned after = heads & ~((2u << lane) - 1u);
+    const int run = (after ? __ffs(after) - 1 : 32) - lane;  // lanes of this one's run from it on
+    for (int d = 1; __any_sync(0xffffffffu, run > d); d <<= 1) {
+#pragma unroll
+      for (int r = 0; r < RV; ++r) {
+        const float v = __shfl_down_sync(0xffffffffu, acc[r], d), e = __shfl_down_sync(0xffffffffu, low[r], d);
+        if (run > d) {
+          const float s = __fadd_rn(acc[r], v), z = __fsub_rn(s, acc[r]);
+          low[r] += __fadd_rn(__fsub_rn(acc[r], __fsub_rn(s, z)), __fsub_rn(v, z)) + e;
+          acc[r] = s;
+        }
+      }
+    }
+  }
+  if (!head || row < 0) return;
+  double* dst = sig + int64_t(row) * R;
+#pragma unroll
+  for (int r = 0; r < RV; ++r)
+    if (r < R) atomicAdd(dst + r, double(acc[r]) + double(low[r]));
 }
 
 // One warp chunk of the closed sigma: the chunk's warp tasks in order, lane i of a task
@@ -775,7 +813,15 @@ __device__ __forceinline__ void cached_lane_warp(const LaneParams& p, const T* _
       load_row<T, RR, RV>(cin + int64_t(__ldg(p.perm + j.kp + s)) * R, R, c);
       add_scaled<T, RV>(acc, v, c);
     }
-    add_rows<T, RR, RV>(sig, j.len > 0 ? j.b : -1, acc, R);
+    const int row = j.len > 0 ? j.b : -1;
+    if constexpr (sizeof(T) == 4 && RV <= 8 && (RR == 0 || RR % 4 != 0)) {
+      if (p.short_jobs && R % 4 != 0)
+        add_runs<RV>(sig, row, acc, R);
+      else
+        add_rows<T, RR, RV>(sig, row, acc, R);
+    } else {
+      add_rows<T, RR, RV>(sig, row, acc, R);
+    }
     val += 32 * int64_t(steps);
   }
 }
@@ -1011,6 +1057,7 @@ static LaneParams make_lane_params(fcg_ctx* ctx, int R) {
   p.cfg = ctx->d_cfg.p;
   p.n_jobs = ctx->plan_jobs;
   p.R = R;
+  p.short_jobs = ctx->plan.lane_kets < kLaneKets[0] ? 1 : 0;
   return p;
 }
 
