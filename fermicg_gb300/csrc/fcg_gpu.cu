@@ -1622,11 +1622,12 @@ namespace {
 std::mutex g_tune_mu;
 std::map<std::string, int> g_tune_cache;  // shape key -> candidate, for this process
 
-std::string tune_key(const fcg_ctx* ctx, int prec, int R) {
+// `jobs`: the lane jobs that are timed (in double some of a plan's items may run as block jobs)
+std::string tune_key(const fcg_ctx* ctx, int prec, int R, int64_t jobs) {
   const Plan& P = ctx->plan;
   return std::to_string(prec) + "/" + std::to_string(R) + "/" + std::to_string(ctx->N) + "/" +
          std::to_string(ctx->n_cfg) + "/" + std::to_string(ctx->n_terms) + "/" + std::to_string(P.n_triples) + "/" +
-         std::to_string(ctx->plan_jobs) + "/" + std::to_string(ctx->device);
+         std::to_string(ctx->plan_jobs) + "/" + std::to_string(jobs) + "/" + std::to_string(ctx->device);
 }
 }  // namespace
 
@@ -1742,7 +1743,12 @@ static int launch_blocks(fcg_ctx* ctx, int R, const double* w, const double* op,
 template <typename T>
 static int tune_closed(fcg_ctx* ctx, int prec, int R, const T* w, const T* op, const T* cin, double* sig) {
   const auto t0 = std::chrono::steady_clock::now();
-  const std::string key = tune_key(ctx, prec, R);
+  const int64_t jobs = use_blocks<T>(ctx) ? ctx->plan.n_direct : ctx->plan_jobs;
+  if (jobs == 0) {  // nothing to time: every item runs as block jobs, or there is none
+    ctx->tuned[prec] = 0;
+    return FCG_OK;
+  }
+  const std::string key = tune_key(ctx, prec, R, jobs);
   {
     std::lock_guard<std::mutex> lock(g_tune_mu);
     auto it = g_tune_cache.find(key);
@@ -1841,7 +1847,7 @@ static int launch_closed(fcg_ctx* ctx, int R, const T* w, const T* op, const T* 
     const int c = ctx->tune_mode >= 0 ? ctx->tune_mode : (ctx->tuned[prec] >= 0 ? ctx->tuned[prec] : 0);
     const int rc = launch_candidate<T>(ctx, c, R, w, op, cin, sig);
     if (rc) return rc;
-    launches += 1;
+    if (!use_blocks<T>(ctx) || ctx->plan.n_direct > 0) launches += 1;
   }
   if (timed) FCG_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
   ctx->stats.kernel_launches = launches;
