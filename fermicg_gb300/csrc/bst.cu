@@ -134,8 +134,9 @@ constexpr int kOpV = 1024, kOpU = 2048, kOpG = 2304;  // largest shared tables o
 //   V[p0, p1] = sum_{p2..} ints[p0, p1, p2..] prod_{a>1} g_a[p_a, q_a]   (two clusters: the ints)
 //   u[p0, q1] = sum_p1 V[p0, p1] g_1[p1, q1]
 //   OP[q0, q1, ..] += sum_p0 g_0[p0, q0] u[p0, q1]
-// with V, u and g_0 in shared memory: every element of a step is one thread's.  The elements of OP
-// are one thread's for all terms, which it adds in term order.
+// with V, u and g_0 in shared memory: every element of a step is one thread's.  The terms are added to
+// OP in term order; another thread may have an element in the next term (its step of q1 depends on the
+// term's p0), so the barrier between terms is what orders the reads and writes of OP.
 //
 // Bound: latency of the short steps.  A thread per tuple of all clusters after the first, with its
 // own u in shared memory and recomputed u for every 16 elements of the first cluster, took 9.7 ms
@@ -2129,9 +2130,12 @@ void bst_lists(fcg_ctx* ctx, int R, size_t elem) {
     }
   }
   // Double groups of more than 72 KB go to the global-workspace kernel too where it has a group for
-  // every SM anyway: a chunk of 384 threads per SM leaves the float64 pipe half idle, but few groups
-  // leave SMs idle there.  32 orbitals, 4 excited clusters, 2 roots: ranks 4-12, 5 / 2 sectors, chunks
-  // 56.2 / 17.0 ms, global 47.3 / 14.4; ranks 4-10, 1 sector, chunks 1.8, global 2.0.
+  // every SM anyway: they fill the SMs that the large groups' long chains, alone in a launch, leave idle.
+  // Without large groups the chunks' shared memory is the faster place.  32 orbitals, 4 excited clusters
+  // (sectors, ranks, roots: large groups; ms with chunks / joined): (2, 4-12, 1: 232) 9.2 / 7.5, (2, 4-12, 2: 232) 16.7 / 14.2, (3, 4-12, 1: 551) 14.6 / 11.8, (2, 9-11, 1: 416) 21.5 / 17.9, (5, 4-12, 2: 1543)
+  // 56.0 / 47.4, (2, 8-12, 2: 4203) 45.4 / 31.5, but (1, 8-12, 1: 1499) 4.5 / 4.8; below the line (1, 4-12, 2: 104)
+  // 3.4 / 3.5, (5, 4-11, 2: 41) 32.6 / 34.2, (2, 4-11, 1: 1) 4.6 / 5.5, (2, 4-10, 2: 0) 5.9 / 7.1, and with up to
+  // three excited clusters (9, 10-15, 1: 0) 28.2 / 37.3.
   if (elem == 8 && n_large >= kLargeEnough)
     for (size_t q = 0; q < ng; ++q)
       if (where[q] < kChunkBuckets && where[q] > kChunkAccMax - 1) {

@@ -800,10 +800,7 @@ struct DavidsonWork {
   int enqueue_fetch(size_t count) {
     fcg_ctx* ctx = this->ctx;
     FCG_REQUIRE(count <= out_cap, FCG_ELIMIT, "Davidson: fetch larger than its buffer");
-    if (grouped()) {
-      fetch_count = count;
-      return FCG_OK;
-    }
+    if (grouped()) fetch_count = count;
     return FCG_OK;
   }
   // queue dst[0 : count) = src[0 : count) to the host (the final vectors)

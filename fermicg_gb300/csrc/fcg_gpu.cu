@@ -13,7 +13,8 @@
 //   vectors      row-major [n_cfg][R]: coefficients in the compute precision, sigma float64
 //
 // Kernels:
-//   dress_kernel         W blocks, once per problem (fcg_set_terms)
+//   dress_kernel         W blocks, once per term set (with the first closed-sigma plan; the open sigma's
+//                        own with its first call)
 //   closed_sigma_lane_kernel  a bra row and up to 32 kets per lane; a matrix element is the W
 //                        column of the dressed cluster contracted with the TDM columns of the
 //                        other active clusters (contract_matrix_element,
@@ -483,17 +484,16 @@ __global__ void __launch_bounds__(kSigmaThreads, MINB)
 constexpr int kBlockWarps = 4;
 constexpr int kBlockTerms = 2;  // terms of one shape whose U are held together
 
-template <typename T>
 struct alignas(16) BlockSmem {
   // at least kBlockBras U columns of the longest length
   static constexpr int kU = 1408;
-  T u[kU];
+  double u[kU];
   int2 ket[32];       // kets of the batch by U index: row, U index | states of the clusters left
   uint32_t bst[32];   // (bw | b_q << 8) of every distinct bra pair
   uint32_t kst[32];   // (kw | k_q << 8) of every distinct ket pair
   int32_t kpos[33];   // first ket of every distinct ket pair
 };
-static_assert(BlockSmem<double>::kU >= kBlockBras * kBlockU, "one U column per bra of a block");
+static_assert(BlockSmem::kU >= kBlockBras * kBlockU, "one U column per bra of a block");
 
 struct BlockParams {
   const BlockJob* jobs;
@@ -525,7 +525,6 @@ __device__ __forceinline__ int warp_exclusive(int v) {
 }
 
 // -x without the floating-point pipe
-__device__ __forceinline__ float flip(float x) { return __int_as_float(__float_as_int(x) ^ int(0x80000000)); }
 __device__ __forceinline__ double flip(double x) {
   return __longlong_as_double(__double_as_longlong(x) ^ (long long)(0x8000000000000000ull));
 }
@@ -535,55 +534,51 @@ __device__ __forceinline__ unsigned div_magic(unsigned n) { return (65535u + n) 
 __device__ __forceinline__ unsigned div_by(unsigned x, unsigned m) { return (x * m) >> 16; }
 
 // 4 consecutive elements of shared memory (16-byte aligned)
-__device__ __forceinline__ void load_u4(const float* p, float* v) {
-  const float4 q = *reinterpret_cast<const float4*>(p);
-  v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
-}
 __device__ __forceinline__ void load_u4(const double* p, double* v) {
   const double2 a = *reinterpret_cast<const double2*>(p), b = *reinterpret_cast<const double2*>(p + 2);
   v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
 }
 
 // U contracted with the columns of the clusters left (one: ga; two: ga, gb)
-template <typename T>
-__device__ __forceinline__ T block_pair(const T* u, int da, int db, const T* __restrict__ ga, const T* __restrict__ gb) {
+__device__ __forceinline__ double block_pair(const double* u, int da, int db, const double* __restrict__ ga,
+                                             const double* __restrict__ gb) {
   if (da == 4) {
-    Vec4<T> av;
+    Vec4<double> av;
     av.load(ga);
-    T x[4];
+    double x[4];
     if (db == 1) {
       load_u4(u, x);
-      T me = x[0] * av.v[0];
+      double me = x[0] * av.v[0];
 #pragma unroll
       for (int i = 1; i < 4; ++i) me = fma(x[i], av.v[i], me);
       return me;
     }
-    T me = T(0);
+    double me = 0.0;
     for (int b = 0; b < db; ++b) {
       load_u4(u + 4 * b, x);
-      T acc = x[0] * av.v[0];
+      double acc = x[0] * av.v[0];
 #pragma unroll
       for (int i = 1; i < 4; ++i) acc = fma(x[i], av.v[i], acc);
       me = fma(acc, __ldg(gb + b), me);
     }
     return me;
   }
-  T me = T(0);
+  double me = 0.0;
   for (int b = 0; b < db; ++b) {
-    T acc = T(0);
+    double acc = 0.0;
     for (int i = 0; i < da; ++i) acc = fma(u[da * b + i], __ldg(ga + i), acc);
     me = db == 1 ? acc : fma(acc, __ldg(gb + b), me);
   }
   return me;
 }
 
-template <typename T, int RR, int RMAX = kMaxR>
+template <int RR, int RMAX = kMaxR>
 __global__ void __launch_bounds__(32 * kBlockWarps)
-    block_sigma_kernel(BlockParams p, const T* __restrict__ w, const T* __restrict__ op, const T* __restrict__ cin,
-                       double* __restrict__ sig) {
+    block_sigma_kernel(BlockParams p, const double* __restrict__ w, const double* __restrict__ op,
+                       const double* __restrict__ cin, double* __restrict__ sig) {
   constexpr int RV = RR > 0 ? RR : RMAX;
-  __shared__ BlockSmem<T> smem[kBlockWarps];
-  BlockSmem<T>& S = smem[threadIdx.x >> 5];
+  __shared__ BlockSmem smem[kBlockWarps];
+  BlockSmem& S = smem[threadIdx.x >> 5];
   const int R = RR > 0 ? RR : p.R;
   const int lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
@@ -609,9 +604,9 @@ __global__ void __launch_bounds__(32 * kBlockWarps)
       mine.y = __shfl_sync(0xffffffffu, rb.y, bl);
       mine.z = __shfl_sync(0xffffffffu, rb.z, bl);
       mine.w = __shfl_sync(0xffffffffu, rb.w, bl);
-      T acc[RV];
+      double acc[RV];
 #pragma unroll
-      for (int r = 0; r < RV; ++r) acc[r] = T(0);
+      for (int r = 0; r < RV; ++r) acc[r] = 0.0;
       for (int k0 = 0; k0 < J.nk; k0 += 32) {
         const int nkb = min(32, int(J.nk) - k0);
         const int krow = lane < nkb ? p.perm[J.ket + k0 + lane] : 0;
@@ -665,18 +660,18 @@ __global__ void __launch_bounds__(32 * kBlockWarps)
           }
           __syncwarp();
           const int du = da * db;
-          if (n_b * du * tg > BlockSmem<T>::kU) tg = 1;  // two terms of long columns: one at a time
-          const int step = min(n_k, BlockSmem<T>::kU / (n_b * du * tg));  // ket pairs of a pass
+          if (n_b * du * tg > BlockSmem::kU) tg = 1;  // two terms of long columns: one at a time
+          const int step = min(n_k, BlockSmem::kU / (n_b * du * tg));  // ket pairs of a pass
           const unsigned m_du = div_magic(unsigned(du)), m_nb = div_magic(unsigned(n_b)), m_da = div_magic(unsigned(da));
           // the contracted cluster and the W columns: stride and length of its index, per-term bases
           const int dq = ts.g_dim[q], sq = q == 0 ? 1 : (q == 1 ? ts.g_dim[0] : ts.g_dim[0] * ts.g_dim[1]);
           const int rest = ts.rest_len, w_mb = ts.w_mb, gq_mb = ts.g_mb[q];
           const TermSector& ts1 = p.ts[J.ts_off + t0 + tg - 1];
-          const T *w0 = w + ts.w_off, *w1 = w + ts1.w_off, *g0 = op + ts.g_off[q], *g1 = op + ts1.g_off[q];
+          const double *w0 = w + ts.w_off, *w1 = w + ts1.w_off, *g0 = op + ts.g_off[q], *g1 = op + ts1.g_off[q];
           const bool neg0 = ts.sign < 0, neg1 = ts1.sign < 0;
           // the bra's columns of the clusters left, per term
-          const T* ga[kBlockTerms];
-          const T* gb[kBlockTerms];
+          const double* ga[kBlockTerms];
+          const double* gb[kBlockTerms];
           int ga_mb = 0, gb_mb = 0;
 #pragma unroll
           for (int t = 0; t < kBlockTerms; ++t) {
@@ -700,11 +695,11 @@ __global__ void __launch_bounds__(32 * kBlockWarps)
                 const int l = int(div_by(unsigned(o), m_da));
                 x = o - l * da + l * da * dq;
               }
-              const T* wx = (t ? w1 : w0) + rest * (int(b & 255u) + w_mb * int(k & 255u)) + x;
-              const T* g = (t ? g1 : g0) + dq * (int(b >> 8) + gq_mb * int(k >> 8));
-              T acc;
+              const double* wx = (t ? w1 : w0) + rest * (int(b & 255u) + w_mb * int(k & 255u)) + x;
+              const double* g = (t ? g1 : g0) + dq * (int(b >> 8) + gq_mb * int(k >> 8));
+              double acc;
               if (dq == 4) {
-                Vec4<T> gv, wv;
+                Vec4<double> gv, wv;
                 gv.load(g);
                 if (sq == 1) {
                   wv.load(wx);
@@ -716,7 +711,7 @@ __global__ void __launch_bounds__(32 * kBlockWarps)
 #pragma unroll
                 for (int i = 1; i < 4; ++i) acc = fma(wv.v[i], gv.v[i], acc);
               } else {
-                acc = T(0);
+                acc = 0.0;
                 for (int i = 0; i < dq; ++i) acc = fma(__ldg(wx + sq * i), __ldg(g + i), acc);
               }
               S.u[e] = (t ? neg1 : neg0) ? flip(acc) : acc;
@@ -726,13 +721,13 @@ __global__ void __launch_bounds__(32 * kBlockWarps)
             if (on)
               for (int at = S.kpos[i0] + sl; at < k_hi; at += slices) {
                 const int2 kk = S.ket[at];
-                const T* u = S.u + (((kk.y & 255) - i0) * n_b + ib) * tg * du;
+                const double* u = S.u + (((kk.y & 255) - i0) * n_b + ib) * tg * du;
                 const int oa = ga_mb * ((kk.y >> 8) & 255), ob = gb_mb * (kk.y >> 16);
-                T me = block_pair<T>(u, da, db, ga[0] + oa, gb[0] + ob);
-                if (tg == 2) me += block_pair<T>(u + du, da, db, ga[1] + oa, gb[1] + ob);
-                T c[RV];
-                load_row<T, RR, RV>(cin + int64_t(kk.x) * R, R, c);
-                add_scaled<T, RV>(acc, me, c);
+                double me = block_pair(u, da, db, ga[0] + oa, gb[0] + ob);
+                if (tg == 2) me += block_pair(u + du, da, db, ga[1] + oa, gb[1] + ob);
+                double c[RV];
+                load_row<double, RR, RV>(cin + int64_t(kk.x) * R, R, c);
+                add_scaled<double, RV>(acc, me, c);
               }
             __syncwarp();
           }
@@ -746,13 +741,13 @@ __global__ void __launch_bounds__(32 * kBlockWarps)
 #pragma unroll
         for (int r = 0; r < RV; ++r) {
           if (RR == 0 && r >= R) break;
-          const T v = __shfl_sync(0xffffffffu, acc[r], src & 31);
+          const double v = __shfl_sync(0xffffffffu, acc[r], src & 31);
           if (sl + h < s) acc[r] += v;
         }
         s = h;
       }
       const int row = __shfl_sync(0xffffffffu, brow, bl);
-      if (sl == 0) add_row<T, RV>(sig, row, acc, R);
+      if (sl == 0) add_row<double, RV>(sig, row, acc, R);
     }
   }
 }
@@ -1719,15 +1714,15 @@ static int launch_blocks(fcg_ctx* ctx, int R, const double* w, const double* op,
   p.cfg = ctx->d_cfg.p;
   p.next = ctx->d_block_next.p;
   p.R = R;
-  auto kernel = R == 1   ? block_sigma_kernel<double, 1>
-                : R == 2 ? block_sigma_kernel<double, 2>
-                : R == 3 ? block_sigma_kernel<double, 3>
-                : R == 4 ? block_sigma_kernel<double, 4>
-                : R == 5 ? block_sigma_kernel<double, 5>
-                : R == 6 ? block_sigma_kernel<double, 6>
-                : R == 7 ? block_sigma_kernel<double, 7>
-                : R == 8 ? block_sigma_kernel<double, 8>
-                : R <= 12 ? block_sigma_kernel<double, 0, 12> : block_sigma_kernel<double, 0>;
+  auto kernel = R == 1   ? block_sigma_kernel<1>
+                : R == 2 ? block_sigma_kernel<2>
+                : R == 3 ? block_sigma_kernel<3>
+                : R == 4 ? block_sigma_kernel<4>
+                : R == 5 ? block_sigma_kernel<5>
+                : R == 6 ? block_sigma_kernel<6>
+                : R == 7 ? block_sigma_kernel<7>
+                : R == 8 ? block_sigma_kernel<8>
+                : R <= 12 ? block_sigma_kernel<0, 12> : block_sigma_kernel<0>;
   int per_sm = 1, n_sm = 152;
   FCG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * kBlockWarps, 0));
   FCG_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, ctx->device));
