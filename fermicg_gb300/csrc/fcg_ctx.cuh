@@ -107,7 +107,8 @@ struct fcg_ctx {
   std::vector<double> term_ints_norm;  // Frobenius norm of each term's integrals (0 for 1-body terms; term_norms)
   int64_t n_ints = 0;
   std::vector<TermDress> dress;
-  OpCells cells;           // the TDM blocks by operator and bra sector
+  OpCells cells;           // the TDM blocks by operator and bra sector, by the first fcg_set_terms
+  bool cells_ready = false;
   Dressing dressing;       // merged terms: the closed sigma's W (d_w64, d_w32)
   Dressing open_dressing;  // a W for every term: the open sigma's (d_ow64, d_ow32), built by its first use
   DevBuf<TermInfo> d_terms;

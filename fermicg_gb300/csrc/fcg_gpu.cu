@@ -1161,7 +1161,7 @@ int fcg_set_ops(fcg_ctx* ctx, int n_clusters, const int32_t* cluster_norb, int64
     ctx->h_blocks[b] = BlockInfo{cursor, int32_t(r[6]), int32_t(r[7]), int32_t(r[8]), 0};
     cursor += r[6] * r[7] * r[8];
   }
-  ctx->cells = op_cells(ctx->norb, ctx->nmax, ctx->opb, ctx->h_blk_index, ctx->h_blocks);
+  ctx->cells_ready = false;
   // the caller's blob goes up once; a kernel places every block at its aligned offset and
   // writes the float copy (the gaps between blocks are zero)
   {
@@ -1356,6 +1356,8 @@ int fcg_set_terms(fcg_ctx* ctx, int n_terms, const int32_t* term_table, int64_t 
   ctx->n_ints = n_ints;
   ctx->term_ints_norm.clear();  // computed when first needed (term_norms)
   {
+    if (!ctx->cells_ready) ctx->cells = op_cells(ctx->norb, ctx->nmax, ctx->opb, ctx->h_blk_index, ctx->h_blocks);
+    ctx->cells_ready = true;
     std::string msg = term_dress(ctx->trm, n_terms, ctx->dress);
     FCG_REQUIRE(msg.empty(), FCG_EINVAL, msg);
     msg = build_dress(ctx->nmax, ctx->trm, n_terms, ctx->cells, ctx->h_blocks, ctx->terms, ctx->dress, true, ctx->dressing);
