@@ -387,7 +387,7 @@ __device__ __forceinline__ void add_rows(double* __restrict__ sig, int row, cons
 // neighbouring lanes of one row, the jobs of a row that has more kets than a job, sum theirs first, in pairs
 // of floats (value and rounding error) that keep what the float64 additions would.  Bound otherwise: those
 // additions, at L2 (4000 rows of 12 orbitals, 116 of a root for every row).  Eight such problems grouped,
-// from stored blocks, 3 / 6 roots: 217 / 360 us with an addition per lane, 179 / 276 so; with jobs of 32
+// from stored blocks, 3 / 6 roots: 217 / 360 us with an addition per lane, 173 / 276 so; with jobs of 32
 // kets few neighbours share a row and the test costs 6 %.
 template <int RV>
 __device__ __forceinline__ void add_runs(double* __restrict__ sig, int row, float* acc, int R) {
@@ -395,21 +395,23 @@ __device__ __forceinline__ void add_runs(double* __restrict__ sig, int row, floa
   const int left = __shfl_up_sync(0xffffffffu, row, 1);
   const bool head = lane == 0 || left != row;
   const unsigned heads = __ballot_sync(0xffffffffu, head);
+  if (heads == 0xffffffffu) {
+    if (row >= 0) add_row<float, RV>(sig, row, acc, R);
+    return;
+  }
   float low[RV];
 #pragma unroll
   for (int r = 0; r < RV; ++r) low[r] = 0.f;
-  if (heads != 0xffffffffu) {
-    const unsigned after = heads & ~((2u << lane) - 1u);
-    const int run = (after ? __ffs(after) - 1 : 32) - lane;  // lanes of this one's run from it on
-    for (int d = 1; __any_sync(0xffffffffu, run > d); d <<= 1) {
+  const unsigned after = heads & ~((2u << lane) - 1u);
+  const int run = (after ? __ffs(after) - 1 : 32) - lane;  // lanes of this one's run from it on
+  for (int d = 1; __any_sync(0xffffffffu, run > d); d <<= 1) {
 #pragma unroll
-      for (int r = 0; r < RV; ++r) {
-        const float v = __shfl_down_sync(0xffffffffu, acc[r], d), e = __shfl_down_sync(0xffffffffu, low[r], d);
-        if (run > d) {
-          const float s = __fadd_rn(acc[r], v), z = __fsub_rn(s, acc[r]);
-          low[r] += __fadd_rn(__fsub_rn(acc[r], __fsub_rn(s, z)), __fsub_rn(v, z)) + e;
-          acc[r] = s;
-        }
+    for (int r = 0; r < RV; ++r) {
+      const float v = __shfl_down_sync(0xffffffffu, acc[r], d), e = __shfl_down_sync(0xffffffffu, low[r], d);
+      if (run > d) {
+        const float s = __fadd_rn(acc[r], v), z = __fsub_rn(s, acc[r]);
+        low[r] += __fadd_rn(__fsub_rn(acc[r], __fsub_rn(s, z)), __fsub_rn(v, z)) + e;
+        acc[r] = s;
       }
     }
   }
@@ -787,7 +789,7 @@ __global__ void __launch_bounds__(kSigmaThreads) hcache_lane_build_kernel(LanePa
 
 // sigma from the stored blocks: the chunk's warp tasks as in closed_lane_warp, one stored value
 // per lane and ket in place of the term loop
-template <typename T, int RR, int RMAX = kMaxR>
+template <typename T, int RR, int RMAX, bool RUNS>
 __device__ __forceinline__ void cached_lane_warp(const LaneParams& p, const T* __restrict__ hc,
                                                  const T* __restrict__ cin, double* __restrict__ sig, int64_t chunk) {
   constexpr int RV = RR > 0 ? RR : RMAX;
@@ -809,7 +811,7 @@ __device__ __forceinline__ void cached_lane_warp(const LaneParams& p, const T* _
       add_scaled<T, RV>(acc, v, c);
     }
     const int row = j.len > 0 ? j.b : -1;
-    if constexpr (sizeof(T) == 4 && RV <= 8 && (RR == 0 || RR % 4 != 0)) {
+    if constexpr (RUNS) {
       if (p.short_jobs && R % 4 != 0)
         add_runs<RV>(sig, row, acc, R);
       else
@@ -821,13 +823,14 @@ __device__ __forceinline__ void cached_lane_warp(const LaneParams& p, const T* _
   }
 }
 
-template <typename T, int RR, int RMAX = kMaxR>
+// RUNS: add_runs for the problems it is for (a variant: its registers and test cost the others 2 to 4 %)
+template <typename T, int RR, int RMAX = kMaxR, bool RUNS = false>
 __global__ void __launch_bounds__(kSigmaThreads) cached_sigma_lane_kernel(LaneParams p, const T* __restrict__ hc,
                                                                           const T* __restrict__ cin,
                                                                           double* __restrict__ sig) {
   const int64_t chunk = int64_t(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5);
   if (chunk >= p.n_chunks) return;
-  cached_lane_warp<T, RR, RMAX>(p, hc, cin, sig, chunk);
+  cached_lane_warp<T, RR, RMAX, RUNS>(p, hc, cin, sig, chunk);
 }
 
 // Many independent problems in one launch: problem q owns CTAs [cta0, cta0 + ceil(its chunks
@@ -857,14 +860,14 @@ __global__ void __launch_bounds__(kSigmaThreads, sizeof(T) == 4 ? 4 : 3)
   closed_lane_warp<T, 0, RMAX>(p, e.w, e.op, e.cin, e.sig, chunk);
 }
 
-template <typename T, int RMAX>
+template <typename T, int RMAX, bool RUNS = false>
 __global__ void __launch_bounds__(kSigmaThreads)
     cached_sigma_grouped_kernel(const GroupEntry<T>* __restrict__ g, const int32_t* __restrict__ cta_problem) {
   const GroupEntry<T>& e = g[__ldg(cta_problem + blockIdx.x)];
   const LaneParams p = e.p;
   const int64_t chunk = (int64_t(blockIdx.x) - e.cta0) * kWarpsPerCta + (threadIdx.x >> 5);
   if (chunk >= p.n_chunks) return;
-  cached_lane_warp<T, 0, RMAX>(p, e.hc, e.cin, e.sig, chunk);
+  cached_lane_warp<T, 0, RMAX, RUNS>(p, e.hc, e.cin, e.sig, chunk);
 }
 
 // problem blockIdx.y: C to the row-major working copy, sigma zeroed
@@ -1637,6 +1640,12 @@ static bool use_blocks(const fcg_ctx* ctx) {
   return sizeof(T) == 8 && ctx->plan_on_device && ctx->n_block_jobs > 0;
 }
 
+// whether a sigma from stored blocks sums neighbouring lanes' rows first (add_runs)
+template <typename T>
+static bool use_runs(const fcg_ctx* ctx, int R) {
+  return sizeof(T) == 4 && R % 4 != 0 && ctx->have_hcache && ctx->plan.lane_kets < kLaneKets[0];
+}
+
 // the finer chunk table of the tuning candidates (built on first use)
 static int fine_chunks(fcg_ctx* ctx, bool direct) {
   const int which = direct ? 1 : 0;
@@ -1785,8 +1794,17 @@ static int tune_closed(fcg_ctx* ctx, int prec, int R, const T* w, const T* op, c
 // (stored blocks of 50,021 rows of 24 orbitals, 6 and 8 roots, while sums were added in float: 252 and
 // 186 us, exact 267 and 226).
 template <typename T>
-static void launch_cached(const LaneParams& p, int64_t grid, int R, const T* hc, const T* cin, double* sig, cudaStream_t s) {
+static void launch_cached(const LaneParams& p, int64_t grid, int R, const T* hc, const T* cin, double* sig, cudaStream_t s,
+                          bool runs) {
   const auto run = [&](auto kernel) { kernel<<<unsigned(grid), kSigmaThreads, 0, s>>>(p, hc, cin, sig); };
+  if constexpr (sizeof(T) == 4) {
+    if (runs && R <= 8) switch (R) {
+        case 1: return run(cached_sigma_lane_kernel<T, 1, kMaxR, true>);
+        case 2: return run(cached_sigma_lane_kernel<T, 2, kMaxR, true>);
+        case 3: return run(cached_sigma_lane_kernel<T, 3, kMaxR, true>);
+        default: return run(cached_sigma_lane_kernel<T, 0, 8, true>);
+      }
+  }
   switch (R) {
     case 1: return run(cached_sigma_lane_kernel<T, 1>);
     case 2: return run(cached_sigma_lane_kernel<T, 2>);
@@ -1830,7 +1848,7 @@ static int launch_closed(fcg_ctx* ctx, int R, const T* w, const T* op, const T* 
   if (timed) FCG_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));
   if (grid > 0 && ctx->have_hcache) {  // from the stored Hamiltonian blocks
     const T* hc = sizeof(T) == 4 ? reinterpret_cast<const T*>(ctx->d_hc32.p) : reinterpret_cast<const T*>(ctx->d_hc64.p);
-    launch_cached<T>(p, grid, R, hc, cin, sig, ctx->stream);
+    launch_cached<T>(p, grid, R, hc, cin, sig, ctx->stream, use_runs<T>(ctx, R));
     FCG_CUDA(cudaGetLastError());
     launches = 1;
   } else if (grid > 0) {
@@ -2033,14 +2051,22 @@ static int grouped_impl(int n, fcg_ctx* const* ctxs, const int* R, const double*
     int rmax = 0;
     for (int q = 0; q < n; ++q) rmax = std::max(rmax, R[q]);
     const int32_t* tab = ctx->d_group_cta.p + cta;
-    if (rmax <= 1)
-      cached_sigma_grouped_kernel<T, 1><<<unsigned(cta_hc), kSigmaThreads, 0, ctx->stream>>>(dg, tab);
-    else if (rmax <= 4)
-      cached_sigma_grouped_kernel<T, 4><<<unsigned(cta_hc), kSigmaThreads, 0, ctx->stream>>>(dg, tab);
-    else if (rmax <= 8)
-      cached_sigma_grouped_kernel<T, 8><<<unsigned(cta_hc), kSigmaThreads, 0, ctx->stream>>>(dg, tab);
-    else
-      cached_sigma_grouped_kernel<T, kMaxR><<<unsigned(cta_hc), kSigmaThreads, 0, ctx->stream>>>(dg, tab);
+    const auto run = [&](auto kernel) { kernel<<<unsigned(cta_hc), kSigmaThreads, 0, ctx->stream>>>(dg, tab); };
+    bool runs = false;
+    for (int q = 0; q < n; ++q) runs = runs || use_runs<T>(ctxs[q], R[q]);
+    if (sizeof(T) == 4 && runs && rmax <= 8) {
+      if constexpr (sizeof(T) == 4)
+        rmax <= 1   ? run(cached_sigma_grouped_kernel<T, 1, true>)
+        : rmax <= 4 ? run(cached_sigma_grouped_kernel<T, 4, true>) : run(cached_sigma_grouped_kernel<T, 8, true>);
+    } else if (rmax <= 1) {
+      run(cached_sigma_grouped_kernel<T, 1>);
+    } else if (rmax <= 4) {
+      run(cached_sigma_grouped_kernel<T, 4>);
+    } else if (rmax <= 8) {
+      run(cached_sigma_grouped_kernel<T, 8>);
+    } else {
+      run(cached_sigma_grouped_kernel<T, kMaxR>);
+    }
     FCG_CUDA(cudaGetLastError());
   }
   FCG_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
