@@ -1132,28 +1132,33 @@ int fcg_set_ops(fcg_ctx* ctx, int n_clusters, const int32_t* cluster_norb, int64
   FCG_REQUIRE(cluster_norb && block_table && (data || n_data == 0) && n_blocks >= 0, FCG_EINVAL, "null pointer");
   FCG_REQUIRE(n_blocks < (int64_t(1) << 31), FCG_ELIMIT, "at most 2^31 - 1 TDM blocks");
   FCG_CUDA(cudaSetDevice(ctx->device));
+  // everything checked before the context changes: a refused set leaves the last one in place
+  int nmax = 0;
+  for (int c = 0; c < n_clusters; ++c) {
+    FCG_REQUIRE(cluster_norb[c] > 0 && cluster_norb[c] <= 15, FCG_ELIMIT, "orbitals per cluster must be in [1, 15]");
+    nmax = std::max(nmax, int(cluster_norb[c]));
+  }
+  for (int64_t b = 0; b < n_blocks; ++b) {
+    const int64_t* r = block_table + b * kOpbCols;
+    FCG_REQUIRE(r[0] >= 0 && r[0] < n_clusters && r[1] >= 0 && r[1] < kNumOps, FCG_EINVAL,
+                "block table: bad cluster or op id");
+    for (int i = 2; i < 6; ++i)
+      FCG_REQUIRE(r[i] >= 0 && r[i] <= cluster_norb[r[0]], FCG_EINVAL, "block table: bad Fock sector");
+    FCG_REQUIRE(r[6] > 0 && r[7] > 0 && r[8] > 0 && r[6] <= 4096 && r[7] <= 256 && r[8] <= 256, FCG_ELIMIT,
+                "block table: block dims out of range");
+    FCG_REQUIRE(r[9] >= 0 && r[9] + r[6] * r[7] * r[8] <= n_data, FCG_EINVAL, "block table: data out of range");
+  }
   ctx->N = n_clusters;
   ctx->norb.assign(cluster_norb, cluster_norb + n_clusters);
-  ctx->nmax = 0;
-  for (int n : ctx->norb) {
-    FCG_REQUIRE(n > 0 && n <= 15, FCG_ELIMIT, "orbitals per cluster must be in [1, 15]");
-    ctx->nmax = std::max(ctx->nmax, n);
-  }
+  ctx->nmax = nmax;
   ctx->opb.assign(block_table, block_table + n_blocks * kOpbCols);
+  ctx->cells_ready = false;
   const int s = ctx->nmax + 1;
   ctx->h_blk_index.assign(size_t(n_clusters) * kNumOps * s * s * s * s, -1);
   ctx->h_blocks.assign(n_blocks, BlockInfo{});
   for (int64_t b = 0; b < n_blocks; ++b) {
     const int64_t* r = &ctx->opb[b * kOpbCols];
-    FCG_REQUIRE(r[0] >= 0 && r[0] < n_clusters && r[1] >= 0 && r[1] < kNumOps, FCG_EINVAL,
-                "block table: bad cluster or op id");
-    for (int i = 2; i < 6; ++i)
-      FCG_REQUIRE(r[i] >= 0 && r[i] <= ctx->norb[r[0]], FCG_EINVAL, "block table: bad Fock sector");
-    FCG_REQUIRE(r[6] > 0 && r[7] > 0 && r[8] > 0 && r[6] <= 4096 && r[7] <= 256 && r[8] <= 256, FCG_ELIMIT,
-                "block table: block dims out of range");
-    FCG_REQUIRE(r[9] >= 0 && r[9] + r[6] * r[7] * r[8] <= n_data, FCG_EINVAL, "block table: data out of range");
-    int64_t i = dense_block_index(s, int(r[0]), int(r[1]), int(r[2]), int(r[3]), int(r[4]), int(r[5]));
-    ctx->h_blk_index[i] = int32_t(b);
+    ctx->h_blk_index[dense_block_index(s, int(r[0]), int(r[1]), int(r[2]), int(r[3]), int(r[4]), int(r[5]))] = int32_t(b);
   }
   // device copy: every block starts on a multiple of kAlign elements (32-byte vector loads
   // of TDM columns whose length is a multiple of 4)
@@ -1164,7 +1169,6 @@ int fcg_set_ops(fcg_ctx* ctx, int n_clusters, const int32_t* cluster_norb, int64
     ctx->h_blocks[b] = BlockInfo{cursor, int32_t(r[6]), int32_t(r[7]), int32_t(r[8]), 0};
     cursor += r[6] * r[7] * r[8];
   }
-  ctx->cells_ready = false;
   // the caller's blob goes up once; a kernel places every block at its aligned offset and
   // writes the float copy (the gaps between blocks are zero)
   {

@@ -177,9 +177,10 @@ class GpuSigma:
         tab = np.ascontiguousarray(packed_ops.table, dtype=np.int64)
         dat = np.ascontiguousarray(packed_ops.data, dtype=np.float64)
         norb = np.ascontiguousarray(packed_ops.cluster_norb, dtype=np.int32)
-        self.N = int(packed_ops.n_clusters)
-        self._check(self.L.fcg_set_ops(self.h, self.N, _ptr(norb), tab.shape[0], _ptr(tab), dat.size, _ptr(dat)),
+        n = int(packed_ops.n_clusters)
+        self._check(self.L.fcg_set_ops(self.h, n, _ptr(norb), tab.shape[0], _ptr(tab), dat.size, _ptr(dat)),
                     "fcg_set_ops")
+        self.N = n  # a refused set leaves the last one in place
 
     def set_terms(self, packed_terms: "pack.PackedTerms"):
         tab = np.ascontiguousarray(packed_terms.table, dtype=np.int32)
