@@ -394,9 +394,13 @@ def bst_benchmark(steps, warmup, cpu_seconds, peaks, n_sectors=5, max_q=4):
 
     ms64, k64, _ = timed("fp64")
     y64 = y.clone()
+    flops_exec = {"fp64": g.stats()["bst_flops_executed"] * R}  # of the order that each group's kernel runs
+    paths = {"fp64": g.bst_paths()}
     ms32, k32, tc32 = timed("fp32")
     rel32 = float((y - y64).abs().max() / y64.abs().max())
     s32 = g.stats()
+    flops_exec["fp32"] = s32["bst_flops_executed"] * R
+    paths["fp32"] = g.bst_paths()
     g.bst_tensor_cores(False)
     ms32c, k32c, _ = timed("fp32")
     relc = float((y - y64).abs().max() / y64.abs().max())
@@ -422,13 +426,12 @@ def bst_benchmark(steps, warmup, cpu_seconds, peaks, n_sectors=5, max_q=4):
     # Executed flops (spectator mode products + group contractions, all roots) over the kernel
     # time, against the nominal CUDA-core peaks of GB300 (152 SMs at 2.07 GHz: 128 FP32 FMA or
     # the FP64 rate per cycle); no measured figure exists for these pipes
-    flops_exec = st["bst_flops_executed"] * R
     nominal = {"fp32": 152 * 128 * 2 * 2.07e9 / 1e12, "fp64": 1.25}
 
     def flop_roof(kms, prec):
-        ach = flops_exec / (kms * 1e-3) / 1e12
+        ach = flops_exec[prec] / (kms * 1e-3) / 1e12
         return {"bound": f"{prec} cuda cores", "achieved": ach, "peak": nominal[prec], "unit": "TFLOP/s",
-                "frac": ach / nominal[prec], "flops_per_sigma": flops_exec,
+                "frac": ach / nominal[prec], "flops_per_sigma": flops_exec[prec],
                 "note": f"executed flops / kernel time, of the nominal {prec} CUDA-core peak (no measured peak)"}
 
     # tensor-core kernel: executed MMA flops (three TF32 products per tile, tiles padded to
@@ -443,7 +446,7 @@ def bst_benchmark(steps, warmup, cpu_seconds, peaks, n_sectors=5, max_q=4):
         "cache_elements": cache, "cache_seconds": st["bst_cache_seconds"], "plan_seconds": st["bst_plan_seconds"],
         "set_wall_s": t_set,
         "flops_reference_per_sigma": st["bst_flops_reference"] * R,
-        "flops_executed_per_sigma": flops_exec,
+        "flops_executed_per_sigma": flops_exec, "groups_by_kernel": paths,
         "fp64": {"value": 1e3 / ms64, "unit": "sigma_builds/s", "ms_per_step": ms64, "kernel_ms": k64,
                  "roofline": roof(k64, 8), "flop_roofline": flop_roof(k64, "fp64")},
         "fp32": {"value": 1e3 / ms32, "unit": "sigma_builds/s", "ms_per_step": ms32, "kernel_ms": k32,
@@ -1041,10 +1044,10 @@ def main():
                      # dram__bytes_read.sum + dram__bytes_write.sum of one float launch on this
                      # exact workload, from the ncu capture summarised in
                      # profiles/closed_sigma_lane_kernel_24o6c.md
-                     "traffic": (334.6e6 + 1.5e6) if (n == 100000 and R == 4) else None,
+                     "traffic": (363.4e6 + 3.7e6) if (n == 100000 and R == 4) else None,
                      "note": "compulsory bytes per launch / closed_sigma_lane_kernel time (fp32), of measured HBM "
-                             "copy peak; the float kernel is bound by the L1 data pipe (87 % of peak) and the "
-                             "double kernel by the FP64 pipe, not by HBM"},
+                             "copy peak; the float kernel is bound by the L1 data pipe (80 % of peak) and the "
+                             "double kernels by the FP64 pipe (82 %), not by HBM"},
         "e2e": {"value": 1e3 / e2e_ms, "unit": "sigma_builds/s", "h2d_bytes_per_step": n * R * 8,
                 "d2h_bytes_per_step": n * R * 8},
         "gpu_launches": int(g.stats()["kernel_launches"]) * a.steps,
@@ -1057,8 +1060,8 @@ def main():
         # sigma, work items) per launch over its CUDA-event time, of the measured HBM copy peak
         stored["roofline"] = {"bound": "hbm", "achieved": stored["hbm_gbs_fp32"], "peak": hbm_peak, "unit": "GB/s",
                               "frac": stored["hbm_gbs_fp32"] / hbm_peak,
-                              "note": "cached_sigma_kernel<float>; bound by the L1 data pipe (ket and C-row "
-                                      "gathers), not HBM"}
+                              "note": "cached_sigma_lane_kernel<float>; bound by the latency of the ket and C-row "
+                                      "gathers (L1 51 % busy) and the row additions, not HBM"}
         out["stored_blocks"] = stored
     if rank == 0 and a.davidson:
         try:

@@ -60,8 +60,9 @@ constexpr int64_t kSplitFma = int64_t(1) << 20;  // larger operator products run
 // One CTA per gamma.  For each orbital multi-index p:  T[p, I, kk] = sum_J G[p, I, J] U_ket[J, kk]
 // staged in shared memory for as many p as fit, then g[p, kb, kk] = sum_I U_bra[I, kb] T[p, I, kk].
 // Consecutive threads take consecutive p (the fastest index of G, of g and of the tile).  Tiles
-// that do not fit the staging buffer for one p use the direct double sum.  Bound: latency; a p at a
-// time, with two barriers each, took 3.2 ms where this takes 0.8 ms (32 orbitals, 3 sectors).
+// that do not fit the staging buffer for one p use the direct double sum.  Bound: the FP64 pipe (96 % busy,
+// 32 orbitals, 1 sector, up to four excited clusters).  A p at a time, with two barriers each, took 3.2 ms
+// where this takes 0.8 ms (32 orbitals, 3 sectors).
 __global__ void __launch_bounds__(kGammaThreads) bst_gamma_kernel(const BstGamma* __restrict__ gam,
                                                                   const BstBlock* __restrict__ blocks,
                                                                   const double* __restrict__ tdm,
@@ -138,7 +139,7 @@ constexpr int kOpV = 1024, kOpU = 2048, kOpG = 2304;  // largest shared tables o
 // OP in term order; another thread may have an element in the next term (its step of q1 depends on the
 // term's p0), so the barrier between terms is what orders the reads and writes of OP.
 //
-// Bound: latency of the short steps.  A thread per tuple of all clusters after the first, with its
+// Bound: the FP64 pipe (84 % busy, 32 orbitals, 1 sector, up to four excited clusters).  A thread per tuple of all clusters after the first, with its
 // own u in shared memory and recomputed u for every 16 elements of the first cluster, took 9.7 ms
 // where this takes 1.9 ms (32 orbitals, 3 sectors, up to three excited clusters, ranks 3-8: 39 150
 // groups, 5.1e6 elements, 3.9e8 multiply-adds), and 193 where this takes 24 ms (5 sectors, up to
@@ -707,7 +708,8 @@ __global__ void __launch_bounds__(kBstThreads, 4) bst_sigma_bra_kernel(const int
 // operator.  Each mode goes to the side of the operator where it is cheaper (post), 30 % fewer
 // multiply-adds than all before it.
 //
-// Bound: instruction issue and the barriers between a group's steps (2 of 4 issue slots used).
+// Bound, FP32: the barriers between a group's steps (45 % of the issue slots used, a barrier the first
+// stall); FP64: those and the FP64 pipe (53 to 68 % busy, by bucket; 32 orbitals, 1 sector, ranks 4-12).
 // 32 orbitals, 5 sectors, cores up to 12^4, 2 roots, FP32: whole sigma 16.1 -> 11.3 ms; ranks 4-10
 // of 2 sectors, FP64: 8.0 -> 5.8 ms; 9 sectors, up to three excited clusters, FP64: 12.4 -> 9.0 ms.
 struct BstEntry {

@@ -480,9 +480,9 @@ __global__ void __launch_bounds__(kSigmaThreads, MINB)
 // place of 84 (four).  Pairs run with a bra per lane; a block of fewer bras gives the other lanes a
 // slice of the kets.  Kets are taken in order of their U index, in passes of as many as fit.
 //
-// Bound: the FP64 pipe (2 multiply-adds a clock per SM; 84 % busy).  24 orbitals, 1e5
+// Bound: the FP64 pipe (2 multiply-adds a clock per SM; 82 % busy at 3e4 configurations of 24 orbitals).  1e5
 // configurations, 4 roots: 3.9 ms for work that took the lane kernel 7.0 ms; whole sigma 9.78 ->
-// 6.58 ms; 32 orbitals, 2e4 configurations, 2 roots: 6.53 -> 4.10 ms.
+// 6.58 ms; 32 orbitals, 2e4 configurations, 2 roots: 6.53 -> 4.10 ms.  With merged terms 3.2 ms of 4.95.
 constexpr int kBlockWarps = 4;
 constexpr int kBlockTerms = 2;  // terms of one shape whose U are held together
 
@@ -1638,7 +1638,8 @@ std::string tune_key(const fcg_ctx* ctx, int prec, int R, int64_t jobs) {
 // whether a direct sigma of this precision runs block jobs and the lane jobs of the other items, or
 // every lane job.  Block jobs are for double: they cut the FP64 multiply-adds that bound it by
 // more than half.  In float the lane kernel is bound by loads, and a block's set-up costs what its
-// shared columns save (24 orbitals, 1e5 configurations, 4 roots: 2.40 ms with, 2.33 ms without).
+// shared columns save (24 orbitals, 1e5 configurations, 4 roots, before terms were merged: 2.40 ms with,
+// 2.33 ms without).
 template <typename T>
 static bool use_blocks(const fcg_ctx* ctx) {
   return sizeof(T) == 8 && ctx->plan_on_device && ctx->n_block_jobs > 0;
