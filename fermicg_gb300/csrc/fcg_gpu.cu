@@ -411,6 +411,7 @@ __device__ __forceinline__ void add_runs(double* __restrict__ sig, int row, floa
       if (run > d) {
         const float s = __fadd_rn(acc[r], v), z = __fsub_rn(s, acc[r]);
         low[r] += __fadd_rn(__fsub_rn(acc[r], __fsub_rn(s, z)), __fsub_rn(v, z)) + e;
+        if (!(fabsf(s) <= 3.402823466e38f)) low[r] = 0.f;  // an infinity stays one
         acc[r] = s;
       }
     }

@@ -58,6 +58,20 @@ def test_closed(closed, R, stored, grouped):
     assert _rms(got, want) < U * (4 if stored else 7) ** 0.5
 
 
+@pytest.mark.parametrize("R", [1, 2, 3, 4, 6])
+def test_infinite_coefficient(closed, R):
+    """A row's one infinite product leaves its sum infinite, beside finite ones, in either precision."""
+    g, f, c = closed
+    g.state_set(f, c)
+    g.cache_hamiltonian()
+    x = np.asfortranarray(np.random.default_rng(R).standard_normal((len(f), R)))
+    x[len(f) // 3] = np.inf
+    want, got = g.sigma_closed(x, "fp64"), g.sigma_closed(x, "fp32")
+    assert np.isinf(want).any() and np.isfinite(want).any()
+    assert np.array_equal(np.isinf(got), np.isinf(want)) and np.array_equal(np.isnan(got), np.isnan(want))
+    assert np.array_equal(np.sign(got[np.isinf(want)]), np.sign(want[np.isinf(want)]))
+
+
 @pytest.mark.parametrize("sectors,max_q,ranks", [(40, 1, (2, 4)), (24, 2, (2, 2)), (1, 4, (4, 6))])
 def test_tucker(sectors, max_q, ranks):
     prob = workloads.config2_problem(0)
