@@ -289,7 +289,7 @@ struct LaneParams {
   const int16_t* cfg;  // [n_cfg][kCfgStride]
   int64_t n_jobs;      // lane jobs to run: the ones past it are left to the block jobs
   int R;
-  int short_jobs;      // 1: lane jobs of less than kLaneKets[0] kets at most
+  int runs;            // 1: add_runs where the rows go out element by element
 };
 
 // R coefficients of one row of a row-major [n][R] array (RR > 0: R == RR, known at compile
@@ -388,7 +388,9 @@ __device__ __forceinline__ void add_rows(double* __restrict__ sig, int row, cons
 // of floats (value and rounding error) that keep what the float64 additions would.  Bound otherwise: those
 // additions, at L2 (4000 rows of 12 orbitals, 116 of a root for every row).  Eight such problems grouped,
 // from stored blocks, 3 / 6 roots: 217 / 360 us with an addition per lane, 173 / 276 so; with jobs of 32
-// kets few neighbours share a row and the test costs 6 %.
+// kets few neighbours share a row and the test costs 6 %, and below kRunJobs lane jobs the launch is latency
+// (500 rows of 12 orbitals, 3 roots: 37 us a call without, 40 with).
+constexpr int64_t kRunJobs = int64_t(1) << 18;
 template <int RV>
 __device__ __forceinline__ void add_runs(double* __restrict__ sig, int row, float* acc, int R) {
   const int lane = threadIdx.x & 31;
@@ -813,7 +815,7 @@ __device__ __forceinline__ void cached_lane_warp(const LaneParams& p, const T* _
     }
     const int row = j.len > 0 ? j.b : -1;
     if constexpr (RUNS) {
-      if (p.short_jobs && R % 4 != 0)
+      if (p.runs && R % 4 != 0)
         add_runs<RV>(sig, row, acc, R);
       else
         add_rows<T, RR, RV>(sig, row, acc, R);
@@ -1056,7 +1058,7 @@ static LaneParams make_lane_params(fcg_ctx* ctx, int R) {
   p.cfg = ctx->d_cfg.p;
   p.n_jobs = ctx->plan_jobs;
   p.R = R;
-  p.short_jobs = ctx->plan.lane_kets < kLaneKets[0] ? 1 : 0;
+  p.runs = ctx->plan.lane_kets < kLaneKets[0] && ctx->plan_jobs >= kRunJobs ? 1 : 0;
   return p;
 }
 
@@ -1648,8 +1650,8 @@ static bool use_blocks(const fcg_ctx* ctx) {
 
 // whether a sigma from stored blocks sums neighbouring lanes' rows first (add_runs)
 template <typename T>
-static bool use_runs(const fcg_ctx* ctx, int R) {
-  return sizeof(T) == 4 && R % 4 != 0 && ctx->have_hcache && ctx->plan.lane_kets < kLaneKets[0];
+static bool use_runs(fcg_ctx* ctx, int R) {
+  return sizeof(T) == 4 && R % 4 != 0 && ctx->have_hcache && make_lane_params(ctx, R).runs;
 }
 
 // the finer chunk table of the tuning candidates (built on first use)

@@ -24,10 +24,10 @@ def _rms(a, b):
     return float(np.linalg.norm(a - b) / np.linalg.norm(b))
 
 
-@pytest.fixture(scope="module")
-def closed():
+@pytest.fixture(scope="module", params=[2000, 4000])  # below and above the lane jobs whose rows are summed in runs
+def closed(request):
     p = workloads.config0_problem()
-    f, c, _, _ = pack.pack_state(workloads.energy_ordered_space(p, 2000, R=1))
+    f, c, _, _ = pack.pack_state(workloads.energy_ordered_space(p, request.param, R=1))
     g = GpuSigma(0)
     g.set_ops(pack.pack_ops(p.ops, p.bases))
     g.set_terms(pack.pack_terms(p.ham))
@@ -45,6 +45,7 @@ def test_closed(closed, R, stored, grouped):
     g.state_set(f, c)
     if stored:
         g.cache_hamiltonian()
+    assert (len(g.plan_arrays()["jobs"]) >= 1 << 18) == (len(f) == 4000)
     x = np.asfortranarray(np.random.default_rng(R).standard_normal((len(f), R)))
     want = g.sigma_closed(x, "fp64")
     if grouped:
